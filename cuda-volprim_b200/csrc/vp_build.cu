@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "vp_internal.h"
+#include "vp_trace8.cuh"
 
 namespace vp {
 namespace {
@@ -25,6 +26,8 @@ struct ErrorWords {
   int bad_scale, bad_density, bad_center;  // lowest failing index (INT_MAX = none)
   unsigned int any_albedo;                 // 1 if some albedo component > 0
   unsigned int opaque_cores;               // Gaussians opaque at their core (vp_tau_order AUTO)
+  unsigned int mixed_albedo;               // 1 if some albedo differs from the first Gaussian's
+  float albedo0[3];                        // the first Gaussian's
 };
 
 // A Gaussian is "opaque at its core" when the optical depth through its centre along its thinnest
@@ -68,6 +71,9 @@ __global__ void k_precompute(uint32_t n, const float* __restrict__ mean,
     ab = clamp_albedo(albedo[3 * i + 2]);
   }
   if (ar > 0.f || ag > 0.f || ab > 0.f) atomicOr(&err->any_albedo, 1u);
+  if (albedo && (ar != clamp_albedo(albedo[0]) || ag != clamp_albedo(albedo[1]) || ab != clamp_albedo(albedo[2])))
+    atomicOr(&err->mixed_albedo, 1u);
+  if (i == 0u) err->albedo0[0] = ar, err->albedo0[1] = ag, err->albedo0[2] = ab;
   const bool scale_ok = sx > 0.f && sy > 0.f && sz > 0.f && isfinite(sx) && isfinite(sy) && isfinite(sz);
   if (!scale_ok) atomicMin(&err->bad_scale, (int)i);
   if (!(M > 0.f) || !isfinite(M)) atomicMin(&err->bad_density, (int)i);
@@ -757,6 +763,235 @@ __global__ void k_collapse(const unsigned int* __restrict__ n_items_dev, const C
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// Compressed 8-wide BVH (vp_trace8.cuh): the same binary tree cut for 8 slots a node with every
+// Gaussian a slot of its own.  The cut minimises the expected cost A (kDp8Node per node, kDp8Prim per
+// Gaussian) over the tree by the same dynamic programme as above, with "at most i slots" costs
+//   C(v, i) = min(C(v, i - 1), D(v, i)),  D(v, i) = min over 1 <= j < i of C(left, j) + C(right, i - j),
+//   C(v, 1) = A(v) kDp8Node + D(v, 8).
+// ------------------------------------------------------------------------------------------
+constexpr float kDp8Node = 1.0f, kDp8Prim = 0.4f;
+
+// Bottom-up, as k_dp_cost.  cost[8 v + i - 1] = C(v, i); choice[8 v + i - 1] = the j of D(v, i), or 0 for
+// C(v, i - 1); choice[8 v] = the j of D(v, 8).
+__global__ void k_dp8_cost(uint32_t n, uint32_t root, const uint32_t* __restrict__ left,
+                           const uint32_t* __restrict__ right, const float4* __restrict__ plo,
+                           const float4* __restrict__ phi, const float4* __restrict__ nlo,
+                           const float4* __restrict__ nhi, const uint32_t* __restrict__ parent,
+                           const uint32_t* __restrict__ parent_leaf, unsigned int* flags, float* cost,
+                           uint8_t* __restrict__ choice) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  uint32_t v = parent_leaf[k];
+  while (true) {
+    __threadfence();
+    if (atomicAdd(&flags[v], 1u) == 0u) return;
+    __threadfence();
+    float C[2][7];
+    const uint32_t ch[2] = {left[v], right[v]};
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (ref_is_leaf(ch[c])) {
+        const uint32_t p = ch[c] & ~kLeafBit;
+        const float a = box_area(plo[p], phi[p]) * kDp8Prim;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) C[c][i] = a;
+      } else {
+        const float4* q = reinterpret_cast<const float4*>(cost + 8ull * ch[c]);
+        const float4 x = __ldcg(q), y = __ldcg(q + 1);
+        C[c][0] = x.x, C[c][1] = x.y, C[c][2] = x.z, C[c][3] = x.w, C[c][4] = y.x, C[c][5] = y.y, C[c][6] = y.z;
+      }
+    }
+    float out[8];
+    uint32_t pick[8];
+    float d8 = INFINITY;
+#pragma unroll
+    for (int i = 2; i <= 8; ++i) {
+      float b = INFINITY;
+      uint32_t bj = 1;
+#pragma unroll
+      for (int j = 1; j < i; ++j) {
+        const float c = C[0][j - 1] + C[1][i - j - 1];
+        if (c < b) {
+          b = c;
+          bj = (uint32_t)j;
+        }
+      }
+      out[i - 1] = b;
+      pick[i - 1] = bj;
+      if (i == 8) d8 = b;
+    }
+    pick[0] = pick[7];
+    out[0] = fmaf(box_area(nlo[v], nhi[v]), kDp8Node, d8);
+#pragma unroll
+    for (int i = 1; i < 8; ++i)
+      if (out[i - 1] <= out[i]) {
+        out[i] = out[i - 1];
+        pick[i] = 0u;
+      }
+    float4* q = reinterpret_cast<float4*>(cost + 8ull * v);
+    __stcg(q, make_float4(out[0], out[1], out[2], out[3]));
+    __stcg(q + 1, make_float4(out[4], out[5], out[6], out[7]));
+    uint32_t lo = 0, hi = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) lo |= pick[i] << (8 * i), hi |= pick[4 + i] << (8 * i);
+    reinterpret_cast<uint2*>(choice)[v] = make_uint2(lo, hi);
+    if (v == root) return;
+    v = parent[v];
+  }
+}
+
+// Origin p < lo and power-of-two quantum q of a node's axis with every plane of [lo, hi] at p + k q,
+// 0 < k < 254 (the exponent byte holds q with a +15 bias).  q grows where p, one quantum below lo, rounds
+// further down than that.
+__device__ __forceinline__ void frame8(float lo, float hi, float& p, float& q) {
+  const uint32_t u = __float_as_uint((hi - lo) * (1.0f / 253.0f));
+  uint32_t e = (u >> 23) + ((u & 0x7FFFFFu) ? 1u : 0u);  // rounded up to a power of two
+  for (e = min(max(e, 1u), 239u);; ++e) {
+    q = __uint_as_float(e << 23);
+    p = __fsub_rd(lo, q);
+    if (hi - p <= 254.0f * q || e >= 239u) return;
+  }
+}
+constexpr float kMaxExtent8 = 1e30f;  // larger nodes do not fit the quantisation: no BVH8 then
+
+struct Item8 {
+  uint32_t bin, slot;  // binary node (or kLeafBit | Gaussian: a tree of one), BVH8 node it becomes
+};
+
+// One level of the cut: each item writes its node and queues its inner children, whose nodes are
+// allocated together.
+__global__ void k_collapse8(const unsigned int* __restrict__ n_items_dev, const Item8* __restrict__ in,
+                            Item8* __restrict__ out, unsigned int* __restrict__ out_count,
+                            unsigned int* __restrict__ slot_counter, const uint32_t* __restrict__ left,
+                            const uint32_t* __restrict__ right, const float4* __restrict__ plo,
+                            const float4* __restrict__ phi, const float4* __restrict__ nlo,
+                            const float4* __restrict__ nhi, const uint32_t* __restrict__ pos,
+                            const uint8_t* __restrict__ choice, uint32_t* __restrict__ nodes, uint32_t max_nodes,
+                            unsigned int* __restrict__ overflow) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= *n_items_dev) return;
+  const Item8 it = in[t];
+  uint32_t refs[8];
+  int cnt = 0;
+  if (ref_is_leaf(it.bin)) {
+    refs[cnt++] = it.bin;
+  } else {
+    uint32_t sv[8];
+    int si[8], sp = 0;
+    {
+      const int j = choice[8ull * it.bin];
+      sv[sp] = right[it.bin], si[sp++] = 8 - j;
+      sv[sp] = left[it.bin], si[sp++] = j;
+    }
+    while (sp > 0 && cnt < 8) {  // the budgets on the stack and the slots taken sum to at most 8
+      --sp;
+      const uint32_t v = sv[sp];
+      int i = si[sp], j = 0;
+      if (!ref_is_leaf(v))
+        while (i > 1 && (j = choice[8ull * v + i - 1]) == 0) --i;
+      if (ref_is_leaf(v) || i == 1) {
+        refs[cnt++] = v;
+        continue;
+      }
+      sv[sp] = right[v], si[sp++] = i - j;
+      sv[sp] = left[v], si[sp++] = j;
+    }
+  }
+  float4 bl[8], bh[8];
+  float3 lo = f3(INFINITY, INFINITY, INFINITY), hi = f3(-INFINITY, -INFINITY, -INFINITY);
+  uint32_t n_inner = 0;
+  for (int c = 0; c < cnt; ++c) {
+    const uint32_t r = refs[c];
+    const bool leaf = ref_is_leaf(r);
+    bl[c] = leaf ? plo[r & ~kLeafBit] : nlo[r];
+    bh[c] = leaf ? phi[r & ~kLeafBit] : nhi[r];
+    lo = f3(fminf(lo.x, bl[c].x), fminf(lo.y, bl[c].y), fminf(lo.z, bl[c].z));
+    hi = f3(fmaxf(hi.x, bh[c].x), fmaxf(hi.y, bh[c].y), fmaxf(hi.z, bh[c].z));
+    n_inner += leaf ? 0u : 1u;
+  }
+  uint32_t first = 0;
+  if (n_inner) {
+    first = atomicAdd(slot_counter, n_inner);
+    if (first + n_inner > max_nodes) {
+      atomicOr(overflow, 1u);
+      return;
+    }
+  }
+  // slots by direction: repeatedly the (child, slot) pair whose child lies furthest towards the slot
+  const float3 mid = f3(0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z));
+  uint32_t free_slots = 0xFFu, left_c = (1u << cnt) - 1u;
+  int slot_of[8];
+  for (int r = 0; r < cnt; ++r) {
+    float best = -INFINITY;
+    int bc = -1, bs = -1;
+    for (int c = 0; c < cnt; ++c) {
+      if (!((left_c >> c) & 1u)) continue;
+      const float x = 0.5f * (bl[c].x + bh[c].x) - mid.x, y = 0.5f * (bl[c].y + bh[c].y) - mid.y,
+                  z = 0.5f * (bl[c].z + bh[c].z) - mid.z;
+      for (int k = 0; k < 8; ++k) {
+        if (!((free_slots >> k) & 1u)) continue;
+        const float v = ((k & 1) ? x : -x) + ((k & 2) ? y : -y) + ((k & 4) ? z : -z);
+        if (bc < 0 || v > best) {
+          best = v;
+          bc = c;
+          bs = k;
+        }
+      }
+    }
+    slot_of[bc] = bs;
+    left_c &= ~(1u << bc);
+    free_slots &= ~(1u << bs);
+  }
+  if (!(fmaxf(hi.x - lo.x, fmaxf(hi.y - lo.y, hi.z - lo.z)) < kMaxExtent8)) {
+    atomicOr(overflow, 1u);
+    return;
+  }
+  float px, py, pz, qx, qy, qz;
+  frame8(lo.x, hi.x, px, qx);
+  frame8(lo.y, hi.y, py, qy);
+  frame8(lo.z, hi.z, pz, qz);
+  uint32_t b[6][2], ref8[8], imask = 0u, next = first;
+  for (int a = 0; a < 6; ++a) b[a][0] = b[a][1] = a < 3 ? 0xFFFFFFFFu : 0u;  // unused: lo 255, hi 0
+  for (int k = 0; k < 8; ++k) ref8[k] = kEmptyRef;
+  for (int c = 0; c < cnt; ++c) {
+    const int k = slot_of[c];
+    // outward to whole quanta with 1/64 of one to spare for the FP32 evaluation of the planes
+    const float lov[3] = {(bl[c].x - px) / qx, (bl[c].y - py) / qy, (bl[c].z - pz) / qz};
+    const float hiv[3] = {(bh[c].x - px) / qx, (bh[c].y - py) / qy, (bh[c].z - pz) / qz};
+    for (int a = 0; a < 3; ++a) {
+      const uint32_t l8 = (uint32_t)fminf(fmaxf(floorf(lov[a] - 0.015625f), 0.f), 255.f);
+      const uint32_t h8 = (uint32_t)fminf(fmaxf(ceilf(hiv[a] + 0.015625f), 0.f), 255.f);
+      const int sh = 8 * (k & 3);
+      b[a][k >> 2] = (b[a][k >> 2] & ~(0xFFu << sh)) | (l8 << sh);
+      b[3 + a][k >> 2] |= h8 << sh;
+    }
+    const uint32_t r = refs[c];
+    if (ref_is_leaf(r)) {
+      ref8[k] = kLeafBit | pos[r & ~kLeafBit];
+    } else {
+      imask |= 1u << k;
+      ref8[k] = next;
+      out[atomicAdd(out_count, 1u)] = Item8{r, next};
+      ++next;
+    }
+  }
+  auto eb = [](float q) { return (__float_as_uint(q) >> 23) + 15u; };
+  uint32_t* w = nodes + (size_t)it.slot * kNode8Words;
+  w[0] = __float_as_uint(px);
+  w[1] = __float_as_uint(py);
+  w[2] = __float_as_uint(pz);
+  w[3] = eb(qx) | (eb(qy) << 8) | (eb(qz) << 16) | (imask << 24);
+  for (int a = 0; a < 6; ++a) w[4 + 2 * a] = b[a][0], w[5 + 2 * a] = b[a][1];
+  for (int k = 0; k < 8; ++k) w[16 + k] = ref8[k];
+}
+
+// Node 0: only a reference to the root, node 1.
+__global__ void k_root8(uint32_t* __restrict__ nodes) {
+  const uint32_t k = threadIdx.x;
+  if (k < kNode8Words) nodes[k] = k == 16u ? 1u : (k >= 17u ? kEmptyRef : 0u);
+}
+
 // Scene order from the collapse's positions: order[pos[m]] = Morton order's caller index.
 __global__ void k_compose(uint32_t n, const uint32_t* __restrict__ morton_order, const uint32_t* __restrict__ pos,
                           uint32_t* __restrict__ order) {
@@ -847,12 +1082,16 @@ vp_status build_empty_scene(vp_context* ctx, const vp_gaussians* g, float sigma_
   v.wide = sc->wide;
   v.bin = sc->bin;
   v.pbox = sc->pbox;
+  v.nodes8 = nullptr;
+  v.depth8 = 0u;
   v.count = 0u;
   v.wide_root = 0u;
   v.bin_root = 0u;
   v.stack_cap = 31u + 2u;
   v.argmin_cap = v.stack_cap + kArgminBestFirstStack + 64u;
   v.albedo_all_zero = 1;
+  v.one_albedo = 1;
+  v.albedo = make_float3(0.f, 0.f, 0.f);
   v.tau_nearest = 0;
   vp_scene_info& info = sc->info;
   info = vp_scene_info{};
@@ -866,6 +1105,77 @@ vp_status build_empty_scene(vp_context* ctx, const vp_gaussians* g, float sigma_
   info.wide_collapse = opt.wide_collapse;
   info.albedo_all_zero = 1;
   info.device_bytes = 64ull + 4ull + 32ull + 32ull + 1024ull + 64ull;
+  return VP_OK;
+}
+
+// The compressed 8-wide BVH of a scene (sc->nodes8, depth8 levels counting node 0), cut from the binary
+// tree the BVH32 comes from.  depth8 = 0: the tree is too deep or too large for it (kMaxDepth8,
+// kMaxNodes8) and the engines use the warp-cooperative queries.
+static vp_status build_bvh8(vp_context* ctx, uint32_t n, uint32_t root, const uint32_t* wl, const uint32_t* wr,
+                            const float4* plo, const float4* phi, const float4* wlo, const float4* whi,
+                            const uint32_t* par, const uint32_t* par_leaf, const uint32_t* pos, vp_scene* sc,
+                            uint32_t& depth8, uint32_t& nodes8) {
+  cudaStream_t st = ctx->stream;
+  depth8 = nodes8 = 0;
+  const int TB = 256;
+  vp_status s;
+  Scratch<float> cost(st);
+  Scratch<uint8_t> choice(st);
+  Scratch<unsigned int> flags(st), ctr(st);
+  if (n > 1u) {
+    if ((s = dev_alloc(&cost.p, 8ull * (n - 1u), st))) return s;
+    if ((s = dev_alloc(&choice.p, 8ull * (n - 1u), st))) return s;
+    if ((s = dev_alloc(&flags.p, n - 1u, st))) return s;
+    VP_CUDA(cudaMemsetAsync(flags.p, 0, sizeof(unsigned int) * (n - 1u), st));
+    k_dp8_cost<<<(n + TB - 1) / TB, TB, 0, st>>>(n, root, wl, wr, plo, phi, wlo, whi, par, par_leaf, flags.p, cost.p,
+                                                 choice.p);
+    VP_CUDA(cudaGetLastError());
+  }
+  // every node has at least two children, so there are fewer nodes than Gaussians (+ node 0 and the root
+  // of a tree of one)
+  const uint32_t max_nodes = std::min(n + 1u, kMaxNodes8);
+  Scratch<uint32_t> nodes(st);
+  Scratch<Item8> qa(st), qb(st);
+  if ((s = dev_alloc(&nodes.p, (size_t)max_nodes * kNode8Words, st))) return s;
+  if ((s = dev_alloc(&qa.p, max_nodes, st))) return s;
+  if ((s = dev_alloc(&qb.p, max_nodes, st))) return s;
+  constexpr uint32_t kLevels = kMaxDepth8;             // levels below node 0 that may hold items
+  if ((s = dev_alloc(&ctr.p, kLevels + 3u, st))) return s;  // items per level, then next node, overflow
+  unsigned int c0[kLevels + 3u] = {};
+  c0[0] = 1u;
+  c0[kLevels + 1u] = 2u;
+  const Item8 root_item{n > 1u ? root : kLeafBit, 1u};
+  VP_CUDA(cudaMemcpyAsync(ctr.p, c0, sizeof(c0), cudaMemcpyHostToDevice, st));
+  VP_CUDA(cudaMemcpyAsync(qa.p, &root_item, sizeof(root_item), cudaMemcpyHostToDevice, st));
+  k_root8<<<1, 32, 0, st>>>(nodes.p);
+  VP_CUDA(cudaGetLastError());
+  uint64_t bound = 1;
+  uint32_t k = 0;
+  unsigned int c[kLevels + 3u];
+  while (true) {
+    // ~9 levels hold a 500k-Gaussian tree, so one read of the counts usually ends the loop
+    for (int i = 0; i < 12 && k < kLevels; ++i, ++k) {
+      Item8* in = (k & 1u) ? qb.p : qa.p;
+      Item8* out = (k & 1u) ? qa.p : qb.p;
+      k_collapse8<<<(unsigned)((bound + 127) / 128), 128, 0, st>>>(ctr.p + k, in, out, ctr.p + k + 1u,
+                                                                 ctr.p + kLevels + 1u, wl, wr, plo, phi, wlo, whi, pos,
+                                                                 choice.p, nodes.p, max_nodes, ctr.p + kLevels + 2u);
+      VP_CUDA(cudaGetLastError());
+      bound = std::min<uint64_t>(bound * 8u, max_nodes);
+    }
+    VP_CUDA(cudaMemcpyAsync(c, ctr.p, sizeof(c), cudaMemcpyDeviceToHost, st));
+    VP_CUDA(cudaStreamSynchronize(st));
+    if (c[kLevels + 2u] != 0u || c[k] == 0u || k == kLevels) break;
+    bound = c[k];
+  }
+  if (c[kLevels + 2u] != 0u || c[k] != 0u) return VP_OK;
+  uint32_t levels = 0;
+  while (c[levels] != 0u) ++levels;
+  if (levels + 1u > kMaxDepth8) return VP_OK;
+  nodes8 = c[kLevels + 1u];
+  if ((s = dev_alloc(&sc->nodes8, (size_t)nodes8 * kNode8Words, st))) return s;
+  VP_CUDA(cudaMemcpyAsync(sc->nodes8, nodes.p, 4ull * kNode8Words * nodes8, cudaMemcpyDeviceToDevice, st));
+  depth8 = levels + 1u;
   return VP_OK;
 }
 
@@ -918,7 +1228,7 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
   if ((s = dev_alloc(&errw.p, 1, st))) return s;
   if ((s = dev_alloc(&bounds.p, 12, st))) return s;
   {
-    ErrorWords e0{0x7FFFFFFF, 0x7FFFFFFF, 0x7FFFFFFF, 0u, 0u};
+    ErrorWords e0{0x7FFFFFFF, 0x7FFFFFFF, 0x7FFFFFFF, 0u, 0u, 0u, {0.f, 0.f, 0.f}};
     VP_CUDA(cudaMemcpyAsync(errw.p, &e0, sizeof(e0), cudaMemcpyHostToDevice, st));
     unsigned int b0[12];
     for (int k = 0; k < 3; ++k) {
@@ -1088,6 +1398,13 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
   sc->wide = wide;
   uint32_t depth = 1, wide_nodes = 1, leaves = 1;
   bool dp_used = false;
+  Scratch<uint32_t> par(st), par_leaf(st);
+  if (n > 1u) {
+    if ((s = dev_alloc(&par.p, n - 1u, st))) return s;
+    if ((s = dev_alloc(&par_leaf.p, n, st))) return s;
+    k_parents<<<(n - 1u + TB - 1) / TB, TB, 0, st>>>(n - 1u, wl, wr, par.p, par_leaf.p);
+    VP_CUDA(cudaGetLastError());
+  }
   if (n <= kLeafMax) {
     k_single_leaf_root<<<1, 32, 0, st>>>(n, plo.p, phi.p, wide);
     VP_CUDA(cudaGetLastError());
@@ -1098,7 +1415,7 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
     const uint32_t nint = n - 1u;
     Scratch<float> dp_cost(st);
     Scratch<uint8_t> dp_split(st), dp_best(st), dp_leaf(st);
-    Scratch<uint32_t> dp_single(st), par(st), par_leaf(st);
+    Scratch<uint32_t> dp_single(st);
     Scratch<unsigned int> dp_flags(st);
     DpTables T{nullptr, nullptr, nullptr, nullptr, nullptr};
     bool dp = opt.wide_collapse == VP_COLLAPSE_SAH && n <= (1u << 24);
@@ -1108,12 +1425,8 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
       if ((s = dev_alloc(&dp_best.p, 32ull * nint, st))) return s;
       if ((s = dev_alloc(&dp_leaf.p, nint, st))) return s;
       if ((s = dev_alloc(&dp_single.p, nint, st))) return s;
-      if ((s = dev_alloc(&par.p, nint, st))) return s;
-      if ((s = dev_alloc(&par_leaf.p, n, st))) return s;
       if ((s = dev_alloc(&dp_flags.p, nint, st))) return s;
       VP_CUDA(cudaMemsetAsync(dp_flags.p, 0, sizeof(unsigned int) * nint, st));
-      k_parents<<<(nint + TB - 1) / TB, TB, 0, st>>>(nint, wl, wr, par.p, par_leaf.p);
-      VP_CUDA(cudaGetLastError());
       T = DpTables{dp_cost.p, dp_split.p, dp_best.p, dp_single.p, dp_leaf.p};
       k_dp_cost<<<nb, TB, 0, st>>>(n, wide_root, wl, wr, plo.p, phi.p, wlo, whi, par.p, par_leaf.p, dp_flags.p, T,
                                    kLeafMax);
@@ -1179,6 +1492,9 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
       dp = false;
     }
   }
+  uint32_t depth8 = 0, nodes8 = 0;
+  if ((s = build_bvh8(ctx, n, wide_root, wl, wr, plo.p, phi.p, wlo, whi, par.p, par_leaf.p, pos.p, sc, depth8, nodes8)))
+    return s;
   // Scene order, then the records, boxes and adjoint inputs gathered into it.
   uint32_t* perm = nullptr;
   if ((s = dev_alloc(&perm, n, st))) return s;
@@ -1235,12 +1551,16 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
   v.wide = wide;
   v.bin = bin;
   v.pbox = pbox;
+  v.nodes8 = sc->nodes8;
+  v.depth8 = depth8;
   v.count = n;
   v.wide_root = 0u;
   v.bin_root = bin_root;
   v.stack_cap = 31u * depth + 2u;
   v.argmin_cap = v.stack_cap + kArgminBestFirstStack + 64u;
   v.albedo_all_zero = eh.any_albedo ? 0 : 1;
+  v.one_albedo = eh.mixed_albedo ? 0 : 1;
+  v.albedo = make_float3(eh.albedo0[0], eh.albedo0[1], eh.albedo0[2]);
   // AUTO: nearest first where rays need many translucent Gaussians to become opaque and the tree
   // has levels below the root's children to order (on a two-level tree the ranking pass costs
   // more than it saves)
@@ -1272,8 +1592,9 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
     info.bounds_min[k] = o2f(bh[6 + k]);
     info.bounds_max[k] = o2f(bh[9 + k]);
   }
-  // records, order, per-Gaussian boxes, adjoint inputs, BVH32, binary LBVH
-  info.device_bytes = 64ull * n + 4ull * n + 32ull * n + 32ull * n + 1024ull * wide_nodes + 64ull * ni;
+  // records, order, per-Gaussian boxes, adjoint inputs, BVH32, binary tree, BVH8
+  info.device_bytes = 64ull * n + 4ull * n + 32ull * n + 32ull * n + 1024ull * wide_nodes + 64ull * ni +
+                      4ull * kNode8Words * nodes8;
   return VP_OK;
 }
 

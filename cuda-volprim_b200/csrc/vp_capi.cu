@@ -305,6 +305,7 @@ vp_status vp_scene_destroy(vp_scene* s) {
   dev_free(s->wide, st);
   dev_free(s->bin, st);
   dev_free(s->pbox, st);
+  dev_free(s->nodes8, st);
   dev_free(s->raw, st);
   dev_free(s->emis, st);
   if (st) cudaStreamSynchronize(st);

@@ -75,6 +75,8 @@ struct SceneView {
   const float4* wide;    // BVH32: node k = 32 lo float4 then 32 hi float4; lo.w = child ref
   const float4* bin;     // binary LBVH: node i = (l_lo, l_hi, r_lo, r_hi); lo.w = child ref
   const float4* pbox;    // per Gaussian (Morton order): 3-sigma box lo, hi (2 float4)
+  const uint32_t* nodes8;  // compressed 8-wide BVH (vp_trace8.cuh), or null when depth8 is 0
+  uint32_t depth8;         // its levels
   uint32_t count;
   uint32_t wide_root;    // ref of the BVH32 root (a node index; 0)
   uint32_t bin_root;     // ref of the binary root
@@ -83,6 +85,8 @@ struct SceneView {
                          // kArgminBestFirstStack + 64 (best-first pops need room beyond the
                          // depth-first bound; see warp_ray_query)
   int32_t albedo_all_zero;
+  int32_t one_albedo;    // every Gaussian has the same albedo: the weighted mean at any point is that one
+  float3 albedo;         // it, when one_albedo
   uint32_t tau_nearest;  // transmittance stacks hit children nearest first (VP_TAU_ORDER_NEAREST)
 };
 
@@ -652,6 +656,13 @@ __device__ __forceinline__ float warp_sum_ff(FF v) {
     v = ff_add(v, w);
   }
   return __fadd_rn(v.hi, v.lo);
+}
+// FP64 sum over the warp: sums carried in FP64 and rounded once give the same FP32 result whatever the
+// order of their terms.
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+  return v;
 }
 __device__ __forceinline__ float warp_min(float v) {
 #pragma unroll

@@ -325,11 +325,13 @@ __global__ void __launch_bounds__(256, 4) k_srv_extend(const SceneView* __restri
     ScatterAlbedo sa;
     sa.valid = false;
     if (!(bounce == 0 && S.albedo_all_zero))
-      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, ((uint64_t)k2.y << 32) | k2.x, status, ws, false, &sa);
+      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, ((uint64_t)k2.y << 32) | k2.x, status, ws, false, &sa,
+                                             bounce ? b.sg[p] : kNoGauss);
     float3 albedo = f3(0.f, 0.f, 0.f);
     if (tstar < kInf) {
       uint32_t ov = sa.overlap;
-      albedo = sa.valid ? sa.albedo : warp_albedo<kAcc>(S, W, fma3(tstar, df, of), ov, status, ws, false);
+      albedo = sa.valid ? sa.albedo : warp_scatter_albedo<kAcc>(S, W, of, df, tstar, ov, status, ws, false);
+      if (S.one_albedo) albedo = S.albedo;
     }
     if (lane == 0) {
       b.alb4[p] = make_float4(albedo.x, albedo.y, albedo.z, tstar);

@@ -1,0 +1,348 @@
+// Thread-per-ray queries over the compressed 8-wide BVH, with the per-Gaussian work of a warp's 32
+// rays pooled: the queries of the wavefront and serving engines and of large transmittance batches.
+//
+// What bounds it, and why this split.  The warp-cooperative query (vp_traverse.cuh) spends 32 lanes
+// on one ray; its chord set-up runs with about two lanes busy.  Here a lane walks its own ray through
+// the inner nodes, and what it finds is shared out over the whole warp:
+//   node step   every lane with nodes left tests the 8 quantised child boxes of one node (64 B + one
+//               child reference); hit inner children stay with the lane (one stack entry a level),
+//               hit Gaussians go to the warp's queue 1 as (lane, node, slot);
+//   chord step  when queue 1 holds 32 entries, lane e loads the e-th Gaussian's record and sets up
+//               its chord against the owner's ray (shuffled over); the few that cross go to queue 2;
+//   value step  when queue 2 holds 32 chords, lane e evaluates the e-th (optical depth, free flight
+//               or albedo weight) and each owner collects its own by shuffles.
+// So box tests, chord set-ups and erf / erfinv evaluations each run with nearly full warps, whatever
+// the 32 rays do.  A warp refills its finished lanes together, after draining both queues.
+//
+// Results do not depend on which rays share a warp or in which order chords are met: the argmin is a
+// minimum, and the sums (optical depth, albedo weights) are carried in FP64 and rounded once.
+#pragma once
+
+#include "vp_traverse.cuh"
+
+namespace vp {
+
+// ---- node layout: 96 B = 24 words ------------------------------------------------------------
+//   words 0..2   box origin p (FP32)
+//   word  3      bytes: 15 + exponent of the x / y / z quantum (biased as a float's), inner mask
+//   words 4..15  child planes, a byte each: lo.x[8] lo.y[8] lo.z[8] hi.x[8] hi.y[8] hi.z[8]
+//   words 16..23 child references: an inner node's index or kLeafBit | Gaussian (scene order)
+// Child slot s holds the child that lies furthest towards (s&1 ? +x : -x, s&2 ? +y : -y, s&4 ? +z : -z),
+// so visiting slots in ascending (s ^ sign bits of the direction) is roughly front to back.
+// An unused slot has lo = 255, hi = 0 (never hit).  Node 0 only points to the root (slot 0).
+constexpr uint32_t kNode8Words = 24;
+constexpr uint32_t kMaxNodes8 = 1u << 24;   // stack entries hold (node << 8 | child mask)
+constexpr uint32_t kMaxDepth8 = 40;         // deeper trees take the warp-cooperative query
+// A value step runs once queue 2 holds this many chords.  Fuller steps cost fewer instructions a chord,
+// earlier ones tighten the free-flight bound (and reach MAX_OPTICAL_DEPTH) sooner: 8 measured fastest or
+// level with 16 on every scene tried (showcase 66.6 / 67.2 / 69.8 ms at 8 / 16 / 32; a 100k-Gaussian image
+// of 361k paths 6.3 / 6.7 / 7.6 ms).
+constexpr int kValueStep = 8;
+constexpr int kQ1Cap = 32 + 256, kQ2Cap = 64, kQ2Words = 7;
+
+// Words of shared memory per warp: stack, queue 1, queue 2, owner masks.
+__host__ __device__ __forceinline__ uint32_t trace8_warp_words(uint32_t depth) {
+  return depth * 32u + kQ1Cap + kQ2Cap * kQ2Words + 32u;
+}
+__host__ __device__ __forceinline__ size_t trace8_smem_bytes(uint32_t depth, int threads) {
+  return (size_t)trace8_warp_words(depth) * 4u * (size_t)(threads / 32);
+}
+
+enum Query8 { kFlight8 = 0, kTau8 = 1, kScatter8 = 2 };
+
+struct Ray8 {
+  float3 o, d;
+  uint64_t key;    // kFlight8: free-flight key
+  float t;         // kScatter8: scatter distance
+  uint32_t seed;   // kTau8: the Gaussian already accounted for; kFlight8: one to start with (kNoGauss: none)
+  float seed_tau;  // its optical depth (0 without one)
+};
+struct Hit8 {
+  float t;          // kFlight8: free-flight minimum (kInf: escape)
+  uint32_t gauss;   // kFlight8: its Gaussian
+  double w, r, g, b;  // kTau8: w = optical depth; kScatter8: sums of weight, weight x albedo
+  uint32_t count;   // kScatter8: Gaussians containing the point
+};
+
+__device__ __forceinline__ float byte_plane(uint32_t word, uint32_t sel) {  // 1 + q / 32768
+  return __uint_as_float(__byte_perm(word, 0x3F800000u, sel));
+}
+
+// One warp's share of n rays.  source(item, ray) fills the ray of an item and returns false when the
+// item needs no query (its sink is not called); sink(item, ray, hit) takes the result.  `rpw` rays are
+// in flight per warp: fewer than 32 when the batch is too small to give every resident warp 32, since
+// the chord and value steps use all lanes anyway.
+template <bool kAcc, int kKind, class Source, class Sink>
+__device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const float4* __restrict__ prims,
+                                       const uint32_t* __restrict__ perm, uint32_t depth, uint32_t* smem, uint32_t n,
+                                       unsigned int* work, int rpw, uint32_t& status, Source&& source, Sink&& sink) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  uint32_t* stack = smem + lane;  // entry k at stack[32 k]: conflict-free whatever the lanes' depths
+  uint32_t* q1 = smem + depth * 32u;
+  uint32_t* q2 = q1 + kQ1Cap;
+  uint32_t* own = q2 + kQ2Cap * kQ2Words;
+  int q1n = 0, q2n = 0;
+  Ray8 ray;
+  ray.o = ray.d = f3(0.f, 0.f, 0.f);
+  ray.key = 0ull;
+  ray.seed = kNoGauss;
+  ray.t = 0.f;
+  float3 inv = f3(0.f, 0.f, 0.f);
+  uint32_t item = 0, node = 0, mask = 0, neg = 0;
+  int sp = 0;
+  bool active = false, more = true;
+  float t_hi = kInf;
+  uint32_t arg = kNoGauss, cnt = 0;
+  double acc = 0.0, ar = 0.0, ag = 0.0, ab = 0.0;
+  const unsigned used = rpw >= 32 ? kFull : ((1u << rpw) - 1u);
+  const int refill = max(1, rpw / 4);
+
+  // value step over the top k chords of queue 2
+  auto values = [&](int k) {
+    const int e = q2n - k + lane;
+    q2n -= k;
+    uint32_t id = 0;
+    float v = kInf, wa = 0.f, wb = 0.f, wc = 0.f;
+    const bool on = lane < k;
+    if (on) id = q2[e];
+    const int ow = (int)(id >> 27) & 31;
+    const uint32_t gi = id & 0x07FFFFFFu;
+    uint64_t key = 0ull;
+    float ts = 0.f;
+    if constexpr (kKind == kFlight8)
+      key = ((uint64_t)__shfl_sync(kFull, (uint32_t)(ray.key >> 32), ow) << 32) |
+            __shfl_sync(kFull, (uint32_t)ray.key, ow);
+    if constexpr (kKind == kScatter8) ts = __shfl_sync(kFull, ray.t, ow);
+    if (on) {
+      Chord ch;
+      ch.tc = __uint_as_float(q2[kQ2Cap + e]);
+      ch.rw = __uint_as_float(q2[2 * kQ2Cap + e]);
+      ch.d2 = __uint_as_float(q2[3 * kQ2Cap + e]);
+      ch.h = __uint_as_float(q2[4 * kQ2Cap + e]);
+      const float icf = __uint_as_float(q2[5 * kQ2Cap + e]);
+      ch.d2lo = kAcc ? __uint_as_float(q2[6 * kQ2Cap + e]) : 0.0f;
+      ch.t_in = fmaf(-ch.h, ch.rw, ch.tc);
+      ch.t_out = fmaf(ch.h, ch.rw, ch.tc);
+      if constexpr (kKind == kTau8) {
+        v = chord_tau<kAcc>(ch.tc, ch.rw, ch.d2, ch.h, chord_u0(ch, 0.0f), fmaxf(ch.t_in, 0.0f), ch.t_out, icf, ch.d2lo);
+      } else if constexpr (kKind == kFlight8) {
+        v = chord_free_flight<kAcc>(ch.tc, ch.rw, ch.d2, ch.h, chord_u0(ch, 0.0f), ch.t_in, ch.t_out, icf,
+                                    free_flight_tau<kAcc>(key, __ldg(perm + gi)), ch.d2lo);
+      } else {
+        const float u = (ts - ch.tc) / ch.rw;
+        v = icf * vexp<kAcc>(-0.5f * fmaf(u, u, ch.d2));
+        const float3 al = load_albedo(prims, gi);
+        wa = al.x, wb = al.y, wc = al.z;
+      }
+    }
+    // each owner finds its chords: the mask of lanes holding them, left in own[] by their lowest lane
+    const unsigned peers = __match_any_sync(kFull, on ? ow : 32 + lane);
+    own[lane] = 0u;
+    __syncwarp();
+    if (on && (peers & lt) == 0u) own[ow] = peers;
+    __syncwarp();
+    unsigned m = own[lane];
+    while (__any_sync(kFull, m != 0u)) {
+      const int j = m ? __ffs(m) - 1 : lane;
+      const float vj = __shfl_sync(kFull, v, j);
+      if constexpr (kKind == kTau8) {
+        if (m) acc += (double)vj;
+      } else if constexpr (kKind == kFlight8) {
+        const uint32_t gj = __shfl_sync(kFull, gi, j);
+        if (m && vj < t_hi) {
+          t_hi = vj;
+          arg = gj;
+        }
+      } else {
+        const float x = __shfl_sync(kFull, wa, j), y = __shfl_sync(kFull, wb, j), z = __shfl_sync(kFull, wc, j);
+        if (m) {
+          acc += (double)vj;
+          ar += (double)vj * (double)x;
+          ag += (double)vj * (double)y;
+          ab += (double)vj * (double)z;
+          ++cnt;
+        }
+      }
+      m &= m - 1u;
+    }
+    __syncwarp();
+    if (kKind == kTau8 && acc >= (double)kMaxOpticalDepth) {  // opaque: the rest of its nodes cannot matter
+      mask = 0u;
+      sp = 0;
+    }
+  };
+
+  // chord step over the top k entries of queue 1
+  auto chords = [&](int k) {
+    const int e = q1n - k + lane;
+    q1n -= k;
+    const uint32_t w = lane < k ? q1[e] : 0u;
+    __syncwarp();
+    const int ow = (int)(w >> 27);
+    const uint32_t at = w & 0x07FFFFFFu;  // node * 8 + slot
+    uint32_t gi = 0;
+    if (lane < k) gi = __ldg(nodes + (size_t)(at >> 3) * kNode8Words + 16u + (at & 7u)) & ~kLeafBit;
+    const float3 o = f3(__shfl_sync(kFull, ray.o.x, ow), __shfl_sync(kFull, ray.o.y, ow), __shfl_sync(kFull, ray.o.z, ow));
+    const float3 d = f3(__shfl_sync(kFull, ray.d.x, ow), __shfl_sync(kFull, ray.d.y, ow), __shfl_sync(kFull, ray.d.z, ow));
+    bool hit = lane < k;
+    float bound = kInf;
+    if constexpr (kKind == kTau8) {
+      const uint32_t seed = __shfl_sync(kFull, ray.seed, ow);
+      hit = hit && gi != seed;
+    } else {
+      bound = __shfl_sync(kFull, kKind == kFlight8 ? t_hi : ray.t, ow);
+    }
+    Chord ch;
+    if (hit) {
+      PrimGeo g;
+      g.a = __ldg(prims + 4u * gi);
+      g.b = __ldg(prims + 4u * gi + 1u);
+      g.c = __ldg(prims + 4u * gi + 2u);
+      hit = chord_setup<kAcc>(g, o, d, ch);
+      if constexpr (kKind == kScatter8) hit = hit && ch.t_in <= bound && bound <= ch.t_out;
+      else hit = hit && ch.t_out > 0.0f && ch.t_in <= bound;
+    }
+    const unsigned hm = __ballot_sync(kFull, hit);
+    if (hm == 0u) return;
+    if (hit) {
+      const int p = q2n + __popc(hm & lt);
+      q2[p] = ((uint32_t)ow << 27) | gi;
+      q2[kQ2Cap + p] = __float_as_uint(ch.tc);
+      q2[2 * kQ2Cap + p] = __float_as_uint(ch.rw);
+      q2[3 * kQ2Cap + p] = __float_as_uint(ch.d2);
+      q2[4 * kQ2Cap + p] = __float_as_uint(ch.h);
+      q2[5 * kQ2Cap + p] = __ldg(reinterpret_cast<const uint32_t*>(prims + 4u * gi + 3u));
+      if (kAcc) q2[6 * kQ2Cap + p] = __float_as_uint(ch.d2lo);
+    }
+    q2n += __popc(hm);
+    __syncwarp();
+    if (q2n >= kValueStep) values(min(q2n, 32));
+  };
+
+  while (true) {
+    const unsigned busy = __ballot_sync(kFull, active && (mask != 0u || sp != 0));
+    const int free_lanes = __popc(used & ~busy);
+    if (busy == 0u || (more && free_lanes >= refill)) {
+      while (q1n > 0) chords(min(q1n, 32));
+      if (q2n > 0) values(q2n);
+      if (active && mask == 0u && sp == 0) {
+        Hit8 h;
+        h.t = t_hi, h.gauss = arg, h.w = acc, h.r = ar, h.g = ag, h.b = ab, h.count = cnt;
+        sink(item, ray, h);
+        active = false;
+      }
+      if (more) {
+        const unsigned want = used & __ballot_sync(kFull, !active);
+        uint32_t first = 0;
+        if (lane == 0) first = atomicAdd(work, (unsigned)__popc(want));
+        first = __shfl_sync(kFull, first, 0);
+        more = first + (uint32_t)__popc(want) < n;
+        if ((want >> lane) & 1u) {
+          item = first + (uint32_t)__popc(want & lt);
+          if (item < n && source(item, ray)) {
+            active = true;
+            inv = safe_inv(ray.d);
+            neg = (inv.x < 0.f ? 1u : 0u) | (inv.y < 0.f ? 2u : 0u) | (inv.z < 0.f ? 4u : 0u);
+            node = 0u;
+            mask = 1u << neg;  // slot 0 of node 0: the root
+            sp = 0;
+            t_hi = kKind == kScatter8 ? ray.t : kInf;
+            arg = kNoGauss;
+            cnt = 0u;
+            acc = ar = ag = ab = 0.0;
+            if constexpr (kKind == kTau8) {
+              if (ray.seed != kNoGauss) acc = (double)ray.seed_tau;
+            }
+            if constexpr (kKind == kFlight8) {
+              // a path that scattered starts inside the Gaussian that scattered it: its free flight
+              // bounds the traversal from the start (showcase: 63 -> 33 nodes a ray with it)
+              if (ray.seed != kNoGauss) {
+                const PrimGeo g = load_geo(prims, ray.seed);
+                Chord ch;
+                if (chord_setup<kAcc>(g, ray.o, ray.d, ch) && ch.t_out > 0.0f) {
+                  const float v = chord_free_flight<kAcc>(ch.tc, ch.rw, ch.d2, ch.h, chord_u0(ch, 0.0f), ch.t_in, ch.t_out,
+                                                          g.icf, free_flight_tau<kAcc>(ray.key, __ldg(perm + ray.seed)),
+                                                          ch.d2lo);
+                  if (v < t_hi) t_hi = v, arg = ray.seed;
+                }
+              }
+            }
+          }
+        }
+      }
+      if (!__any_sync(kFull, active) && !more) break;
+      continue;
+    }
+    // node step
+    uint32_t leaf = 0u;
+    if (active && (mask != 0u || sp != 0)) {
+      if (mask == 0u) {
+        const uint32_t e = stack[32 * --sp];
+        node = e >> 8;
+        mask = e & 0xFFu;
+      }
+      const uint32_t b = (uint32_t)__ffs(mask) - 1u;
+      mask &= mask - 1u;
+      const uint32_t cur = __ldg(nodes + (size_t)node * kNode8Words + 16u + (b ^ neg));
+      if (mask != 0u) {
+        if ((uint32_t)sp >= depth) {  // cannot happen for a tree of the recorded depth
+          status |= kStatusStackOverflow;
+        } else {
+          stack[32 * sp++] = (node << 8) | mask;
+        }
+      }
+      const float4* p4 = reinterpret_cast<const float4*>(nodes + (size_t)cur * kNode8Words);
+      const float4 h = __ldg(p4);
+      const uint4 a = __ldg(reinterpret_cast<const uint4*>(p4) + 1), bq = __ldg(reinterpret_cast<const uint4*>(p4) + 2),
+                  c = __ldg(reinterpret_cast<const uint4*>(p4) + 3);
+      const uint32_t ew = __float_as_uint(h.w);
+      const float ax = __uint_as_float((ew & 0xFFu) << 23) * inv.x;
+      const float ay = __uint_as_float((ew & 0xFF00u) << 15) * inv.y;
+      const float az = __uint_as_float((ew & 0xFF0000u) << 7) * inv.z;
+      const float bx = fmaf(h.x - ray.o.x, inv.x, -ax), by = fmaf(h.y - ray.o.y, inv.y, -ay),
+                  bz = fmaf(h.z - ray.o.z, inv.z, -az);
+      const bool nx = neg & 1u, ny = neg & 2u, nz = neg & 4u;
+      // near / far planes by the direction's signs: (lo.x, hi.x) = (a.xy, bq.zw), (lo.y, hi.y) = (a.zw, c.xy),
+      // (lo.z, hi.z) = (bq.xy, c.zw)
+      const uint32_t nxw[2] = {nx ? bq.z : a.x, nx ? bq.w : a.y}, fxw[2] = {nx ? a.x : bq.z, nx ? a.y : bq.w};
+      const uint32_t nyw[2] = {ny ? c.x : a.z, ny ? c.y : a.w}, fyw[2] = {ny ? a.z : c.x, ny ? a.w : c.y};
+      const uint32_t nzw[2] = {nz ? c.z : bq.x, nz ? c.w : bq.y}, fzw[2] = {nz ? bq.x : c.z, nz ? bq.y : c.w};
+      const float lo_t = kKind == kScatter8 ? ray.t : 0.0f;
+      uint32_t hits = 0u;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t sel = 0x7604u | ((uint32_t)(j & 3) << 4);
+        const float tn = fmax3f(fmaf(byte_plane(nxw[j >> 2], sel), ax, bx), fmaf(byte_plane(nyw[j >> 2], sel), ay, by),
+                                fmaxf(fmaf(byte_plane(nzw[j >> 2], sel), az, bz), lo_t));
+        const float tf = fmin3f(fmaf(byte_plane(fxw[j >> 2], sel), ax, bx), fmaf(byte_plane(fyw[j >> 2], sel), ay, by),
+                                fminf(fmaf(byte_plane(fzw[j >> 2], sel), az, bz), t_hi));
+        if (tn <= tf) hits |= 1u << j;
+      }
+      // slots -> visiting order (bit s moves to bit s ^ neg)
+      uint32_t im = ((ew >> 24) << 8) | hits;
+      if (nx) im = ((im & 0x5555u) << 1) | ((im >> 1) & 0x5555u);
+      if (ny) im = ((im & 0x3333u) << 2) | ((im >> 2) & 0x3333u);
+      if (nz) im = ((im & 0x0F0Fu) << 4) | ((im >> 4) & 0x0F0Fu);
+      const uint32_t inner = im >> 8, ph = im & 0xFFu;
+      node = cur;
+      mask = ph & inner;
+      leaf = ph & ~inner;
+    }
+    // hit Gaussians to queue 1
+    unsigned bal;
+    while ((bal = __ballot_sync(kFull, leaf != 0u)) != 0u) {
+      if (leaf != 0u) {
+        const uint32_t b = (uint32_t)__ffs(leaf) - 1u;
+        leaf &= leaf - 1u;
+        q1[q1n + __popc(bal & lt)] = ((uint32_t)lane << 27) | (node << 3) | (b ^ neg);
+      }
+      q1n += __popc(bal);
+    }
+    __syncwarp();
+    while (q1n >= 32) chords(32);
+    if (__any_sync(kFull, status != 0u)) break;
+  }
+}
+
+}  // namespace vp

@@ -171,6 +171,11 @@ __device__ __forceinline__ float point_r2(const PrimGeo& g, float3 x) {
   }
 }
 
+// Mean albedo of FP64 sums of weight and weight x albedo.
+__device__ __forceinline__ float3 mean_albedo(double w, double r, double g, double b) {
+  return w > 0.0 ? f3((float)(r / w), (float)(g / w), (float)(b / w)) : f3(0.f, 0.f, 0.f);
+}
+
 struct WarpStats {
   unsigned long long crossings = 0, nodes = 0, leaves = 0;
   unsigned long long kind_nodes[3] = {0, 0, 0}, kind_leaves[3] = {0, 0, 0};
@@ -211,17 +216,18 @@ __device__ __forceinline__ float seed_chord_tau(const SceneView& S, uint32_t see
 // evaluate_albedo (:257-283), with the whitened radius from the chord frame,
 // |y|^2 = d2 + ((t* - t_c)|w|)^2.  Every Gaussian containing the scatter point was processed (its
 // chord starts before t* <= t), so the set is complete; if the retained chords outgrow the
-// buffer, sa->valid stays false and the caller runs the point query instead.
+// buffer, sa->valid stays false and the caller runs warp_scatter_albedo instead.
 //
 // The optical depth is summed over the warp in FP32 after every leaf step (for the stop at
-// MAX_OPTICAL_DEPTH); under kAcc each lane also keeps a compensated float-pair sum of its own
-// chords, reduced once at the end, so thousands of overlapping chords keep the 1e-5
-// transmittance bound.
+// MAX_OPTICAL_DEPTH); each lane also keeps an FP64 sum of its own chords, reduced once at the end and
+// rounded once, so the result does not depend on the order of the chords (the thread-per-ray queries
+// of vp_trace8.cuh give the same one) and thousands of them keep the 1e-5 transmittance bound.
 //
 // A kTau query whose origin lies inside a known Gaussian (`seed`, the one whose free flight put
 // the path there) evaluates that chord first (or takes its value, seed_tau, when the caller
 // evaluated it already): in a dense medium it alone usually reaches MAX_OPTICAL_DEPTH and the
-// traversal is skipped; otherwise the traversal skips it at its leaf.
+// traversal is skipped; otherwise the traversal skips it at its leaf.  A kArgmin query from there starts
+// with that Gaussian's free flight as its bound (and meets it again at its leaf).
 template <bool kAcc, int kKind>
 __device__ float warp_ray_query(const SceneView& S, const WarpSmem& W, float3 o, float3 d,
                                 uint64_t key, uint32_t& status, WarpStats& ws, bool measure,
@@ -231,17 +237,23 @@ __device__ float warp_ray_query(const SceneView& S, const WarpSmem& W, float3 o,
   const RayBox rb = ray_box(o, d);
   float t_hi = kInf;
   float acc = 0.0f;
-  FF lane_tau = {0.0f, 0.0f};  // kAcc: this lane's chords as a compensated float pair
-  auto tau_total = [&]() -> float {
-    if constexpr (kAcc) return warp_sum_ff(lane_tau);
-    else return acc;
-  };
+  double lane_tau = 0.0;  // this lane's chords
+  auto tau_total = [&]() -> float { return (float)warp_sum(lane_tau); };
   uint32_t arg = kNoGauss;  // kArgmin: the Gaussian of the current minimum
+  if (kKind == kArgmin && seed != kNoGauss) {  // the same on every lane
+    const PrimGeo g = load_geo(S.prims, seed);
+    Chord ch;
+    if (chord_setup<kAcc>(g, o, d, ch) && ch.t_out > 0.0f) {
+      const float v = chord_free_flight<kAcc>(ch.tc, ch.rw, ch.d2, ch.h, chord_u0(ch, 0.0f), ch.t_in, ch.t_out, g.icf,
+                                              free_flight_tau<kAcc>(key, __ldg(S.perm + seed)), ch.d2lo) + 0.0f;
+      if (v < t_hi) t_hi = v, arg = seed;
+    }
+  }
   if (kKind == kTau && seed != kNoGauss) {
     float v = 0.0f;  // seed_tau >= 0: evaluated ahead of the query (seed_chord_tau)
     if (lane == 0) v = seed_tau >= 0.0f ? seed_tau : seed_chord_tau<kAcc>(S, seed, o, d);
     acc = __shfl_sync(kFull, v, 0);
-    if (kAcc) lane_tau.hi = v;  // v is 0 on lanes other than 0
+    lane_tau = (double)v;  // v is 0 on lanes other than 0
     if (measure) ws.crossings += 1;
     if (acc >= kMaxOpticalDepth) {
       if (measure) {
@@ -255,7 +267,8 @@ __device__ float warp_ray_query(const SceneView& S, const WarpSmem& W, float3 o,
   // best-first pops while the stack holds at most bf_limit entries (negative: never, for a warp
   // stack without the argmin's extra room)
   const int bf_limit = min((int)kArgminBestFirstStack, (int)W.st_cap - (int)S.stack_cap - 64);
-  bool keep = (kKind == kArgmin) && sa != nullptr;
+  // a scene of one albedo needs no set at the scatter point, except to measure its overlap
+  bool keep = (kKind == kArgmin) && sa != nullptr && (!S.one_albedo || measure);
   unsigned int hits_seen = 0;
   // The node to visit next is kept in registers (the nearest hit child of the last inner node);
   // only its siblings go through the shared-memory stack.
@@ -369,7 +382,7 @@ __device__ float warp_ray_query(const SceneView& S, const WarpSmem& W, float3 o,
       Chord ch;
       float icf = 0.f;
       bool boxed = false;
-      if (lane < total && pi != seed) {  // the Gaussian's own 3-sigma box first (32 B), then its record
+      if (lane < total && (kKind == kArgmin || pi != seed)) {  // the Gaussian's own 3-sigma box first (32 B), then its record
         float tb;
         boxed = slab<kKind == kArgmin>(rb, __ldg(S.pbox + 2u * pi), __ldg(S.pbox + 2u * pi + 1u), 0.0f, t_hi, tb);
       }
@@ -393,7 +406,7 @@ __device__ float warp_ray_query(const SceneView& S, const WarpSmem& W, float3 o,
                                                 ch.t_out, icf, ch.d2lo)
                               : 0.0f;
           acc += warp_sum(v);
-          if (kAcc) ff_accumulate(lane_tau, v);
+          lane_tau += (double)v;
           hits_seen += __popc(m);
           if (measure) ws.crossings += (unsigned)__popc(m);
           if (acc >= kMaxOpticalDepth) break;
@@ -427,7 +440,7 @@ __device__ float warp_ray_query(const SceneView& S, const WarpSmem& W, float3 o,
           const int nr = __popc(rm);
           if (nr != 0 && hb + nr > W.hit_cap) {  // make room: drop chords that start beyond t_hi
             compact();
-            if (hb + nr > W.hit_cap) {  // still full: stop retaining, the caller will query the point
+            if (hb + nr > W.hit_cap) {  // still full: stop retaining, the caller will run warp_scatter_albedo
               keep = false;
               kept = hb = 0;
             }
@@ -520,18 +533,18 @@ __device__ float warp_ray_query(const SceneView& S, const WarpSmem& W, float3 o,
       sa->gauss = t_hi < kInf ? arg : kNoGauss;
       if (keep && t_hi < kInf) {
         const float ts = t_hi;
-        float aw = 0.f, ar = 0.f, ag = 0.f, ab = 0.f;
+        double aw = 0.0, ar = 0.0, ag = 0.0, ab = 0.0;
         unsigned int cnt = 0;
         for (int base = 0; base < kept; base += 32) {
           const int e = base + lane;
           if (e < kept && W.hb_tin[e] <= ts && ts <= W.hb_tout[e]) {
             const float u = (ts - W.hb_tc[e]) / W.hb_rw[e];
-            const float wgt = W.hb_icf[e] * vexp<kAcc>(-0.5f * fmaf(u, u, W.hb_d2[e]));
+            const double wgt = (double)(W.hb_icf[e] * vexp<kAcc>(-0.5f * fmaf(u, u, W.hb_d2[e])));
             const float3 al = load_albedo(S.prims, W.hb_idx[e]);
             aw += wgt;
-            ar += wgt * al.x;
-            ag += wgt * al.y;
-            ab += wgt * al.z;
+            ar += wgt * (double)al.x;
+            ag += wgt * (double)al.y;
+            ab += wgt * (double)al.z;
             ++cnt;
           }
         }
@@ -540,16 +553,94 @@ __device__ float warp_ray_query(const SceneView& S, const WarpSmem& W, float3 o,
         ag = warp_sum(ag);
         ab = warp_sum(ab);
         for (int off = 16; off > 0; off >>= 1) cnt += __shfl_xor_sync(kFull, cnt, off);
-        const float r = aw > 0.f ? __frcp_rn(aw) : 0.f;
-        sa->albedo = aw > 0.f ? f3(ar * r, ag * r, ab * r) : f3(0.f, 0.f, 0.f);
+        sa->albedo = mean_albedo(aw, ar, ag, ab);
         sa->overlap = cnt;
         sa->valid = true;
       }
+      if (S.one_albedo && !measure) {
+        sa->overlap = 0u;
+        sa->valid = true;
+      }
+      if (S.one_albedo) sa->albedo = S.albedo;
     }
   }
   __syncwarp();
   if constexpr (kKind == kArgmin) return t_hi;
   else return tau_total();
+}
+
+// Albedo at distance t along a ray: the sum over the chords containing t that an argmin query takes from
+// its own retained chords, found by a traversal of its own -- for the rays whose chords outgrew the hit
+// buffer.  The same terms in FP64, so the same result.
+template <bool kAcc>
+__device__ float3 warp_scatter_albedo(const SceneView& S, const WarpSmem& W, float3 o, float3 d, float t,
+                                      uint32_t& overlap, uint32_t& status, WarpStats& ws, bool measure) {
+  const int lane = threadIdx.x & 31;
+  const RayBox rb = ray_box(o, d);
+  double aw = 0.0, ar = 0.0, ag = 0.0, ab = 0.0;
+  unsigned int cnt = 0;
+  int sp = 1;
+  if (lane == 0) W.st_ref[0] = S.wide_root;
+  __syncwarp();
+  while (sp > 0) {
+    --sp;
+    const uint32_t ref = W.st_ref[sp];
+    __syncwarp();
+    float tn;
+    if (ref_is_leaf(ref)) {
+      const uint32_t first = wide_leaf_first(ref), count = wide_leaf_count(ref);
+      if (measure) {
+        ws.leaves++;
+        ws.kind_leaves[2]++;
+        ws.kind_prims[2] += count;
+      }
+      const uint32_t pi = first + lane;
+      const bool boxed = (uint32_t)lane < count &&
+                         slab(rb, __ldg(S.pbox + 2u * pi), __ldg(S.pbox + 2u * pi + 1u), t, t, tn);
+      if (measure) ws.kind_geo[2] += __popc(__ballot_sync(kFull, boxed));
+      Chord ch;
+      if (boxed) {
+        const PrimGeo g = load_geo(S.prims, pi);
+        if (chord_setup<kAcc>(g, o, d, ch) && ch.t_in <= t && t <= ch.t_out) {
+          const float u = (t - ch.tc) / ch.rw;
+          const double wgt = (double)(g.icf * vexp<kAcc>(-0.5f * fmaf(u, u, ch.d2)));
+          const float3 al = load_albedo(S.prims, pi);
+          aw += wgt;
+          ar += wgt * (double)al.x;
+          ag += wgt * (double)al.y;
+          ab += wgt * (double)al.z;
+          ++cnt;
+        }
+      }
+    } else {
+      if (measure) {
+        ws.nodes++;
+        ws.kind_nodes[2]++;
+      }
+      const float4* node = S.wide + (size_t)ref * 64u;
+      const float4 lo = __ldg(node + lane);
+      const float4 hi = __ldg(node + 32 + lane);
+      const uint32_t cref = __float_as_uint(lo.w);
+      const bool hit = (cref != kEmptyRef) && slab(rb, lo, hi, t, t, tn);
+      const unsigned m = __ballot_sync(kFull, hit);
+      const int nh = __popc(m);
+      if ((uint32_t)(sp + nh) > S.stack_cap) {
+        status |= kStatusStackOverflow;
+        break;
+      }
+      if (hit) W.st_ref[sp + __popc(m & ((1u << lane) - 1u))] = cref;
+      sp += nh;
+      __syncwarp();
+    }
+  }
+  __syncwarp();
+  for (int k = 16; k > 0; k >>= 1) cnt += __shfl_xor_sync(kFull, cnt, k);
+  overlap = cnt;
+  aw = warp_sum(aw);
+  ar = warp_sum(ar);
+  ag = warp_sum(ag);
+  ab = warp_sum(ab);
+  return mean_albedo(aw, ar, ag, ab);
 }
 
 // Albedo at a point: sigma_t * pdf weighted mean over the ellipsoids containing it
@@ -707,7 +798,7 @@ struct ThreadQueries {
     }
     return (kKind == kArgmin) ? t_hi : tau_value(acc);
   }
-  __device__ float argmin(float3 o, float3 d, uint64_t key, ScatterAlbedo* sa) {
+  __device__ float argmin(float3 o, float3 d, uint64_t key, ScatterAlbedo* sa, uint32_t /*seed*/) {
     sa->valid = false;  // the plain megakernel evaluates the albedo with its own point query
     sa->gauss = kNoGauss;
     return ray<kArgmin>(o, d, key);
@@ -716,6 +807,7 @@ struct ThreadQueries {
     const float tau = ray<kTau>(o, d, 0ull);
     return tau >= kMaxOpticalDepth ? 0.0f : expf(-tau);
   }
+  __device__ float3 albedo_along(float3 o, float3 d, float t, uint32_t& overlap) { return albedo(fma3(t, d, o), overlap); }
   __device__ float3 albedo(float3 x, uint32_t& overlap) {
     uint32_t stack[kBinStack];
     int sp = 0;

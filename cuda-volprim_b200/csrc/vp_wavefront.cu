@@ -10,7 +10,12 @@
 //     shadow  (warp per query)   transmittance over the BVH32 with early exit at tau >= 88
 //     gather  (thread per path)  radiance += weight x T in query order; finished paths write
 //                                their sample
-//   welford   (thread per pixel) running mean over the batch's samples in sample order
+//   tail      (warp per path)    once few paths are left: each runs to its end in one launch; then, a
+//                                thread per pixel, the running mean over the batch's samples in order
+//
+// extend and shadow have a second form for long queues (kTrace8Min): thread per ray over the compressed
+// 8-wide BVH (vp_trace8.cuh), with the same results.  In it the scatter-point albedo is the scene's, when
+// all its Gaussians share one, or a stage of its own (k_wf_scatter8).
 //
 // Each kernel is a fraction of the fused path loop's code and registers, so more warps are
 // resident per SM to hide the latency of the dependent node loads.  The reference found a
@@ -22,9 +27,11 @@
 // same order of radiance accumulation.
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "vp_internal.h"
-#include "vp_path.cuh"
-#include "vp_traverse.cuh"
+#include "vp_pathloop.cuh"
+#include "vp_trace8.cuh"
 
 namespace vp {
 namespace {
@@ -53,6 +60,20 @@ constexpr int kExtendHitCap = VP_WF_EXTEND_HIT_CAP;
 #define VP_WF_SORT_MIN 65536
 #endif
 constexpr uint32_t kSortMinPaths = VP_WF_SORT_MIN;
+// Queues of at least this many paths take the thread-per-ray stages.  Below it the launch ends with its
+// longest rays, whose lanes walk alone, and a whole warp on each ray is sooner done.  Measured on 8-bounce
+// images (thread-per-ray / warp-per-ray, ms): 65k paths 2.7 / 1.9 (50k-Gaussian cloud), 5.0 / 3.8 (500k),
+// 6.6 / 4.7 (200k in clusters); 131k paths 3.0 / 3.3, 5.7 / 6.5, 8.1 / 8.3; 524k paths 5.0 / 11.2, 9.5 / 22.8,
+// 15.0 / 29.2.
+constexpr uint32_t kTrace8Min = 7u << 14;
+// At most this many paths go to the tail kernel: as stages, a bounce of few paths is launches, polls and each
+// stage's slowest ray; as whole paths it is one launch, but a warp shades alone and holds more registers.
+// 64-bounce images, ms as stages / with the tail from 16k paths / from 40k: 4k paths 4.4 / 2.2 / 2.1 (50k-
+// Gaussian cloud), 7.6 / 5.0 / 5.1 (500k); 65k paths 7.0 / 5.2 / 7.7, 12.7 / 10.5 / 13.3.
+constexpr uint32_t kTailMax = 16384;
+// Resident blocks per SM of its register budget: 2 (128 registers, no spills to speak of) against 3 or 4:
+// 4k paths 1.75 / 2.13 / 2.34 ms (50k), 4.4 / 5.1 / 5.0 (500k).
+constexpr int kTailBlocks = 2;
 
 __device__ __forceinline__ uint32_t meta_bounce(uint32_t m) { return m & 0xFFFFu; }
 __device__ __forceinline__ uint32_t meta_nshadow(uint32_t m) { return (m >> 16) & 3u; }
@@ -108,7 +129,7 @@ __global__ void k_wf_generate(CameraView C, ParamsView P, uint32_t spp_offset, u
   if (!adaptive) {
     if (p == 0) {
       b.ctr[0] = P.max_bounces > 0 ? n : 0u;
-      b.ctr[1] = b.ctr[2] = b.ctr[3] = b.ctr[4] = 0u;
+      b.ctr[1] = b.ctr[2] = b.ctr[3] = b.ctr[4] = b.ctr[5] = 0u;
     }
     if (p >= n) return;
   } else {
@@ -164,11 +185,13 @@ __global__ void __launch_bounds__(256, VP_WF_MIN_BLOCKS) k_wf_extend(SceneView S
     ScatterAlbedo sa;
     sa.valid = false;
     if (!(bounce == 0 && S.albedo_all_zero))
-      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, ((uint64_t)k2.y << 32) | k2.x, status, ws, measure, &sa);
+      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, ((uint64_t)k2.y << 32) | k2.x, status, ws, measure, &sa,
+                                             bounce ? b.sg[p] : kNoGauss);
     float3 albedo = f3(0.f, 0.f, 0.f);
     if (tstar < kInf) {
       uint32_t ov = sa.overlap;
-      albedo = sa.valid ? sa.albedo : warp_albedo<kAcc>(S, W, fma3(tstar, df, of), ov, status, ws, measure);
+      albedo = sa.valid ? sa.albedo : warp_scatter_albedo<kAcc>(S, W, of, df, tstar, ov, status, ws, measure);
+      if (S.one_albedo) albedo = S.albedo;
       max_overlap = max(max_overlap, ov);
       ++scatters;
     }
@@ -197,6 +220,105 @@ __global__ void __launch_bounds__(256, VP_WF_MIN_BLOCKS) k_wf_extend(SceneView S
       }
     }
   }
+}
+
+// ---- thread-per-ray stages (vp_trace8.cuh) -----------------------------------------------------
+// Resident blocks per SM their register budget is sized for: 3 (80 registers).  4 (64 registers) spills and
+// leaves less of the SM's memory to L1: the showcase batch took 93 ms at 4, 86 at 3, 83 at 2 with later
+// changes ahead of 3 (70).
+constexpr int kT8Blocks = 3;
+constexpr int kT8Threads = 256;
+
+// Rays in flight per warp: 32, or an even share of a batch too small for that.
+__device__ __forceinline__ int rays_per_warp(uint32_t n) {
+  const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+  return (int)min(32u, max(4u, (n + warps - 1u) / warps));
+}
+
+template <bool kAcc>
+__global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_wf_extend8(SceneView S, WfBuffers b, const uint32_t* q,
+                                                                        const uint32_t* count, unsigned int* work,
+                                                                        Counters* ctr) {
+  uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(S.depth8);
+  const uint32_t n = *count;
+  uint32_t status = 0;
+  trace8<kAcc, kFlight8>(
+      S.nodes8, S.prims, S.perm, S.depth8, smem, n, work, rays_per_warp(n), status,
+      [&](uint32_t item, Ray8& ray) {
+        const uint32_t p = __ldg(q + item);
+        const uint32_t bounce = meta_bounce(b.meta[p]);
+        if (S.albedo_all_zero && bounce == 0u) {  // a scatter would end the path with nothing
+          b.alb4[p] = make_float4(0.f, 0.f, 0.f, kInf);
+          b.sg[p] = kNoGauss;
+          return false;
+        }
+        const float4 o = b.o4[p], d = b.d4[p];
+        const uint2 k2 = b.key2[p];
+        ray.o = f3(o.x, o.y, o.z);
+        ray.d = f3(d.x, d.y, d.z);
+        ray.key = ((uint64_t)k2.y << 32) | k2.x;
+        ray.seed = bounce ? b.sg[p] : kNoGauss;
+        return true;
+      },
+      [&](uint32_t item, const Ray8&, const Hit8& h) {
+        const uint32_t p = __ldg(q + item);
+        const float3 a = h.t < kInf ? S.albedo : f3(0.f, 0.f, 0.f);  // k_wf_scatter8 replaces it in mixed scenes
+        b.alb4[p] = make_float4(a.x, a.y, a.z, h.t);
+        b.sg[p] = h.gauss;
+      });
+  if (status) atomicOr(&ctr->status, status);
+}
+
+// Albedo at the scatter points of a scene whose Gaussians differ in it: the sigma_t * pdf-weighted
+// mean over the chords containing the scatter distance (evaluate_albedo over the rebuilt active set,
+// sampling.cuh:257-283, 422-458).
+template <bool kAcc>
+__global__ void __launch_bounds__(kT8Threads) k_wf_scatter8(SceneView S, WfBuffers b, const uint32_t* q,
+                                                           const uint32_t* count, unsigned int* work, Counters* ctr) {
+  uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(S.depth8);
+  const uint32_t n = *count;
+  uint32_t status = 0;
+  trace8<kAcc, kScatter8>(
+      S.nodes8, S.prims, S.perm, S.depth8, smem, n, work, rays_per_warp(n), status,
+      [&](uint32_t item, Ray8& ray) {
+        const uint32_t p = __ldg(q + item);
+        const float t = b.alb4[p].w;
+        if (!(t < kInf)) return false;
+        const float4 o = b.o4[p], d = b.d4[p];
+        ray.o = f3(o.x, o.y, o.z);
+        ray.d = f3(d.x, d.y, d.z);
+        ray.t = t;
+        return true;
+      },
+      [&](uint32_t item, const Ray8& ray, const Hit8& h) {
+        const float3 a = mean_albedo(h.w, h.r, h.g, h.b);
+        b.alb4[__ldg(q + item)] = make_float4(a.x, a.y, a.z, ray.t);
+      });
+  if (status) atomicOr(&ctr->status, status);
+}
+
+template <bool kAcc>
+__global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_wf_shadow8(SceneView S, WfBuffers b, const uint32_t* count,
+                                                                        unsigned int* work, Counters* ctr) {
+  uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(S.depth8);
+  const uint32_t n = *count;
+  uint32_t status = 0;
+  trace8<kAcc, kTau8>(
+      S.nodes8, S.prims, S.perm, S.depth8, smem, n, work, rays_per_warp(n), status,
+      [&](uint32_t item, Ray8& ray) {
+        const uint32_t slot = __ldg(b.qs + item);
+        const float4 o = b.so4[slot], d = b.sd4[slot];
+        ray.o = f3(o.x, o.y, o.z);
+        ray.d = f3(d.x, d.y, d.z);
+        ray.seed = __float_as_uint(d.w);
+        ray.seed_tau = o.w;
+        return true;
+      },
+      [&](uint32_t item, const Ray8&, const Hit8& h) {
+        const float tau = (float)h.w;
+        b.so4[__ldg(b.qs + item)].w = tau >= kMaxOpticalDepth ? 0.0f : expf(-tau);
+      });
+  if (status) atomicOr(&ctr->status, status);
 }
 
 // The shadow rays' seed chords are evaluated here, one thread per ray (seed_chord_tau): a ray
@@ -340,15 +462,15 @@ __global__ void k_wf_advance(uint32_t* ctr) {
   ctr[2] = 0u;
   ctr[3] = 0u;
   ctr[4] = 0u;
+  ctr[5] = 0u;
 }
 
-// Welford mean over the batch's samples of each pixel, in sample order (raygen.cuh:214-242).
+// Welford mean over the batch's samples of one pixel, in sample order (raygen.cuh:214-242).
 // With adaptive sampling it also keeps M2, and a pixel that k_wf_generate found converged (the
 // same test on the same, still unchanged state) keeps its state.
-__global__ void k_wf_welford(ParamsView P, WfBuffers b, uint32_t batch, uint32_t n_pix, float4* __restrict__ mean,
-                             float4* __restrict__ m2, uint32_t* __restrict__ count) {
-  const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= n_pix) return;
+__device__ __forceinline__ void welford_pixel(const ParamsView& P, const WfBuffers& b, uint32_t batch, uint32_t pix,
+                                              float4* __restrict__ mean, float4* __restrict__ m2,
+                                              uint32_t* __restrict__ count) {
   const bool adaptive = P.adaptive_threshold > 0.0f;
   const uint32_t prev = count[pix];
   const float4 m4 = mean[pix];
@@ -362,6 +484,49 @@ __global__ void k_wf_welford(ParamsView P, WfBuffers b, uint32_t batch, uint32_t
   mean[pix] = make_float4(m.x, m.y, m.z, 0.f);
   if (adaptive) m2[pix] = make_float4(q.x, q.y, q.z, 0.f);
   count[pix] = prev + batch;
+}
+
+// The end of a batch, one cooperative launch: the paths still queued run to their ends, a warp on each
+// (the warp engine's path loop: no launches, queues or path state in memory between bounces), and once
+// all have finished the pixels' means take the batch's samples.
+template <bool kAcc, bool kMeasure>
+__global__ void __launch_bounds__(256, kTailBlocks) k_wf_tail(SceneView S, EnvView E, ParamsView P, WfBuffers b, const uint32_t* q,
+                                                 const uint32_t* count, unsigned int* work, Counters* ctr,
+                                                 uint32_t batch, uint32_t n_pix, float4* __restrict__ mean,
+                                                 float4* __restrict__ m2, uint32_t* __restrict__ pix_count) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  WarpSmem W = carve(vp_dyn_smem + kRootStageBytes + warp * warp_smem_bytes(S.argmin_cap, kExtendHitCap), S.argmin_cap,
+                     kExtendHitCap);
+  if constexpr (VP_STAGE_ROOT) {
+    stage_root(S.wide, S.wide_root);
+    W.root_staged = true;
+  }
+  if constexpr (!kMeasure) P.measure = 0;
+  const uint32_t n = *count;
+  uint32_t status = 0;
+  WarpStats ws;
+  PathStats ps;
+  const bool measure = kMeasure && P.measure != 0;
+  if (measure) ws.hist = &ctr->hits_hist[0][0];
+  WarpQueries<kAcc> queries{S, W, status, ws, measure};
+  while (n != 0u) {
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(work, 1u);
+    item = __shfl_sync(kFull, item, 0);
+    if (item >= n) break;
+    const uint32_t p = __ldg(q + item);
+    const uint32_t bounce = meta_bounce(b.meta[p]);
+    PathState s = load_path(b, p, bounce);
+    const uint2 k2 = b.key2[p];
+    run_path(S, E, P, queries, s, ((uint64_t)k2.y << 32) | k2.x, bounce ? b.sg[p] : kNoGauss, ps);
+    const float3 L = finalize_sample(P, s.rad);
+    if (lane == 0) b.L4[p] = make_float4(L.x, L.y, L.z, 0.f);
+    if (status) break;
+  }
+  if (lane == 0) flush_stats(ctr, ps, ws, status, measure);
+  cooperative_groups::this_grid().sync();
+  for (uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x; pix < n_pix; pix += gridDim.x * blockDim.x)
+    welford_pixel(P, b, batch, pix, mean, m2, pix_count);
 }
 
 // Morton key (10 bits per axis) of each queued path's origin over the scene bounds: sorting the
@@ -484,6 +649,21 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
   const int ext_blocks = ctx->sm_count * resident_blocks(ext, threads, smem);
   const int shd_blocks = ctx->sm_count * resident_blocks(shd, threads, smem_sh);
   const int thr_blocks = ctx->sm_count * 8;
+  // Thread-per-ray stages above kTrace8Min paths; the counting variants are the warp-cooperative ones.
+  const bool can8 = s->view.depth8 != 0u && !P.measure;
+  const size_t smem8 = trace8_smem_bytes(s->view.depth8, kT8Threads);
+  auto ext8 = P.accurate ? k_wf_extend8<true> : k_wf_extend8<false>;
+  auto sca8 = P.accurate ? k_wf_scatter8<true> : k_wf_scatter8<false>;
+  auto shd8 = P.accurate ? k_wf_shadow8<true> : k_wf_shadow8<false>;
+  int ext8_blocks = 0, sca8_blocks = 0, shd8_blocks = 0;
+  if (can8) {
+    if (smem8 > 48 * 1024)
+      for (auto k : {(const void*)ext8, (const void*)sca8, (const void*)shd8})
+        VP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem8));
+    ext8_blocks = ctx->sm_count * resident_blocks(ext8, kT8Threads, smem8);
+    sca8_blocks = ctx->sm_count * resident_blocks(sca8, kT8Threads, smem8);
+    shd8_blocks = ctx->sm_count * resident_blocks(shd8, kT8Threads, smem8);
+  }
   // VP_MEASURE_STAGES: events around the extend and shadow launches of each iteration (a ring of 4 iterations,
   // read back at every poll, when the stream has drained)
   cudaEvent_t* ev = ctx->stage_ev;
@@ -503,7 +683,7 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
     pending = 0;
     return cudaSuccess;
   };
-  if (P.adaptive_threshold > 0.0f) VP_CUDA(cudaMemsetAsync(b.ctr, 0, 5 * sizeof(uint32_t), st));
+  if (P.adaptive_threshold > 0.0f) VP_CUDA(cudaMemsetAsync(b.ctr, 0, 6 * sizeof(uint32_t), st));
   k_wf_generate<<<(paths + 255) / 256, 256, 0, st>>>(cam, P, spp_offset, spp_count, paths, b, img->mean, img->m2,
                                                      img->count, ctx->counters);
   VP_CUDA(cudaGetLastError());
@@ -518,8 +698,14 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
   const float3 binv = make_float3(inv_ext1(si.bounds_min[0], si.bounds_max[0]),
                                   inv_ext1(si.bounds_min[1], si.bounds_max[1]),
                                   inv_ext1(si.bounds_min[2], si.bounds_max[2]));
+  auto tail = P.accurate ? (P.measure ? k_wf_tail<true, true> : k_wf_tail<true, false>)
+                         : (P.measure ? k_wf_tail<false, true> : k_wf_tail<false, false>);
+  if (smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   uint32_t polled = paths;
   for (uint32_t it = 0; it < P.max_bounces; ++it) {
+    // Few paths left (the count last read), or none that can be (a scatter in an albedo-0 scene ends its
+    // path): the tail takes over.  The first bounce always runs as stages.
+    if (it != 0u && (polled <= kTailMax || s->view.albedo_all_zero)) break;
     if (it != 0u && (it & 3u) == 0u && polled >= kSortMinPaths) {  // (camera rays share one origin)
       k_wf_sort_keys<<<(polled + 255) / 256, 256, 0, st>>>(polled, qcur, b.o4, blo, binv, b.sk_a);
       vp_status r = radix_sort_pairs(b.sk_a, qcur, polled, 30, ctx->wf.sort_tmp, ctx->wf.sort_tmp_bytes, st,
@@ -528,12 +714,25 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
     }
     cudaEvent_t* e4 = ev + 4 * (it & 3u);
     if (timed) VP_CUDA(cudaEventRecord(e4[0], st));
-    ext<<<ext_blocks, threads, smem, st>>>(s->view, P, b, qcur, b.ctr + 0, b.ctr + 3, ctx->counters);
+    const bool use8 = can8 && polled >= kTrace8Min;
+    if (use8) {
+      ext8<<<ext8_blocks, kT8Threads, smem8, st>>>(s->view, b, qcur, b.ctr + 0, b.ctr + 3, ctx->counters);
+      if (!s->view.one_albedo) {
+        sca8<<<sca8_blocks, kT8Threads, smem8, st>>>(s->view, b, qcur, b.ctr + 0, b.ctr + 5, ctx->counters);
+        ctx->launches += 1;
+        ctx->stage_launches[0] += 1;
+      }
+    } else {
+      ext<<<ext_blocks, threads, smem, st>>>(s->view, P, b, qcur, b.ctr + 0, b.ctr + 3, ctx->counters);
+    }
     if (timed) VP_CUDA(cudaEventRecord(e4[1], st));
     k_wf_shade<<<thr_blocks, threads, 0, st>>>(s->view, e->view, P, b, qcur, b.ctr + 0, qnext, b.ctr + 1,
                                                ctx->counters);
     if (timed) VP_CUDA(cudaEventRecord(e4[2], st));
-    shd<<<shd_blocks, threads, smem_sh, st>>>(s->view, b, b.ctr + 2, b.ctr + 4, ctx->counters, P.measure);
+    if (use8)
+      shd8<<<shd8_blocks, kT8Threads, smem8, st>>>(s->view, b, b.ctr + 2, b.ctr + 4, ctx->counters);
+    else
+      shd<<<shd_blocks, threads, smem_sh, st>>>(s->view, b, b.ctr + 2, b.ctr + 4, ctx->counters, P.measure);
     if (timed) VP_CUDA(cudaEventRecord(e4[3], st));
     k_wf_gather<<<thr_blocks, threads, 0, st>>>(P, b, qcur, b.ctr + 0);
     k_wf_advance<<<1, 1, 0, st>>>(b.ctr);
@@ -551,8 +750,18 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
       if (polled == 0u) break;
     }
   }
-  k_wf_welford<<<(n_pix + 255) / 256, 256, 0, st>>>(P, b, spp_count, n_pix, img->mean, img->m2, img->count);
-  VP_CUDA(cudaGetLastError());
+  {
+    const uint32_t* tcount = b.ctr + 0;
+    unsigned int* twork = b.ctr + 3;
+    Counters* tctr = ctx->counters;
+    SceneView tS = s->view;
+    EnvView tE = e->view;
+    ParamsView tP = P;
+    uint32_t tbatch = spp_count, tpix = n_pix;
+    void* args[] = {&tS, &tE, &tP, &b, &qcur, &tcount, &twork, &tctr, &tbatch, &tpix, &img->mean, &img->m2, &img->count};
+    VP_CUDA(cudaLaunchCooperativeKernel((const void*)tail, dim3(ctx->sm_count * resident_blocks(tail, threads, smem)),
+                                        dim3(threads), args, smem, st));
+  }
   ctx->launches += 1;
   if (timed && pending) {
     VP_CUDA(cudaStreamSynchronize(st));

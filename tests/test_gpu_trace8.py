@@ -1,0 +1,85 @@
+"""GPU: the thread-per-ray stages over the compressed 8-wide BVH (wavefront engine, queues of at least
+114,688 paths) against the warp engine, which traverses the BVH32 one path a warp.
+
+Both engines take the same samples, evaluate the same chords with the same arithmetic and carry their
+sums in FP64 rounded once, so a pixel differs only where a transmittance reaches MAX_OPTICAL_DEPTH in
+one order of summation and not in the other (T below 1e-38), or where a sum lies within 1e-16 of a
+rounding boundary.  Hence: every pixel within 1e-5 of the image's mean.
+"""
+import math
+
+import numpy as np
+import pytest
+
+import volprim_b200 as vp
+from volprim_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+W, H = 409, 281  # 114,929 paths: the first iterations take the thread-per-ray stages, the tail the others
+
+
+def gaussians(n, seed, layout="box", mixed=True):
+    rng = np.random.default_rng(seed)
+    scale = np.exp(rng.normal(math.log(0.1), 0.5, (n, 3)))
+    mean = rng.uniform(-0.6, 0.6, (n, 3))
+    if layout == "nested":      # a chain: deeper than the 8-wide tree's limit, so the warp queries run
+        scale = np.repeat((0.01 * 1.003 ** np.arange(n))[:, None], 3, 1)
+        mean = np.zeros((n, 3))
+    elif layout == "same":      # identical boxes
+        scale, mean = np.full((n, 3), 0.2), np.full((n, 3), 0.1)
+    elif layout == "spread":    # extents from 1e-4 to 1e2 in one tree
+        scale = np.exp(rng.uniform(math.log(3e-5), math.log(30.0), (n, 1))) * np.exp(rng.normal(0, 0.3, (n, 3)))
+    elif layout == "plate":     # thin in one axis, aligned with it
+        scale = np.stack([np.full(n, 0.1), np.full(n, 1e-5), np.full(n, 0.1)], 1)
+        mean[:, 1] = 0.25
+    quat = scenes.uniform_quaternions(rng, n) if layout != "plate" else np.tile(np.array([1.0, 0, 0, 0]), (n, 1))
+    dens = np.exp(rng.normal(-1.0, 0.5, n)) * (8.0 / max(n, 8)) * (scale.prod(1) / 1e-3) ** (2.0 / 3.0)
+    albedo = rng.uniform(0.2, 0.95, (n, 3)) if mixed else np.tile(np.array([0.9, 0.8, 0.7]), (n, 1))
+    return vp.Gaussians(*(a.astype(np.float32) for a in (mean, scale, quat, dens, albedo)))
+
+
+def images(ctx, g, sigma=1.0, camera=None, **kw):
+    sc = vp.Scene(ctx, g, sigma)
+    env = vp.Environment(ctx, rgb=scenes.procedural_env(64, 32, sun_radiance=50.0, sun_radius_deg=8.0))
+    out = {}
+    for engine in ("wavefront", "warp"):
+        cfg = vp.Config(num_samples_per_pixel=1, image_width=W, image_height=H, seed=5, engine=engine, max_bounces=16,
+                        rr_depth=4, **kw)
+        out[engine] = vp.Renderer(cfg, sc, camera or scenes.negz_camera(3.0, 40.0), env=env, ctx=ctx).render()[..., :3]
+    sc.close()
+    return out["wavefront"], out["warp"]
+
+
+def check(a, b):
+    assert np.isfinite(a).all() and b.mean() > 1e-3
+    assert np.abs(a - b).max() <= 1e-5 * b.mean(), (np.abs(a - b).max(), np.mean(a != b))
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 24, 25, 64, 65, 3000])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_sizes(vp_ctx, n, mixed):
+    check(*images(vp_ctx, gaussians(n, n, mixed=mixed), hg_g=0.6))
+
+
+@pytest.mark.parametrize("layout", ["nested", "same", "spread", "plate"])
+def test_layouts(vp_ctx, layout):
+    check(*images(vp_ctx, gaussians(600, 3, layout), hg_g=0.0))
+
+
+@pytest.mark.parametrize("nee", ["mis", "phase", "ris", "none"])
+@pytest.mark.parametrize("precision", ["fast", "accurate"])
+def test_estimators(vp_ctx, nee, precision):
+    check(*images(vp_ctx, gaussians(500, 9), sigma=3.0, nee=nee, precision=precision, hg_g=0.85))
+
+
+def test_camera_inside_and_axis_aligned_rays(vp_ctx):
+    """An orthographic camera along an axis (two direction components 0), from inside the cloud."""
+    cam = vp.Camera.orthographic_camera((0.0, 0.0, -0.2), (0.0, 0.0, 1.0), (0.0, 1.0, 0.0), 1.0)
+    check(*images(vp_ctx, gaussians(800, 4), camera=cam, hg_g=0.0))
+
+
+def test_empty_scene(vp_ctx):
+    g = vp.Gaussians(np.zeros((0, 3), np.float32), np.zeros((0, 3), np.float32), np.zeros((0, 4), np.float32),
+                     np.zeros(0, np.float32))
+    check(*images(vp_ctx, g))

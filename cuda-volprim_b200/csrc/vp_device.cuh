@@ -609,8 +609,8 @@ __device__ __forceinline__ float mis_balance(float a, float b) {
 // ---- camera (device/params/camera.h:33-57, random.cuh:55-72) ------------------------------
 // IEEE-rounded operations only (no contraction, correctly rounded normalisation) so the
 // host oracle reproduces every camera ray bit for bit.
-__device__ __forceinline__ void camera_ray(const CameraView& C, const ParamsView& P, uint32_t px,
-                                           uint32_t py, Pcg32& rng, float3& o, float3& d) {
+// Jittered pixel coordinates of one sample.
+__device__ __forceinline__ void camera_jitter(const ParamsView& P, uint32_t px, uint32_t py, Pcg32& rng, float& x, float& y) {
   float jx, jy;
   if (P.filter_stddev > 0.0f) {
     const float u1 = fmaxf(rng.uniform(), 1e-7f);
@@ -624,11 +624,16 @@ __device__ __forceinline__ void camera_ray(const CameraView& C, const ParamsView
     jx = __fsub_rn(rng.uniform(), 0.5f);
     jy = __fsub_rn(rng.uniform(), 0.5f);
   }
-  const float x = __fadd_rn((float)px, jx);
-  const float y = __fadd_rn((float)py, jy);
-  const float3 off = f3(fmaf(x, C.du.x, fmaf(y, C.dv.x, C.p00.x)),
-                        fmaf(x, C.du.y, fmaf(y, C.dv.y, C.p00.y)),
-                        fmaf(x, C.du.z, fmaf(y, C.dv.z, C.p00.z)));
+  x = __fadd_rn((float)px, jx);
+  y = __fadd_rn((float)py, jy);
+}
+// Point of the image plane at pixel coordinates (x, y), relative to the eye.
+__device__ __forceinline__ float3 camera_offset(const CameraView& C, float x, float y) {
+  return f3(fmaf(x, C.du.x, fmaf(y, C.dv.x, C.p00.x)), fmaf(x, C.du.y, fmaf(y, C.dv.y, C.p00.y)),
+            fmaf(x, C.du.z, fmaf(y, C.dv.z, C.p00.z)));
+}
+__device__ __forceinline__ void camera_ray_at(const CameraView& C, float x, float y, float3& o, float3& d) {
+  const float3 off = camera_offset(C, x, y);
   if (C.ortho) {
     o = f3(__fadd_rn(C.eye.x, off.x), __fadd_rn(C.eye.y, off.y), __fadd_rn(C.eye.z, off.z));
     d = C.view_dir;
@@ -638,6 +643,12 @@ __device__ __forceinline__ void camera_ray(const CameraView& C, const ParamsView
     o = C.eye;
     d = f3(__fmul_rn(off.x, inv), __fmul_rn(off.y, inv), __fmul_rn(off.z, inv));
   }
+}
+__device__ __forceinline__ void camera_ray(const CameraView& C, const ParamsView& P, uint32_t px,
+                                           uint32_t py, Pcg32& rng, float3& o, float3& d) {
+  float x, y;
+  camera_jitter(P, px, py, rng, x, y);
+  camera_ray_at(C, x, y, o, d);
 }
 
 // ---- warp helpers -------------------------------------------------------------------------

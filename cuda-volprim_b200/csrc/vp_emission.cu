@@ -26,6 +26,8 @@
 // sum g_tau dtau/dp (3, for the mean), sum g_tau tau (1, for density and the scale
 // normaliser), dLoss/de (3); a finishing kernel maps them to mean / scale / quaternion /
 // density / emission gradients in the caller's order.
+#include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 #include <vector>
@@ -36,20 +38,114 @@
 namespace vp {
 namespace {
 
-// Warp-cooperative visit of every Gaussian whose 3-sigma chord overlaps [0, inf) of the ray.  The
-// warp walks the BVH32 with the first hit child of each inner node kept in registers and the
-// others on the warp's shared-memory stack (no ordering: the image model is order-independent).
-// At a leaf (packed with the leaves next on the stack while they fit in 32 lanes), lane j takes the
-// j-th Gaussian of the ranges laid end to end: box pre-test, chord set-up, then f(pi, g, ch) on
-// that lane alone.
+// Packets.  A warp takes the samples of a small tile of pixels -- up to 32 camera rays that cross nearly the
+// same Gaussians -- and walks the BVH32 once for all of them: at an inner node lane c tests child c's box
+// against the packet's frustum, at a leaf lane j tests the j-th Gaussian's, and each candidate is then met
+// by all 32 rays at once (its record one broadcast load, every lane setting up its own ray's chord).  One
+// ray a warp instead left about two lanes busy in the chord work, and the adjoint issued its 64 bytes of
+// atomics per (ray, Gaussian) where a packet reduces its rays' gradients first.
+//
+// Tile of the packet: k = min(spp, 32) samples of 2^floor(log2(32 / k)) pixels, near square.
+struct Tiling {
+  uint32_t k, tw, th, tiles_x, tiles;
+};
+
+// A block of kGroup warps shares a packet: the critical path is the tile whose rays cross the densest part
+// (some thousand Gaussians one after the other), so the tree's first levels are expanded into a list of
+// subtrees that the block's warps take one at a time, each with all 32 rays.
+constexpr uint32_t kFrontier = 96;  // list capacity; expansion stops when another node's 32 children may not fit
+constexpr uint32_t kShares = 48;    // subtrees that are enough to share
+
+// The packet's bounds, in shared memory (read by every lane at every step): the four side planes of its
+// frustum (n, w): inside where n . x + w >= 0, with w already widened by the tolerance; its middle ray and
+// how far the others are from it: |o - oc| <= r0, |d - dc| <= r1.
+struct PacketBounds {
+  float4 plane[4];
+  float4 oc;  // origin, r0
+  float4 dc;  // direction, r1
+};
+
+__device__ __forceinline__ float3 cross3(float3 a, float3 b) {
+  return f3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
+}
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFull, v, o));
+  return v;
+}
+
+// extent: the largest |coordinate| of the scene's boxes.  The side planes go through the pixel coordinates
+// of the outermost samples, moved out by 0.02 pixels; their FP32 evaluation at a box corner is within
+// 1e-6 (|n|_1 extent + |w|), which the tolerance covers.
+__device__ __forceinline__ void packet_bounds(const CameraView& C, float extent, bool active, float x, float y, float3 o,
+                                              float3 d, PacketBounds* B) {
+  const int lane = threadIdx.x & 31;
+  const float x0 = -warp_max(active ? -x : -kInf) - 0.02f, x1 = warp_max(active ? x : -kInf) + 0.02f;
+  const float y0 = -warp_max(active ? -y : -kInf) - 0.02f, y1 = warp_max(active ? y : -kInf) + 0.02f;
+  float3 oc, dc;
+  camera_ray_at(C, 0.5f * (x0 + x1), 0.5f * (y0 + y1), oc, dc);
+  const float3 eo = sub(o, oc), ed = sub(d, dc);
+  const float r0 = warp_max(active ? sqrtf(dot3(eo, eo)) : 0.f), r1 = warp_max(active ? sqrtf(dot3(ed, ed)) : 0.f);
+  if (lane < 4) {
+    const bool vertical = lane < 2;                     // planes of constant x, else of constant y
+    const float px = (lane == 1) ? x1 : x0, py = (lane == 3) ? y1 : y0;
+    const float3 corner = camera_offset(C, px, py);
+    const float3 along = vertical ? C.dv : C.du;
+    float3 inward = vertical ? C.du : C.dv;
+    if (lane & 1) inward = mul(inward, -1.0f);
+    float3 n = cross3(C.ortho ? C.view_dir : corner, along);
+    n = mul(n, rsqrtf(fmaxf(dot3(n, n), 1e-37f)));
+    if (dot3(n, inward) < 0.f) n = mul(n, -1.0f);
+    const float3 at = C.ortho ? add(C.eye, corner) : C.eye;
+    const float w = -dot3(n, at);
+    const float tol = 1e-6f * ((fabsf(n.x) + fabsf(n.y) + fabsf(n.z)) * extent + fabsf(w));
+    B->plane[lane] = make_float4(n.x, n.y, n.z, w + tol);
+  }
+  if (lane == 4) B->oc = make_float4(oc.x, oc.y, oc.z, r0 * 1.001f + 1e-6f * extent);
+  if (lane == 5) B->dc = make_float4(dc.x, dc.y, dc.z, r1 * 1.001f + 1e-6f);
+  __syncwarp();
+}
+
+__device__ __forceinline__ bool in_frustum(const PacketBounds* B, float4 lo, float4 hi) {
+  bool in = true;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float4 n = B->plane[k];
+    const float s = fmaxf(n.x * lo.x, n.x * hi.x) + fmaxf(n.y * lo.y, n.y * hi.y) + fmaxf(n.z * lo.z, n.z * hi.z) + n.w;
+    in = in && !(s < 0.f);
+  }
+  return in;
+}
+
+// Whether some ray of the packet can meet the Gaussian's 3-sigma ellipsoid.  At such a ray's point x(t), t at
+// most the distance to the far side of the Gaussian's box, the middle ray is within r0 + t r1, so its
+// whitened distance from the centre is at most 3 + |W| (r0 + t r1); |W| is bounded by the Frobenius norm.
+__device__ __forceinline__ bool near_packet(const PacketBounds* B, const PrimGeo& g, float4 lo, float4 hi) {
+  const float4 oc = B->oc, dc = B->dc;
+  const float3 d = f3(dc.x, dc.y, dc.z), v = sub(f3(oc.x, oc.y, oc.z), f3(g.a.x, g.a.y, g.a.z));
+  const float ex = hi.x - lo.x, ey = hi.y - lo.y, ez = hi.z - lo.z;
+  const float t = sqrtf(dot3(v, v)) + oc.w + 0.5f * sqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
+  const float3 w = whiten(g, d);
+  const float a2 = dot3(w, w);
+  const float tc = -dot3(whiten(g, v), w) * __frcp_rn(a2);
+  const float3 p = whiten(g, fma3(tc, d, v));
+  const float w2 = g.a.w * g.a.w + g.b.x * g.b.x + g.b.y * g.b.y + g.b.z * g.b.z + g.b.w * g.b.w + g.c.x * g.c.x +
+                   g.c.y * g.c.y + g.c.z * g.c.z + g.c.w * g.c.w;
+  const float wn = sqrtf(w2);
+  // 1e-6 |W| t covers the FP32 rounding of the middle ray's own closest approach
+  const float reach = 3.001f + wn * (oc.w + t * dc.w + 2e-6f * t);
+  return !(dot3(p, p) > reach * reach);
+}
+
+// f(pi, g, ch, hit) for every Gaussian under the sp references on the stack that some active ray's chord
+// crosses over [0, inf); `hit` and `ch` are the lane's own, all lanes call it.
 template <bool kAcc, class F>
-__device__ void warp_visit(const SceneView& S, uint32_t* stack, float3 o, float3 d, uint32_t& status, F&& f) {
+__device__ __forceinline__ void packet_visit(const SceneView& S, uint32_t* stack, const PacketBounds* B, float3 o, float3 d,
+                                             bool active, uint32_t& status, int sp, F&& f) {
   const int lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const RayBox rb = ray_box(o, d);
-  int sp = 0;
-  uint32_t ref = S.wide_root;
-  bool have = true;
+  uint32_t ref = 0u;
+  bool have = false;
   while (true) {
     if (!have) {
       if (sp == 0) break;
@@ -71,25 +167,31 @@ __device__ void warp_visit(const SceneView& S, uint32_t* stack, float3 o, float3
         total += c2;
       }
       __syncwarp();
+      bool candidate = false;
       if (lane < total) {
-        float tb;
-        if (slab(rb, __ldg(S.pbox + 2u * pi), __ldg(S.pbox + 2u * pi + 1u), 0.0f, kInf, tb)) {
-          const PrimGeo g = load_geo(S.prims, pi);
-          Chord ch;
-          if (chord_setup<kAcc>(g, o, d, ch) && ch.t_out > 0.0f) f(pi, g, ch);
-        }
+        const float4 lo = __ldg(S.pbox + 2u * pi), hi = __ldg(S.pbox + 2u * pi + 1u);
+        if (in_frustum(B, lo, hi)) candidate = near_packet(B, load_geo(S.prims, pi), lo, hi);
+      }
+      unsigned cm = __ballot_sync(kFull, candidate);
+      while (cm != 0u) {
+        const int j = __ffs(cm) - 1;
+        cm &= cm - 1u;
+        const uint32_t gi = __shfl_sync(kFull, pi, j);
+        const PrimGeo g = load_geo(S.prims, gi);
+        Chord ch;
+        const bool hit = active && chord_setup<kAcc>(g, o, d, ch) && ch.t_out > 0.0f;
+        if (__any_sync(kFull, hit)) f(gi, g, ch, hit);
       }
     } else {
       const float4* node = S.wide + (size_t)ref * 64u;
       const float4 lo = __ldg(node + lane);
       const float4 hi = __ldg(node + 32 + lane);
       const uint32_t cref = __float_as_uint(lo.w);
-      float tnear = 0.f;
-      const bool hit = (cref != kEmptyRef) && slab(rb, lo, hi, 0.0f, kInf, tnear);
+      const bool hit = (cref != kEmptyRef) && in_frustum(B, lo, hi);
       const unsigned m = __ballot_sync(kFull, hit);
       const int nh = __popc(m);
       if (nh > 0) {
-        if ((uint32_t)(sp + nh) > S.stack_cap) {  // cannot happen for a BVH of the recorded depth
+        if ((uint32_t)(sp + nh) > S.stack_cap + 1u) {  // cannot happen for a BVH of the recorded depth
           status |= kStatusStackOverflow;
           break;
         }
@@ -112,35 +214,157 @@ __device__ __forceinline__ float chord_tau0(const Chord& ch, float icf) {
                          ch.d2lo);
 }
 
-// The ray of (pixel, sample): the renderer's jittered camera ray (raygen.cuh:82-99).
-__device__ __forceinline__ void pixel_ray(const CameraView& C, const ParamsView& P, uint32_t pix, uint32_t s,
-                                          float3& o, float3& d) {
-  const uint32_t px = pix % P.width, py = pix / P.width;
-  Pcg32 rng = pcg_init(P.seed, seq_hash((uint64_t)pix * (uint64_t)P.spp_total + s));
-  camera_ray(C, P, px, py, rng, o, d);
+// This lane's ray of a packet: sample s of its pixel (the renderer's jittered camera ray,
+// raygen.cuh:82-99).  A lane without one takes part with any ray.
+struct PacketRay {
+  float x, y;
+  float3 o, d;
+};
+__device__ __forceinline__ PacketRay packet_ray(const CameraView& C, const ParamsView& P, uint32_t px, uint32_t py,
+                                                uint32_t s) {
+  PacketRay r;
+  Pcg32 rng = pcg_init(P.seed, seq_hash(((uint64_t)py * P.width + px) * (uint64_t)P.spp_total + s));
+  camera_jitter(P, px, py, rng, r.x, r.y);
+  camera_ray_at(C, r.x, r.y, r.o, r.d);
+  return r;
+}
+struct PacketLane {
+  uint32_t px, py, s;  // pixel, sample of the first pass
+  bool on;             // has a pixel of the image
+};
+__device__ __forceinline__ PacketLane packet_lane(const Tiling& T, const ParamsView& P, uint32_t tile) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t p = lane / T.k;
+  PacketLane l;
+  l.s = lane - p * T.k;
+  const uint32_t ty = tile / T.tiles_x, tx = tile - ty * T.tiles_x;
+  l.px = tx * T.tw + p % T.tw;
+  l.py = ty * T.th + p / T.tw;
+  l.on = p < T.tw * T.th && l.px < P.width && l.py < P.height;
+  return l;
 }
 
 struct RaySums {
   float S, r, g, b;  // sum tau, sum tau * e (RGB)
 };
 
-template <bool kAcc>
-__device__ RaySums ray_sums(const SceneView& S, const float4* __restrict__ emis, uint32_t* stack, float3 o, float3 d,
-                            uint32_t& status, unsigned long long& crossings) {
-  float s = 0.f, r = 0.f, g = 0.f, b = 0.f;
-  unsigned int nc = 0;
-  warp_visit<kAcc>(S, stack, o, d, status, [&](uint32_t pi, const PrimGeo& geo, const Chord& ch) {
-    const float tau = chord_tau0<kAcc>(ch, geo.icf);
-    const float4 e = __ldg(emis + pi);
-    s += tau;
-    r = fmaf(tau, e.x, r);
-    g = fmaf(tau, e.y, g);
-    b = fmaf(tau, e.z, b);
-    ++nc;
-  });
-  for (int off = 16; off > 0; off >>= 1) nc += __shfl_xor_sync(kFull, nc, off);
+// Gaussians a warp met in the packet's first traversal, for the adjoint's second pass (n beyond the
+// capacity: not all, and it traverses its subtrees again).
+constexpr uint32_t kListCap = 512;
+
+// Shared memory of a block: the packet, its frontier and the warps' partial sums.
+template <int kGroup>
+struct PacketShared {
+  PacketBounds bounds;
+  uint32_t tile, n_front, next, pad;
+  uint32_t front[kFrontier];
+  uint8_t owner[kFrontier];  // the warp that took each
+  double sums[kGroup][4][32];
+};
+// Words after PacketShared, per warp: stack, Gaussian list (adjoint).
+__host__ __device__ __forceinline__ uint32_t packet_words(uint32_t stack_cap, bool list) {
+  return ((stack_cap + 4u) & ~3u) + (list ? kListCap : 0u);
+}
+template <int kGroup>
+constexpr size_t packet_smem(uint32_t stack_cap, bool list) {
+  return sizeof(PacketShared<kGroup>) + 4u * (size_t)kGroup * packet_words(stack_cap, list);
+}
+
+// The block's first warp lists the subtrees below the tree's first levels that the packet meets.
+template <int kGroup>
+__device__ __forceinline__ void expand_frontier(const SceneView& S, PacketShared<kGroup>& sh) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) sh.front[0] = S.wide_root;
+  __syncwarp();
+  uint32_t n = 1, at = 0;
+  while (at < n && n + 31u <= kFrontier) {
+    const uint32_t ref = sh.front[at];
+    __syncwarp();
+    if (ref_is_leaf(ref)) {
+      ++at;
+      continue;
+    }
+    const float4* node = S.wide + (size_t)ref * 64u;
+    const float4 lo = __ldg(node + lane);
+    const float4 hi = __ldg(node + 32 + lane);
+    const uint32_t cref = __float_as_uint(lo.w);
+    const bool hit = cref != kEmptyRef && in_frustum(&sh.bounds, lo, hi);
+    const unsigned m = __ballot_sync(kFull, hit);
+    // its children take its place and the list's end
+    if (m == 0u) {
+      if (lane == 0) sh.front[at] = sh.front[n - 1u];
+      --n;
+    } else {
+      const int rank = __popc(m & ((1u << lane) - 1u));
+      if (hit) sh.front[rank == 0 ? at : n + (uint32_t)rank - 1u] = cref;
+      if (n > 1u) ++at;  // on to its siblings
+      n += (uint32_t)__popc(m) - 1u;
+    }
+    __syncwarp();
+    if (n >= kShares) break;
+  }
+  if (lane == 0) {
+    sh.n_front = n;
+    sh.next = 0u;
+  }
+  for (uint32_t i = lane; i < n; i += 32u) sh.owner[i] = 0xFFu;
+}
+
+// Sums of this lane's ray over the packet's Gaussians, by the whole block: on every warp.  They run over up
+// to thousands of Gaussians one after the other, so they are carried in FP64 (eight terms at a time).
+template <bool kAcc, bool kList, int kGroup>
+__device__ __forceinline__ RaySums packet_sums(const SceneView& S, const float4* __restrict__ emis, uint32_t* stack,
+                                               PacketShared<kGroup>& sh, float3 o, float3 d, bool active, uint32_t& status,
+                                               unsigned long long& crossings, uint32_t* list, uint32_t& n) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double s = 0.0, r = 0.0, g = 0.0, b = 0.0;
+  float fs = 0.f, fr = 0.f, fg = 0.f, fb = 0.f;  // the last few terms
+  unsigned int nc = 0, met = 0;
+  auto flush = [&]() {
+    s += (double)fs, r += (double)fr, g += (double)fg, b += (double)fb;
+    fs = fr = fg = fb = 0.f;
+  };
+  n = 0;
+  if (warp == 0) expand_frontier(S, sh);
+  __syncthreads();
+  const uint32_t n_front = sh.n_front;
+  while (true) {
+    uint32_t i = 0;
+    if (lane == 0) i = atomicAdd(&sh.next, 1u);
+    i = __shfl_sync(kFull, i, 0);
+    if (i >= n_front) break;
+    if (lane == 0) {
+      stack[0] = sh.front[i];
+      if (kList) sh.owner[i] = (uint8_t)warp;
+    }
+    __syncwarp();
+    packet_visit<kAcc>(S, stack, &sh.bounds, o, d, active, status, 1,
+                       [&](uint32_t gi, const PrimGeo& geo, const Chord& ch, bool hit) {
+      if (kList) {
+        if (n < kListCap && lane == 0) list[n] = gi;
+        ++n;
+      }
+      if (hit) {
+        const float tau = chord_tau0<kAcc>(ch, geo.icf);
+        const float4 e = __ldg(emis + gi);
+        fs += tau;
+        fr = fmaf(tau, e.x, fr);
+        fg = fmaf(tau, e.y, fg);
+        fb = fmaf(tau, e.z, fb);
+        ++nc;
+      }
+      if ((++met & 7u) == 0u) flush();
+    });
+  }
+  flush();
   crossings += nc;
-  return RaySums{warp_sum(s), warp_sum(r), warp_sum(g), warp_sum(b)};
+  sh.sums[warp][0][lane] = s, sh.sums[warp][1][lane] = r, sh.sums[warp][2][lane] = g, sh.sums[warp][3][lane] = b;
+  __syncthreads();
+  s = r = g = b = 0.0;
+#pragma unroll
+  for (int w = 0; w < kGroup; ++w)
+    s += sh.sums[w][0][lane], r += sh.sums[w][1][lane], g += sh.sums[w][2][lane], b += sh.sums[w][3][lane];
+  return RaySums{(float)s, (float)r, (float)g, (float)b};
 }
 
 // (1 - T) / S and (T - (1 - T) / S) / S for S >= 0, with their series below 1e-3.
@@ -161,47 +385,47 @@ __device__ __forceinline__ float3 ray_radiance(const RaySums& rs, float3 env) {
   return f3(fmaf(a, rs.r, T * env.x), fmaf(a, rs.g, T * env.y), fmaf(a, rs.b, T * env.z));
 }
 
-// Resident 256-thread blocks per SM the FP32 emission kernels' register budgets are sized for
-// (64 registers; the ACCURATE float-pair variants keep 2, which holds their ~100 registers).  On the differentiation workload 4 blocks take the
-// forward from 56.5 to 49.2 ms and the adjoint from 127 to 114 ms against the compiler's own
-// budgets (76 and 80 registers: 3 blocks).
-#ifndef VP_EMIS_FWD_BLOCKS
-#define VP_EMIS_FWD_BLOCKS 4
-#endif
-#ifndef VP_EMIS_BWD_BLOCKS
-#define VP_EMIS_BWD_BLOCKS 4
-#endif
+// Resident warps per SM the FP32 kernels' register budgets are sized for (16 for the ACCURATE ones).  On the
+// 100k-Gaussian cloud: forward 256x256 4.1 / 3.5 ms at 24 / 32; adjoint of two 160x120 views 8.4 / 8.1 ms at
+// 20 / 24.
+constexpr int kFwdWarps = 32, kBwdWarps = 24;
 
-template <bool kAcc>
-__global__ void __launch_bounds__(256, kAcc ? 2 : VP_EMIS_FWD_BLOCKS) k_emis_forward(SceneView S, EnvView E, CameraView C, ParamsView P,
-                                                      const float4* __restrict__ emis, float4* __restrict__ out,
-                                                      unsigned int* work, Counters* ctr) {
-  extern __shared__ uint32_t stacks[];
+template <bool kAcc, int kGroup>
+__global__ void __launch_bounds__(32 * kGroup, (kAcc ? 16 : kFwdWarps) / kGroup) k_emis_forward(SceneView S, EnvView E, CameraView C, ParamsView P,
+                                                      Tiling T, float extent, const float4* __restrict__ emis,
+                                                      float4* __restrict__ out, unsigned int* work, Counters* ctr) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t* stack = stacks + warp * S.stack_cap;
-  const uint32_t n_pix = P.width * P.height;
-  uint32_t status = 0;
+  auto& sh = *reinterpret_cast<PacketShared<kGroup>*>(vp_dyn_smem);
+  uint32_t* stack = reinterpret_cast<uint32_t*>(vp_dyn_smem + sizeof(sh)) + warp * packet_words(S.stack_cap, false);
+  uint32_t status = 0, n_list;
   unsigned long long crossings = 0;
   while (true) {
-    uint32_t pix = 0;
-    if (lane == 0) pix = atomicAdd(work, 1u);
-    pix = __shfl_sync(kFull, pix, 0);
-    if (pix >= n_pix) break;
+    if (threadIdx.x == 0) sh.tile = atomicAdd(work, 1u);
+    __syncthreads();
+    const uint32_t tile = sh.tile;
+    if (tile >= T.tiles) break;
+    const PacketLane l = packet_lane(T, P, tile);
     float3 sum = f3(0.f, 0.f, 0.f);
-    for (uint32_t s = 0; s < P.spp_total; ++s) {
-      float3 o, d;
-      pixel_ray(C, P, pix, s, o, d);
-      const RaySums rs = ray_sums<kAcc>(S, emis, stack, o, d, status, crossings);
-      sum = add(sum, ray_radiance(rs, env_lookup(E, d)));
+    for (uint32_t s0 = 0; s0 < P.spp_total; s0 += T.k) {
+      const uint32_t k = min(T.k, P.spp_total - s0);  // samples of this pass
+      const bool active = l.on && l.s < k;
+      const PacketRay r = packet_ray(C, P, l.px, l.py, s0 + l.s);
+      if (warp == 0) packet_bounds(C, extent, active, r.x, r.y, r.o, r.d, &sh.bounds);
+      const RaySums rs = packet_sums<kAcc, false, kGroup>(S, emis, stack, sh, r.o, r.d, active, status, crossings, nullptr, n_list);
+      const float3 L = ray_radiance(rs, env_lookup(E, r.d));
+      // the pixel's samples in order
+      const int base = lane - (int)l.s;
+      for (uint32_t j = 0; j < k; ++j)
+        sum = add(sum, f3(__shfl_sync(kFull, L.x, (base + (int)j) & 31), __shfl_sync(kFull, L.y, (base + (int)j) & 31),
+                          __shfl_sync(kFull, L.z, (base + (int)j) & 31)));
     }
     const float inv = 1.0f / (float)P.spp_total;
-    if (lane == 0) out[pix] = make_float4(sum.x * inv, sum.y * inv, sum.z * inv, 1.0f);
-    if (status) break;
+    if (warp == 0 && l.on && l.s == 0u)
+      out[(size_t)l.py * P.width + l.px] = make_float4(sum.x * inv, sum.y * inv, sum.z * inv, 1.0f);
+    if (__syncthreads_or(status != 0u)) break;
   }
-  if (lane == 0) {
-    if (status) atomicOr(&ctr->status, status);
-    if (P.measure) atomicAdd(&ctr->crossings, crossings);
-  }
+  if (status) atomicOr(&ctr->status, status);
+  if (P.measure) atomicAdd(&ctr->crossings, crossings);
 }
 
 // dtau/dp and dtau/dw of one chord, with tau itself, where p = W (x0 - mu), w = W d and x0 is a
@@ -278,59 +502,104 @@ __device__ __forceinline__ bool tau_grad(const PrimGeo& g, const Chord& ch, floa
   return true;
 }
 
-template <bool kAcc>
-__global__ void __launch_bounds__(256, kAcc ? 2 : VP_EMIS_BWD_BLOCKS) k_emis_backward(SceneView S, EnvView E, CameraView C, ParamsView P,
-                                                       const float4* __restrict__ emis,
+// Sums of 16 values over the warp, two lanes a value: lane l returns the sum of v[(l >> 1)], bits of the index
+// from the top (15 shuffles halve the values a lane carries, one adds the last pair).
+__device__ __forceinline__ float warp_sum16(float (&v)[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int half = 8, bit = 16; half > 0; half >>= 1, bit >>= 1) {
+    const bool up = (lane & bit) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float send = up ? v[i] : v[half + i];
+      const float keep = up ? v[half + i] : v[i];
+      v[i] = keep + __shfl_xor_sync(kFull, send, bit);
+    }
+  }
+  return v[0] + __shfl_xor_sync(kFull, v[0], 1);
+}
+
+template <bool kAcc, int kGroup>
+__global__ void __launch_bounds__(32 * kGroup, (kAcc ? 16 : kBwdWarps) / kGroup) k_emis_backward(SceneView S, EnvView E, CameraView C, ParamsView P,
+                                                       Tiling T, float extent, const float4* __restrict__ emis,
                                                        const float4* __restrict__ dl_dpix, float4* __restrict__ acc,
                                                        unsigned int* work, Counters* ctr) {
-  extern __shared__ uint32_t stacks[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t* stack = stacks + warp * S.stack_cap;
-  const uint32_t n_pix = P.width * P.height;
+  auto& sh = *reinterpret_cast<PacketShared<kGroup>*>(vp_dyn_smem);
+  uint32_t* stack = reinterpret_cast<uint32_t*>(vp_dyn_smem + sizeof(sh)) + warp * packet_words(S.stack_cap, true);
+  uint32_t* list = stack + ((S.stack_cap + 4u) & ~3u);
   const float inv_spp = 1.0f / (float)P.spp_total;
   uint32_t status = 0;
   unsigned long long crossings = 0;
   while (true) {
-    uint32_t pix = 0;
-    if (lane == 0) pix = atomicAdd(work, 1u);
-    pix = __shfl_sync(kFull, pix, 0);
-    if (pix >= n_pix) break;
-    const float4 gp = __ldg(dl_dpix + pix);
-    if (gp.x == 0.0f && gp.y == 0.0f && gp.z == 0.0f) continue;  // nothing flows back (e.g. a crop)
+    if (threadIdx.x == 0) sh.tile = atomicAdd(work, 1u);
+    __syncthreads();
+    const uint32_t tile = sh.tile;
+    if (tile >= T.tiles) break;
+    const PacketLane l = packet_lane(T, P, tile);
+    const float4 gp = l.on ? __ldg(dl_dpix + (size_t)l.py * P.width + l.px) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool wanted = gp.x != 0.0f || gp.y != 0.0f || gp.z != 0.0f;  // else nothing flows back (e.g. a crop)
     const float3 G = f3(gp.x * inv_spp, gp.y * inv_spp, gp.z * inv_spp);
-    for (uint32_t s = 0; s < P.spp_total; ++s) {
-      float3 o, d;
-      pixel_ray(C, P, pix, s, o, d);
-      const RaySums rs = ray_sums<kAcc>(S, emis, stack, o, d, status, crossings);
+    for (uint32_t s0 = 0; s0 < P.spp_total; s0 += T.k) {
+      const uint32_t k = min(T.k, P.spp_total - s0);
+      const bool active = wanted && l.s < k;
+      if (!__any_sync(kFull, active)) continue;
+      const PacketRay r = packet_ray(C, P, l.px, l.py, s0 + l.s);
+      const float3 o = r.o, d = r.d;
+      if (warp == 0) packet_bounds(C, extent, active, r.x, r.y, o, d, &sh.bounds);
+      uint32_t n = 0;
+      const RaySums rs = packet_sums<kAcc, true, kGroup>(S, emis, stack, sh, o, d, active, status, crossings, list, n);
       const float3 env = env_lookup(E, d);
-      float T, a, q;
-      opacity_terms(rs.S, T, a, q);
-      const float gS = G.x * fmaf(rs.r, q, -T * env.x) + G.y * fmaf(rs.g, q, -T * env.y) +
-                       G.z * fmaf(rs.b, q, -T * env.z);
+      float Tr, a, q;
+      opacity_terms(rs.S, Tr, a, q);
+      const float gS = G.x * fmaf(rs.r, q, -Tr * env.x) + G.y * fmaf(rs.g, q, -Tr * env.y) +
+                       G.z * fmaf(rs.b, q, -Tr * env.z);
       const float3 gC = mul(G, a);
-      warp_visit<kAcc>(S, stack, o, d, status, [&](uint32_t pi, const PrimGeo& geo, const Chord& ch) {
+      auto scatter = [&](uint32_t gi, const PrimGeo& geo, const Chord& ch, bool hit) {
+        float v16[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v16[i] = 0.f;
         float tau;
         float3 v, dp, dw;
-        if (!tau_grad<kAcc>(geo, ch, o, d, tau, v, dp, dw)) return;
-        const float4 e = __ldg(emis + pi);
-        const float gt = gS + gC.x * e.x + gC.y * e.y + gC.z * e.z;
-        const float3 gp3 = mul(dp, gt), gw3 = mul(dw, gt);
-        // dLoss/dW_kl = gp_k v_l + gw_k d_l
-        float4* a4 = acc + 4u * pi;
-        atomicAdd(a4 + 0, make_float4(fmaf(gp3.x, v.x, gw3.x * d.x), fmaf(gp3.x, v.y, gw3.x * d.y),
-                                      fmaf(gp3.x, v.z, gw3.x * d.z), fmaf(gp3.y, v.x, gw3.y * d.x)));
-        atomicAdd(a4 + 1, make_float4(fmaf(gp3.y, v.y, gw3.y * d.y), fmaf(gp3.y, v.z, gw3.y * d.z),
-                                      fmaf(gp3.z, v.x, gw3.z * d.x), fmaf(gp3.z, v.y, gw3.z * d.y)));
-        atomicAdd(a4 + 2, make_float4(fmaf(gp3.z, v.z, gw3.z * d.z), gp3.x, gp3.y, gp3.z));
-        atomicAdd(a4 + 3, make_float4(gt * tau, gC.x * tau, gC.y * tau, gC.z * tau));
-      });
+        if (hit && tau_grad<kAcc>(geo, ch, o, d, tau, v, dp, dw)) {
+          const float4 e = __ldg(emis + gi);
+          const float gt = gS + gC.x * e.x + gC.y * e.y + gC.z * e.z;
+          const float3 gp3 = mul(dp, gt), gw3 = mul(dw, gt);
+          // dLoss/dW_kl = gp_k v_l + gw_k d_l
+          v16[0] = fmaf(gp3.x, v.x, gw3.x * d.x), v16[1] = fmaf(gp3.x, v.y, gw3.x * d.y);
+          v16[2] = fmaf(gp3.x, v.z, gw3.x * d.z), v16[3] = fmaf(gp3.y, v.x, gw3.y * d.x);
+          v16[4] = fmaf(gp3.y, v.y, gw3.y * d.y), v16[5] = fmaf(gp3.y, v.z, gw3.y * d.z);
+          v16[6] = fmaf(gp3.z, v.x, gw3.z * d.x), v16[7] = fmaf(gp3.z, v.y, gw3.z * d.y);
+          v16[8] = fmaf(gp3.z, v.z, gw3.z * d.z);
+          v16[9] = gp3.x, v16[10] = gp3.y, v16[11] = gp3.z;
+          v16[12] = gt * tau, v16[13] = gC.x * tau, v16[14] = gC.y * tau, v16[15] = gC.z * tau;
+        }
+        const float sum = warp_sum16(v16);
+        if (!(lane & 1)) atomicAdd(reinterpret_cast<float*>(acc + 4u * gi) + (lane >> 1), sum);
+      };
+      __syncwarp();
+      if (n <= kListCap) {
+        for (uint32_t i = 0; i < n; ++i) {
+          const uint32_t gi = list[i];
+          const PrimGeo g = load_geo(S.prims, gi);
+          Chord ch;
+          const bool hit = active && chord_setup<kAcc>(g, o, d, ch) && ch.t_out > 0.0f;
+          scatter(gi, g, ch, hit);
+        }
+      } else {
+        for (uint32_t i = 0; i < sh.n_front; ++i) {
+          if (sh.owner[i] != (uint8_t)warp) continue;
+          if (lane == 0) stack[0] = sh.front[i];
+          __syncwarp();
+          packet_visit<kAcc>(S, stack, &sh.bounds, o, d, active, status, 1, scatter);
+        }
+      }
+      __syncthreads();  // the packet's shared state is the next pass's
     }
-    if (status) break;
+    if (__syncthreads_or(status != 0u)) break;
   }
-  if (lane == 0) {
-    if (status) atomicOr(&ctr->status, status);
-    if (P.measure) atomicAdd(&ctr->crossings, crossings);
-  }
+  if (status) atomicOr(&ctr->status, status);
+  if (P.measure) atomicAdd(&ctr->crossings, crossings);
 }
 
 // Per-Gaussian accumulators (internal order) -> gradients of the caller's parameters (caller
@@ -415,8 +684,33 @@ vp_status ensure_emission(vp_scene* s) {
 struct Common {
   CameraView cv;
   ParamsView P;
-  size_t smem;
+  Tiling tiles;
+  float extent;
 };
+
+// Warps a packet's block has: more where there are few tiles to fill the chip and hide the dense ones, fewer
+// where they only wait for one another at the block's barriers.  Forward, 100k-Gaussian cloud: 16,384 tiles
+// 3.0 / 3.3 ms with 2 / 4 warps; 4,800 tiles 2.0 / 1.6 ms.
+// A tree so deep that the warps' stacks do not fit a block takes fewer.
+template <class F>
+vp_status with_group(uint32_t tiles, uint32_t stack_cap, F&& f) {
+  constexpr size_t kMost = 200 * 1024;
+  if (tiles >= 10240u || packet_smem<4>(stack_cap, true) > kMost) return f(std::integral_constant<int, 2>{});
+  if (tiles >= 1024u || packet_smem<8>(stack_cap, true) > kMost) return f(std::integral_constant<int, 4>{});
+  return f(std::integral_constant<int, 8>{});
+}
+
+Tiling tiling(uint32_t width, uint32_t height, uint32_t spp) {
+  Tiling t{};
+  t.k = std::min(spp, 32u);
+  uint32_t log = 0;
+  while ((2u << log) * t.k <= 32u) ++log;  // 2^log pixels
+  t.tw = 1u << ((log + 1u) / 2u);
+  t.th = 1u << (log / 2u);
+  t.tiles_x = (width + t.tw - 1u) / t.tw;
+  t.tiles = t.tiles_x * ((height + t.th - 1u) / t.th);
+  return t;
+}
 
 vp_status prepare(vp_scene* s, vp_env* e, const vp_camera* cam, const vp_render_params* p, Common& c) {
   if (!s || !e || !cam || !p) return fail(VP_ERROR_INVALID_ARGUMENT, "NULL argument");
@@ -428,8 +722,12 @@ vp_status prepare(vp_scene* s, vp_env* e, const vp_camera* cam, const vp_render_
   VP_CUDA(cudaSetDevice(s->ctx->device));
   build_camera(*cam, p->width, p->height, c.cv);
   c.P = make_params(*p, s);
-  c.smem = (size_t)8 * s->view.stack_cap * 4u;
-  if (c.smem > 200 * 1024) return fail(VP_ERROR_LIMIT, "BVH too deep for the shared-memory stack");
+  if (packet_smem<2>(s->view.stack_cap, true) > 200 * 1024 || (size_t)8 * s->view.stack_cap * 4u > 200 * 1024)
+    return fail(VP_ERROR_LIMIT, "BVH too deep for the shared-memory stack");
+  c.tiles = tiling(p->width, p->height, p->spp);
+  c.extent = 0.0f;
+  for (int k = 0; k < 3; ++k)
+    c.extent = std::max({c.extent, (float)std::fabs(s->info.bounds_min[k]), (float)std::fabs(s->info.bounds_max[k])});
   vp_status r;
   if ((r = ensure_emission(s))) return r;
   return VP_OK;
@@ -505,10 +803,17 @@ vp_status vp_render_emission(vp_scene* s, vp_env* e, const vp_camera* cam, const
   VP_CUDA(cudaMemsetAsync(ctx->counters, 0, sizeof(Counters), st));
   VP_CUDA(cudaMemsetAsync(ctx->work_counter, 0, sizeof(unsigned int), st));
   VP_CUDA(cudaEventRecord(ctx->ev0, st));
-  auto kern = c.P.accurate ? k_emis_forward<true> : k_emis_forward<false>;
-  if (c.smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
-  const int blocks = ctx->sm_count * blocks_per_sm(kern, 256, c.smem);
-  kern<<<blocks, 256, c.smem, st>>>(s->view, e->view, c.cv, c.P, s->emis, out, ctx->work_counter, ctx->counters);
+  const vp_status lr = with_group(c.tiles.tiles, s->view.stack_cap, [&](auto group) -> vp_status {
+    constexpr int G = decltype(group)::value;
+    auto kern = c.P.accurate ? k_emis_forward<true, G> : k_emis_forward<false, G>;
+    const size_t smem = packet_smem<G>(s->view.stack_cap, false);
+    if (smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int blocks = ctx->sm_count * blocks_per_sm(kern, 32 * G, smem);
+    kern<<<blocks, 32 * G, smem, st>>>(s->view, e->view, c.cv, c.P, c.tiles, c.extent, s->emis, out, ctx->work_counter,
+                                       ctx->counters);
+    return VP_OK;
+  });
+  if (lr) return lr;
   VP_CUDA(cudaGetLastError());
   r = finish_stats(ctx, p, 1, stats);
   if (tmp) {
@@ -569,10 +874,17 @@ vp_status vp_render_emission_backward(vp_scene* s, vp_env* e, const vp_camera* c
   VP_CUDA(cudaMemsetAsync(ctx->counters, 0, sizeof(Counters), st));
   VP_CUDA(cudaMemsetAsync(ctx->work_counter, 0, sizeof(unsigned int), st));
   VP_CUDA(cudaEventRecord(ctx->ev0, st));
-  auto kern = c.P.accurate ? k_emis_backward<true> : k_emis_backward<false>;
-  if (c.smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
-  const int blocks = ctx->sm_count * blocks_per_sm(kern, 256, c.smem);
-  kern<<<blocks, 256, c.smem, st>>>(s->view, e->view, c.cv, c.P, s->emis, dsrc, acc, ctx->work_counter, ctx->counters);
+  const vp_status lr = with_group(c.tiles.tiles, s->view.stack_cap, [&](auto group) -> vp_status {
+    constexpr int G = decltype(group)::value;
+    auto kern = c.P.accurate ? k_emis_backward<true, G> : k_emis_backward<false, G>;
+    const size_t smem = packet_smem<G>(s->view.stack_cap, true);
+    if (smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int blocks = ctx->sm_count * blocks_per_sm(kern, 32 * G, smem);
+    kern<<<blocks, 32 * G, smem, st>>>(s->view, e->view, c.cv, c.P, c.tiles, c.extent, s->emis, dsrc, acc, ctx->work_counter,
+                                       ctx->counters);
+    return VP_OK;
+  });
+  if (lr) return cleanup(), lr;
   VP_CUDA(cudaGetLastError());
   k_emis_finish<<<(n + 255) / 256, 256, 0, st>>>(n, s->perm, s->prims, s->raw, acc, s->scale_is_log, gm, gs, gq, gd, ge);
   VP_CUDA(cudaGetLastError());

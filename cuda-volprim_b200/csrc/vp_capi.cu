@@ -4,8 +4,10 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "vp_internal.h"
@@ -14,6 +16,17 @@ namespace vp {
 
 namespace {
 thread_local std::string g_last_error;
+
+// Streams of the live contexts and their pools.
+std::mutex g_pools_mutex;
+std::vector<std::pair<cudaStream_t, cudaMemPool_t>> g_pools;
+}  // namespace
+
+cudaMemPool_t pool_of(cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(g_pools_mutex);
+  for (const auto& p : g_pools)
+    if (p.first == s) return p.second;
+  return nullptr;
 }
 
 void set_error(const std::string& msg) { g_last_error = msg; }
@@ -198,6 +211,21 @@ vp_status vp_context_create(int32_t device, vp_context** out) {
   c->device = device;
   cudaError_t e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+  if (e == cudaSuccess) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    e = cudaMemPoolCreate(&c->pool, &props);
+  }
+  if (e == cudaSuccess) {
+    uint64_t keep = kPoolKeep;
+    e = cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
+  if (e == cudaSuccess) {
+    std::lock_guard<std::mutex> lock(g_pools_mutex);
+    g_pools.emplace_back(c->stream, c->pool);
+  }
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
   if (e == cudaSuccess) e = cudaMalloc(&c->counters, sizeof(Counters));
@@ -222,6 +250,15 @@ vp_status vp_context_destroy(vp_context* c) {
     if (ev) cudaEventDestroy(ev);
   free_wavefront(c);
   if (c->wf.host_count) cudaFreeHost(c->wf.host_count);
+  {
+    std::lock_guard<std::mutex> lock(g_pools_mutex);
+    for (size_t i = 0; i < g_pools.size(); ++i)
+      if (g_pools[i].first == c->stream && g_pools[i].second == c->pool) {
+        g_pools.erase(g_pools.begin() + (std::ptrdiff_t)i);
+        break;
+      }
+  }
+  if (c->pool) cudaMemPoolDestroy(c->pool);  // (memory still held by the caller's objects goes when they free it)
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return VP_OK;

@@ -1,19 +1,18 @@
-// Device-wide primitives of the scene build and the wavefront re-sort, written for sm_100a:
+// Device-wide sort of the scene build and the wavefront re-sort, written for sm_100a:
 //
 //   radix_sort_pairs   stable LSD radix sort of (key, value) pairs, 8-bit digits, keys of 32 or
 //                      64 bits (only the digits covering [0, end_bit) are sorted)
-//   exclusive_scan     exclusive prefix sum of 32- or 64-bit counts
 //
 // Sort pass over one 8-bit digit (tiles of 2048 items, 256 threads, 8 warps):
 //   k_rs_upsweep    per-tile digit histogram (shared-memory atomics) -> hist[digit * tiles + tile]
-//   exclusive_scan  over hist: digit-major order gives every (digit, tile) its first output slot
+//   exclusive scan  over hist: digit-major order gives every (digit, tile) its first output slot
 //   k_rs_scatter    each warp ranks its 256 items in index order with __match_any_sync on the
 //                   digit (lanes with equal digits see one another; the rank is the number of
 //                   equal-digit lanes below plus the warp's running count of that digit), the
 //                   warps' counts are scanned per digit in the block, and every item goes to
 //                   hist[digit, tile] + (equal digits in earlier warps) + its warp rank.  Items
 //                   keep their order within a digit, so the sort is stable.
-// Scan of 32- or 64-bit counts (tiles of 4096 items, 1024 threads): per-tile sums, one block
+// Scan of counts (tiles of 4096 items, 1024 threads): per-tile sums, one block
 // scans the tile sums, then each tile scans itself from its offset.
 #include <algorithm>
 
@@ -105,7 +104,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* __restrict__
   }
 }
 
-// ---- exclusive scan of 32- or 64-bit counts ---------------------------------------------------
+// ---- exclusive scan of counts ---------------------------------------------------
 template <class T>
 __device__ __forceinline__ T block_scan_excl(T v, T* warp_tot, T& total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -254,16 +253,6 @@ vp_status exclusive_scan_t(const T* in, T* out, size_t n, void* tmp, size_t tmp_
 
 }  // namespace
 
-vp_status exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* tmp, size_t tmp_bytes, cudaStream_t st,
-                         uint32_t* launches) {
-  return exclusive_scan_t<uint32_t>(in, out, n, tmp, tmp_bytes, st, launches);
-}
-vp_status exclusive_scan(const unsigned long long* in, unsigned long long* out, size_t n, void* tmp, size_t tmp_bytes,
-                         cudaStream_t st, uint32_t* launches) {
-  return exclusive_scan_t<unsigned long long>(in, out, n, tmp, tmp_bytes, st, launches);
-}
-
-size_t exclusive_scan_tmp_bytes(size_t n) { return scan_tmp_bytes(n); }
 size_t radix_sort_tmp_bytes_u64(size_t n) { return sort_tmp_bytes_t<uint64_t>(n); }
 size_t radix_sort_tmp_bytes_u32(size_t n) { return sort_tmp_bytes_t<uint32_t>(n); }
 

@@ -570,6 +570,12 @@ vp_status ensure_workspace(vp_context* ctx, size_t paths) {
   const size_t per_path = 4 * 16 + 16 + 8 + 4 + 16 + 4 + 3 * 48 + 16 + 4 * 3 + 3 * 4;
   const size_t bytes = paths * per_path + 64 * 256 + 4096;
   cudaError_t e = cudaMalloc(&w.base, bytes);
+  if (e == cudaErrorMemoryAllocation) {  // give back what the context's pool keeps, and try again
+    (void)cudaGetLastError();
+    VP_CUDA(cudaStreamSynchronize(ctx->stream));
+    VP_CUDA(cudaMemPoolTrimTo(ctx->pool, 0));
+    e = cudaMalloc(&w.base, bytes);
+  }
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     w.base = nullptr;

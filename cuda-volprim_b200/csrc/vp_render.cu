@@ -25,6 +25,7 @@
 
 #include "vp_internal.h"
 #include "vp_pathloop.cuh"
+#include "vp_trace8.cuh"
 
 namespace vp {
 namespace {
@@ -204,6 +205,27 @@ __global__ void k_albedo_thread(SceneView S, const float* __restrict__ pts, uint
   if (status) atomicOr(&ctr->status, status);
 }
 
+// The same query, thread per ray (vp_trace8.cuh), for batches of at least kTrace8Min rays.
+template <bool kAcc>
+__global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_tau8(SceneView S, const float* __restrict__ org,
+                                                               const float* __restrict__ dir, uint32_t n,
+                                                               float* __restrict__ out, unsigned int* work, Counters* ctr) {
+  uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(S.depth8);
+  uint32_t status = 0;
+  trace8<kAcc, kTau8>(
+      OneScene8{scene8_of(S)}, S.depth8, smem, n, work, rays_per_warp(n), status,
+      [&](uint32_t i, Ray8& ray) {
+        ray.o = f3(org[3 * i], org[3 * i + 1], org[3 * i + 2]);
+        ray.d = f3(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
+        return true;
+      },
+      [&](uint32_t i, const Ray8&, const Hit8& h) {
+        const float tau = (float)h.w;
+        out[i] = tau >= kMaxOpticalDepth ? 0.0f : expf(-tau);
+      });
+  if (status) atomicOr(&ctr->status, status);
+}
+
 // normalize_accumulator_kernel (device/kernels/normalize_accumulator.cu:16-25)
 __global__ void k_normalize(float4* __restrict__ out, const float4* __restrict__ in, size_t n, float s) {
   const size_t stride = (size_t)blockDim.x * gridDim.x;
@@ -262,7 +284,14 @@ vp_status launch_transmittance(vp_scene* s, const float* o, const float* d, uint
   vp_context* ctx = s->ctx;
   cudaStream_t st = ctx->stream;
   if (n == 0) return VP_OK;
-  if (engine == VP_ENGINE_WARP) {
+  if (engine == VP_ENGINE_WARP && s->view.depth8 != 0u && n >= kTrace8Min) {
+    auto kern = accurate ? k_tau8<true> : k_tau8<false>;
+    const size_t smem = trace8_smem_bytes(s->view.depth8, kT8Threads);
+    VP_CUDA(cudaMemsetAsync(ctx->work_counter, 0, sizeof(unsigned int), st));
+    if (smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int blocks = ctx->sm_count * occupancy_blocks(kern, kT8Threads, smem);
+    kern<<<blocks, kT8Threads, smem, st>>>(s->view, o, d, n, out, ctx->work_counter, ctx->counters);
+  } else if (engine == VP_ENGINE_WARP) {
     const int threads = 256;
     const size_t smem = (size_t)(threads / 32) * warp_smem_bytes(s->view.stack_cap, 32);
     VP_CUDA(cudaMemsetAsync(ctx->work_counter, 0, sizeof(unsigned int), st));

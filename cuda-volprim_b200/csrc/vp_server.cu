@@ -7,9 +7,10 @@
 //                                requests that still have unstarted paths (the schedule)
 //   regen    (thread per path)   new paths: owning request from the share prefix sums, camera
 //                                ray, PCG32 stream, first free-flight key -- appended to the queue
-//   extend   (warp per path)     free-flight argmin + scatter albedo on the path's own scene
+//   extend   (warp per path)     free-flight argmin + scatter albedo on the path's own scene; from
+//                                kTrace8Min paths on in thread-per-ray form (vp_trace8.cuh)
 //   shade    (thread per path)   phase / NEE / roulette with the request's own controls
-//   shadow   (warp per query)    transmittance on the query's scene
+//   shadow   (warp per query)    transmittance on the query's scene; thread-per-ray likewise
 //   gather   (thread per path)   radiance += weight x T; a finished path adds its sample to its
 //                                request's pixel sum, counts itself done and frees its slot
 // so paths of different requests, scenes, resolutions and sample counts share every launch, and
@@ -38,7 +39,7 @@
 
 #include "vp_internal.h"
 #include "vp_path.cuh"
-#include "vp_traverse.cuh"
+#include "vp_trace8.cuh"
 
 namespace vp {
 namespace {
@@ -65,7 +66,7 @@ struct SrvCtl {  // device control block of the iteration
   uint32_t regen_m;     // paths started by the current iteration
   uint32_t regen_from;  // free-stack index of the first slot they take
   uint32_t survivors;   // paths carried over from the previous iteration
-  uint32_t ctr[8];      // [0] paths this iteration, [1] next, [2] shadow queries, [3..4] work heads
+  uint32_t ctr[8];      // [0] paths this iteration, [1] next, [2] shadow queries, [3..5] work heads
   unsigned long long total_started;  // paths the lane has started (the clock of SRPT aging)
 };
 
@@ -265,7 +266,7 @@ __global__ void k_srv_advance(SrvCtl* c, const SrvRequest* __restrict__ table, u
     c->regen_from = F - m;
     c->free_count = F - m;
     c->ctr[0] = s_surv + m;
-    c->ctr[1] = c->ctr[2] = c->ctr[3] = c->ctr[4] = 0u;
+    c->ctr[1] = c->ctr[2] = c->ctr[3] = c->ctr[4] = c->ctr[5] = 0u;
     c->total_started += m;
   }
 }
@@ -303,11 +304,12 @@ template <bool kAcc>
 __global__ void __launch_bounds__(256, 4) k_srv_extend(const SceneView* __restrict__ scenes,
                                                        const SrvRequest* __restrict__ table, SrvPaths b,
                                                        const uint32_t* __restrict__ q, SrvCtl* c, uint32_t max_cap,
-                                                       Counters* ctr) {
+                                                       uint32_t below, Counters* ctr) {
   extern __shared__ unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const WarpSmem W = carve(smem + warp * warp_smem_bytes(max_cap, kSrvHitCap), max_cap, kSrvHitCap);
   const uint32_t n = c->ctr[0];
+  if (n >= below) return;  // k_srv_extend8 takes the iteration
   uint32_t status = 0;
   WarpStats ws;
   while (true) {
@@ -340,6 +342,113 @@ __global__ void __launch_bounds__(256, 4) k_srv_extend(const SceneView* __restri
     if (status) break;
   }
   if (lane == 0 && status) atomicOr(&ctr->status, status);
+}
+
+// ---- thread-per-ray forms of extend and shadow, in every iteration's launches beside the others: which of
+// the two runs is decided by the iteration's count on the device ----
+// Shared memory after the warps' own: what the queries read of each resident scene.
+__device__ __forceinline__ ManyScenes8 stage_scenes(const SceneView* __restrict__ scenes, uint32_t n_scenes, uint32_t depth) {
+  Scene8* t = reinterpret_cast<Scene8*>(vp_dyn_smem + trace8_smem_bytes(depth, kT8Threads));
+  for (uint32_t k = threadIdx.x; k < n_scenes; k += blockDim.x) t[k] = scene8_of(scenes[k]);
+  __syncthreads();
+  return ManyScenes8{t};
+}
+
+template <bool kAcc>
+__global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_srv_extend8(const SceneView* __restrict__ scenes, uint32_t n_scenes,
+                                                                      const SrvRequest* __restrict__ table, SrvPaths b,
+                                                                      const uint32_t* __restrict__ q, SrvCtl* c,
+                                                                      uint32_t depth, Counters* ctr) {
+  const uint32_t n = c->ctr[0];
+  if (n < kTrace8Min) return;
+  const ManyScenes8 many = stage_scenes(scenes, n_scenes, depth);
+  uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(depth);
+  uint32_t status = 0;
+  trace8<kAcc, kFlight8>(
+      many, depth, smem, n, &c->ctr[3], rays_per_warp(n), status,
+      [&](uint32_t item, Ray8& ray) {
+        const uint32_t p = __ldg(q + item);
+        ray.scene = table[b.req[p]].scene;
+        const uint32_t bounce = b.meta[p] & 0xFFFFu;
+        if (bounce == 0u && scenes[ray.scene].albedo_all_zero) {
+          b.alb4[p] = make_float4(0.f, 0.f, 0.f, kInf);
+          b.sg[p] = kNoGauss;
+          return false;
+        }
+        const float4 o = b.o4[p], d = b.d4[p];
+        const uint2 k2 = b.key2[p];
+        ray.o = f3(o.x, o.y, o.z);
+        ray.d = f3(d.x, d.y, d.z);
+        ray.key = ((uint64_t)k2.y << 32) | k2.x;
+        ray.seed = bounce ? b.sg[p] : kNoGauss;
+        return true;
+      },
+      [&](uint32_t item, const Ray8& ray, const Hit8& h) {
+        const uint32_t p = __ldg(q + item);
+        // k_srv_scatter8 replaces the albedo where the scene's Gaussians differ in it
+        const float3 a = h.t < kInf ? scenes[ray.scene].albedo : f3(0.f, 0.f, 0.f);
+        b.alb4[p] = make_float4(a.x, a.y, a.z, h.t);
+        b.sg[p] = h.gauss;
+      });
+  if (status) atomicOr(&ctr->status, status);
+}
+
+// Launched when some resident scene's Gaussians differ in albedo.
+template <bool kAcc>
+__global__ void __launch_bounds__(kT8Threads) k_srv_scatter8(const SceneView* __restrict__ scenes, uint32_t n_scenes,
+                                                            const SrvRequest* __restrict__ table, SrvPaths b,
+                                                            const uint32_t* __restrict__ q, SrvCtl* c, uint32_t depth,
+                                                            Counters* ctr) {
+  const uint32_t n = c->ctr[0];
+  if (n < kTrace8Min) return;
+  const ManyScenes8 many = stage_scenes(scenes, n_scenes, depth);
+  uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(depth);
+  uint32_t status = 0;
+  trace8<kAcc, kScatter8>(
+      many, depth, smem, n, &c->ctr[5], rays_per_warp(n), status,
+      [&](uint32_t item, Ray8& ray) {
+        const uint32_t p = __ldg(q + item);
+        ray.scene = table[b.req[p]].scene;
+        ray.t = b.alb4[p].w;
+        if (!(ray.t < kInf) || scenes[ray.scene].one_albedo) return false;
+        const float4 o = b.o4[p], d = b.d4[p];
+        ray.o = f3(o.x, o.y, o.z);
+        ray.d = f3(d.x, d.y, d.z);
+        return true;
+      },
+      [&](uint32_t item, const Ray8& ray, const Hit8& h) {
+        const float3 a = mean_albedo(h.w, h.r, h.g, h.b);
+        b.alb4[__ldg(q + item)] = make_float4(a.x, a.y, a.z, ray.t);
+      });
+  if (status) atomicOr(&ctr->status, status);
+}
+
+template <bool kAcc>
+__global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_srv_shadow8(const SceneView* __restrict__ scenes, uint32_t n_scenes,
+                                                                      const SrvRequest* __restrict__ table, SrvPaths b,
+                                                                      SrvCtl* c, uint32_t depth, Counters* ctr) {
+  const uint32_t n = c->ctr[2];
+  if (n < kTrace8Min) return;
+  const ManyScenes8 many = stage_scenes(scenes, n_scenes, depth);
+  uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(depth);
+  uint32_t status = 0;
+  trace8<kAcc, kTau8>(
+      many, depth, smem, n, &c->ctr[4], rays_per_warp(n), status,
+      [&](uint32_t item, Ray8& ray) {
+        const uint32_t slot = __ldg(b.qs + item);
+        ray.scene = table[b.req[slot / 3u]].scene;
+        const float4 o = b.so4[slot], d = b.sd4[slot];
+        ray.o = f3(o.x, o.y, o.z);
+        ray.d = f3(d.x, d.y, d.z);
+        ray.seed = __float_as_uint(d.w);
+        ray.seed_tau = o.w;
+        return true;
+      },
+      [&](uint32_t item, const Ray8&, const Hit8& h) {
+        const float tau = (float)h.w;
+        b.so4[__ldg(b.qs + item)].w = tau >= kMaxOpticalDepth ? 0.0f : expf(-tau);
+      });
+  if (status) atomicOr(&ctr->status, status);
 }
 
 // As the offline engine's shade stage, the shadow rays' seed chords are evaluated here, one
@@ -396,11 +505,12 @@ __global__ void __launch_bounds__(256) k_srv_shade(const SceneView* __restrict__
 template <bool kAcc>
 __global__ void __launch_bounds__(256, 4) k_srv_shadow(const SceneView* __restrict__ scenes,
                                                        const SrvRequest* __restrict__ table, SrvPaths b, SrvCtl* c,
-                                                       uint32_t max_cap, Counters* ctr) {
+                                                       uint32_t max_cap, uint32_t below, Counters* ctr) {
   extern __shared__ unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const WarpSmem W = carve(smem + warp * warp_smem_bytes(max_cap, 32), max_cap, 32);
   const uint32_t n = c->ctr[2];
+  if (n >= below) return;  // k_srv_shadow8 takes the iteration
   uint32_t status = 0;
   WarpStats ws;
   while (true) {
@@ -491,6 +601,10 @@ struct vp_server {
                                                 // entry's first iteration (~0 until then)
   // pinned staging of the table entries (each reaches the device by a stream-ordered copy)
   SrvRequest* h_table = nullptr;
+  uint32_t max_depth8 = 0;      // deepest BVH8 over the scenes, 0 when some scene has none
+  bool mixed_albedo = false;    // some scene's Gaussians differ in albedo
+  int ext8_blocks = 0, sca8_blocks = 0, shd8_blocks = 0;
+  size_t smem8 = 0;
   int ext_blocks = 0, shd_blocks = 0, thr_blocks = 0;
   size_t smem_ext = 0, smem_shd = 0;
   cudaStream_t copy_stream = nullptr;  // output copies of completed requests
@@ -629,19 +743,30 @@ vp_status enqueue_iteration(vp_server* s, uint32_t l, bool even) {
   k_srv_advance<<<1, R, 0, st>>>(L.d_ctl, s->d_table, s->d_started, s->d_age_base, L.d_alloc_off,
                                  L.d_alloc_start, s->cfg.schedule, s->cfg.srpt_reserve, s->cfg.srpt_aging, l, nl);
   k_srv_regen<<<s->thr_blocks, 256, 0, st>>>(L.d_ctl, s->d_table, L.d_alloc_off, L.d_alloc_start, R, L.paths, qcur);
-  if (s->accurate)
-    k_srv_extend<true><<<s->ext_blocks, 256, s->smem_ext, st>>>(s->d_scenes, s->d_table, L.paths, qcur, L.d_ctl,
-                                                               s->max_argmin_cap, ctr);
-  else
-    k_srv_extend<false><<<s->ext_blocks, 256, s->smem_ext, st>>>(s->d_scenes, s->d_table, L.paths, qcur, L.d_ctl,
-                                                                s->max_argmin_cap, ctr);
+  // an iteration of at least kTrace8Min paths (or shadow queries) takes the thread-per-ray form
+  const uint32_t below = s->max_depth8 ? kTrace8Min : 0xFFFFFFFFu;
+  const uint32_t n_scenes = (uint32_t)s->scenes.size();
+  auto ext = s->accurate ? k_srv_extend<true> : k_srv_extend<false>;
+  auto shd = s->accurate ? k_srv_shadow<true> : k_srv_shadow<false>;
+  auto ext8 = s->accurate ? k_srv_extend8<true> : k_srv_extend8<false>;
+  auto sca8 = s->accurate ? k_srv_scatter8<true> : k_srv_scatter8<false>;
+  auto shd8 = s->accurate ? k_srv_shadow8<true> : k_srv_shadow8<false>;
+  const bool both = s->max_depth8 && L.slots >= kTrace8Min;  // (a smaller pool never reaches the count)
+  ext<<<s->ext_blocks, 256, s->smem_ext, st>>>(s->d_scenes, s->d_table, L.paths, qcur, L.d_ctl, s->max_argmin_cap,
+                                              below, ctr);
+  if (both) {
+    ext8<<<s->ext8_blocks, kT8Threads, s->smem8, st>>>(s->d_scenes, n_scenes, s->d_table, L.paths, qcur, L.d_ctl,
+                                                      s->max_depth8, ctr);
+    if (s->mixed_albedo)
+      sca8<<<s->sca8_blocks, kT8Threads, s->smem8, st>>>(s->d_scenes, n_scenes, s->d_table, L.paths, qcur, L.d_ctl,
+                                                        s->max_depth8, ctr);
+  }
   k_srv_shade<<<s->thr_blocks, 256, 0, st>>>(s->d_scenes, s->d_envs, s->d_table, L.paths, qcur, L.d_ctl, qnext);
-  if (s->accurate)
-    k_srv_shadow<true><<<s->shd_blocks, 256, s->smem_shd, st>>>(s->d_scenes, s->d_table, L.paths, L.d_ctl,
-                                                               s->max_cap, ctr);
-  else
-    k_srv_shadow<false><<<s->shd_blocks, 256, s->smem_shd, st>>>(s->d_scenes, s->d_table, L.paths, L.d_ctl,
-                                                                s->max_cap, ctr);
+  shd<<<s->shd_blocks, 256, s->smem_shd, st>>>(s->d_scenes, s->d_table, L.paths, L.d_ctl, s->max_cap, below, ctr);
+  // (three shadow queries a path at most)
+  if (s->max_depth8 && 3ull * L.slots >= kTrace8Min)
+    shd8<<<s->shd8_blocks, kT8Threads, s->smem8, st>>>(s->d_scenes, n_scenes, s->d_table, L.paths, L.d_ctl,
+                                                      s->max_depth8, ctr);
   k_srv_gather<<<s->thr_blocks, 256, 0, st>>>(s->d_table, L.paths, qcur, L.d_ctl, s->d_done);
   VP_CUDA(cudaGetLastError());
   return VP_OK;
@@ -653,9 +778,28 @@ vp_status prepare_launch(vp_server* s) {
   vp_context* ctx = s->ctx;
   s->max_cap = 2;
   s->max_argmin_cap = 2;
+  bool can8 = true;
+  s->max_depth8 = 0;
+  s->mixed_albedo = false;
   for (vp_scene* sc : s->scenes) {
+    can8 = can8 && sc->view.depth8 != 0u;
+    s->max_depth8 = std::max(s->max_depth8, sc->view.depth8);
+    s->mixed_albedo = s->mixed_albedo || !sc->view.one_albedo;
     s->max_cap = std::max(s->max_cap, sc->view.stack_cap);
     s->max_argmin_cap = std::max(s->max_argmin_cap, sc->view.argmin_cap);
+  }
+  if (!can8) s->max_depth8 = 0;
+  if (s->max_depth8) {
+    s->smem8 = trace8_smem_bytes(s->max_depth8, kT8Threads) + s->scenes.size() * sizeof(Scene8);
+    auto ext8 = s->accurate ? k_srv_extend8<true> : k_srv_extend8<false>;
+    auto sca8 = s->accurate ? k_srv_scatter8<true> : k_srv_scatter8<false>;
+    auto shd8 = s->accurate ? k_srv_shadow8<true> : k_srv_shadow8<false>;
+    if (s->smem8 > 48 * 1024)
+      for (auto k : {(const void*)ext8, (const void*)sca8, (const void*)shd8})
+        VP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem8));
+    s->ext8_blocks = ctx->sm_count * srv_blocks(ext8, kT8Threads, s->smem8);
+    s->sca8_blocks = ctx->sm_count * srv_blocks(sca8, kT8Threads, s->smem8);
+    s->shd8_blocks = ctx->sm_count * srv_blocks(shd8, kT8Threads, s->smem8);
   }
   s->smem_ext = (size_t)8 * warp_smem_bytes(s->max_argmin_cap, kSrvHitCap);
   s->smem_shd = (size_t)8 * warp_smem_bytes(s->max_cap, 32);

@@ -50,10 +50,28 @@ __host__ __device__ __forceinline__ size_t trace8_smem_bytes(uint32_t depth, int
 
 enum Query8 { kFlight8 = 0, kTau8 = 1, kScatter8 = 2 };
 
+// What a query reads of a scene.
+struct Scene8 {
+  const uint32_t* nodes;
+  const float4* prims;
+  const uint32_t* perm;
+};
+__device__ __forceinline__ Scene8 scene8_of(const SceneView& S) { return Scene8{S.nodes8, S.prims, S.perm}; }
+// The scene of every ray of a launch, or (the serving engine) each ray's own, from a table in shared memory.
+struct OneScene8 {
+  Scene8 s;
+  __device__ __forceinline__ Scene8 of(uint32_t) const { return s; }
+};
+struct ManyScenes8 {
+  const Scene8* table;
+  __device__ __forceinline__ Scene8 of(uint32_t k) const { return table[k]; }
+};
+
 struct Ray8 {
   float3 o, d;
   uint64_t key;    // kFlight8: free-flight key
   float t;         // kScatter8: scatter distance
+  uint32_t scene;  // ManyScenes8: index into the table
   uint32_t seed;   // kTau8: the Gaussian already accounted for; kFlight8: one to start with (kNoGauss: none)
   float seed_tau;  // its optical depth (0 without one)
 };
@@ -72,10 +90,10 @@ __device__ __forceinline__ float byte_plane(uint32_t word, uint32_t sel) {  // 1
 // item needs no query (its sink is not called); sink(item, ray, hit) takes the result.  `rpw` rays are
 // in flight per warp: fewer than 32 when the batch is too small to give every resident warp 32, since
 // the chord and value steps use all lanes anyway.
-template <bool kAcc, int kKind, class Source, class Sink>
-__device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const float4* __restrict__ prims,
-                                       const uint32_t* __restrict__ perm, uint32_t depth, uint32_t* smem, uint32_t n,
+template <bool kAcc, int kKind, class Scenes, class Source, class Sink>
+__device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uint32_t* smem, uint32_t n,
                                        unsigned int* work, int rpw, uint32_t& status, Source&& source, Sink&& sink) {
+  constexpr bool kMany = std::is_same_v<Scenes, ManyScenes8>;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   uint32_t* stack = smem + lane;  // entry k at stack[32 k]: conflict-free whatever the lanes' depths
@@ -88,6 +106,9 @@ __device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const
   ray.key = 0ull;
   ray.seed = kNoGauss;
   ray.t = 0.f;
+  ray.scene = 0u;
+  // the scene of another lane's ray
+  auto scene_of = [&](int ow) { return scenes.of(kMany ? __shfl_sync(kFull, ray.scene, ow) : 0u); };
   float3 inv = f3(0.f, 0.f, 0.f);
   uint32_t item = 0, node = 0, mask = 0, neg = 0;
   int sp = 0;
@@ -108,6 +129,7 @@ __device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const
     if (on) id = q2[e];
     const int ow = (int)(id >> 27) & 31;
     const uint32_t gi = id & 0x07FFFFFFu;
+    const Scene8 sc = scene_of(ow);
     uint64_t key = 0ull;
     float ts = 0.f;
     if constexpr (kKind == kFlight8)
@@ -128,11 +150,11 @@ __device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const
         v = chord_tau<kAcc>(ch.tc, ch.rw, ch.d2, ch.h, chord_u0(ch, 0.0f), fmaxf(ch.t_in, 0.0f), ch.t_out, icf, ch.d2lo);
       } else if constexpr (kKind == kFlight8) {
         v = chord_free_flight<kAcc>(ch.tc, ch.rw, ch.d2, ch.h, chord_u0(ch, 0.0f), ch.t_in, ch.t_out, icf,
-                                    free_flight_tau<kAcc>(key, __ldg(perm + gi)), ch.d2lo);
+                                    free_flight_tau<kAcc>(key, __ldg(sc.perm + gi)), ch.d2lo);
       } else {
         const float u = (ts - ch.tc) / ch.rw;
         v = icf * vexp<kAcc>(-0.5f * fmaf(u, u, ch.d2));
-        const float3 al = load_albedo(prims, gi);
+        const float3 al = load_albedo(sc.prims, gi);
         wa = al.x, wb = al.y, wc = al.z;
       }
     }
@@ -181,8 +203,9 @@ __device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const
     __syncwarp();
     const int ow = (int)(w >> 27);
     const uint32_t at = w & 0x07FFFFFFu;  // node * 8 + slot
+    const Scene8 sc = scene_of(ow);
     uint32_t gi = 0;
-    if (lane < k) gi = __ldg(nodes + (size_t)(at >> 3) * kNode8Words + 16u + (at & 7u)) & ~kLeafBit;
+    if (lane < k) gi = __ldg(sc.nodes + (size_t)(at >> 3) * kNode8Words + 16u + (at & 7u)) & ~kLeafBit;
     const float3 o = f3(__shfl_sync(kFull, ray.o.x, ow), __shfl_sync(kFull, ray.o.y, ow), __shfl_sync(kFull, ray.o.z, ow));
     const float3 d = f3(__shfl_sync(kFull, ray.d.x, ow), __shfl_sync(kFull, ray.d.y, ow), __shfl_sync(kFull, ray.d.z, ow));
     bool hit = lane < k;
@@ -196,9 +219,9 @@ __device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const
     Chord ch;
     if (hit) {
       PrimGeo g;
-      g.a = __ldg(prims + 4u * gi);
-      g.b = __ldg(prims + 4u * gi + 1u);
-      g.c = __ldg(prims + 4u * gi + 2u);
+      g.a = __ldg(sc.prims + 4u * gi);
+      g.b = __ldg(sc.prims + 4u * gi + 1u);
+      g.c = __ldg(sc.prims + 4u * gi + 2u);
       hit = chord_setup<kAcc>(g, o, d, ch);
       if constexpr (kKind == kScatter8) hit = hit && ch.t_in <= bound && bound <= ch.t_out;
       else hit = hit && ch.t_out > 0.0f && ch.t_in <= bound;
@@ -212,7 +235,7 @@ __device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const
       q2[2 * kQ2Cap + p] = __float_as_uint(ch.rw);
       q2[3 * kQ2Cap + p] = __float_as_uint(ch.d2);
       q2[4 * kQ2Cap + p] = __float_as_uint(ch.h);
-      q2[5 * kQ2Cap + p] = __ldg(reinterpret_cast<const uint32_t*>(prims + 4u * gi + 3u));
+      q2[5 * kQ2Cap + p] = __ldg(reinterpret_cast<const uint32_t*>(sc.prims + 4u * gi + 3u));
       if (kAcc) q2[6 * kQ2Cap + p] = __float_as_uint(ch.d2lo);
     }
     q2n += __popc(hm);
@@ -258,11 +281,12 @@ __device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const
               // a path that scattered starts inside the Gaussian that scattered it: its free flight
               // bounds the traversal from the start (showcase: 63 -> 33 nodes a ray with it)
               if (ray.seed != kNoGauss) {
-                const PrimGeo g = load_geo(prims, ray.seed);
+                const Scene8 sc = scenes.of(ray.scene);
+                const PrimGeo g = load_geo(sc.prims, ray.seed);
                 Chord ch;
                 if (chord_setup<kAcc>(g, ray.o, ray.d, ch) && ch.t_out > 0.0f) {
                   const float v = chord_free_flight<kAcc>(ch.tc, ch.rw, ch.d2, ch.h, chord_u0(ch, 0.0f), ch.t_in, ch.t_out,
-                                                          g.icf, free_flight_tau<kAcc>(ray.key, __ldg(perm + ray.seed)),
+                                                          g.icf, free_flight_tau<kAcc>(ray.key, __ldg(sc.perm + ray.seed)),
                                                           ch.d2lo);
                   if (v < t_hi) t_hi = v, arg = ray.seed;
                 }
@@ -276,6 +300,7 @@ __device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const
     }
     // node step
     uint32_t leaf = 0u;
+    const uint32_t* nodes = scenes.of(ray.scene).nodes;
     if (active && (mask != 0u || sp != 0)) {
       if (mask == 0u) {
         const uint32_t e = stack[32 * --sp];
@@ -343,6 +368,27 @@ __device__ __forceinline__ void trace8(const uint32_t* __restrict__ nodes, const
     while (q1n >= 32) chords(32);
     if (__any_sync(kFull, status != 0u)) break;
   }
+}
+
+
+// Batches of at least this many rays take the thread-per-ray form.  Below it a launch ends with its longest
+// rays, whose lanes walk alone, and a whole warp on each ray is sooner done.  Transmittance batches
+// (thread-per-ray / warp-per-ray, ms): 65k rays 0.29 / 0.24 (100k-Gaussian cloud), 0.37 / 0.32 (500k), 0.57 /
+// 0.42 (100k in clusters); 130k 0.33 / 0.38, 0.44 / 0.53, 0.70 / 0.72; 250k 0.39 / 0.63, 0.55 / 0.93, 0.94 /
+// 1.25.  8-bounce images: 65k paths 2.7 / 1.9 (50k-Gaussian cloud), 5.0 / 3.8 (500k),
+// 6.6 / 4.7 (200k in clusters); 131k paths 3.0 / 3.3, 5.7 / 6.5, 8.1 / 8.3; 524k paths 5.0 / 11.2, 9.5 / 22.8,
+// 15.0 / 29.2.
+constexpr uint32_t kTrace8Min = 7u << 14;
+// Threads of a block of the stages, and the resident blocks per SM of their register budget: 3 (80 registers).
+// 4 (64 registers) spills and leaves less of the SM's memory to L1, 2 hides less latency: the showcase batch
+// took 93 ms at 4 against 86 at 3, and 83 ms at 2 against 70 at 3.
+constexpr int kT8Blocks = 3;
+constexpr int kT8Threads = 256;
+
+// Rays in flight per warp: 32, or an even share of a batch too small for that.
+__device__ __forceinline__ int rays_per_warp(uint32_t n) {
+  const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+  return (int)min(32u, max(4u, (n + warps - 1u) / warps));
 }
 
 }  // namespace vp

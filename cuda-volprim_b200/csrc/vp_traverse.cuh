@@ -569,6 +569,32 @@ __device__ float warp_ray_query(const SceneView& S, const WarpSmem& W, float3 o,
   else return tau_total();
 }
 
+// A leaf step's Gaussians: the leaf's own and those of the leaves next on the stack while they fit in the 32
+// lanes.  Returns how many; pi is the lane's.
+__device__ __forceinline__ uint32_t packed_leaves(const uint32_t* stack, int& sp, uint32_t ref, uint32_t& pi,
+                                                  WarpStats& ws, bool measure) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t total = wide_leaf_count(ref), packed = 1u;
+  pi = wide_leaf_first(ref) + lane;
+  while (VP_LEAF_PACK && sp > 0) {
+    const uint32_t r2 = stack[sp - 1];
+    if (!ref_is_leaf(r2)) break;
+    const uint32_t c2 = wide_leaf_count(r2);
+    if (total + c2 > 32u) break;
+    --sp;
+    if (lane >= total && lane < total + c2) pi = wide_leaf_first(r2) + (lane - total);
+    total += c2;
+    ++packed;
+  }
+  __syncwarp();
+  if (measure) {
+    ws.leaves += packed;
+    ws.kind_leaves[2] += packed;
+    ws.kind_prims[2] += total;
+  }
+  return total;
+}
+
 // Albedo at distance t along a ray: the sum over the chords containing t that an argmin query takes from
 // its own retained chords, found by a traversal of its own -- for the rays whose chords outgrew the hit
 // buffer.  The same terms in FP64, so the same result.
@@ -588,13 +614,8 @@ __device__ float3 warp_scatter_albedo(const SceneView& S, const WarpSmem& W, flo
     __syncwarp();
     float tn;
     if (ref_is_leaf(ref)) {
-      const uint32_t first = wide_leaf_first(ref), count = wide_leaf_count(ref);
-      if (measure) {
-        ws.leaves++;
-        ws.kind_leaves[2]++;
-        ws.kind_prims[2] += count;
-      }
-      const uint32_t pi = first + lane;
+      uint32_t pi;
+      const uint32_t count = packed_leaves(W.st_ref, sp, ref, pi, ws, measure);
       const bool boxed = (uint32_t)lane < count &&
                          slab(rb, __ldg(S.pbox + 2u * pi), __ldg(S.pbox + 2u * pi + 1u), t, t, tn);
       if (measure) ws.kind_geo[2] += __popc(__ballot_sync(kFull, boxed));
@@ -650,7 +671,7 @@ template <bool kAcc>
 __device__ float3 warp_albedo(const SceneView& S, const WarpSmem& W, float3 x, uint32_t& overlap,
                               uint32_t& status, WarpStats& ws, bool measure) {
   const int lane = threadIdx.x & 31;
-  float aw = 0.f, ar = 0.f, ag = 0.f, ab = 0.f;
+  double aw = 0.0, ar = 0.0, ag = 0.0, ab = 0.0;
   unsigned int cnt = 0;
   int sp = 1;
   if (lane == 0) W.st_ref[0] = S.wide_root;
@@ -660,13 +681,8 @@ __device__ float3 warp_albedo(const SceneView& S, const WarpSmem& W, float3 x, u
     const uint32_t ref = W.st_ref[sp];
     __syncwarp();
     if (ref_is_leaf(ref)) {
-      const uint32_t first = wide_leaf_first(ref), count = wide_leaf_count(ref);
-      if (measure) {
-        ws.leaves++;
-        ws.kind_leaves[2]++;
-        ws.kind_prims[2] += count;
-      }
-      const uint32_t pi = first + lane;
+      uint32_t pi;
+      const uint32_t count = packed_leaves(W.st_ref, sp, ref, pi, ws, measure);
       const bool boxed = (uint32_t)lane < count &&
                          box_contains(__ldg(S.pbox + 2u * pi), __ldg(S.pbox + 2u * pi + 1u), x);
       if (measure) ws.kind_geo[2] += __popc(__ballot_sync(kFull, boxed));
@@ -674,12 +690,12 @@ __device__ float3 warp_albedo(const SceneView& S, const WarpSmem& W, float3 x, u
         const PrimGeo g = load_geo(S.prims, pi);
         const float r2 = point_r2<kAcc>(g, x);
         if (r2 <= kExtent2) {  // point_inside_bvh_bound (intersection.h:56-61)
-          const float wgt = g.icf * vexp<kAcc>(-0.5f * r2);
+          const double wgt = (double)(g.icf * vexp<kAcc>(-0.5f * r2));
           const float3 al = load_albedo(S.prims, pi);
           aw += wgt;
-          ar += wgt * al.x;
-          ag += wgt * al.y;
-          ab += wgt * al.z;
+          ar += wgt * (double)al.x;
+          ag += wgt * (double)al.y;
+          ab += wgt * (double)al.z;
           ++cnt;
         }
       }
@@ -711,9 +727,7 @@ __device__ float3 warp_albedo(const SceneView& S, const WarpSmem& W, float3 x, u
   ab = warp_sum(ab);
   for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(kFull, cnt, o);
   overlap = cnt;
-  if (!(aw > 0.f)) return f3(0.f, 0.f, 0.f);
-  const float r = __frcp_rn(aw);
-  return f3(ar * r, ag * r, ab * r);
+  return mean_albedo(aw, ar, ag, ab);
 }
 
 

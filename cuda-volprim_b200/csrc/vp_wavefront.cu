@@ -60,12 +60,6 @@ constexpr int kExtendHitCap = VP_WF_EXTEND_HIT_CAP;
 #define VP_WF_SORT_MIN 65536
 #endif
 constexpr uint32_t kSortMinPaths = VP_WF_SORT_MIN;
-// Queues of at least this many paths take the thread-per-ray stages.  Below it the launch ends with its
-// longest rays, whose lanes walk alone, and a whole warp on each ray is sooner done.  Measured on 8-bounce
-// images (thread-per-ray / warp-per-ray, ms): 65k paths 2.7 / 1.9 (50k-Gaussian cloud), 5.0 / 3.8 (500k),
-// 6.6 / 4.7 (200k in clusters); 131k paths 3.0 / 3.3, 5.7 / 6.5, 8.1 / 8.3; 524k paths 5.0 / 11.2, 9.5 / 22.8,
-// 15.0 / 29.2.
-constexpr uint32_t kTrace8Min = 7u << 14;
 // At most this many paths go to the tail kernel: as stages, a bounce of few paths is launches, polls and each
 // stage's slowest ray; as whole paths it is one launch, but a warp shades alone and holds more registers.
 // 64-bounce images, ms as stages / with the tail from 16k paths / from 40k: 4k paths 4.4 / 2.2 / 2.1 (50k-
@@ -223,17 +217,6 @@ __global__ void __launch_bounds__(256, VP_WF_MIN_BLOCKS) k_wf_extend(SceneView S
 }
 
 // ---- thread-per-ray stages (vp_trace8.cuh) -----------------------------------------------------
-// Resident blocks per SM their register budget is sized for: 3 (80 registers).  4 (64 registers) spills and
-// leaves less of the SM's memory to L1: the showcase batch took 93 ms at 4, 86 at 3, 83 at 2 with later
-// changes ahead of 3 (70).
-constexpr int kT8Blocks = 3;
-constexpr int kT8Threads = 256;
-
-// Rays in flight per warp: 32, or an even share of a batch too small for that.
-__device__ __forceinline__ int rays_per_warp(uint32_t n) {
-  const uint32_t warps = gridDim.x * (blockDim.x / 32u);
-  return (int)min(32u, max(4u, (n + warps - 1u) / warps));
-}
 
 template <bool kAcc>
 __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_wf_extend8(SceneView S, WfBuffers b, const uint32_t* q,
@@ -243,7 +226,7 @@ __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_wf_extend8(SceneView 
   const uint32_t n = *count;
   uint32_t status = 0;
   trace8<kAcc, kFlight8>(
-      S.nodes8, S.prims, S.perm, S.depth8, smem, n, work, rays_per_warp(n), status,
+      OneScene8{scene8_of(S)}, S.depth8, smem, n, work, rays_per_warp(n), status,
       [&](uint32_t item, Ray8& ray) {
         const uint32_t p = __ldg(q + item);
         const uint32_t bounce = meta_bounce(b.meta[p]);
@@ -279,7 +262,7 @@ __global__ void __launch_bounds__(kT8Threads) k_wf_scatter8(SceneView S, WfBuffe
   const uint32_t n = *count;
   uint32_t status = 0;
   trace8<kAcc, kScatter8>(
-      S.nodes8, S.prims, S.perm, S.depth8, smem, n, work, rays_per_warp(n), status,
+      OneScene8{scene8_of(S)}, S.depth8, smem, n, work, rays_per_warp(n), status,
       [&](uint32_t item, Ray8& ray) {
         const uint32_t p = __ldg(q + item);
         const float t = b.alb4[p].w;
@@ -304,7 +287,7 @@ __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_wf_shadow8(SceneView 
   const uint32_t n = *count;
   uint32_t status = 0;
   trace8<kAcc, kTau8>(
-      S.nodes8, S.prims, S.perm, S.depth8, smem, n, work, rays_per_warp(n), status,
+      OneScene8{scene8_of(S)}, S.depth8, smem, n, work, rays_per_warp(n), status,
       [&](uint32_t item, Ray8& ray) {
         const uint32_t slot = __ldg(b.qs + item);
         const float4 o = b.so4[slot], d = b.sd4[slot];

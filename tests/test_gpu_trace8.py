@@ -83,3 +83,50 @@ def test_empty_scene(vp_ctx):
     g = vp.Gaussians(np.zeros((0, 3), np.float32), np.zeros((0, 3), np.float32), np.zeros((0, 4), np.float32),
                      np.zeros(0, np.float32))
     check(*images(vp_ctx, g))
+
+
+def test_large_transmittance_batch(vp_ctx):
+    """vp_transmittance takes the thread-per-ray form from 114,688 rays on: the same values as in smaller calls."""
+    sc = vp.Scene(vp_ctx, gaussians(1500, 21), 0.2)
+    rng = np.random.default_rng(22)
+    n = 114_700
+    o = np.where((np.arange(n) % 2 == 0)[:, None], rng.normal(0, 2.0, (n, 3)), rng.uniform(-0.5, 0.5, (n, 3)))
+    d = rng.normal(0, 1, (n, 3))
+    d[::7, 0] = 0.0  # axis-parallel components
+    d = d / np.linalg.norm(d, axis=1, keepdims=True)
+    o, d = o.astype(np.float32), d.astype(np.float32)
+    for precision in (vp.VP_PRECISION_FAST, vp.VP_PRECISION_ACCURATE):
+        got = sc.transmittance(o, d, precision=precision)
+        want = np.concatenate([sc.transmittance(o[k:k + 50_000], d[k:k + 50_000], precision=precision)
+                               for k in range(0, n, 50_000)])
+        assert (want < 0.9).sum() > 1000 and (want > 0.99).sum() > 1000
+        assert np.abs(got - want).max() <= 1e-7, np.abs(got - want).max()
+    sc.close()
+
+
+def test_served_requests_match_renders(vp_ctx):
+    """Two scenes -- one of one albedo, one mixed -- and a pool of path slots above the threshold: every request
+    equals its own render up to the order of its pixel sums."""
+    from volprim_b200 import serving
+    env = vp.Environment(vp_ctx, rgb=scenes.procedural_env(64, 32, sun_radiance=50.0, sun_radius_deg=8.0))
+    scs = [vp.Scene(vp_ctx, gaussians(700, 31 + k, mixed=bool(k))) for k in range(2)]
+    server = serving.Server(vp_ctx, path_slots=1 << 18)
+    for s in scs:
+        server.add_scene(s, env)
+    reqs = []
+    for k, (w, h, spp) in enumerate([(300, 250, 2), (301, 203, 2), (64, 64, 4), (257, 129, 3)]):
+        cfg = vp.Config(num_samples_per_pixel=spp, image_width=w, image_height=h, seed=k, hg_g=0.3, max_bounces=12,
+                        rr_depth=12, precision="fast")
+        cam = serving.random_camera(np.random.default_rng(k), 3.0)
+        reqs.append((server.submit(k % 2, cam, cfg), k % 2, cam, cfg))
+    left = len(reqs)
+    while left:
+        server.step()
+        left -= len(server.poll())
+    for rid, k, cam, cfg in reqs:
+        got = server.result(rid)[..., :3]
+        want = vp.Renderer(cfg, scs[k], cam, env=env, ctx=vp_ctx).render()[..., :3]
+        assert np.abs(got - want).max() <= 1e-5 * want.max() + 1e-6
+    server.close()
+    for s in scs:
+        s.close()

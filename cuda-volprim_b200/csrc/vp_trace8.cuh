@@ -29,7 +29,7 @@ namespace vp {
 //   words 16..23 child references: an inner node's index or kLeafBit | Gaussian (scene order)
 // Child slot s holds the child that lies furthest towards (s&1 ? +x : -x, s&2 ? +y : -y, s&4 ? +z : -z),
 // so visiting slots in ascending (s ^ sign bits of the direction) is roughly front to back.
-// An unused slot has lo = 255, hi = 0 (never hit).  Node 0 only points to the root (slot 0).
+// An unused slot has lo = 255, hi = 0 and no reference (a hit of it is dropped).  Node 0 only points to the root (slot 0).
 constexpr uint32_t kNode8Words = 24;
 constexpr uint32_t kMaxNodes8 = 1u << 24;   // stack entries hold (node << 8 | child mask)
 constexpr uint32_t kMaxDepth8 = 40;         // deeper trees take the warp-cooperative query
@@ -204,11 +204,13 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
     const int ow = (int)(w >> 27);
     const uint32_t at = w & 0x07FFFFFFu;  // node * 8 + slot
     const Scene8 sc = scene_of(ow);
-    uint32_t gi = 0;
-    if (lane < k) gi = __ldg(sc.nodes + (size_t)(at >> 3) * kNode8Words + 16u + (at & 7u)) & ~kLeafBit;
+    uint32_t gi = kEmptyRef;
+    if (lane < k) gi = __ldg(sc.nodes + (size_t)(at >> 3) * kNode8Words + 16u + (at & 7u));
+    // an unused slot's planes (lo 255, hi 0) coincide when the ray's distance rounds the whole node away
+    bool hit = gi != kEmptyRef;
+    gi &= ~kLeafBit;
     const float3 o = f3(__shfl_sync(kFull, ray.o.x, ow), __shfl_sync(kFull, ray.o.y, ow), __shfl_sync(kFull, ray.o.z, ow));
     const float3 d = f3(__shfl_sync(kFull, ray.d.x, ow), __shfl_sync(kFull, ray.d.y, ow), __shfl_sync(kFull, ray.d.z, ow));
-    bool hit = lane < k;
     float bound = kInf;
     if constexpr (kKind == kTau8) {
       const uint32_t seed = __shfl_sync(kFull, ray.seed, ow);

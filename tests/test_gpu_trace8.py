@@ -130,3 +130,13 @@ def test_served_requests_match_renders(vp_ctx):
     server.close()
     for s in scs:
         s.close()
+
+
+def test_nodes_below_the_distance_rounding(vp_ctx):
+    """A node far smaller than an ulp of the ray's distance to it: all its planes round to one distance, those of
+    its unused slots too, and only its three Gaussians may be met."""
+    c = np.array([[0.0, 0.0, 0.0], [2e-8, 0.0, 0.0], [0.0, 2e-8, 1e-8]], np.float32)
+    g = vp.Gaussians(c, np.full((3, 3), 1e-8, np.float32), np.tile(np.array([1.0, 0, 0, 0], np.float32), (3, 1)),
+                     np.full(3, 1e-16, np.float32), np.full((3, 3), 0.5, np.float32))
+    cam = vp.Camera.orthographic_camera((0.0, 0.0, -100.0), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 2e-7)
+    check(*images(vp_ctx, g, camera=cam, hg_g=0.0))

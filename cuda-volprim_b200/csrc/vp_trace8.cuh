@@ -86,6 +86,17 @@ __device__ __forceinline__ float byte_plane(uint32_t word, uint32_t sel) {  // 1
   return __uint_as_float(__byte_perm(word, 0x3F800000u, sel));
 }
 
+// Two FMAs in one instruction (sm_100).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{.reg .b64 ra, rb, rc, rd;\n\t"
+      "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%6, %7};\n\t"
+      "fma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
 // One warp's share of n rays.  source(item, ray) fills the ray of an item and returns false when the
 // item needs no query (its sink is not called); sink(item, ray, hit) takes the result.  `rpw` rays are
 // in flight per warp: fewer than 32 when the batch is too small to give every resident warp 32, since
@@ -94,6 +105,15 @@ template <bool kAcc, int kKind, class Scenes, class Source, class Sink>
 __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uint32_t* smem, uint32_t n,
                                        unsigned int* work, int rpw, uint32_t& status, Source&& source, Sink&& sink) {
   constexpr bool kMany = std::is_same_v<Scenes, ManyScenes8>;
+  // order[sign bits << 8 | child mask]: the mask's first slot in the direction's visiting order
+  __shared__ uint8_t order[2048];
+  for (uint32_t k = threadIdx.x; k < 2048u; k += blockDim.x) {
+    uint32_t s = 0u;
+    for (uint32_t b = 8u; b-- > 0u;)
+      if ((k >> (b ^ (k >> 8))) & 1u) s = b ^ (k >> 8);
+    order[k] = (uint8_t)s;
+  }
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   uint32_t* stack = smem + lane;  // entry k at stack[32 k]: conflict-free whatever the lanes' depths
@@ -246,6 +266,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
   };
 
   while (true) {
+    if (status) mask = 0u, sp = 0;  // (raised below: the lane gives its ray up)
     const unsigned busy = __ballot_sync(kFull, active && (mask != 0u || sp != 0));
     const int free_lanes = __popc(used & ~busy);
     if (busy == 0u || (more && free_lanes >= refill)) {
@@ -268,9 +289,9 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
           if (item < n && source(item, ray)) {
             active = true;
             inv = safe_inv(ray.d);
-            neg = (inv.x < 0.f ? 1u : 0u) | (inv.y < 0.f ? 2u : 0u) | (inv.z < 0.f ? 4u : 0u);
+            neg = (inv.x < 0.f ? 0x100u : 0u) | (inv.y < 0.f ? 0x200u : 0u) | (inv.z < 0.f ? 0x400u : 0u);
             node = 0u;
-            mask = 1u << neg;  // slot 0 of node 0: the root
+            mask = 1u;  // slot 0 of node 0: the root
             sp = 0;
             t_hi = kKind == kScatter8 ? ray.t : kInf;
             arg = kNoGauss;
@@ -309,9 +330,9 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
         node = e >> 8;
         mask = e & 0xFFu;
       }
-      const uint32_t b = (uint32_t)__ffs(mask) - 1u;
-      mask &= mask - 1u;
-      const uint32_t cur = __ldg(nodes + (size_t)node * kNode8Words + 16u + (b ^ neg));
+      const uint32_t slot = order[neg | mask];
+      mask &= ~(1u << slot);
+      const uint32_t cur = __ldg(nodes + (size_t)node * kNode8Words + 16u + slot);
       if (mask != 0u) {
         if ((uint32_t)sp >= depth) {  // cannot happen for a tree of the recorded depth
           status |= kStatusStackOverflow;
@@ -329,46 +350,65 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
       const float az = __uint_as_float((ew & 0xFF0000u) << 7) * inv.z;
       const float bx = fmaf(h.x - ray.o.x, inv.x, -ax), by = fmaf(h.y - ray.o.y, inv.y, -ay),
                   bz = fmaf(h.z - ray.o.z, inv.z, -az);
-      const bool nx = neg & 1u, ny = neg & 2u, nz = neg & 4u;
+      const bool nx = inv.x < 0.f, ny = inv.y < 0.f, nz = inv.z < 0.f;
       // near / far planes by the direction's signs: (lo.x, hi.x) = (a.xy, bq.zw), (lo.y, hi.y) = (a.zw, c.xy),
       // (lo.z, hi.z) = (bq.xy, c.zw)
       const uint32_t nxw[2] = {nx ? bq.z : a.x, nx ? bq.w : a.y}, fxw[2] = {nx ? a.x : bq.z, nx ? a.y : bq.w};
       const uint32_t nyw[2] = {ny ? c.x : a.z, ny ? c.y : a.w}, fyw[2] = {ny ? a.z : c.x, ny ? a.w : c.y};
       const uint32_t nzw[2] = {nz ? c.z : bq.x, nz ? c.w : bq.y}, fzw[2] = {nz ? bq.x : c.z, nz ? bq.y : c.w};
-      const float lo_t = kKind == kScatter8 ? ray.t : 0.0f;
-      uint32_t hits = 0u;
+      // child j is missed when far - near is negative: the signs are shifted into a mask, child 0's last
+      uint32_t miss = 0u;
+      const float2 a2x = make_float2(ax, ax), a2y = make_float2(ay, ay), a2z = make_float2(az, az);
+      const float2 b2x = make_float2(bx, bx), b2y = make_float2(by, by), b2z = make_float2(bz, bz);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const uint32_t sel = 0x7604u | ((uint32_t)(j & 3) << 4);
-        const float tn = fmax3f(fmaf(byte_plane(nxw[j >> 2], sel), ax, bx), fmaf(byte_plane(nyw[j >> 2], sel), ay, by),
-                                fmaxf(fmaf(byte_plane(nzw[j >> 2], sel), az, bz), lo_t));
-        const float tf = fmin3f(fmaf(byte_plane(fxw[j >> 2], sel), ax, bx), fmaf(byte_plane(fyw[j >> 2], sel), ay, by),
-                                fminf(fmaf(byte_plane(fzw[j >> 2], sel), az, bz), t_hi));
-        if (tn <= tf) hits |= 1u << j;
+      for (int j = 6; j >= 0; j -= 2) {  // two children at a time: packed FMAs
+        const uint32_t s0 = 0x7604u | ((uint32_t)(j & 3) << 4), s1 = 0x7604u | ((uint32_t)((j + 1) & 3) << 4);
+        const int w = j >> 2;
+        auto plane2 = [&](uint32_t word, float2 A, float2 B) {
+          return fma2(make_float2(byte_plane(word, s0), byte_plane(word, s1)), A, B);
+        };
+        const float2 nx2 = plane2(nxw[w], a2x, b2x), ny2 = plane2(nyw[w], a2y, b2y), nz2 = plane2(nzw[w], a2z, b2z);
+        const float2 fx2 = plane2(fxw[w], a2x, b2x), fy2 = plane2(fyw[w], a2y, b2y);
+        float2 fz2 = plane2(fzw[w], a2z, b2z);
+        const float t0 = kKind == kScatter8 ? ray.t : 0.0f;
+        if constexpr (kKind != kTau8) fz2 = make_float2(fminf(fz2.x, t_hi), fminf(fz2.y, t_hi));  // a transmittance query has no far end
+        const float d1 = fmin3f(fx2.y, fy2.y, fz2.y) - fmax3f(nx2.y, ny2.y, fmaxf(nz2.y, t0));
+        const float d0 = fmin3f(fx2.x, fy2.x, fz2.x) - fmax3f(nx2.x, ny2.x, fmaxf(nz2.x, t0));
+        miss = __funnelshift_l(__float_as_uint(d1), miss, 1);
+        miss = __funnelshift_l(__float_as_uint(d0), miss, 1);
       }
-      // slots -> visiting order (bit s moves to bit s ^ neg)
-      uint32_t im = ((ew >> 24) << 8) | hits;
-      if (nx) im = ((im & 0x5555u) << 1) | ((im >> 1) & 0x5555u);
-      if (ny) im = ((im & 0x3333u) << 2) | ((im >> 2) & 0x3333u);
-      if (nz) im = ((im & 0x0F0Fu) << 4) | ((im >> 4) & 0x0F0Fu);
-      const uint32_t inner = im >> 8, ph = im & 0xFFu;
+      const uint32_t hits = ~miss & 0xFFu, inner = ew >> 24;
       node = cur;
-      mask = ph & inner;
-      leaf = ph & ~inner;
+      mask = hits & inner;
+      leaf = hits & ~inner;
     }
-    // hit Gaussians to queue 1
-    unsigned bal;
-    while ((bal = __ballot_sync(kFull, leaf != 0u)) != 0u) {
+    // hit Gaussians to queue 1: a vote per round, or (faster for transmittance, whose rays meet more of them;
+    // 33.3 / 34.9 ms of the showcase, but 19.9 / 19.2 for the argmin) one shared-memory atomic per lane
+    if constexpr (kKind == kTau8) {
+      if (lane == 0) own[0] = (uint32_t)q1n;
+      __syncwarp();
       if (leaf != 0u) {
-        const uint32_t b = (uint32_t)__ffs(leaf) - 1u;
-        leaf &= leaf - 1u;
-        q1[q1n + __popc(bal & lt)] = ((uint32_t)lane << 27) | (node << 3) | (b ^ neg);
+        uint32_t at = atomicAdd(own, (uint32_t)__popc(leaf));
+        do {
+          q1[at++] = ((uint32_t)lane << 27) | (node << 3) | ((uint32_t)__ffs(leaf) - 1u);
+          leaf &= leaf - 1u;
+        } while (leaf != 0u);
       }
-      q1n += __popc(bal);
+      __syncwarp();
+      q1n = (int)own[0];
+    } else {
+      unsigned bal;
+      while ((bal = __ballot_sync(kFull, leaf != 0u)) != 0u) {
+        if (leaf != 0u) {
+          const uint32_t b = (uint32_t)__ffs(leaf) - 1u;
+          leaf &= leaf - 1u;
+          q1[q1n + __popc(bal & lt)] = ((uint32_t)lane << 27) | (node << 3) | b;
+        }
+        q1n += __popc(bal);
+      }
     }
     __syncwarp();
     while (q1n >= 32) chords(32);
-    if (__any_sync(kFull, status != 0u)) break;
   }
 }
 

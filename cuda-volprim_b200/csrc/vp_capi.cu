@@ -39,6 +39,15 @@ vp_status cuda_fail(cudaError_t e, const char* what) {
   return e == cudaErrorMemoryAllocation ? VP_ERROR_OUT_OF_MEMORY : VP_ERROR_CUDA;
 }
 
+vp_status clear_counters(vp_context* ctx) {
+  VP_CUDA(cudaMemsetAsync(ctx->counters, 0, kCountersBytes + sizeof(unsigned int), ctx->stream));
+  return VP_OK;
+}
+vp_status fetch_counters(vp_context* ctx) {
+  VP_CUDA(cudaMemcpyAsync(ctx->host_counters, ctx->counters, sizeof(Counters), cudaMemcpyDeviceToHost, ctx->stream));
+  return VP_OK;
+}
+
 // ---- host float3 arithmetic in the reference's operation order (math.h) --------------------
 namespace hm {
 struct V {
@@ -228,8 +237,11 @@ vp_status vp_context_create(int32_t device, vp_context** out) {
   }
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&c->ev1);
-  if (e == cudaSuccess) e = cudaMalloc(&c->counters, sizeof(Counters));
-  if (e == cudaSuccess) e = cudaMalloc(&c->work_counter, sizeof(unsigned int));
+  if (e == cudaSuccess) e = cudaMalloc(&c->counters, kCountersBytes + 16);
+  if (e == cudaSuccess) {
+    c->work_counter = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(c->counters) + kCountersBytes);
+    e = cudaMallocHost(&c->host_counters, sizeof(Counters));
+  }
   if (e != cudaSuccess) {
     vp_context_destroy(c);
     return cuda_fail(e, "vp_context_create");
@@ -243,7 +255,7 @@ vp_status vp_context_destroy(vp_context* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->counters) cudaFree(c->counters);
-  if (c->work_counter) cudaFree(c->work_counter);
+  if (c->host_counters) cudaFreeHost(c->host_counters);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   for (cudaEvent_t ev : c->stage_ev)
@@ -569,7 +581,7 @@ vp_status vp_render_accumulate(vp_scene* s, vp_env* e, const vp_camera* cam, con
   ctx->time_stages = (p->measure & VP_MEASURE_STAGES) != 0;
   ctx->stage_ms[0] = ctx->stage_ms[1] = 0.0;
   ctx->stage_launches[0] = ctx->stage_launches[1] = 0;
-  VP_CUDA(cudaMemsetAsync(ctx->counters, 0, sizeof(Counters), ctx->stream));
+  if ((st = clear_counters(ctx))) return st;
   VP_CUDA(cudaEventRecord(ctx->ev0, ctx->stream));
   const uint32_t batch = p->batch_spp ? p->batch_spp : spp_count;
   for (uint32_t off = 0; off < spp_count; off += batch) {
@@ -581,9 +593,9 @@ vp_status vp_render_accumulate(vp_scene* s, vp_env* e, const vp_camera* cam, con
     }
   }
   VP_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
-  VP_CUDA(cudaEventSynchronize(ctx->ev1));
-  Counters c{};
-  VP_CUDA(cudaMemcpy(&c, ctx->counters, sizeof(c), cudaMemcpyDeviceToHost));
+  if ((st = fetch_counters(ctx))) return st;
+  VP_CUDA(cudaStreamSynchronize(ctx->stream));
+  const Counters& c = *ctx->host_counters;
   if (stats) {
     float ms = 0.f;
     VP_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
@@ -649,8 +661,8 @@ vp_status vp_transmittance(vp_scene* s, const float* origins, const float* dirs,
   VP_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
   const bool accurate = precision == VP_PRECISION_ACCURATE || (precision == VP_PRECISION_AUTO && s->view.albedo_all_zero);
-  VP_CUDA(cudaMemsetAsync(ctx->counters, 0, sizeof(Counters), st));
   vp_status r;
+  if ((r = clear_counters(ctx))) return r;
   if (memory == VP_MEMORY_DEVICE) {
     if ((r = launch_transmittance(s, origins, dirs, n, accurate, engine, out))) return r;
   } else if (memory == VP_MEMORY_HOST) {
@@ -673,9 +685,9 @@ vp_status vp_transmittance(vp_scene* s, const float* origins, const float* dirs,
   } else {
     return fail(VP_ERROR_INVALID_ARGUMENT, "bad memory kind");
   }
+  if ((r = fetch_counters(ctx))) return r;
   VP_CUDA(cudaStreamSynchronize(st));
-  Counters c{};
-  VP_CUDA(cudaMemcpy(&c, ctx->counters, sizeof(c), cudaMemcpyDeviceToHost));
+  const Counters& c = *ctx->host_counters;
   if (c.status) return fail(VP_ERROR_DEVICE_STATUS, "transmittance kernel raised device status " + std::to_string(c.status));
   return VP_OK;
 }
@@ -736,8 +748,8 @@ vp_status vp_albedo_at(vp_scene* s, const float* points, uint32_t n, int32_t pre
   VP_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
   const bool accurate = precision == VP_PRECISION_ACCURATE || (precision == VP_PRECISION_AUTO && s->view.albedo_all_zero);
-  VP_CUDA(cudaMemsetAsync(ctx->counters, 0, sizeof(Counters), st));
-  vp_status r = VP_OK;
+  vp_status r;
+  if ((r = clear_counters(ctx))) return r;
   if (memory == VP_MEMORY_DEVICE) {
     if ((r = launch_albedo(s, points, n, accurate, engine, out_rgb, out_overlap))) return r;
   } else if (memory == VP_MEMORY_HOST) {
@@ -761,9 +773,9 @@ vp_status vp_albedo_at(vp_scene* s, const float* points, uint32_t n, int32_t pre
   } else {
     return fail(VP_ERROR_INVALID_ARGUMENT, "bad memory kind");
   }
+  if ((r = fetch_counters(ctx))) return r;
   VP_CUDA(cudaStreamSynchronize(st));
-  Counters c{};
-  VP_CUDA(cudaMemcpy(&c, ctx->counters, sizeof(c), cudaMemcpyDeviceToHost));
+  const Counters& c = *ctx->host_counters;
   if (c.status) return fail(VP_ERROR_DEVICE_STATUS, "albedo kernel raised device status " + std::to_string(c.status));
   return VP_OK;
 }

@@ -735,9 +735,10 @@ vp_status prepare(vp_scene* s, vp_env* e, const vp_camera* cam, const vp_render_
 
 vp_status finish_stats(vp_context* ctx, const vp_render_params* p, uint32_t launches, vp_render_stats* stats) {
   VP_CUDA(cudaEventRecord(ctx->ev1, ctx->stream));
-  VP_CUDA(cudaEventSynchronize(ctx->ev1));
-  Counters c{};
-  VP_CUDA(cudaMemcpy(&c, ctx->counters, sizeof(c), cudaMemcpyDeviceToHost));
+  vp_status r;
+  if ((r = fetch_counters(ctx))) return r;
+  VP_CUDA(cudaStreamSynchronize(ctx->stream));
+  const Counters& c = *ctx->host_counters;
   if (stats) {
     float ms = 0.f;
     VP_CUDA(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
@@ -800,8 +801,7 @@ vp_status vp_render_emission(vp_scene* s, vp_env* e, const vp_camera* cam, const
     if ((r = dev_alloc(&tmp, n_pix, st))) return r;
     out = tmp;
   }
-  VP_CUDA(cudaMemsetAsync(ctx->counters, 0, sizeof(Counters), st));
-  VP_CUDA(cudaMemsetAsync(ctx->work_counter, 0, sizeof(unsigned int), st));
+  if ((r = clear_counters(ctx))) return r;
   VP_CUDA(cudaEventRecord(ctx->ev0, st));
   const vp_status lr = with_group(c.tiles.tiles, s->view.stack_cap, [&](auto group) -> vp_status {
     constexpr int G = decltype(group)::value;
@@ -871,8 +871,7 @@ vp_status vp_render_emission_backward(vp_scene* s, vp_env* e, const vp_camera* c
     ge = grads->emission ? gout + 11ull * n : nullptr;
   }
   VP_CUDA(cudaMemsetAsync(acc, 0, 64ull * n, st));
-  VP_CUDA(cudaMemsetAsync(ctx->counters, 0, sizeof(Counters), st));
-  VP_CUDA(cudaMemsetAsync(ctx->work_counter, 0, sizeof(unsigned int), st));
+  if ((r = clear_counters(ctx))) return cleanup(), r;
   VP_CUDA(cudaEventRecord(ctx->ev0, st));
   const vp_status lr = with_group(c.tiles.tiles, s->view.stack_cap, [&](auto group) -> vp_status {
     constexpr int G = decltype(group)::value;

@@ -205,7 +205,7 @@ __global__ void k_albedo_thread(SceneView S, const float* __restrict__ pts, uint
   if (status) atomicOr(&ctr->status, status);
 }
 
-// The same query, thread per ray (vp_trace8.cuh), for batches of at least kTrace8Min rays.
+// The same query, thread per ray (vp_trace8.cuh); k_tau_warp serves scenes too deep for the 8-wide BVH.
 template <bool kAcc>
 __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_tau8(SceneView S, const float* __restrict__ org,
                                                                const float* __restrict__ dir, uint32_t n,
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_tau8(SceneView S, con
   uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(S.depth8);
   uint32_t status = 0;
   trace8<kAcc, kTau8>(
-      OneScene8{scene8_of(S)}, S.depth8, smem, n, work, rays_per_warp(n), status,
+      OneScene8{scene8_of(S)}, S.depth8, smem, stage_order8(), n, work, grid_warps(), rays_per_warp(n, grid_warps()), status,
       [&](uint32_t i, Ray8& ray) {
         ray.o = f3(org[3 * i], org[3 * i + 1], org[3 * i + 2]);
         ray.d = f3(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
@@ -279,22 +279,21 @@ vp_status launch_render(vp_scene* s, vp_env* e, const CameraView& cam, const Par
   return VP_OK;
 }
 
+// (The caller has cleared the counters and the work-queue head.)
 vp_status launch_transmittance(vp_scene* s, const float* o, const float* d, uint32_t n, bool accurate,
                                int32_t engine, float* out) {
   vp_context* ctx = s->ctx;
   cudaStream_t st = ctx->stream;
   if (n == 0) return VP_OK;
-  if (engine == VP_ENGINE_WARP && s->view.depth8 != 0u && n >= kTrace8Min) {
+  if (engine == VP_ENGINE_WARP && s->view.depth8 != 0u) {
     auto kern = accurate ? k_tau8<true> : k_tau8<false>;
     const size_t smem = trace8_smem_bytes(s->view.depth8, kT8Threads);
-    VP_CUDA(cudaMemsetAsync(ctx->work_counter, 0, sizeof(unsigned int), st));
     if (smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int blocks = ctx->sm_count * occupancy_blocks(kern, kT8Threads, smem);
     kern<<<blocks, kT8Threads, smem, st>>>(s->view, o, d, n, out, ctx->work_counter, ctx->counters);
   } else if (engine == VP_ENGINE_WARP) {
     const int threads = 256;
     const size_t smem = (size_t)(threads / 32) * warp_smem_bytes(s->view.stack_cap, 32);
-    VP_CUDA(cudaMemsetAsync(ctx->work_counter, 0, sizeof(unsigned int), st));
     if (accurate) {
       if (smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(k_tau_warp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       const int blocks = ctx->sm_count * occupancy_blocks(k_tau_warp<true>, threads, smem);
@@ -322,7 +321,6 @@ vp_status launch_albedo(vp_scene* s, const float* pts, uint32_t n, bool accurate
   if (engine == VP_ENGINE_WARP) {
     const int threads = 256;
     const size_t smem = (size_t)(threads / 32) * warp_smem_bytes(s->view.stack_cap, 32);
-    VP_CUDA(cudaMemsetAsync(ctx->work_counter, 0, sizeof(unsigned int), st));
     if (accurate) {
       if (smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(k_albedo_warp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       const int blocks = ctx->sm_count * occupancy_blocks(k_albedo_warp<true>, threads, smem);

@@ -7,10 +7,10 @@
 //                                requests that still have unstarted paths (the schedule)
 //   regen    (thread per path)   new paths: owning request from the share prefix sums, camera
 //                                ray, PCG32 stream, first free-flight key -- appended to the queue
-//   extend   (warp per path)     free-flight argmin + scatter albedo on the path's own scene; from
-//                                kTrace8Min paths on in thread-per-ray form (vp_trace8.cuh)
+//   extend   (thread per path)   free-flight argmin + scatter albedo on the path's own scene (vp_trace8.cuh;
+//                                warp per path over the BVH32 when some scene is too deep for the 8-wide one)
 //   shade    (thread per path)   phase / NEE / roulette with the request's own controls
-//   shadow   (warp per query)    transmittance on the query's scene; thread-per-ray likewise
+//   shadow   (thread per query)  transmittance on the query's scene, likewise
 //   gather   (thread per path)   radiance += weight x T; a finished path adds its sample to its
 //                                request's pixel sum, counts itself done and frees its slot
 // so paths of different requests, scenes, resolutions and sample counts share every launch, and
@@ -66,7 +66,7 @@ struct SrvCtl {  // device control block of the iteration
   uint32_t regen_m;     // paths started by the current iteration
   uint32_t regen_from;  // free-stack index of the first slot they take
   uint32_t survivors;   // paths carried over from the previous iteration
-  uint32_t ctr[8];      // [0] paths this iteration, [1] next, [2] shadow queries, [3..5] work heads
+  uint32_t ctr[8];      // [0] paths this iteration, [1] next, [2] shadow queries, [3..4] work heads
   unsigned long long total_started;  // paths the lane has started (the clock of SRPT aging)
 };
 
@@ -266,7 +266,7 @@ __global__ void k_srv_advance(SrvCtl* c, const SrvRequest* __restrict__ table, u
     c->regen_from = F - m;
     c->free_count = F - m;
     c->ctr[0] = s_surv + m;
-    c->ctr[1] = c->ctr[2] = c->ctr[3] = c->ctr[4] = c->ctr[5] = 0u;
+    c->ctr[1] = c->ctr[2] = c->ctr[3] = c->ctr[4] = 0u;
     c->total_started += m;
   }
 }
@@ -304,12 +304,11 @@ template <bool kAcc>
 __global__ void __launch_bounds__(256, 4) k_srv_extend(const SceneView* __restrict__ scenes,
                                                        const SrvRequest* __restrict__ table, SrvPaths b,
                                                        const uint32_t* __restrict__ q, SrvCtl* c, uint32_t max_cap,
-                                                       uint32_t below, Counters* ctr) {
+                                                       Counters* ctr) {
   extern __shared__ unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const WarpSmem W = carve(smem + warp * warp_smem_bytes(max_cap, kSrvHitCap), max_cap, kSrvHitCap);
   const uint32_t n = c->ctr[0];
-  if (n >= below) return;  // k_srv_extend8 takes the iteration
   uint32_t status = 0;
   WarpStats ws;
   while (true) {
@@ -344,8 +343,7 @@ __global__ void __launch_bounds__(256, 4) k_srv_extend(const SceneView* __restri
   if (lane == 0 && status) atomicOr(&ctr->status, status);
 }
 
-// ---- thread-per-ray forms of extend and shadow, in every iteration's launches beside the others: which of
-// the two runs is decided by the iteration's count on the device ----
+// ---- thread-per-ray forms of extend and shadow ----
 // Shared memory after the warps' own: what the queries read of each resident scene.
 __device__ __forceinline__ ManyScenes8 stage_scenes(const SceneView* __restrict__ scenes, uint32_t n_scenes, uint32_t depth) {
   Scene8* t = reinterpret_cast<Scene8*>(vp_dyn_smem + trace8_smem_bytes(depth, kT8Threads));
@@ -354,18 +352,17 @@ __device__ __forceinline__ ManyScenes8 stage_scenes(const SceneView* __restrict_
   return ManyScenes8{t};
 }
 
-template <bool kAcc>
-__global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_srv_extend8(const SceneView* __restrict__ scenes, uint32_t n_scenes,
+// kMixed: some resident scene's Gaussians differ in albedo.
+template <bool kAcc, bool kMixed>
+__global__ void __launch_bounds__(kT8Threads, kMixed ? 2 : kT8Blocks) k_srv_extend8(const SceneView* __restrict__ scenes, uint32_t n_scenes,
                                                                       const SrvRequest* __restrict__ table, SrvPaths b,
                                                                       const uint32_t* __restrict__ q, SrvCtl* c,
                                                                       uint32_t depth, Counters* ctr) {
-  const uint32_t n = c->ctr[0];
-  if (n < kTrace8Min) return;
   const ManyScenes8 many = stage_scenes(scenes, n_scenes, depth);
   uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(depth);
   uint32_t status = 0;
-  trace8<kAcc, kFlight8>(
-      many, depth, smem, n, &c->ctr[3], rays_per_warp(n), status,
+  extend8<kAcc, kMixed>(
+      many, depth, smem, c->ctr[0], &c->ctr[3], status,
       [&](uint32_t item, Ray8& ray) {
         const uint32_t p = __ldg(q + item);
         ray.scene = table[b.req[p]].scene;
@@ -385,27 +382,10 @@ __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_srv_extend8(const Sce
       },
       [&](uint32_t item, const Ray8& ray, const Hit8& h) {
         const uint32_t p = __ldg(q + item);
-        // k_srv_scatter8 replaces the albedo where the scene's Gaussians differ in it
         const float3 a = h.t < kInf ? scenes[ray.scene].albedo : f3(0.f, 0.f, 0.f);
         b.alb4[p] = make_float4(a.x, a.y, a.z, h.t);
         b.sg[p] = h.gauss;
-      });
-  if (status) atomicOr(&ctr->status, status);
-}
-
-// Launched when some resident scene's Gaussians differ in albedo.
-template <bool kAcc>
-__global__ void __launch_bounds__(kT8Threads) k_srv_scatter8(const SceneView* __restrict__ scenes, uint32_t n_scenes,
-                                                            const SrvRequest* __restrict__ table, SrvPaths b,
-                                                            const uint32_t* __restrict__ q, SrvCtl* c, uint32_t depth,
-                                                            Counters* ctr) {
-  const uint32_t n = c->ctr[0];
-  if (n < kTrace8Min) return;
-  const ManyScenes8 many = stage_scenes(scenes, n_scenes, depth);
-  uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(depth);
-  uint32_t status = 0;
-  trace8<kAcc, kScatter8>(
-      many, depth, smem, n, &c->ctr[5], rays_per_warp(n), status,
+      },
       [&](uint32_t item, Ray8& ray) {
         const uint32_t p = __ldg(q + item);
         ray.scene = table[b.req[p]].scene;
@@ -416,10 +396,7 @@ __global__ void __launch_bounds__(kT8Threads) k_srv_scatter8(const SceneView* __
         ray.d = f3(d.x, d.y, d.z);
         return true;
       },
-      [&](uint32_t item, const Ray8& ray, const Hit8& h) {
-        const float3 a = mean_albedo(h.w, h.r, h.g, h.b);
-        b.alb4[__ldg(q + item)] = make_float4(a.x, a.y, a.z, ray.t);
-      });
+      [&](uint32_t item, const Ray8& ray, float3 a) { b.alb4[__ldg(q + item)] = make_float4(a.x, a.y, a.z, ray.t); });
   if (status) atomicOr(&ctr->status, status);
 }
 
@@ -428,12 +405,11 @@ __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_srv_shadow8(const Sce
                                                                       const SrvRequest* __restrict__ table, SrvPaths b,
                                                                       SrvCtl* c, uint32_t depth, Counters* ctr) {
   const uint32_t n = c->ctr[2];
-  if (n < kTrace8Min) return;
   const ManyScenes8 many = stage_scenes(scenes, n_scenes, depth);
   uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(depth);
   uint32_t status = 0;
   trace8<kAcc, kTau8>(
-      many, depth, smem, n, &c->ctr[4], rays_per_warp(n), status,
+      many, depth, smem, stage_order8(), n, &c->ctr[4], grid_warps(), rays_per_warp(n, grid_warps()), status,
       [&](uint32_t item, Ray8& ray) {
         const uint32_t slot = __ldg(b.qs + item);
         ray.scene = table[b.req[slot / 3u]].scene;
@@ -505,12 +481,11 @@ __global__ void __launch_bounds__(256) k_srv_shade(const SceneView* __restrict__
 template <bool kAcc>
 __global__ void __launch_bounds__(256, 4) k_srv_shadow(const SceneView* __restrict__ scenes,
                                                        const SrvRequest* __restrict__ table, SrvPaths b, SrvCtl* c,
-                                                       uint32_t max_cap, uint32_t below, Counters* ctr) {
+                                                       uint32_t max_cap, Counters* ctr) {
   extern __shared__ unsigned char smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const WarpSmem W = carve(smem + warp * warp_smem_bytes(max_cap, 32), max_cap, 32);
   const uint32_t n = c->ctr[2];
-  if (n >= below) return;  // k_srv_shadow8 takes the iteration
   uint32_t status = 0;
   WarpStats ws;
   while (true) {
@@ -603,7 +578,7 @@ struct vp_server {
   SrvRequest* h_table = nullptr;
   uint32_t max_depth8 = 0;      // deepest BVH8 over the scenes, 0 when some scene has none
   bool mixed_albedo = false;    // some scene's Gaussians differ in albedo
-  int ext8_blocks = 0, sca8_blocks = 0, shd8_blocks = 0;
+  int ext8_blocks = 0, shd8_blocks = 0;
   size_t smem8 = 0;
   int ext_blocks = 0, shd_blocks = 0, thr_blocks = 0;
   size_t smem_ext = 0, smem_shd = 0;
@@ -732,6 +707,11 @@ void srv_free(vp_server* s) {
   delete s;
 }
 
+auto extend8_kernel(const vp_server* s) {
+  return s->accurate ? (s->mixed_albedo ? k_srv_extend8<true, true> : k_srv_extend8<true, false>)
+                     : (s->mixed_albedo ? k_srv_extend8<false, true> : k_srv_extend8<false, false>);
+}
+
 // One wavefront iteration of lane l with the queues in the given roles.
 vp_status enqueue_iteration(vp_server* s, uint32_t l, bool even) {
   vp_server::Lane& L = s->lanes[l];
@@ -743,30 +723,24 @@ vp_status enqueue_iteration(vp_server* s, uint32_t l, bool even) {
   k_srv_advance<<<1, R, 0, st>>>(L.d_ctl, s->d_table, s->d_started, s->d_age_base, L.d_alloc_off,
                                  L.d_alloc_start, s->cfg.schedule, s->cfg.srpt_reserve, s->cfg.srpt_aging, l, nl);
   k_srv_regen<<<s->thr_blocks, 256, 0, st>>>(L.d_ctl, s->d_table, L.d_alloc_off, L.d_alloc_start, R, L.paths, qcur);
-  // an iteration of at least kTrace8Min paths (or shadow queries) takes the thread-per-ray form
-  const uint32_t below = s->max_depth8 ? kTrace8Min : 0xFFFFFFFFu;
   const uint32_t n_scenes = (uint32_t)s->scenes.size();
-  auto ext = s->accurate ? k_srv_extend<true> : k_srv_extend<false>;
-  auto shd = s->accurate ? k_srv_shadow<true> : k_srv_shadow<false>;
-  auto ext8 = s->accurate ? k_srv_extend8<true> : k_srv_extend8<false>;
-  auto sca8 = s->accurate ? k_srv_scatter8<true> : k_srv_scatter8<false>;
-  auto shd8 = s->accurate ? k_srv_shadow8<true> : k_srv_shadow8<false>;
-  const bool both = s->max_depth8 && L.slots >= kTrace8Min;  // (a smaller pool never reaches the count)
-  ext<<<s->ext_blocks, 256, s->smem_ext, st>>>(s->d_scenes, s->d_table, L.paths, qcur, L.d_ctl, s->max_argmin_cap,
-                                              below, ctr);
-  if (both) {
+  if (s->max_depth8) {
+    auto ext8 = extend8_kernel(s);
     ext8<<<s->ext8_blocks, kT8Threads, s->smem8, st>>>(s->d_scenes, n_scenes, s->d_table, L.paths, qcur, L.d_ctl,
                                                       s->max_depth8, ctr);
-    if (s->mixed_albedo)
-      sca8<<<s->sca8_blocks, kT8Threads, s->smem8, st>>>(s->d_scenes, n_scenes, s->d_table, L.paths, qcur, L.d_ctl,
-                                                        s->max_depth8, ctr);
+  } else {
+    auto ext = s->accurate ? k_srv_extend<true> : k_srv_extend<false>;
+    ext<<<s->ext_blocks, 256, s->smem_ext, st>>>(s->d_scenes, s->d_table, L.paths, qcur, L.d_ctl, s->max_argmin_cap, ctr);
   }
   k_srv_shade<<<s->thr_blocks, 256, 0, st>>>(s->d_scenes, s->d_envs, s->d_table, L.paths, qcur, L.d_ctl, qnext);
-  shd<<<s->shd_blocks, 256, s->smem_shd, st>>>(s->d_scenes, s->d_table, L.paths, L.d_ctl, s->max_cap, below, ctr);
-  // (three shadow queries a path at most)
-  if (s->max_depth8 && 3ull * L.slots >= kTrace8Min)
+  if (s->max_depth8) {
+    auto shd8 = s->accurate ? k_srv_shadow8<true> : k_srv_shadow8<false>;
     shd8<<<s->shd8_blocks, kT8Threads, s->smem8, st>>>(s->d_scenes, n_scenes, s->d_table, L.paths, L.d_ctl,
                                                       s->max_depth8, ctr);
+  } else {
+    auto shd = s->accurate ? k_srv_shadow<true> : k_srv_shadow<false>;
+    shd<<<s->shd_blocks, 256, s->smem_shd, st>>>(s->d_scenes, s->d_table, L.paths, L.d_ctl, s->max_cap, ctr);
+  }
   k_srv_gather<<<s->thr_blocks, 256, 0, st>>>(s->d_table, L.paths, qcur, L.d_ctl, s->d_done);
   VP_CUDA(cudaGetLastError());
   return VP_OK;
@@ -791,14 +765,12 @@ vp_status prepare_launch(vp_server* s) {
   if (!can8) s->max_depth8 = 0;
   if (s->max_depth8) {
     s->smem8 = trace8_smem_bytes(s->max_depth8, kT8Threads) + s->scenes.size() * sizeof(Scene8);
-    auto ext8 = s->accurate ? k_srv_extend8<true> : k_srv_extend8<false>;
-    auto sca8 = s->accurate ? k_srv_scatter8<true> : k_srv_scatter8<false>;
+    auto ext8 = extend8_kernel(s);
     auto shd8 = s->accurate ? k_srv_shadow8<true> : k_srv_shadow8<false>;
     if (s->smem8 > 48 * 1024)
-      for (auto k : {(const void*)ext8, (const void*)sca8, (const void*)shd8})
+      for (auto k : {(const void*)ext8, (const void*)shd8})
         VP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem8));
     s->ext8_blocks = ctx->sm_count * srv_blocks(ext8, kT8Threads, s->smem8);
-    s->sca8_blocks = ctx->sm_count * srv_blocks(sca8, kT8Threads, s->smem8);
     s->shd8_blocks = ctx->sm_count * srv_blocks(shd8, kT8Threads, s->smem8);
   }
   s->smem_ext = (size_t)8 * warp_smem_bytes(s->max_argmin_cap, kSrvHitCap);

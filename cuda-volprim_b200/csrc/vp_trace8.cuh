@@ -1,5 +1,5 @@
 // Thread-per-ray queries over the compressed 8-wide BVH, with the per-Gaussian work of a warp's 32
-// rays pooled: the queries of the wavefront and serving engines and of large transmittance batches.
+// rays pooled: the queries of the wavefront and serving engines and of vp_transmittance.
 //
 // What bounds it, and why this split.  The warp-cooperative query (vp_traverse.cuh) spends 32 lanes
 // on one ray; its chord set-up runs with about two lanes busy.  Here a lane walks its own ray through
@@ -12,7 +12,12 @@
 //   value step  when queue 2 holds 32 chords, lane e evaluates the e-th (optical depth, free flight
 //               or albedo weight) and each owner collects its own by shuffles.
 // So box tests, chord set-ups and erf / erfinv evaluations each run with nearly full warps, whatever
-// the 32 rays do.  A warp refills its finished lanes together, after draining both queues.
+// the 32 rays do.  A warp refills its finished lanes together, after draining both queues; once there is
+// nothing left to fetch, its idle lanes take over subtrees of the rays still walking.  Without that, a batch
+// ended with its longest rays, whose lanes walked alone, and below some 115k rays a whole warp on each ray
+// was sooner done; with it this form is the faster one at every size measured (transmittance of 1k / 65k /
+// 250k rays through a 100k-Gaussian cloud: 0.08 / 0.14 / 0.26 ms, 0.10 / 0.29 / 0.39 without, 0.10 / 0.24 /
+// 0.63 with a warp on each ray; the 2M-Gaussian stress image 64 / 77 / 180 ms).
 //
 // Results do not depend on which rays share a warp or in which order chords are met: the argmin is a
 // minimum, and the sums (optical depth, albedo weights) are carried in FP64 and rounded once.
@@ -40,9 +45,9 @@ constexpr uint32_t kMaxDepth8 = 40;         // deeper trees take the warp-cooper
 constexpr int kValueStep = 8;
 constexpr int kQ1Cap = 32 + 256, kQ2Cap = 64, kQ2Words = 7;
 
-// Words of shared memory per warp: stack, queue 1, queue 2, owner masks.
+// Words of shared memory per warp: stack, queue 1, queue 2, owner masks, a work counter of its own.
 __host__ __device__ __forceinline__ uint32_t trace8_warp_words(uint32_t depth) {
-  return depth * 32u + kQ1Cap + kQ2Cap * kQ2Words + 32u;
+  return depth * 32u + kQ1Cap + kQ2Cap * kQ2Words + 33u;
 }
 __host__ __device__ __forceinline__ size_t trace8_smem_bytes(uint32_t depth, int threads) {
   return (size_t)trace8_warp_words(depth) * 4u * (size_t)(threads / 32);
@@ -86,6 +91,32 @@ __device__ __forceinline__ float byte_plane(uint32_t word, uint32_t sel) {  // 1
   return __uint_as_float(__byte_perm(word, 0x3F800000u, sel));
 }
 
+// order[sign bits << 8 | child mask]: the mask's first slot in the direction's visiting order.
+struct Order8 {
+  alignas(16) uint8_t slot[2048];
+};
+constexpr Order8 make_order8() {
+  Order8 t{};
+  for (uint32_t k = 0; k < 2048u; ++k) {
+    const uint32_t neg = k >> 8;
+    uint32_t s = 0u;
+    for (uint32_t b = 8u; b-- > 0u;)
+      if ((k >> (b ^ neg)) & 1u) s = b ^ neg;
+    t.slot[k] = (uint8_t)s;
+  }
+  return t;
+}
+static __device__ const Order8 g_order8 = make_order8();
+
+// The table in shared memory.  All threads of the block call it, before any of its trace8 calls.
+__device__ __forceinline__ const uint8_t* stage_order8() {
+  __shared__ Order8 order;
+  for (uint32_t k = threadIdx.x; k < sizeof(Order8) / 16u; k += blockDim.x)
+    reinterpret_cast<uint4*>(order.slot)[k] = reinterpret_cast<const uint4*>(g_order8.slot)[k];
+  __syncthreads();
+  return order.slot;
+}
+
 // Two FMAs in one instruction (sm_100).
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   float2 d;
@@ -97,23 +128,15 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return d;
 }
 
-// One warp's share of n rays.  source(item, ray) fills the ray of an item and returns false when the
+// One warp's share of n rays, handed out through *work to `warps` warps.  source(item, ray) fills the ray of an item and returns false when the
 // item needs no query (its sink is not called); sink(item, ray, hit) takes the result.  `rpw` rays are
 // in flight per warp: fewer than 32 when the batch is too small to give every resident warp 32, since
 // the chord and value steps use all lanes anyway.
 template <bool kAcc, int kKind, class Scenes, class Source, class Sink>
-__device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uint32_t* smem, uint32_t n,
-                                       unsigned int* work, int rpw, uint32_t& status, Source&& source, Sink&& sink) {
+__device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uint32_t* smem, const uint8_t* order,
+                                       uint32_t n, unsigned int* work, uint32_t warps, int rpw, uint32_t& status,
+                                       Source&& source, Sink&& sink) {
   constexpr bool kMany = std::is_same_v<Scenes, ManyScenes8>;
-  // order[sign bits << 8 | child mask]: the mask's first slot in the direction's visiting order
-  __shared__ uint8_t order[2048];
-  for (uint32_t k = threadIdx.x; k < 2048u; k += blockDim.x) {
-    uint32_t s = 0u;
-    for (uint32_t b = 8u; b-- > 0u;)
-      if ((k >> (b ^ (k >> 8))) & 1u) s = b ^ (k >> 8);
-    order[k] = (uint8_t)s;
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   uint32_t* stack = smem + lane;  // entry k at stack[32 k]: conflict-free whatever the lanes' depths
@@ -129,9 +152,10 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
   ray.scene = 0u;
   // the scene of another lane's ray
   auto scene_of = [&](int ow) { return scenes.of(kMany ? __shfl_sync(kFull, ray.scene, ow) : 0u); };
-  float3 inv = f3(0.f, 0.f, 0.f);
-  uint32_t item = 0, node = 0, mask = 0, neg = 0;
-  int sp = 0;
+  // what this lane walks: its own ray or, late in a batch, part of another lane's (owner)
+  float3 no = f3(0.f, 0.f, 0.f), inv = f3(0.f, 0.f, 0.f);
+  uint32_t item = 0, node = 0, mask = 0, neg = 0, walk_scene = 0;
+  int sp = 0, sb = 0, owner = lane;  // its stack entries are [sb, sp)
   bool active = false, more = true;
   float t_hi = kInf;
   uint32_t arg = kNoGauss, cnt = 0;
@@ -209,10 +233,6 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
       m &= m - 1u;
     }
     __syncwarp();
-    if (kKind == kTau8 && acc >= (double)kMaxOpticalDepth) {  // opaque: the rest of its nodes cannot matter
-      mask = 0u;
-      sp = 0;
-    }
   };
 
   // chord step over the top k entries of queue 1
@@ -266,13 +286,19 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
   };
 
   while (true) {
-    if (status) mask = 0u, sp = 0;  // (raised below: the lane gives its ray up)
-    const unsigned busy = __ballot_sync(kFull, active && (mask != 0u || sp != 0));
+    if (status) mask = 0u, sp = sb;  // (raised below: the lane gives its ray up)
+    if constexpr (kKind == kTau8) {  // opaque: the rest of the ray's nodes cannot matter
+      const bool opaque = acc >= (double)kMaxOpticalDepth;
+      if (__any_sync(kFull, opaque)) {
+        if (__shfl_sync(kFull, (int)opaque, owner)) mask = 0u, sp = sb;
+      }
+    }
+    unsigned busy = __ballot_sync(kFull, mask != 0u || sp != sb);
     const int free_lanes = __popc(used & ~busy);
     if (busy == 0u || (more && free_lanes >= refill)) {
       while (q1n > 0) chords(min(q1n, 32));
       if (q2n > 0) values(q2n);
-      if (active && mask == 0u && sp == 0) {
+      if (active && mask == 0u && sp == sb) {
         Hit8 h;
         h.t = t_hi, h.gauss = arg, h.w = acc, h.r = ar, h.g = ag, h.b = ab, h.count = cnt;
         sink(item, ray, h);
@@ -283,16 +309,20 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
         uint32_t first = 0;
         if (lane == 0) first = atomicAdd(work, (unsigned)__popc(want));
         first = __shfl_sync(kFull, first, 0);
-        more = first + (uint32_t)__popc(want) < n;
+        // (where every warp's first share covers the batch, there is nothing more to fetch)
+        more = first + (uint32_t)__popc(want) < n && n > (uint32_t)rpw * warps;
         if ((want >> lane) & 1u) {
           item = first + (uint32_t)__popc(want & lt);
           if (item < n && source(item, ray)) {
             active = true;
             inv = safe_inv(ray.d);
             neg = (inv.x < 0.f ? 0x100u : 0u) | (inv.y < 0.f ? 0x200u : 0u) | (inv.z < 0.f ? 0x400u : 0u);
+            no = ray.o;
+            walk_scene = ray.scene;
+            owner = lane;
             node = 0u;
             mask = 1u;  // slot 0 of node 0: the root
-            sp = 0;
+            sp = sb = 0;
             t_hi = kKind == kScatter8 ? ray.t : kInf;
             arg = kNoGauss;
             cnt = 0u;
@@ -321,10 +351,45 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
       if (!__any_sync(kFull, active) && !more) break;
       continue;
     }
+    if (!more && busy != kFull) {
+      // No rays left to fetch: lanes without nodes take the oldest stack entry -- the largest subtree -- of
+      // lanes that have more than one thing to do, and walk it for its owner.  Queue entries carry the owner,
+      // so nothing else changes; the warp's last rays no longer walk alone.
+      const unsigned donors = __ballot_sync(kFull, sp - sb + (mask != 0u ? 1 : 0) >= 2 && sp != sb);
+      if (donors != 0u) {
+        const bool give = (donors >> lane) & 1u, idle = !((busy >> lane) & 1u);
+        const int rank = __popc((give ? donors : ~busy) & lt), pairs = min(__popc(donors), __popc(~busy));
+        if (give && rank < pairs) own[rank] = (uint32_t)lane;
+        __syncwarp();
+        const bool take = idle && rank < pairs;
+        const int from = take ? (int)own[rank] : lane;
+        const int at = __shfl_sync(kFull, sb, from);
+        const float ox = __shfl_sync(kFull, no.x, from), oy = __shfl_sync(kFull, no.y, from), oz = __shfl_sync(kFull, no.z, from);
+        const float ix = __shfl_sync(kFull, inv.x, from), iy = __shfl_sync(kFull, inv.y, from), iz = __shfl_sync(kFull, inv.z, from);
+        const uint32_t ng = __shfl_sync(kFull, neg, from);
+        const int ow = __shfl_sync(kFull, owner, from);
+        const uint32_t ws = kMany ? __shfl_sync(kFull, walk_scene, from) : 0u;
+        if (take) {
+          const uint32_t e = smem[32 * at + from];
+          node = e >> 8;
+          mask = e & 0xFFu;
+          no = f3(ox, oy, oz);
+          inv = f3(ix, iy, iz);
+          neg = ng;
+          owner = ow;
+          walk_scene = ws;
+          sp = sb = 0;
+        }
+        if (give && rank < pairs) ++sb;
+        __syncwarp();
+      }
+    }
     // node step
     uint32_t leaf = 0u;
-    const uint32_t* nodes = scenes.of(ray.scene).nodes;
-    if (active && (mask != 0u || sp != 0)) {
+    const uint32_t* nodes = scenes.of(walk_scene).nodes;
+    const float far_t = kKind == kFlight8 ? __shfl_sync(kFull, t_hi, owner) : 0.f;
+    const float at_t = kKind == kScatter8 ? __shfl_sync(kFull, ray.t, owner) : 0.f;
+    if (mask != 0u || sp != sb) {
       if (mask == 0u) {
         const uint32_t e = stack[32 * --sp];
         node = e >> 8;
@@ -348,8 +413,8 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
       const float ax = __uint_as_float((ew & 0xFFu) << 23) * inv.x;
       const float ay = __uint_as_float((ew & 0xFF00u) << 15) * inv.y;
       const float az = __uint_as_float((ew & 0xFF0000u) << 7) * inv.z;
-      const float bx = fmaf(h.x - ray.o.x, inv.x, -ax), by = fmaf(h.y - ray.o.y, inv.y, -ay),
-                  bz = fmaf(h.z - ray.o.z, inv.z, -az);
+      const float bx = fmaf(h.x - no.x, inv.x, -ax), by = fmaf(h.y - no.y, inv.y, -ay),
+                  bz = fmaf(h.z - no.z, inv.z, -az);
       const bool nx = inv.x < 0.f, ny = inv.y < 0.f, nz = inv.z < 0.f;
       // near / far planes by the direction's signs: (lo.x, hi.x) = (a.xy, bq.zw), (lo.y, hi.y) = (a.zw, c.xy),
       // (lo.z, hi.z) = (bq.xy, c.zw)
@@ -370,8 +435,11 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
         const float2 nx2 = plane2(nxw[w], a2x, b2x), ny2 = plane2(nyw[w], a2y, b2y), nz2 = plane2(nzw[w], a2z, b2z);
         const float2 fx2 = plane2(fxw[w], a2x, b2x), fy2 = plane2(fyw[w], a2y, b2y);
         float2 fz2 = plane2(fzw[w], a2z, b2z);
-        const float t0 = kKind == kScatter8 ? ray.t : 0.0f;
-        if constexpr (kKind != kTau8) fz2 = make_float2(fminf(fz2.x, t_hi), fminf(fz2.y, t_hi));  // a transmittance query has no far end
+        const float t0 = at_t;  // 0 but for kScatter8
+        if constexpr (kKind != kTau8) {
+          const float t1 = kKind == kScatter8 ? at_t : far_t;
+          fz2 = make_float2(fminf(fz2.x, t1), fminf(fz2.y, t1));
+        }  // a transmittance query has no far end
         const float d1 = fmin3f(fx2.y, fy2.y, fz2.y) - fmax3f(nx2.y, ny2.y, fmaxf(nz2.y, t0));
         const float d0 = fmin3f(fx2.x, fy2.x, fz2.x) - fmax3f(nx2.x, ny2.x, fmaxf(nz2.x, t0));
         miss = __funnelshift_l(__float_as_uint(d1), miss, 1);
@@ -390,7 +458,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
       if (leaf != 0u) {
         uint32_t at = atomicAdd(own, (uint32_t)__popc(leaf));
         do {
-          q1[at++] = ((uint32_t)lane << 27) | (node << 3) | ((uint32_t)__ffs(leaf) - 1u);
+          q1[at++] = ((uint32_t)owner << 27) | (node << 3) | ((uint32_t)__ffs(leaf) - 1u);
           leaf &= leaf - 1u;
         } while (leaf != 0u);
       }
@@ -402,7 +470,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
         if (leaf != 0u) {
           const uint32_t b = (uint32_t)__ffs(leaf) - 1u;
           leaf &= leaf - 1u;
-          q1[q1n + __popc(bal & lt)] = ((uint32_t)lane << 27) | (node << 3) | b;
+          q1[q1n + __popc(bal & lt)] = ((uint32_t)owner << 27) | (node << 3) | b;
         }
         q1n += __popc(bal);
       }
@@ -412,25 +480,60 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
   }
 }
 
-
-// Batches of at least this many rays take the thread-per-ray form.  Below it a launch ends with its longest
-// rays, whose lanes walk alone, and a whole warp on each ray is sooner done.  Transmittance batches
-// (thread-per-ray / warp-per-ray, ms): 65k rays 0.29 / 0.24 (100k-Gaussian cloud), 0.37 / 0.32 (500k), 0.57 /
-// 0.42 (100k in clusters); 130k 0.33 / 0.38, 0.44 / 0.53, 0.70 / 0.72; 250k 0.39 / 0.63, 0.55 / 0.93, 0.94 /
-// 1.25.  8-bounce images: 65k paths 2.7 / 1.9 (50k-Gaussian cloud), 5.0 / 3.8 (500k),
-// 6.6 / 4.7 (200k in clusters); 131k paths 3.0 / 3.3, 5.7 / 6.5, 8.1 / 8.3; 524k paths 5.0 / 11.2, 9.5 / 22.8,
-// 15.0 / 29.2.
-constexpr uint32_t kTrace8Min = 7u << 14;
 // Threads of a block of the stages, and the resident blocks per SM of their register budget: 3 (80 registers).
 // 4 (64 registers) spills and leaves less of the SM's memory to L1, 2 hides less latency: the showcase batch
 // took 93 ms at 4 against 86 at 3, and 83 ms at 2 against 70 at 3.
 constexpr int kT8Blocks = 3;
 constexpr int kT8Threads = 256;
 
+__device__ __forceinline__ uint32_t grid_warps() { return gridDim.x * (blockDim.x / 32u); }
 // Rays in flight per warp: 32, or an even share of a batch too small for that.
-__device__ __forceinline__ int rays_per_warp(uint32_t n) {
-  const uint32_t warps = gridDim.x * (blockDim.x / 32u);
-  return (int)min(32u, max(4u, (n + warps - 1u) / warps));
+__device__ __forceinline__ int rays_per_warp(uint32_t n, uint32_t warps) {
+  return (int)min(32u, max(1u, (n + warps - 1u) / warps));
+}
+
+// The extend stage of one path queue: free flights and then, where a scene's Gaussians differ in albedo
+// (kMixed), the albedo at the scatter points -- the sigma_t * pdf-weighted mean over the chords containing the
+// scatter distance (evaluate_albedo over the rebuilt active set, sampling.cuh:257-283, 422-458).  With kMixed
+// a warp takes a share of the queue at a time through both.  load(item, ray) and store(item, ray, hit) are
+// the flights' source and sink; at(item, ray) fills a scattered path's ray and distance (false: nothing to
+// look up) and albedo(item, ray, rgb) takes the result.
+constexpr uint32_t kMixedShare = 256;
+template <bool kAcc, bool kMixed, class Scenes, class Load, class Store, class At, class Albedo>
+__device__ __forceinline__ void extend8(const Scenes& scenes, uint32_t depth, uint32_t* smem, uint32_t n,
+                                        unsigned int* work, uint32_t& status, Load&& load, Store&& store, At&& at,
+                                        Albedo&& albedo) {
+  const uint8_t* order = stage_order8();
+  const uint32_t warps = grid_warps();
+  if constexpr (!kMixed) {
+    trace8<kAcc, kFlight8>(scenes, depth, smem, order, n, work, warps, rays_per_warp(n, warps), status, load, store);
+  } else {
+    const int lane = threadIdx.x & 31;
+    unsigned int* next = smem + trace8_warp_words(depth) - 1u;
+    const uint32_t share = min(kMixedShare, max(1u, (n + warps - 1u) / warps));
+    while (!__any_sync(kFull, status != 0u)) {
+      uint32_t first = 0;
+      if (lane == 0) first = atomicAdd(work, share);
+      first = __shfl_sync(kFull, first, 0);
+      if (first >= n) break;
+      const uint32_t m = min(share, n - first);
+      const int rpw = (int)min(32u, m);
+      if (lane == 0) *next = 0u;
+      __syncwarp();
+      trace8<kAcc, kFlight8>(
+          scenes, depth, smem, order, m, next, 1u, rpw, status,
+          [&](uint32_t i, Ray8& ray) { return load(first + i, ray); },
+          [&](uint32_t i, const Ray8& ray, const Hit8& h) { store(first + i, ray, h); });
+      __syncwarp();
+      if (lane == 0) *next = 0u;
+      __syncwarp();
+      trace8<kAcc, kScatter8>(
+          scenes, depth, smem, order, m, next, 1u, rpw, status,
+          [&](uint32_t i, Ray8& ray) { return at(first + i, ray); },
+          [&](uint32_t i, const Ray8& ray, const Hit8& h) { albedo(first + i, ray, mean_albedo(h.w, h.r, h.g, h.b)); });
+      __syncwarp();
+    }
+  }
 }
 
 }  // namespace vp

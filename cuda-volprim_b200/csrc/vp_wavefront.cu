@@ -13,9 +13,10 @@
 //   tail      (warp per path)    once few paths are left: each runs to its end in one launch; then, a
 //                                thread per pixel, the running mean over the batch's samples in order
 //
-// extend and shadow have a second form for long queues (kTrace8Min): thread per ray over the compressed
-// 8-wide BVH (vp_trace8.cuh), with the same results.  In it the scatter-point albedo is the scene's, when
-// all its Gaussians share one, or a stage of its own (k_wf_scatter8).
+//   extend and shadow run thread per ray over the compressed 8-wide BVH (vp_trace8.cuh); the scatter-point
+//   albedo is then the scene's, when all its Gaussians share one, or a second traversal.
+//   Their warp-per-ray forms over the BVH32 give the same results: they count (VP_MEASURE_COUNTERS) and
+//   serve scenes too deep for the 8-wide tree.
 //
 // Each kernel is a fraction of the fused path loop's code and registers, so more warps are
 // resident per SM to hide the latency of the dependent node loads.  The reference found a
@@ -62,9 +63,10 @@ constexpr int kExtendHitCap = VP_WF_EXTEND_HIT_CAP;
 constexpr uint32_t kSortMinPaths = VP_WF_SORT_MIN;
 // At most this many paths go to the tail kernel: as stages, a bounce of few paths is launches, polls and each
 // stage's slowest ray; as whole paths it is one launch, but a warp shades alone and holds more registers.
-// 64-bounce images, ms as stages / with the tail from 16k paths / from 40k: 4k paths 4.4 / 2.2 / 2.1 (50k-
-// Gaussian cloud), 7.6 / 5.0 / 5.1 (500k); 65k paths 7.0 / 5.2 / 7.7, 12.7 / 10.5 / 13.3.
-constexpr uint32_t kTailMax = 16384;
+// 64-bounce images, ms as stages / with the tail from 8k paths / from 16k: 4k paths 4.4 / 1.7 / 1.9 (50k-
+// Gaussian cloud), 5.3 / 4.3 / 4.4 (500k); 16k paths 4.8 / 2.9 / 2.8, 5.8 / 4.8 / 5.7; 65k paths 5.6 / 3.8 / 3.9,
+// 7.3 / 6.9 / 6.8.
+constexpr uint32_t kTailMax = 8192;
 // Resident blocks per SM of its register budget: 2 (128 registers, no spills to speak of) against 3 or 4:
 // 4k paths 1.75 / 2.13 / 2.34 ms (50k), 4.4 / 5.1 / 5.0 (500k).
 constexpr int kTailBlocks = 2;
@@ -123,7 +125,7 @@ __global__ void k_wf_generate(CameraView C, ParamsView P, uint32_t spp_offset, u
   if (!adaptive) {
     if (p == 0) {
       b.ctr[0] = P.max_bounces > 0 ? n : 0u;
-      b.ctr[1] = b.ctr[2] = b.ctr[3] = b.ctr[4] = b.ctr[5] = 0u;
+      b.ctr[1] = b.ctr[2] = b.ctr[3] = b.ctr[4] = 0u;
     }
     if (p >= n) return;
   } else {
@@ -218,15 +220,14 @@ __global__ void __launch_bounds__(256, VP_WF_MIN_BLOCKS) k_wf_extend(SceneView S
 
 // ---- thread-per-ray stages (vp_trace8.cuh) -----------------------------------------------------
 
-template <bool kAcc>
-__global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_wf_extend8(SceneView S, WfBuffers b, const uint32_t* q,
-                                                                        const uint32_t* count, unsigned int* work,
-                                                                        Counters* ctr) {
+template <bool kAcc, bool kMixed>
+__global__ void __launch_bounds__(kT8Threads, kMixed ? 2 : kT8Blocks) k_wf_extend8(SceneView S, WfBuffers b, const uint32_t* q,
+                                                                     const uint32_t* count, unsigned int* work,
+                                                                     Counters* ctr) {
   uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(S.depth8);
-  const uint32_t n = *count;
   uint32_t status = 0;
-  trace8<kAcc, kFlight8>(
-      OneScene8{scene8_of(S)}, S.depth8, smem, n, work, rays_per_warp(n), status,
+  extend8<kAcc, kMixed>(
+      OneScene8{scene8_of(S)}, S.depth8, smem, *count, work, status,
       [&](uint32_t item, Ray8& ray) {
         const uint32_t p = __ldg(q + item);
         const uint32_t bounce = meta_bounce(b.meta[p]);
@@ -245,38 +246,20 @@ __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_wf_extend8(SceneView 
       },
       [&](uint32_t item, const Ray8&, const Hit8& h) {
         const uint32_t p = __ldg(q + item);
-        const float3 a = h.t < kInf ? S.albedo : f3(0.f, 0.f, 0.f);  // k_wf_scatter8 replaces it in mixed scenes
+        const float3 a = h.t < kInf ? S.albedo : f3(0.f, 0.f, 0.f);
         b.alb4[p] = make_float4(a.x, a.y, a.z, h.t);
         b.sg[p] = h.gauss;
-      });
-  if (status) atomicOr(&ctr->status, status);
-}
-
-// Albedo at the scatter points of a scene whose Gaussians differ in it: the sigma_t * pdf-weighted
-// mean over the chords containing the scatter distance (evaluate_albedo over the rebuilt active set,
-// sampling.cuh:257-283, 422-458).
-template <bool kAcc>
-__global__ void __launch_bounds__(kT8Threads) k_wf_scatter8(SceneView S, WfBuffers b, const uint32_t* q,
-                                                           const uint32_t* count, unsigned int* work, Counters* ctr) {
-  uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + (threadIdx.x >> 5) * trace8_warp_words(S.depth8);
-  const uint32_t n = *count;
-  uint32_t status = 0;
-  trace8<kAcc, kScatter8>(
-      OneScene8{scene8_of(S)}, S.depth8, smem, n, work, rays_per_warp(n), status,
+      },
       [&](uint32_t item, Ray8& ray) {
         const uint32_t p = __ldg(q + item);
-        const float t = b.alb4[p].w;
-        if (!(t < kInf)) return false;
+        ray.t = b.alb4[p].w;
+        if (!(ray.t < kInf)) return false;
         const float4 o = b.o4[p], d = b.d4[p];
         ray.o = f3(o.x, o.y, o.z);
         ray.d = f3(d.x, d.y, d.z);
-        ray.t = t;
         return true;
       },
-      [&](uint32_t item, const Ray8& ray, const Hit8& h) {
-        const float3 a = mean_albedo(h.w, h.r, h.g, h.b);
-        b.alb4[__ldg(q + item)] = make_float4(a.x, a.y, a.z, ray.t);
-      });
+      [&](uint32_t item, const Ray8& ray, float3 a) { b.alb4[__ldg(q + item)] = make_float4(a.x, a.y, a.z, ray.t); });
   if (status) atomicOr(&ctr->status, status);
 }
 
@@ -287,7 +270,7 @@ __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_wf_shadow8(SceneView 
   const uint32_t n = *count;
   uint32_t status = 0;
   trace8<kAcc, kTau8>(
-      OneScene8{scene8_of(S)}, S.depth8, smem, n, work, rays_per_warp(n), status,
+      OneScene8{scene8_of(S)}, S.depth8, smem, stage_order8(), n, work, grid_warps(), rays_per_warp(n, grid_warps()), status,
       [&](uint32_t item, Ray8& ray) {
         const uint32_t slot = __ldg(b.qs + item);
         const float4 o = b.so4[slot], d = b.sd4[slot];
@@ -445,7 +428,6 @@ __global__ void k_wf_advance(uint32_t* ctr) {
   ctr[2] = 0u;
   ctr[3] = 0u;
   ctr[4] = 0u;
-  ctr[5] = 0u;
 }
 
 // Welford mean over the batch's samples of one pixel, in sample order (raygen.cuh:214-242).
@@ -638,19 +620,19 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
   const int ext_blocks = ctx->sm_count * resident_blocks(ext, threads, smem);
   const int shd_blocks = ctx->sm_count * resident_blocks(shd, threads, smem_sh);
   const int thr_blocks = ctx->sm_count * 8;
-  // Thread-per-ray stages above kTrace8Min paths; the counting variants are the warp-cooperative ones.
-  const bool can8 = s->view.depth8 != 0u && !P.measure;
+  // The thread-per-ray stages, but for a scene without the 8-wide BVH and for the counting variants.
+  const bool use8 = s->view.depth8 != 0u && !P.measure;
   const size_t smem8 = trace8_smem_bytes(s->view.depth8, kT8Threads);
-  auto ext8 = P.accurate ? k_wf_extend8<true> : k_wf_extend8<false>;
-  auto sca8 = P.accurate ? k_wf_scatter8<true> : k_wf_scatter8<false>;
+  const bool mixed = s->view.one_albedo == 0;
+  auto ext8 = P.accurate ? (mixed ? k_wf_extend8<true, true> : k_wf_extend8<true, false>)
+                         : (mixed ? k_wf_extend8<false, true> : k_wf_extend8<false, false>);
   auto shd8 = P.accurate ? k_wf_shadow8<true> : k_wf_shadow8<false>;
-  int ext8_blocks = 0, sca8_blocks = 0, shd8_blocks = 0;
-  if (can8) {
+  int ext8_blocks = 0, shd8_blocks = 0;
+  if (use8) {
     if (smem8 > 48 * 1024)
-      for (auto k : {(const void*)ext8, (const void*)sca8, (const void*)shd8})
+      for (auto k : {(const void*)ext8, (const void*)shd8})
         VP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem8));
     ext8_blocks = ctx->sm_count * resident_blocks(ext8, kT8Threads, smem8);
-    sca8_blocks = ctx->sm_count * resident_blocks(sca8, kT8Threads, smem8);
     shd8_blocks = ctx->sm_count * resident_blocks(shd8, kT8Threads, smem8);
   }
   // VP_MEASURE_STAGES: events around the extend and shadow launches of each iteration (a ring of 4 iterations,
@@ -672,7 +654,7 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
     pending = 0;
     return cudaSuccess;
   };
-  if (P.adaptive_threshold > 0.0f) VP_CUDA(cudaMemsetAsync(b.ctr, 0, 6 * sizeof(uint32_t), st));
+  if (P.adaptive_threshold > 0.0f) VP_CUDA(cudaMemsetAsync(b.ctr, 0, 5 * sizeof(uint32_t), st));
   k_wf_generate<<<(paths + 255) / 256, 256, 0, st>>>(cam, P, spp_offset, spp_count, paths, b, img->mean, img->m2,
                                                      img->count, ctx->counters);
   VP_CUDA(cudaGetLastError());
@@ -703,14 +685,8 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
     }
     cudaEvent_t* e4 = ev + 4 * (it & 3u);
     if (timed) VP_CUDA(cudaEventRecord(e4[0], st));
-    const bool use8 = can8 && polled >= kTrace8Min;
     if (use8) {
       ext8<<<ext8_blocks, kT8Threads, smem8, st>>>(s->view, b, qcur, b.ctr + 0, b.ctr + 3, ctx->counters);
-      if (!s->view.one_albedo) {
-        sca8<<<sca8_blocks, kT8Threads, smem8, st>>>(s->view, b, qcur, b.ctr + 0, b.ctr + 5, ctx->counters);
-        ctx->launches += 1;
-        ctx->stage_launches[0] += 1;
-      }
     } else {
       ext<<<ext_blocks, threads, smem, st>>>(s->view, P, b, qcur, b.ctr + 0, b.ctr + 3, ctx->counters);
     }

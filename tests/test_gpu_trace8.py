@@ -1,5 +1,5 @@
-"""GPU: the thread-per-ray stages over the compressed 8-wide BVH (wavefront engine, queues of at least
-114,688 paths) against the warp engine, which traverses the BVH32 one path a warp.
+"""GPU: the thread-per-ray stages over the compressed 8-wide BVH (wavefront engine) against the warp engine,
+which traverses the BVH32 one path a warp.
 
 Both engines take the same samples, evaluate the same chords with the same arithmetic and carry their
 sums in FP64 rounded once, so a pixel differs only where a transmittance reaches MAX_OPTICAL_DEPTH in
@@ -16,7 +16,7 @@ from volprim_b200 import scenes
 
 pytestmark = pytest.mark.gpu
 
-W, H = 409, 281  # 114,929 paths: the first iterations take the thread-per-ray stages, the tail the others
+W, H = 409, 281  # 114,929 paths: more than one refill of every warp; the tail kernel takes the last 8,192
 
 
 def gaussians(n, seed, layout="box", mixed=True):
@@ -85,11 +85,11 @@ def test_empty_scene(vp_ctx):
     check(*images(vp_ctx, g))
 
 
-def test_large_transmittance_batch(vp_ctx):
-    """vp_transmittance takes the thread-per-ray form from 114,688 rays on: the same values as in smaller calls."""
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 1000, 114_700])
+def test_transmittance_batches(vp_ctx, n):
+    """vp_transmittance (thread per ray) against vp_transmittance_static (warp per ray over the BVH32)."""
     sc = vp.Scene(vp_ctx, gaussians(1500, 21), 0.2)
     rng = np.random.default_rng(22)
-    n = 114_700
     o = np.where((np.arange(n) % 2 == 0)[:, None], rng.normal(0, 2.0, (n, 3)), rng.uniform(-0.5, 0.5, (n, 3)))
     d = rng.normal(0, 1, (n, 3))
     d[::7, 0] = 0.0  # axis-parallel components
@@ -97,9 +97,9 @@ def test_large_transmittance_batch(vp_ctx):
     o, d = o.astype(np.float32), d.astype(np.float32)
     for precision in (vp.VP_PRECISION_FAST, vp.VP_PRECISION_ACCURATE):
         got = sc.transmittance(o, d, precision=precision)
-        want = np.concatenate([sc.transmittance(o[k:k + 50_000], d[k:k + 50_000], precision=precision)
+        want = np.concatenate([sc.transmittance_static(o[k:k + 50_000], d[k:k + 50_000], precision=precision)
                                for k in range(0, n, 50_000)])
-        assert (want < 0.9).sum() > 1000 and (want > 0.99).sum() > 1000
+        assert n < 1000 or ((want < 0.9).sum() > n // 100 and (want > 0.99).sum() > n // 100)
         assert np.abs(got - want).max() <= 1e-7, np.abs(got - want).max()
     sc.close()
 

@@ -205,7 +205,7 @@ __global__ void k_albedo_thread(SceneView S, const float* __restrict__ pts, uint
   if (status) atomicOr(&ctr->status, status);
 }
 
-// The same query, thread per ray (vp_trace8.cuh); k_tau_warp serves scenes too deep for the 8-wide BVH.
+// The same query, thread per ray (vp_trace8.cuh); k_tau_warp takes small calls and scenes too deep for the 8-wide BVH.
 template <bool kAcc>
 __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_tau8(SceneView S, const float* __restrict__ org,
                                                                const float* __restrict__ dir, uint32_t n,
@@ -285,10 +285,13 @@ vp_status launch_transmittance(vp_scene* s, const float* o, const float* d, uint
   vp_context* ctx = s->ctx;
   cudaStream_t st = ctx->stream;
   if (n == 0) return VP_OK;
-  if (engine == VP_ENGINE_WARP && s->view.depth8 != 0u) {
+  // Few rays through a small scene end sooner with a warp on each: 1,000 rays 59 / 71 us (1,000 Gaussians), 52 /
+  // 62 us (10k); at 65k rays it is 152 / 139 and 134 / 97 us, at 100k Gaussians 98 / 82 us for 1,000 rays.
+  const bool small = n <= 16384u && s->view.count < 32768u;
+  if (engine == VP_ENGINE_WARP && s->view.depth8 != 0u && !small) {
     auto kern = accurate ? k_tau8<true> : k_tau8<false>;
     const size_t smem = trace8_smem_bytes(s->view.depth8, kT8Threads);
-    if (smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kSmem8Default) VP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int blocks = ctx->sm_count * occupancy_blocks(kern, kT8Threads, smem);
     kern<<<blocks, kT8Threads, smem, st>>>(s->view, o, d, n, out, ctx->work_counter, ctx->counters);
   } else if (engine == VP_ENGINE_WARP) {

@@ -767,7 +767,7 @@ vp_status prepare_launch(vp_server* s) {
     s->smem8 = trace8_smem_bytes(s->max_depth8, kT8Threads) + s->scenes.size() * sizeof(Scene8);
     auto ext8 = extend8_kernel(s);
     auto shd8 = s->accurate ? k_srv_shadow8<true> : k_srv_shadow8<false>;
-    if (s->smem8 > 48 * 1024)
+    if (s->smem8 > kSmem8Default)
       for (auto k : {(const void*)ext8, (const void*)shd8})
         VP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->smem8));
     s->ext8_blocks = ctx->sm_count * srv_blocks(ext8, kT8Threads, s->smem8);

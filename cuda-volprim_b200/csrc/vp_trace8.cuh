@@ -53,7 +53,7 @@ __host__ __device__ __forceinline__ size_t trace8_smem_bytes(uint32_t depth, int
   return (size_t)trace8_warp_words(depth) * 4u * (size_t)(threads / 32);
 }
 
-enum Query8 { kFlight8 = 0, kTau8 = 1, kScatter8 = 2 };
+enum Query8 { kFlight8 = 0, kTau8 = 1, kScatter8 = 2, kBoth8 = 3 /* flights and transmittances by Ray8::flight */ };
 
 // What a query reads of a scene.
 struct Scene8 {
@@ -77,6 +77,7 @@ struct Ray8 {
   uint64_t key;    // kFlight8: free-flight key
   float t;         // kScatter8: scatter distance
   uint32_t scene;  // ManyScenes8: index into the table
+  bool flight;     // kBoth8: a free flight, else a transmittance
   uint32_t seed;   // kTau8: the Gaussian already accounted for; kFlight8: one to start with (kNoGauss: none)
   float seed_tau;  // its optical depth (0 without one)
 };
@@ -137,6 +138,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
                                        uint32_t n, unsigned int* work, uint32_t warps, int rpw, uint32_t& status,
                                        Source&& source, Sink&& sink) {
   constexpr bool kMany = std::is_same_v<Scenes, ManyScenes8>;
+  constexpr bool kFlights = kKind == kFlight8 || kKind == kBoth8, kTaus = kKind == kTau8 || kKind == kBoth8;
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   uint32_t* stack = smem + lane;  // entry k at stack[32 k]: conflict-free whatever the lanes' depths
@@ -150,6 +152,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
   ray.seed = kNoGauss;
   ray.t = 0.f;
   ray.scene = 0u;
+  ray.flight = kKind == kFlight8;
   // the scene of another lane's ray
   auto scene_of = [&](int ow) { return scenes.of(kMany ? __shfl_sync(kFull, ray.scene, ow) : 0u); };
   // what this lane walks: its own ray or, late in a batch, part of another lane's (owner)
@@ -176,7 +179,9 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
     const Scene8 sc = scene_of(ow);
     uint64_t key = 0ull;
     float ts = 0.f;
-    if constexpr (kKind == kFlight8)
+    bool flight = kKind == kFlight8;
+    if constexpr (kKind == kBoth8) flight = __shfl_sync(kFull, (int)ray.flight, ow) != 0;
+    if constexpr (kFlights)
       key = ((uint64_t)__shfl_sync(kFull, (uint32_t)(ray.key >> 32), ow) << 32) |
             __shfl_sync(kFull, (uint32_t)ray.key, ow);
     if constexpr (kKind == kScatter8) ts = __shfl_sync(kFull, ray.t, ow);
@@ -190,9 +195,9 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
       ch.d2lo = kAcc ? __uint_as_float(q2[6 * kQ2Cap + e]) : 0.0f;
       ch.t_in = fmaf(-ch.h, ch.rw, ch.tc);
       ch.t_out = fmaf(ch.h, ch.rw, ch.tc);
-      if constexpr (kKind == kTau8) {
+      if (kTaus && !flight) {
         v = chord_tau<kAcc>(ch.tc, ch.rw, ch.d2, ch.h, chord_u0(ch, 0.0f), fmaxf(ch.t_in, 0.0f), ch.t_out, icf, ch.d2lo);
-      } else if constexpr (kKind == kFlight8) {
+      } else if (kFlights) {
         v = chord_free_flight<kAcc>(ch.tc, ch.rw, ch.d2, ch.h, chord_u0(ch, 0.0f), ch.t_in, ch.t_out, icf,
                                     free_flight_tau<kAcc>(key, __ldg(sc.perm + gi)), ch.d2lo);
       } else {
@@ -212,13 +217,14 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
     while (__any_sync(kFull, m != 0u)) {
       const int j = m ? __ffs(m) - 1 : lane;
       const float vj = __shfl_sync(kFull, v, j);
-      if constexpr (kKind == kTau8) {
-        if (m) acc += (double)vj;
-      } else if constexpr (kKind == kFlight8) {
-        const uint32_t gj = __shfl_sync(kFull, gi, j);
-        if (m && vj < t_hi) {
-          t_hi = vj;
-          arg = gj;
+      if constexpr (kKind != kScatter8) {
+        if (kTaus && m && !ray.flight) acc += (double)vj;
+        if constexpr (kFlights) {
+          const uint32_t gj = __shfl_sync(kFull, gi, j);
+          if (m && ray.flight && vj < t_hi) {
+            t_hi = vj;
+            arg = gj;
+          }
         }
       } else {
         const float x = __shfl_sync(kFull, wa, j), y = __shfl_sync(kFull, wb, j), z = __shfl_sync(kFull, wc, j);
@@ -252,12 +258,11 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
     const float3 o = f3(__shfl_sync(kFull, ray.o.x, ow), __shfl_sync(kFull, ray.o.y, ow), __shfl_sync(kFull, ray.o.z, ow));
     const float3 d = f3(__shfl_sync(kFull, ray.d.x, ow), __shfl_sync(kFull, ray.d.y, ow), __shfl_sync(kFull, ray.d.z, ow));
     float bound = kInf;
-    if constexpr (kKind == kTau8) {
+    if constexpr (kTaus) {
       const uint32_t seed = __shfl_sync(kFull, ray.seed, ow);
       hit = hit && gi != seed;
-    } else {
-      bound = __shfl_sync(kFull, kKind == kFlight8 ? t_hi : ray.t, ow);
     }
+    if constexpr (kKind != kTau8) bound = __shfl_sync(kFull, kKind == kScatter8 ? ray.t : t_hi, ow);
     Chord ch;
     if (hit) {
       PrimGeo g;
@@ -287,7 +292,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
 
   while (true) {
     if (status) mask = 0u, sp = sb;  // (raised below: the lane gives its ray up)
-    if constexpr (kKind == kTau8) {  // opaque: the rest of the ray's nodes cannot matter
+    if constexpr (kTaus) {  // opaque: the rest of the ray's nodes cannot matter
       const bool opaque = acc >= (double)kMaxOpticalDepth;
       if (__any_sync(kFull, opaque)) {
         if (__shfl_sync(kFull, (int)opaque, owner)) mask = 0u, sp = sb;
@@ -327,13 +332,13 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
             arg = kNoGauss;
             cnt = 0u;
             acc = ar = ag = ab = 0.0;
-            if constexpr (kKind == kTau8) {
-              if (ray.seed != kNoGauss) acc = (double)ray.seed_tau;
+            if constexpr (kTaus) {
+              if (!ray.flight && ray.seed != kNoGauss) acc = (double)ray.seed_tau;
             }
-            if constexpr (kKind == kFlight8) {
+            if constexpr (kFlights) {
               // a path that scattered starts inside the Gaussian that scattered it: its free flight
               // bounds the traversal from the start (showcase: 63 -> 33 nodes a ray with it)
-              if (ray.seed != kNoGauss) {
+              if (ray.flight && ray.seed != kNoGauss) {
                 const Scene8 sc = scenes.of(ray.scene);
                 const PrimGeo g = load_geo(sc.prims, ray.seed);
                 Chord ch;
@@ -343,6 +348,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
                                                           ch.d2lo);
                   if (v < t_hi) t_hi = v, arg = ray.seed;
                 }
+                ray.seed = kNoGauss;  // (the traversal meets it again)
               }
             }
           }
@@ -387,7 +393,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
     // node step
     uint32_t leaf = 0u;
     const uint32_t* nodes = scenes.of(walk_scene).nodes;
-    const float far_t = kKind == kFlight8 ? __shfl_sync(kFull, t_hi, owner) : 0.f;
+    const float far_t = kFlights ? __shfl_sync(kFull, t_hi, owner) : 0.f;
     const float at_t = kKind == kScatter8 ? __shfl_sync(kFull, ray.t, owner) : 0.f;
     if (mask != 0u || sp != sb) {
       if (mask == 0u) {
@@ -452,7 +458,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
     }
     // hit Gaussians to queue 1: a vote per round, or (faster for transmittance, whose rays meet more of them;
     // 33.3 / 34.9 ms of the showcase, but 19.9 / 19.2 for the argmin) one shared-memory atomic per lane
-    if constexpr (kKind == kTau8) {
+    if constexpr (kTaus) {
       if (lane == 0) own[0] = (uint32_t)q1n;
       __syncwarp();
       if (leaf != 0u) {
@@ -479,6 +485,9 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
     while (q1n >= 32) chords(32);
   }
 }
+
+// Dynamic shared memory above which a kernel has to ask for it: 48 KB less its static part (the order table).
+constexpr size_t kSmem8Default = 48 * 1024 - sizeof(Order8) - 1024;
 
 // Threads of a block of the stages, and the resident blocks per SM of their register budget: 3 (80 registers).
 // 4 (64 registers) spills and leaves less of the SM's memory to L1, 2 hides less latency: the showcase batch

@@ -10,7 +10,7 @@
 //     shadow  (warp per query)   transmittance over the BVH32 with early exit at tau >= 88
 //     gather  (thread per path)  radiance += weight x T in query order; finished paths write
 //                                their sample
-//   tail      (warp per path)    once few paths are left: each runs to its end in one launch; then, a
+//   tail      (a few paths a warp) once few paths are left: they run to their ends in one launch; then, a
 //                                thread per pixel, the running mean over the batch's samples in order
 //
 //   extend and shadow run thread per ray over the compressed 8-wide BVH (vp_trace8.cuh); the scatter-point
@@ -61,14 +61,13 @@ constexpr int kExtendHitCap = VP_WF_EXTEND_HIT_CAP;
 #define VP_WF_SORT_MIN 65536
 #endif
 constexpr uint32_t kSortMinPaths = VP_WF_SORT_MIN;
-// At most this many paths go to the tail kernel: as stages, a bounce of few paths is launches, polls and each
-// stage's slowest ray; as whole paths it is one launch, but a warp shades alone and holds more registers.
-// 64-bounce images, ms as stages / with the tail from 8k paths / from 16k: 4k paths 4.4 / 1.7 / 1.9 (50k-
-// Gaussian cloud), 5.3 / 4.3 / 4.4 (500k); 16k paths 4.8 / 2.9 / 2.8, 5.8 / 4.8 / 5.7; 65k paths 5.6 / 3.8 / 3.9,
-// 7.3 / 6.9 / 6.8.
-constexpr uint32_t kTailMax = 8192;
-// Resident blocks per SM of its register budget: 2 (128 registers, no spills to speak of) against 3 or 4:
-// 4k paths 1.75 / 2.13 / 2.34 ms (50k), 4.4 / 5.1 / 5.0 (500k).
+// At most this many paths go to the tail: as stages, a bounce of few paths is launches, polls and each stage's
+// slowest ray.  64-bounce images, ms as stages / with the tail from 16k / 64k / 128k paths: 4k paths 4.4 / 1.9 /
+// 1.9 / 1.8 (50k-Gaussian cloud), 5.3 / 2.5 / 2.4 / 2.4 (500k); 65k paths 5.6 / 3.5 / 3.0 / 3.2, 7.3 / 5.0 / 4.6 /
+// 4.4; a 12-bounce image of 361k paths 4.4 from 64k, 5.0 from 128k.
+constexpr uint32_t kTailMax = 65536;
+// Resident blocks per SM of its register budget: 2 (128 registers) against 3: 4k paths 1.9 / 2.2 ms (50k), 2.4 /
+// 2.8 (500k).
 constexpr int kTailBlocks = 2;
 
 __device__ __forceinline__ uint32_t meta_bounce(uint32_t m) { return m & 0xFFFFu; }
@@ -287,9 +286,43 @@ __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_wf_shadow8(SceneView 
   if (status) atomicOr(&ctr->status, status);
 }
 
-// The shadow rays' seed chords are evaluated here, one thread per ray (seed_chord_tau): a ray
-// whose seed chord alone reaches MAX_OPTICAL_DEPTH gets T = 0 and never enters the shadow queue;
-// the others carry the seed's optical depth to the transmittance query in so4.w.
+// A path's vertex, by one thread: phase sample, NEE and roulette; the path's next ray, its transmittance
+// queries (so4, sd4, sw4) and its meta word.  Returns which of the queries need a traversal (bit k) and sets
+// ns and alive.  The shadow rays' seed chords are evaluated here, one thread per ray (seed_chord_tau): a ray
+// whose seed chord alone reaches MAX_OPTICAL_DEPTH gets T = 0 at once; the others carry the seed's optical
+// depth to the query in so4.w.
+__device__ __forceinline__ unsigned shade_path(const SceneView& S, const EnvView& E, const ParamsView& P,
+                                               const WfBuffers& b, uint32_t p, int& ns, bool& alive,
+                                               unsigned long long& opaque) {
+  PathState s = load_path(b, p, meta_bounce(b.meta[p]));
+  const float4 a = b.alb4[p];
+  const bool scattered = a.w < kInf;
+  ShadowSet sh;
+  alive = shade_bounce(E, P, s, scattered, a.w, f3(a.x, a.y, a.z), sh, b.sg[p]);
+  ns = sh.n;
+  unsigned queued = 0u;
+  for (int k = 0; k < sh.n; ++k) {
+    float seed_tau = -1.0f;  // no seed
+    if (sh.seed[k] != kNoGauss)
+      seed_tau = P.accurate ? seed_chord_tau<true>(S, sh.seed[k], sh.o[k], sh.d[k])
+                            : seed_chord_tau<false>(S, sh.seed[k], sh.o[k], sh.d[k]);
+    const bool opaque_k = seed_tau >= kMaxOpticalDepth;
+    // .w of the origin: the seed's optical depth for the query, or T = 0 already
+    b.so4[3u * p + k] = make_float4(sh.o[k].x, sh.o[k].y, sh.o[k].z, opaque_k ? 0.0f : seed_tau);
+    b.sd4[3u * p + k] = make_float4(sh.d[k].x, sh.d[k].y, sh.d[k].z, __uint_as_float(sh.seed[k]));
+    b.sw4[3u * p + k] = make_float4(sh.w[k].x, sh.w[k].y, sh.w[k].z, 0.f);
+    if (!opaque_k) queued |= 1u << k;
+    else opaque += 1;
+  }
+  if (alive) {
+    const uint64_t key = draw_bounce_key(s.rng);
+    b.key2[p] = make_uint2((uint32_t)key, (uint32_t)(key >> 32));
+  }
+  store_path(b, p, s);
+  b.meta[p] = (s.bounce & 0xFFFFu) | ((uint32_t)sh.n << 16) | (alive ? kAliveBit : 0u);
+  return queued;
+}
+
 __global__ void __launch_bounds__(256) k_wf_shade(SceneView S, EnvView E, ParamsView P, WfBuffers b,
                                                   const uint32_t* q, const uint32_t* count, uint32_t* qnext,
                                                   uint32_t* cnext, Counters* ctr) {
@@ -308,31 +341,7 @@ __global__ void __launch_bounds__(256) k_wf_shade(SceneView S, EnvView E, Params
     bool alive = false;
     if (valid) {
       p = q[i];
-      PathState s = load_path(b, p, meta_bounce(b.meta[p]));
-      const float4 a = b.alb4[p];
-      const bool scattered = a.w < kInf;
-      ShadowSet sh;
-      alive = shade_bounce(E, P, s, scattered, a.w, f3(a.x, a.y, a.z), sh, b.sg[p]);
-      ns = sh.n;
-      for (int k = 0; k < sh.n; ++k) {
-        float seed_tau = -1.0f;  // no seed
-        if (sh.seed[k] != kNoGauss)
-          seed_tau = P.accurate ? seed_chord_tau<true>(S, sh.seed[k], sh.o[k], sh.d[k])
-                                : seed_chord_tau<false>(S, sh.seed[k], sh.o[k], sh.d[k]);
-        const bool opaque_k = seed_tau >= kMaxOpticalDepth;
-        // .w of the origin: the seed's optical depth for the query, or T = 0 already
-        b.so4[3u * p + k] = make_float4(sh.o[k].x, sh.o[k].y, sh.o[k].z, opaque_k ? 0.0f : seed_tau);
-        b.sd4[3u * p + k] = make_float4(sh.d[k].x, sh.d[k].y, sh.d[k].z, __uint_as_float(sh.seed[k]));
-        b.sw4[3u * p + k] = make_float4(sh.w[k].x, sh.w[k].y, sh.w[k].z, 0.f);
-        if (!opaque_k) queued |= 1u << k;
-        else opaque += 1;
-      }
-      if (alive) {
-        const uint64_t key = draw_bounce_key(s.rng);
-        b.key2[p] = make_uint2((uint32_t)key, (uint32_t)(key >> 32));
-      }
-      store_path(b, p, s);
-      b.meta[p] = (s.bounce & 0xFFFFu) | ((uint32_t)sh.n << 16) | (alive ? kAliveBit : 0u);
+      queued = shade_path(S, E, P, b, p, ns, alive, opaque);
     }
     shadows += (unsigned)ns;
     uint32_t slot = queue_reserve(b.ctr + 2, (uint32_t)__popc(queued));
@@ -399,25 +408,29 @@ __global__ void __launch_bounds__(256, kAcc ? VP_WF_MIN_BLOCKS : VP_WF_SHADOW_MI
   }
 }
 
+// radiance += weight x T over a path's queries, in their order; an ended path writes its sample.
+__device__ __forceinline__ void gather_path(const ParamsView& P, const WfBuffers& b, uint32_t p) {
+  const uint32_t m = b.meta[p];
+  const int ns = (int)meta_nshadow(m);
+  const float4 r = b.rad4[p];
+  float3 rad = f3(r.x, r.y, r.z);
+  for (int k = 0; k < ns; ++k) {
+    const float4 w = b.sw4[3u * p + k];
+    rad = add(rad, mul(f3(w.x, w.y, w.z), b.so4[3u * p + k].w));
+  }
+  if (m & kAliveBit) {
+    b.rad4[p] = make_float4(rad.x, rad.y, rad.z, 0.f);
+  } else {
+    const float3 L = finalize_sample(P, rad);
+    b.L4[p] = make_float4(L.x, L.y, L.z, 0.f);
+  }
+}
+
 __global__ void __launch_bounds__(256) k_wf_gather(ParamsView P, WfBuffers b, const uint32_t* q,
                                                    const uint32_t* count) {
   const uint32_t n = *count;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t p = q[i];
-    const uint32_t m = b.meta[p];
-    const int ns = (int)meta_nshadow(m);
-    const float4 r = b.rad4[p];
-    float3 rad = f3(r.x, r.y, r.z);
-    for (int k = 0; k < ns; ++k) {
-      const float4 w = b.sw4[3u * p + k];
-      rad = add(rad, mul(f3(w.x, w.y, w.z), b.so4[3u * p + k].w));
-    }
-    if (m & kAliveBit) {
-      b.rad4[p] = make_float4(rad.x, rad.y, rad.z, 0.f);
-    } else {
-      const float3 L = finalize_sample(P, rad);
-      b.L4[p] = make_float4(L.x, L.y, L.z, 0.f);
-    }
+    gather_path(P, b, q[i]);
   }
 }
 
@@ -451,9 +464,9 @@ __device__ __forceinline__ void welford_pixel(const ParamsView& P, const WfBuffe
   count[pix] = prev + batch;
 }
 
-// The end of a batch, one cooperative launch: the paths still queued run to their ends, a warp on each
-// (the warp engine's path loop: no launches, queues or path state in memory between bounces), and once
-// all have finished the pixels' means take the batch's samples.
+// The end of a batch, one cooperative launch: the paths still queued run to their ends, and once all have
+// finished the pixels' means take the batch's samples.  This form, a warp on each path over the BVH32 (the
+// warp engine's path loop), counts and serves scenes too deep for the 8-wide tree.
 template <bool kAcc, bool kMeasure>
 __global__ void __launch_bounds__(256, kTailBlocks) k_wf_tail(SceneView S, EnvView E, ParamsView P, WfBuffers b, const uint32_t* q,
                                                  const uint32_t* count, unsigned int* work, Counters* ctr,
@@ -489,6 +502,145 @@ __global__ void __launch_bounds__(256, kTailBlocks) k_wf_tail(SceneView S, EnvVi
     if (status) break;
   }
   if (lane == 0) flush_stats(ctr, ps, ws, status, measure);
+  cooperative_groups::this_grid().sync();
+  for (uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x; pix < n_pix; pix += gridDim.x * blockDim.x)
+    welford_pixel(P, b, batch, pix, mean, m2, pix_count);
+}
+
+// The same, thread per ray (vp_trace8.cuh): a warp keeps up to `share` of the queued paths and runs its own
+// little wavefront over them -- one traversal for the paths' next free flights and the transmittance
+// queries of their last vertices together, then a lane per path gathers and shades -- so no bounce waits for
+// another warp's.  kMixed: the scene's Gaussians differ in albedo.
+constexpr uint32_t kTailShare = 16;
+struct TailWarp {  // in shared memory, after the traversal's
+  uint32_t path[32];               // this round's paths: flying ones first, then those that only have queries left
+  uint32_t query[3 * kTailShare];  // shadow-query slots to trace
+  uint32_t next;
+};
+template <bool kAcc, bool kMixed>
+__global__ void __launch_bounds__(kT8Threads, kTailBlocks) k_wf_tail8(SceneView S, EnvView E, ParamsView P, WfBuffers b,
+                                                                     const uint32_t* q, const uint32_t* count,
+                                                                     unsigned int* work, Counters* ctr, uint32_t batch,
+                                                                     uint32_t n_pix, float4* __restrict__ mean,
+                                                                     float4* __restrict__ m2,
+                                                                     uint32_t* __restrict__ pix_count) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  uint32_t* smem = reinterpret_cast<uint32_t*>(vp_dyn_smem) + warp * trace8_warp_words(S.depth8);
+  TailWarp& T = reinterpret_cast<TailWarp*>(vp_dyn_smem + trace8_smem_bytes(S.depth8, kT8Threads))[warp];
+  const uint8_t* order = stage_order8();
+  const OneScene8 scene{scene8_of(S)};
+  const uint32_t n = *count, warps = grid_warps();
+  const uint32_t share = min(kTailShare, max(1u, (n + warps - 1u) / warps));
+  uint32_t status = 0, flying = 0, ending = 0, queries = 0;  // the warp's paths and queries in T
+  bool more = n != 0u;
+  unsigned long long opaque = 0;
+  while (true) {
+    if (more && flying + ending < share) {  // (ending paths leave after this round)
+      const uint32_t want = share - flying - ending;
+      uint32_t first = 0;
+      if (lane == 0) first = atomicAdd(work, want);
+      first = __shfl_sync(kFull, first, 0);
+      const uint32_t got = first < n ? min(want, n - first) : 0u;
+      more = first + want < n;
+      // new paths go behind the flying ones, in front of the ending
+      uint32_t keep = 0;
+      if ((uint32_t)lane < ending) keep = T.path[flying + lane];
+      __syncwarp();
+      if ((uint32_t)lane < got) {
+        const uint32_t p = __ldg(q + first + lane);
+        T.path[flying + lane] = p;
+        b.meta[p] &= ~(3u << 16);  // its last vertex's queries are gathered already
+      }
+      if ((uint32_t)lane < ending) T.path[flying + got + lane] = keep;
+      flying += got;
+    }
+    if (flying + ending == 0u) break;
+    if (lane == 0) T.next = 0u;
+    __syncwarp();
+    const uint32_t rays = flying + queries;
+    trace8<kAcc, kBoth8>(
+        scene, S.depth8, smem, order, rays, &T.next, 1u, (int)min(32u, rays), status,
+        [&](uint32_t i, Ray8& ray) {
+          ray.flight = i < flying;
+          if (ray.flight) {
+            const uint32_t p = T.path[i];
+            const uint32_t bounce = meta_bounce(b.meta[p]);
+            const float4 o = b.o4[p], d = b.d4[p];
+            const uint2 k2 = b.key2[p];
+            ray.o = f3(o.x, o.y, o.z);
+            ray.d = f3(d.x, d.y, d.z);
+            ray.key = ((uint64_t)k2.y << 32) | k2.x;
+            ray.seed = bounce ? b.sg[p] : kNoGauss;
+          } else {
+            const uint32_t slot = T.query[i - flying];
+            const float4 o = b.so4[slot], d = b.sd4[slot];
+            ray.o = f3(o.x, o.y, o.z);
+            ray.d = f3(d.x, d.y, d.z);
+            ray.seed = __float_as_uint(d.w);
+            ray.seed_tau = o.w;
+          }
+          return true;
+        },
+        [&](uint32_t i, const Ray8&, const Hit8& h) {
+          if (i < flying) {
+            const uint32_t p = T.path[i];
+            const float3 a = h.t < kInf ? S.albedo : f3(0.f, 0.f, 0.f);
+            b.alb4[p] = make_float4(a.x, a.y, a.z, h.t);
+            b.sg[p] = h.gauss;
+          } else {
+            const float tau = (float)h.w;
+            b.so4[T.query[i - flying]].w = tau >= kMaxOpticalDepth ? 0.0f : expf(-tau);
+          }
+        });
+    __syncwarp();
+    if constexpr (kMixed) {
+      if (lane == 0) T.next = 0u;
+      __syncwarp();
+      trace8<kAcc, kScatter8>(
+          scene, S.depth8, smem, order, flying, &T.next, 1u, (int)min(32u, max(flying, 1u)), status,
+          [&](uint32_t i, Ray8& ray) {
+            const uint32_t p = T.path[i];
+            ray.t = b.alb4[p].w;
+            if (!(ray.t < kInf)) return false;
+            const float4 o = b.o4[p], d = b.d4[p];
+            ray.o = f3(o.x, o.y, o.z);
+            ray.d = f3(d.x, d.y, d.z);
+            return true;
+          },
+          [&](uint32_t i, const Ray8& ray, const Hit8& h) {
+            const float3 a = mean_albedo(h.w, h.r, h.g, h.b);
+            b.alb4[T.path[i]] = make_float4(a.x, a.y, a.z, ray.t);
+          });
+      __syncwarp();
+    }
+    if (__any_sync(kFull, status != 0u)) break;
+    // gather the last vertices' queries, shade the new ones
+    const bool mine = (uint32_t)lane < flying + ending, fly = (uint32_t)lane < flying;
+    const uint32_t p = mine ? T.path[lane] : 0u;
+    int ns = 0;
+    unsigned queued = 0u;
+    bool alive = false;
+    if (mine) gather_path(P, b, p);
+    if (fly) queued = shade_path(S, E, P, b, p, ns, alive, opaque);
+    // a path that ends here without a query to trace is finished at once
+    if (fly && !alive && queued == 0u) gather_path(P, b, p);
+    __syncwarp();
+    const unsigned am = __ballot_sync(kFull, fly && alive), em = __ballot_sync(kFull, fly && !alive && queued != 0u);
+    if ((am >> lane) & 1u) T.path[__popc(am & lt)] = p;
+    if ((em >> lane) & 1u) T.path[__popc(am) + __popc(em & lt)] = p;
+    flying = (uint32_t)__popc(am);
+    ending = (uint32_t)__popc(em);
+    queries = 0u;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const unsigned qm = __ballot_sync(kFull, (queued >> k) & 1u);
+      if ((qm >> lane) & 1u) T.query[queries + __popc(qm & lt)] = 3u * p + k;
+      queries += (uint32_t)__popc(qm);
+    }
+    __syncwarp();
+  }
+  if (status) atomicOr(&ctr->status, status);
   cooperative_groups::this_grid().sync();
   for (uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x; pix < n_pix; pix += gridDim.x * blockDim.x)
     welford_pixel(P, b, batch, pix, mean, m2, pix_count);
@@ -629,7 +781,7 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
   auto shd8 = P.accurate ? k_wf_shadow8<true> : k_wf_shadow8<false>;
   int ext8_blocks = 0, shd8_blocks = 0;
   if (use8) {
-    if (smem8 > 48 * 1024)
+    if (smem8 > kSmem8Default)
       for (auto k : {(const void*)ext8, (const void*)shd8})
         VP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem8));
     ext8_blocks = ctx->sm_count * resident_blocks(ext8, kT8Threads, smem8);
@@ -671,7 +823,14 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
                                   inv_ext1(si.bounds_min[2], si.bounds_max[2]));
   auto tail = P.accurate ? (P.measure ? k_wf_tail<true, true> : k_wf_tail<true, false>)
                          : (P.measure ? k_wf_tail<false, true> : k_wf_tail<false, false>);
-  if (smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  size_t smem_tail = smem;
+  if (use8) {
+    tail = P.accurate ? (mixed ? k_wf_tail8<true, true> : k_wf_tail8<true, false>)
+                      : (mixed ? k_wf_tail8<false, true> : k_wf_tail8<false, false>);
+    smem_tail = smem8 + (kT8Threads / 32) * sizeof(TailWarp);
+  }
+  if (smem_tail > kSmem8Default)
+    VP_CUDA(cudaFuncSetAttribute(tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_tail));
   uint32_t polled = paths;
   for (uint32_t it = 0; it < P.max_bounces; ++it) {
     // Few paths left (the count last read), or none that can be (a scatter in an albedo-0 scene ends its
@@ -724,8 +883,8 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
     ParamsView tP = P;
     uint32_t tbatch = spp_count, tpix = n_pix;
     void* args[] = {&tS, &tE, &tP, &b, &qcur, &tcount, &twork, &tctr, &tbatch, &tpix, &img->mean, &img->m2, &img->count};
-    VP_CUDA(cudaLaunchCooperativeKernel((const void*)tail, dim3(ctx->sm_count * resident_blocks(tail, threads, smem)),
-                                        dim3(threads), args, smem, st));
+    VP_CUDA(cudaLaunchCooperativeKernel((const void*)tail, dim3(ctx->sm_count * resident_blocks(tail, threads, smem_tail)),
+                                        dim3(threads), args, smem_tail, st));
   }
   ctx->launches += 1;
   if (timed && pending) {

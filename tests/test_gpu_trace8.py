@@ -16,7 +16,7 @@ from volprim_b200 import scenes
 
 pytestmark = pytest.mark.gpu
 
-W, H = 409, 281  # 114,929 paths: more than one refill of every warp; the tail kernel takes the last 8,192
+W, H = 409, 281  # 114,929 paths: more than one refill of every warp; the tail kernel takes the last 65,536
 
 
 def gaussians(n, seed, layout="box", mixed=True):
@@ -60,6 +60,15 @@ def check(a, b):
 @pytest.mark.parametrize("mixed", [False, True])
 def test_sizes(vp_ctx, n, mixed):
     check(*images(vp_ctx, gaussians(n, n, mixed=mixed), hg_g=0.6))
+
+
+@pytest.mark.parametrize("w, h", [(1, 1), (3, 1), (31, 3), (67, 41), (211, 250)])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_tail(vp_ctx, monkeypatch, w, h, mixed):
+    """Images whose paths all go to the tail after their first bounce: from one path to 22 a warp."""
+    monkeypatch.setitem(globals(), "W", w)
+    monkeypatch.setitem(globals(), "H", h)
+    check(*images(vp_ctx, gaussians(400, 12, mixed=mixed), sigma=2.0, hg_g=0.3, camera=scenes.negz_camera(1.2, 30.0)))
 
 
 @pytest.mark.parametrize("layout", ["nested", "same", "spread", "plate"])

@@ -54,17 +54,20 @@ void dev_free(T*& p, cudaStream_t s) {
 }  // namespace vp
 
 namespace vp {
-// Wavefront path state (structure of arrays, one entry per path of a launch batch) and queues.
-struct WfBuffers {
-  float4 *o4, *d4, *thr4, *rad4;  // ray origin / direction / throughput / radiance (.w unused)
-  uint4* rng4;                    // PCG32 state (lo, hi) and increment (lo, hi)
-  uint2* key2;                    // free-flight key of the next bounce
-  uint32_t* meta;                 // bounce | shadow count << 16 | alive << 18
-  float4* alb4;                   // albedo at the scatter point, scatter distance
-  uint32_t* sg;                   // the Gaussian of the scatter (scene order) or kNoGauss
-  float4 *so4, *sd4, *sw4;        // 3 transmittance queries per path: origin (.w: the seed chord's
-                                  // optical depth, -1 without a seed; then T), dir (+ the
-                                  // seed Gaussian's bits in .w), weight
+// The state of paths in flight (wavefront and serving engines; accessors in vp_pathstore.cuh).  What a stage
+// needs of a path lies in whole 32-byte sectors: after the first bounces the queues hold paths in the order of
+// their places in the scene, and every field that is an array of its own costs a sector a path.
+struct PathStore {
+  float4* ray;  // 2 per path: origin, direction; the free-flight key of the next bounce (lo, hi) in their .w
+  float4* st;   // 4 per path: throughput (.w: bounce | shadow count << 16 | alive << 18 | request << 19); radiance
+                // (.w: the Gaussian of the scatter, scene order, or kNoGauss); PCG32 state (lo, hi) and
+                // increment (lo, hi); albedo at the scatter point, scatter distance
+  float4* sq;   // 3 transmittance queries per path, 2 each: origin (.w: the seed chord's optical depth, -1
+                // without a seed), direction (.w: the seed Gaussian's bits)
+  float4* sw;   // the queries' weights; T in .w
+};
+// The wavefront engine's paths and queues.
+struct WfBuffers : PathStore {
   float4* L4;                     // finished sample radiance
   uint32_t *qa, *qb, *qs;         // path queues (current / next) and shadow-query queue
   uint32_t* sk_a;                 // sorting: the Morton keys of path origins

@@ -38,13 +38,12 @@
 #include <vector>
 
 #include "vp_internal.h"
-#include "vp_path.cuh"
+#include "vp_pathstore.cuh"
 #include "vp_trace8.cuh"
 
 namespace vp {
 namespace {
 
-constexpr uint32_t kAlive = 1u << 18;
 constexpr int kSrvHitCap = 64;        // extend hit buffer, as the offline wavefront's
 constexpr uint32_t kMaxScenes = 64;
 constexpr uint32_t kMaxRequests = 1024;  // the share computation is one block
@@ -70,54 +69,10 @@ struct SrvCtl {  // device control block of the iteration
   unsigned long long total_started;  // paths the lane has started (the clock of SRPT aging)
 };
 
-struct SrvPaths {  // per path slot
-  float4 *o4, *d4, *thr4, *rad4, *alb4;
-  uint32_t* sg;  // the Gaussian of the scatter (scene order) or kNoGauss
-  uint4* rng4;
-  uint2* key2;
-  uint32_t* meta;  // bounce | shadow count << 16 | alive << 18
-  uint32_t *req, *pix;
-  float4 *so4, *sd4, *sw4;  // 3 transmittance queries per slot
+struct SrvPaths : PathStore {  // per path slot; the meta word's upper bits name the request-table entry
+  uint32_t* pix;
   uint32_t *qa, *qb, *qs, *free_stack;
 };
-
-__device__ __forceinline__ void srv_store(const SrvPaths& b, uint32_t p, const PathState& s) {
-  b.o4[p] = make_float4(s.o.x, s.o.y, s.o.z, 0.f);
-  b.d4[p] = make_float4(s.d.x, s.d.y, s.d.z, 0.f);
-  b.thr4[p] = make_float4(s.thr.x, s.thr.y, s.thr.z, 0.f);
-  b.rad4[p] = make_float4(s.rad.x, s.rad.y, s.rad.z, 0.f);
-  b.rng4[p] = make_uint4((uint32_t)s.rng.state, (uint32_t)(s.rng.state >> 32), (uint32_t)s.rng.inc,
-                         (uint32_t)(s.rng.inc >> 32));
-}
-
-__device__ __forceinline__ PathState srv_load(const SrvPaths& b, uint32_t p, uint32_t bounce) {
-  PathState s;
-  const float4 o = b.o4[p], d = b.d4[p], t = b.thr4[p], r = b.rad4[p];
-  const uint4 g = b.rng4[p];
-  s.o = f3(o.x, o.y, o.z);
-  s.d = f3(d.x, d.y, d.z);
-  s.thr = f3(t.x, t.y, t.z);
-  s.rad = f3(r.x, r.y, r.z);
-  s.rng.state = ((uint64_t)g.y << 32) | g.x;
-  s.rng.inc = ((uint64_t)g.w << 32) | g.z;
-  s.bounce = bounce;
-  return s;
-}
-
-// Warp-aggregated queue append (all 32 lanes call it): this lane's first slot for n entries.
-__device__ __forceinline__ uint32_t srv_reserve(uint32_t* counter, uint32_t n) {
-  const int lane = threadIdx.x & 31;
-  uint32_t incl = n;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o) incl += v;
-  }
-  const uint32_t total = __shfl_sync(kFull, incl, 31);
-  uint32_t base = 0;
-  if (lane == 31 && total) base = atomicAdd(counter, total);
-  base = __shfl_sync(kFull, base, 31);
-  return base + incl - n;
-}
 
 __global__ void k_srv_init(SrvCtl* c, uint32_t* free_stack, uint32_t slots) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -291,10 +246,7 @@ __global__ void k_srv_regen(const SrvCtl* __restrict__ c, const SrvRequest* __re
     const uint32_t pix = (uint32_t)(local / spp), s = (uint32_t)(local % spp);
     PathState st = start_path(r.cam, r.P, pix % r.P.width, pix / r.P.width, s);
     const uint64_t key = draw_bounce_key(st.rng);
-    srv_store(b, slot, st);
-    b.key2[slot] = make_uint2((uint32_t)key, (uint32_t)(key >> 32));
-    b.meta[slot] = kAlive;
-    b.req[slot] = e;
+    store_path(b, slot, st, key, kAliveBit | (e << 19), kNoGauss);
     b.pix[slot] = pix;
     q[surv + i] = slot;
   }
@@ -317,27 +269,24 @@ __global__ void __launch_bounds__(256, 4) k_srv_extend(const SceneView* __restri
     item = __shfl_sync(kFull, item, 0);
     if (item >= n) break;
     const uint32_t p = __ldg(q + item);
-    const SceneView S = scenes[table[b.req[p]].scene];
-    const float4 o = b.o4[p], d = b.d4[p];
-    const uint2 k2 = b.key2[p];
-    const uint32_t bounce = b.meta[p] & 0xFFFFu;
-    const float3 of = f3(o.x, o.y, o.z), df = f3(d.x, d.y, d.z);
+    const uint32_t meta = path_meta(b, p), bounce = meta_bounce(meta);
+    const SceneView S = scenes[table[meta_request(meta)].scene];
+    float3 of, df;
+    uint64_t key;
+    path_ray(b, p, of, df, key);
     float tstar = kInf;
     ScatterAlbedo sa;
     sa.valid = false;
     if (!(bounce == 0 && S.albedo_all_zero))
-      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, ((uint64_t)k2.y << 32) | k2.x, status, ws, false, &sa,
-                                             bounce ? b.sg[p] : kNoGauss);
+      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, key, status, ws, false, &sa,
+                                             bounce ? path_gauss(b, p) : kNoGauss);
     float3 albedo = f3(0.f, 0.f, 0.f);
     if (tstar < kInf) {
       uint32_t ov = sa.overlap;
       albedo = sa.valid ? sa.albedo : warp_scatter_albedo<kAcc>(S, W, of, df, tstar, ov, status, ws, false);
       if (S.one_albedo) albedo = S.albedo;
     }
-    if (lane == 0) {
-      b.alb4[p] = make_float4(albedo.x, albedo.y, albedo.z, tstar);
-      b.sg[p] = tstar < kInf ? sa.gauss : kNoGauss;
-    }
+    if (lane == 0) set_scatter(b, p, albedo, tstar, tstar < kInf ? sa.gauss : kNoGauss);
     if (status) break;
   }
   if (lane == 0 && status) atomicOr(&ctr->status, status);
@@ -365,38 +314,31 @@ __global__ void __launch_bounds__(kT8Threads, kMixed ? 2 : kT8Blocks) k_srv_exte
       many, depth, smem, c->ctr[0], &c->ctr[3], status,
       [&](uint32_t item, Ray8& ray) {
         const uint32_t p = __ldg(q + item);
-        ray.scene = table[b.req[p]].scene;
-        const uint32_t bounce = b.meta[p] & 0xFFFFu;
+        const uint32_t meta = path_meta(b, p), bounce = meta_bounce(meta);
+        ray.scene = table[meta_request(meta)].scene;
         if (bounce == 0u && scenes[ray.scene].albedo_all_zero) {
-          b.alb4[p] = make_float4(0.f, 0.f, 0.f, kInf);
-          b.sg[p] = kNoGauss;
+          set_scatter(b, p, f3(0.f, 0.f, 0.f), kInf, kNoGauss);
           return false;
         }
-        const float4 o = b.o4[p], d = b.d4[p];
-        const uint2 k2 = b.key2[p];
-        ray.o = f3(o.x, o.y, o.z);
-        ray.d = f3(d.x, d.y, d.z);
-        ray.key = ((uint64_t)k2.y << 32) | k2.x;
-        ray.seed = bounce ? b.sg[p] : kNoGauss;
+        path_ray(b, p, ray.o, ray.d, ray.key);
+        ray.seed = bounce ? path_gauss(b, p) : kNoGauss;
         return true;
       },
       [&](uint32_t item, const Ray8& ray, const Hit8& h) {
         const uint32_t p = __ldg(q + item);
-        const float3 a = h.t < kInf ? scenes[ray.scene].albedo : f3(0.f, 0.f, 0.f);
-        b.alb4[p] = make_float4(a.x, a.y, a.z, h.t);
-        b.sg[p] = h.gauss;
+        set_scatter(b, p, h.t < kInf ? scenes[ray.scene].albedo : f3(0.f, 0.f, 0.f), h.t, h.gauss);
       },
       [&](uint32_t item, Ray8& ray) {
         const uint32_t p = __ldg(q + item);
-        ray.scene = table[b.req[p]].scene;
-        ray.t = b.alb4[p].w;
+        ray.scene = table[meta_request(path_meta(b, p))].scene;
+        ray.t = path_scatter_t(b, p);
         if (!(ray.t < kInf) || scenes[ray.scene].one_albedo) return false;
-        const float4 o = b.o4[p], d = b.d4[p];
-        ray.o = f3(o.x, o.y, o.z);
-        ray.d = f3(d.x, d.y, d.z);
+        path_ray(b, p, ray.o, ray.d, ray.key);
         return true;
       },
-      [&](uint32_t item, const Ray8& ray, float3 a) { b.alb4[__ldg(q + item)] = make_float4(a.x, a.y, a.z, ray.t); });
+      [&](uint32_t item, const Ray8& ray, float3 a) {
+        b.st[4u * __ldg(q + item) + 3u] = make_float4(a.x, a.y, a.z, ray.t);
+      });
   if (status) atomicOr(&ctr->status, status);
 }
 
@@ -412,18 +354,11 @@ __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_srv_shadow8(const Sce
       many, depth, smem, stage_order8(), n, &c->ctr[4], grid_warps(), rays_per_warp(n, grid_warps()), status,
       [&](uint32_t item, Ray8& ray) {
         const uint32_t slot = __ldg(b.qs + item);
-        ray.scene = table[b.req[slot / 3u]].scene;
-        const float4 o = b.so4[slot], d = b.sd4[slot];
-        ray.o = f3(o.x, o.y, o.z);
-        ray.d = f3(d.x, d.y, d.z);
-        ray.seed = __float_as_uint(d.w);
-        ray.seed_tau = o.w;
+        ray.scene = table[meta_request(path_meta(b, slot / 3u))].scene;
+        query_ray(b, slot, ray.o, ray.d, ray.seed, ray.seed_tau);
         return true;
       },
-      [&](uint32_t item, const Ray8&, const Hit8& h) {
-        const float tau = (float)h.w;
-        b.so4[__ldg(b.qs + item)].w = tau >= kMaxOpticalDepth ? 0.0f : expf(-tau);
-      });
+      [&](uint32_t item, const Ray8&, const Hit8& h) { set_transmittance(b, __ldg(b.qs + item), (float)h.w); });
   if (status) atomicOr(&ctr->status, status);
 }
 
@@ -444,36 +379,16 @@ __global__ void __launch_bounds__(256) k_srv_shade(const SceneView* __restrict__
     int ns = 0;
     unsigned queued = 0u;
     bool alive = false;
+    unsigned long long opaque = 0;
     if (i < n) {
       p = q[i];
-      const SrvRequest& r = table[b.req[p]];
-      PathState s = srv_load(b, p, b.meta[p] & 0xFFFFu);
-      const float4 a = b.alb4[p];
-      ShadowSet sh;
-      alive = shade_bounce(envs[r.scene], r.P, s, a.w < kInf, a.w, f3(a.x, a.y, a.z), sh, b.sg[p]);
-      ns = sh.n;
-      for (int k = 0; k < sh.n; ++k) {
-        float seed_tau = -1.0f;  // no seed
-        if (sh.seed[k] != kNoGauss)
-          seed_tau = r.P.accurate ? seed_chord_tau<true>(scenes[r.scene], sh.seed[k], sh.o[k], sh.d[k])
-                                  : seed_chord_tau<false>(scenes[r.scene], sh.seed[k], sh.o[k], sh.d[k]);
-        const bool opaque_k = seed_tau >= kMaxOpticalDepth;
-        b.so4[3u * p + k] = make_float4(sh.o[k].x, sh.o[k].y, sh.o[k].z, opaque_k ? 0.0f : seed_tau);
-        b.sd4[3u * p + k] = make_float4(sh.d[k].x, sh.d[k].y, sh.d[k].z, __uint_as_float(sh.seed[k]));
-        b.sw4[3u * p + k] = make_float4(sh.w[k].x, sh.w[k].y, sh.w[k].z, 0.f);
-        if (!opaque_k) queued |= 1u << k;
-      }
-      if (alive) {
-        const uint64_t key = draw_bounce_key(s.rng);
-        b.key2[p] = make_uint2((uint32_t)key, (uint32_t)(key >> 32));
-      }
-      srv_store(b, p, s);
-      b.meta[p] = (s.bounce & 0xFFFFu) | ((uint32_t)sh.n << 16) | (alive ? kAlive : 0u);
+      const SrvRequest& r = table[meta_request(path_meta(b, p))];
+      queued = shade_path(scenes[r.scene], envs[r.scene], r.P, b, p, ns, alive, opaque);
     }
-    uint32_t slot = srv_reserve(&c->ctr[2], (uint32_t)__popc(queued));
+    uint32_t slot = queue_reserve(&c->ctr[2], (uint32_t)__popc(queued));
     for (int k = 0; k < ns; ++k)
       if (queued & (1u << k)) b.qs[slot++] = 3u * p + k;
-    const uint32_t qslot = srv_reserve(&c->ctr[1], alive ? 1u : 0u);
+    const uint32_t qslot = queue_reserve(&c->ctr[1], alive ? 1u : 0u);
     if (alive) qnext[qslot] = p;
   }
 }
@@ -494,11 +409,13 @@ __global__ void __launch_bounds__(256, 4) k_srv_shadow(const SceneView* __restri
     item = __shfl_sync(kFull, item, 0);
     if (item >= n) break;
     const uint32_t qslot = __ldg(b.qs + item);
-    const SceneView S = scenes[table[b.req[qslot / 3u]].scene];
-    const float4 o = b.so4[qslot], d = b.sd4[qslot];
-    const float tau = warp_ray_query<kAcc, kTau>(S, W, f3(o.x, o.y, o.z), f3(d.x, d.y, d.z), 0ull, status, ws, false,
-                                                 nullptr, __float_as_uint(d.w), o.w);
-    if (lane == 0) b.so4[qslot].w = tau >= kMaxOpticalDepth ? 0.0f : expf(-tau);
+    const SceneView S = scenes[table[meta_request(path_meta(b, qslot / 3u))].scene];
+    float3 o, d;
+    uint32_t seed;
+    float seed_tau;
+    query_ray(b, qslot, o, d, seed, seed_tau);
+    const float tau = warp_ray_query<kAcc, kTau>(S, W, o, d, 0ull, status, ws, false, nullptr, seed, seed_tau);
+    if (lane == 0) set_transmittance(b, qslot, tau);
     if (status) break;
   }
   if (lane == 0 && status) atomicOr(&ctr->status, status);
@@ -510,18 +427,9 @@ __global__ void __launch_bounds__(256) k_srv_gather(const SrvRequest* __restrict
   const uint32_t n = c->ctr[0];
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint32_t p = q[i];
-    const uint32_t m = b.meta[p];
-    const int ns = (int)((m >> 16) & 3u);
-    const float4 r4 = b.rad4[p];
-    float3 rad = f3(r4.x, r4.y, r4.z);
-    for (int k = 0; k < ns; ++k) {
-      const float4 w = b.sw4[3u * p + k];
-      rad = add(rad, mul(f3(w.x, w.y, w.z), b.so4[3u * p + k].w));
-    }
-    if (m & kAlive) {
-      b.rad4[p] = make_float4(rad.x, rad.y, rad.z, 0.f);
-    } else {
-      const uint32_t e = b.req[p];
+    float3 rad;
+    if (!gather_radiance(b, p, rad)) {
+      const uint32_t e = meta_request(path_meta(b, p));
       const SrvRequest& r = table[e];
       const float3 L = finalize_sample(r.P, rad);
       atomicAdd(r.sum + b.pix[p], make_float4(L.x, L.y, L.z, 0.f));
@@ -551,7 +459,7 @@ void srv_carve(char*& cur, T*& out, size_t count) {
   cur += (count * sizeof(T) + 255) & ~size_t(255);
 }
 
-constexpr size_t kSlotBytes = 5 * 16 + 4 + 16 + 8 + 4 + 4 + 4 + 3 * 48 + 4 * 2 + 3 * 4 + 4;
+constexpr size_t kSlotBytes = 2 * 16 + 4 * 16 + 3 * 48 + 4 + 4 * 2 + 3 * 4 + 4;
 
 }  // namespace
 }  // namespace vp
@@ -1098,20 +1006,11 @@ vp_status vp_server_create(vp_context* ctx, const vp_server_config* config, vp_s
   vp_server::Lane& L = s->lanes[l];
   char* cur = static_cast<char*>(L.path_mem);
   SrvPaths& b = L.paths;
-  srv_carve(cur, b.o4, P);
-  srv_carve(cur, b.d4, P);
-  srv_carve(cur, b.thr4, P);
-  srv_carve(cur, b.rad4, P);
-  srv_carve(cur, b.alb4, P);
-  srv_carve(cur, b.sg, P);
-  srv_carve(cur, b.rng4, P);
-  srv_carve(cur, b.key2, P);
-  srv_carve(cur, b.meta, P);
-  srv_carve(cur, b.req, P);
+  srv_carve(cur, b.ray, 2ull * P);
+  srv_carve(cur, b.st, 4ull * P);
+  srv_carve(cur, b.sq, 6ull * P);
+  srv_carve(cur, b.sw, 3ull * P);
   srv_carve(cur, b.pix, P);
-  srv_carve(cur, b.so4, 3ull * P);
-  srv_carve(cur, b.sd4, 3ull * P);
-  srv_carve(cur, b.sw4, 3ull * P);
   srv_carve(cur, b.qa, P);
   srv_carve(cur, b.qb, P);
   srv_carve(cur, b.qs, 3ull * P);

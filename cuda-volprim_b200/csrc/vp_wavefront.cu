@@ -3,17 +3,17 @@
 //
 //   generate  (thread per path)  camera ray, PCG32 stream, first free-flight key
 //   per bounce, while any path is alive:
-//     extend  (warp per path)    free-flight argmin over the BVH32 + albedo at the scatter point
+//     extend  (thread per path)  free-flight argmin over the 8-wide BVH + albedo at the scatter point
 //     shade   (thread per path)  phase sample, NEE sampling, escape rule, roulette; compacts
 //                                surviving paths into the next queue and the bounce's
 //                                transmittance queries into the shadow queue
-//     shadow  (warp per query)   transmittance over the BVH32 with early exit at tau >= 88
+//     shadow  (thread per query) transmittance over the 8-wide BVH with early exit at tau >= 88
 //     gather  (thread per path)  radiance += weight x T in query order; finished paths write
 //                                their sample
 //   tail      (a few paths a warp) once few paths are left: they run to their ends in one launch; then, a
 //                                thread per pixel, the running mean over the batch's samples in order
 //
-//   extend and shadow run thread per ray over the compressed 8-wide BVH (vp_trace8.cuh); the scatter-point
+//   extend, shadow and tail run thread per ray over the compressed 8-wide BVH (vp_trace8.cuh); the scatter-point
 //   albedo is then the scene's, when all its Gaussians share one, or a second traversal.
 //   Their warp-per-ray forms over the BVH32 give the same results: they count (VP_MEASURE_COUNTERS) and
 //   serve scenes too deep for the 8-wide tree.
@@ -22,8 +22,8 @@
 // resident per SM to hide the latency of the dependent node loads.  The reference found a
 // wavefront 100x slower than its megakernel because ~352 B of per-ray sets and hit buffers
 // streamed through DRAM each bounce (latex/chapters/06-optimization.tex:438-446); here no hit
-// buffer or active set survives a stage (the queries rebuild them from geometry), so a path
-// carries ~290 B in total and the traffic is negligible next to the traversal.  Results are
+// buffer or active set survives a stage (the queries rebuild them from geometry), and the ~280 B a
+// path carries are laid out by what the stages read together (vp_pathstore.cuh).  Results are
 // those of the warp engine: the same shading code (vp_path.cuh), the same queries, and the
 // same order of radiance accumulation.
 #include <algorithm>
@@ -32,17 +32,15 @@
 
 #include "vp_internal.h"
 #include "vp_pathloop.cuh"
+#include "vp_pathstore.cuh"
 #include "vp_trace8.cuh"
 
 namespace vp {
 namespace {
 
-constexpr uint32_t kAliveBit = 1u << 18;
-
-// Resident 256-thread blocks per SM the extend / shadow kernels' register budgets are sized for:
-// 4 (64 registers) for extend; 5 (48 registers, 52 B of spills) for the FP32 shadow kernel, whose
-// smaller state gains more from the extra warps than it loses to the spills (-2% shadow time on
-// the showcase; extend at 5 spills 116 B and loses 9%).  The ACCURATE (float-pair) shadow kernel keeps
+// Resident 256-thread blocks per SM the warp-per-ray extend / shadow kernels' register budgets are sized for:
+// 4 (64 registers) for extend; 5 (48 registers, some spills) for the FP32 shadow kernel, whose
+// smaller state gains more from the extra warps than it loses to the spills.  The ACCURATE shadow kernel keeps
 // the extend budget.
 #ifndef VP_WF_MIN_BLOCKS
 #define VP_WF_MIN_BLOCKS 4
@@ -70,47 +68,7 @@ constexpr uint32_t kTailMax = 65536;
 // 2.8 (500k).
 constexpr int kTailBlocks = 2;
 
-__device__ __forceinline__ uint32_t meta_bounce(uint32_t m) { return m & 0xFFFFu; }
-__device__ __forceinline__ uint32_t meta_nshadow(uint32_t m) { return (m >> 16) & 3u; }
 
-__device__ __forceinline__ void store_path(const WfBuffers& b, uint32_t p, const PathState& s) {
-  b.o4[p] = make_float4(s.o.x, s.o.y, s.o.z, 0.f);
-  b.d4[p] = make_float4(s.d.x, s.d.y, s.d.z, 0.f);
-  b.thr4[p] = make_float4(s.thr.x, s.thr.y, s.thr.z, 0.f);
-  b.rad4[p] = make_float4(s.rad.x, s.rad.y, s.rad.z, 0.f);
-  b.rng4[p] = make_uint4((uint32_t)s.rng.state, (uint32_t)(s.rng.state >> 32), (uint32_t)s.rng.inc,
-                         (uint32_t)(s.rng.inc >> 32));
-}
-
-__device__ __forceinline__ PathState load_path(const WfBuffers& b, uint32_t p, uint32_t bounce) {
-  PathState s;
-  const float4 o = b.o4[p], d = b.d4[p], t = b.thr4[p], r = b.rad4[p];
-  const uint4 g = b.rng4[p];
-  s.o = f3(o.x, o.y, o.z);
-  s.d = f3(d.x, d.y, d.z);
-  s.thr = f3(t.x, t.y, t.z);
-  s.rad = f3(r.x, r.y, r.z);
-  s.rng.state = ((uint64_t)g.y << 32) | g.x;
-  s.rng.inc = ((uint64_t)g.w << 32) | g.z;
-  s.bounce = bounce;
-  return s;
-}
-
-// Warp-aggregated queue append, called by all 32 lanes: returns this lane's first slot for its
-// `n` (possibly 0) entries; one atomic per warp.
-__device__ __forceinline__ uint32_t queue_reserve(uint32_t* counter, uint32_t n) {
-  const int lane = threadIdx.x & 31;
-  uint32_t incl = n;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t v = __shfl_up_sync(kFull, incl, o);
-    if (lane >= o) incl += v;
-  }
-  const uint32_t total = __shfl_sync(kFull, incl, 31);
-  uint32_t base = 0;
-  if (lane == 31 && total) base = atomicAdd(counter, total);
-  base = __shfl_sync(kFull, base, 31);
-  return base + incl - n;
-}
 
 // Path p is sample p % batch of pixel p / batch.  Without adaptive sampling every path starts
 // and queue slot p holds path p.  With it, the host has cleared the counters and only the paths
@@ -140,9 +98,7 @@ __global__ void k_wf_generate(CameraView C, ParamsView P, uint32_t spp_offset, u
   const uint32_t pixel = p / batch, s = p % batch;
   PathState st = start_path(C, P, pixel % P.width, pixel / P.width, (uint64_t)spp_offset + s);
   const uint64_t key = draw_bounce_key(st.rng);
-  store_path(b, p, st);
-  b.key2[p] = make_uint2((uint32_t)key, (uint32_t)(key >> 32));
-  b.meta[p] = 0u | kAliveBit;
+  store_path(b, p, st, key, kAliveBit, kNoGauss);
   b.qa[slot] = p;
   b.L4[p] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
@@ -172,16 +128,16 @@ __global__ void __launch_bounds__(256, VP_WF_MIN_BLOCKS) k_wf_extend(SceneView S
     item = __shfl_sync(kFull, item, 0);
     if (item >= n) break;
     const uint32_t p = __ldg(q + item);
-    const float4 o = b.o4[p], d = b.d4[p];
-    const uint2 k2 = b.key2[p];
-    const uint32_t bounce = meta_bounce(b.meta[p]);
-    const float3 of = f3(o.x, o.y, o.z), df = f3(d.x, d.y, d.z);
+    const uint32_t bounce = meta_bounce(path_meta(b, p));
+    float3 of, df;
+    uint64_t key;
+    path_ray(b, p, of, df, key);
     float tstar = kInf;
     ScatterAlbedo sa;
     sa.valid = false;
     if (!(bounce == 0 && S.albedo_all_zero))
-      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, ((uint64_t)k2.y << 32) | k2.x, status, ws, measure, &sa,
-                                             bounce ? b.sg[p] : kNoGauss);
+      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, key, status, ws, measure, &sa,
+                                             bounce ? path_gauss(b, p) : kNoGauss);
     float3 albedo = f3(0.f, 0.f, 0.f);
     if (tstar < kInf) {
       uint32_t ov = sa.overlap;
@@ -191,10 +147,7 @@ __global__ void __launch_bounds__(256, VP_WF_MIN_BLOCKS) k_wf_extend(SceneView S
       ++scatters;
     }
     ++bounces;
-    if (lane == 0) {
-      b.alb4[p] = make_float4(albedo.x, albedo.y, albedo.z, tstar);
-      b.sg[p] = tstar < kInf ? sa.gauss : kNoGauss;
-    }
+    if (lane == 0) set_scatter(b, p, albedo, tstar, tstar < kInf ? sa.gauss : kNoGauss);
     if (status) break;
   }
   if (lane == 0) {
@@ -229,36 +182,29 @@ __global__ void __launch_bounds__(kT8Threads, kMixed ? 2 : kT8Blocks) k_wf_exten
       OneScene8{scene8_of(S)}, S.depth8, smem, *count, work, status,
       [&](uint32_t item, Ray8& ray) {
         const uint32_t p = __ldg(q + item);
-        const uint32_t bounce = meta_bounce(b.meta[p]);
+        const uint32_t bounce = meta_bounce(path_meta(b, p));
         if (S.albedo_all_zero && bounce == 0u) {  // a scatter would end the path with nothing
-          b.alb4[p] = make_float4(0.f, 0.f, 0.f, kInf);
-          b.sg[p] = kNoGauss;
+          set_scatter(b, p, f3(0.f, 0.f, 0.f), kInf, kNoGauss);
           return false;
         }
-        const float4 o = b.o4[p], d = b.d4[p];
-        const uint2 k2 = b.key2[p];
-        ray.o = f3(o.x, o.y, o.z);
-        ray.d = f3(d.x, d.y, d.z);
-        ray.key = ((uint64_t)k2.y << 32) | k2.x;
-        ray.seed = bounce ? b.sg[p] : kNoGauss;
+        path_ray(b, p, ray.o, ray.d, ray.key);
+        ray.seed = bounce ? path_gauss(b, p) : kNoGauss;
         return true;
       },
       [&](uint32_t item, const Ray8&, const Hit8& h) {
         const uint32_t p = __ldg(q + item);
-        const float3 a = h.t < kInf ? S.albedo : f3(0.f, 0.f, 0.f);
-        b.alb4[p] = make_float4(a.x, a.y, a.z, h.t);
-        b.sg[p] = h.gauss;
+        set_scatter(b, p, h.t < kInf ? S.albedo : f3(0.f, 0.f, 0.f), h.t, h.gauss);
       },
       [&](uint32_t item, Ray8& ray) {
         const uint32_t p = __ldg(q + item);
-        ray.t = b.alb4[p].w;
+        ray.t = path_scatter_t(b, p);
         if (!(ray.t < kInf)) return false;
-        const float4 o = b.o4[p], d = b.d4[p];
-        ray.o = f3(o.x, o.y, o.z);
-        ray.d = f3(d.x, d.y, d.z);
+        path_ray(b, p, ray.o, ray.d, ray.key);
         return true;
       },
-      [&](uint32_t item, const Ray8& ray, float3 a) { b.alb4[__ldg(q + item)] = make_float4(a.x, a.y, a.z, ray.t); });
+      [&](uint32_t item, const Ray8& ray, float3 a) {
+        b.st[4u * __ldg(q + item) + 3u] = make_float4(a.x, a.y, a.z, ray.t);
+      });
   if (status) atomicOr(&ctr->status, status);
 }
 
@@ -271,58 +217,16 @@ __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_wf_shadow8(SceneView 
   trace8<kAcc, kTau8>(
       OneScene8{scene8_of(S)}, S.depth8, smem, stage_order8(), n, work, grid_warps(), rays_per_warp(n, grid_warps()), status,
       [&](uint32_t item, Ray8& ray) {
-        const uint32_t slot = __ldg(b.qs + item);
-        const float4 o = b.so4[slot], d = b.sd4[slot];
-        ray.o = f3(o.x, o.y, o.z);
-        ray.d = f3(d.x, d.y, d.z);
-        ray.seed = __float_as_uint(d.w);
-        ray.seed_tau = o.w;
+        query_ray(b, __ldg(b.qs + item), ray.o, ray.d, ray.seed, ray.seed_tau);
         return true;
       },
-      [&](uint32_t item, const Ray8&, const Hit8& h) {
-        const float tau = (float)h.w;
-        b.so4[__ldg(b.qs + item)].w = tau >= kMaxOpticalDepth ? 0.0f : expf(-tau);
-      });
+      [&](uint32_t item, const Ray8&, const Hit8& h) { set_transmittance(b, __ldg(b.qs + item), (float)h.w); });
   if (status) atomicOr(&ctr->status, status);
 }
 
-// A path's vertex, by one thread: phase sample, NEE and roulette; the path's next ray, its transmittance
-// queries (so4, sd4, sw4) and its meta word.  Returns which of the queries need a traversal (bit k) and sets
-// ns and alive.  The shadow rays' seed chords are evaluated here, one thread per ray (seed_chord_tau): a ray
-// whose seed chord alone reaches MAX_OPTICAL_DEPTH gets T = 0 at once; the others carry the seed's optical
-// depth to the query in so4.w.
-__device__ __forceinline__ unsigned shade_path(const SceneView& S, const EnvView& E, const ParamsView& P,
-                                               const WfBuffers& b, uint32_t p, int& ns, bool& alive,
-                                               unsigned long long& opaque) {
-  PathState s = load_path(b, p, meta_bounce(b.meta[p]));
-  const float4 a = b.alb4[p];
-  const bool scattered = a.w < kInf;
-  ShadowSet sh;
-  alive = shade_bounce(E, P, s, scattered, a.w, f3(a.x, a.y, a.z), sh, b.sg[p]);
-  ns = sh.n;
-  unsigned queued = 0u;
-  for (int k = 0; k < sh.n; ++k) {
-    float seed_tau = -1.0f;  // no seed
-    if (sh.seed[k] != kNoGauss)
-      seed_tau = P.accurate ? seed_chord_tau<true>(S, sh.seed[k], sh.o[k], sh.d[k])
-                            : seed_chord_tau<false>(S, sh.seed[k], sh.o[k], sh.d[k]);
-    const bool opaque_k = seed_tau >= kMaxOpticalDepth;
-    // .w of the origin: the seed's optical depth for the query, or T = 0 already
-    b.so4[3u * p + k] = make_float4(sh.o[k].x, sh.o[k].y, sh.o[k].z, opaque_k ? 0.0f : seed_tau);
-    b.sd4[3u * p + k] = make_float4(sh.d[k].x, sh.d[k].y, sh.d[k].z, __uint_as_float(sh.seed[k]));
-    b.sw4[3u * p + k] = make_float4(sh.w[k].x, sh.w[k].y, sh.w[k].z, 0.f);
-    if (!opaque_k) queued |= 1u << k;
-    else opaque += 1;
-  }
-  if (alive) {
-    const uint64_t key = draw_bounce_key(s.rng);
-    b.key2[p] = make_uint2((uint32_t)key, (uint32_t)(key >> 32));
-  }
-  store_path(b, p, s);
-  b.meta[p] = (s.bounce & 0xFFFFu) | ((uint32_t)sh.n << 16) | (alive ? kAliveBit : 0u);
-  return queued;
-}
-
+// Bound by the latency of its path records (DRAM: random after the first sort) at 2 resident blocks; more blocks
+// only widen the set of records in L2: 3 / 4 / 5 blocks an SM took 9.6 / 10.7 / 11.9 ms against 9.0 (with gather and
+// sort; 4.2M paths, 500k Gaussians), so what helps is fewer sectors a path (vp_pathstore.cuh).
 __global__ void __launch_bounds__(256) k_wf_shade(SceneView S, EnvView E, ParamsView P, WfBuffers b,
                                                   const uint32_t* q, const uint32_t* count, uint32_t* qnext,
                                                   uint32_t* cnext, Counters* ctr) {
@@ -385,10 +289,12 @@ __global__ void __launch_bounds__(256, kAcc ? VP_WF_MIN_BLOCKS : VP_WF_SHADOW_MI
     item = __shfl_sync(kFull, item, 0);
     if (item >= n) break;
     const uint32_t slot = __ldg(b.qs + item);
-    const float4 o = b.so4[slot], d = b.sd4[slot];
-    const float tau = warp_ray_query<kAcc, kTau>(S, W, f3(o.x, o.y, o.z), f3(d.x, d.y, d.z), 0ull, status, ws,
-                                                 measure, nullptr, __float_as_uint(d.w), o.w);
-    if (lane == 0) b.so4[slot].w = tau >= kMaxOpticalDepth ? 0.0f : expf(-tau);
+    float3 o, d;
+    uint32_t seed;
+    float seed_tau;
+    query_ray(b, slot, o, d, seed, seed_tau);
+    const float tau = warp_ray_query<kAcc, kTau>(S, W, o, d, 0ull, status, ws, measure, nullptr, seed, seed_tau);
+    if (lane == 0) set_transmittance(b, slot, tau);
     if (status) break;
   }
   if (lane == 0) {
@@ -410,17 +316,8 @@ __global__ void __launch_bounds__(256, kAcc ? VP_WF_MIN_BLOCKS : VP_WF_SHADOW_MI
 
 // radiance += weight x T over a path's queries, in their order; an ended path writes its sample.
 __device__ __forceinline__ void gather_path(const ParamsView& P, const WfBuffers& b, uint32_t p) {
-  const uint32_t m = b.meta[p];
-  const int ns = (int)meta_nshadow(m);
-  const float4 r = b.rad4[p];
-  float3 rad = f3(r.x, r.y, r.z);
-  for (int k = 0; k < ns; ++k) {
-    const float4 w = b.sw4[3u * p + k];
-    rad = add(rad, mul(f3(w.x, w.y, w.z), b.so4[3u * p + k].w));
-  }
-  if (m & kAliveBit) {
-    b.rad4[p] = make_float4(rad.x, rad.y, rad.z, 0.f);
-  } else {
+  float3 rad;
+  if (!gather_radiance(b, p, rad)) {
     const float3 L = finalize_sample(P, rad);
     b.L4[p] = make_float4(L.x, L.y, L.z, 0.f);
   }
@@ -493,10 +390,10 @@ __global__ void __launch_bounds__(256, kTailBlocks) k_wf_tail(SceneView S, EnvVi
     item = __shfl_sync(kFull, item, 0);
     if (item >= n) break;
     const uint32_t p = __ldg(q + item);
-    const uint32_t bounce = meta_bounce(b.meta[p]);
-    PathState s = load_path(b, p, bounce);
-    const uint2 k2 = b.key2[p];
-    run_path(S, E, P, queries, s, ((uint64_t)k2.y << 32) | k2.x, bounce ? b.sg[p] : kNoGauss, ps);
+    uint64_t key;
+    uint32_t meta;
+    PathState s = load_path(b, p, key, meta);
+    run_path(S, E, P, queries, s, key, s.bounce ? path_gauss(b, p) : kNoGauss, ps);
     const float3 L = finalize_sample(P, s.rad);
     if (lane == 0) b.L4[p] = make_float4(L.x, L.y, L.z, 0.f);
     if (status) break;
@@ -550,7 +447,7 @@ __global__ void __launch_bounds__(kT8Threads, kTailBlocks) k_wf_tail8(SceneView 
       if ((uint32_t)lane < got) {
         const uint32_t p = __ldg(q + first + lane);
         T.path[flying + lane] = p;
-        b.meta[p] &= ~(3u << 16);  // its last vertex's queries are gathered already
+        b.st[4u * p].w = __uint_as_float(path_meta(b, p) & ~(3u << 16));  // its last vertex's queries are gathered already
       }
       if ((uint32_t)lane < ending) T.path[flying + got + lane] = keep;
       flying += got;
@@ -565,32 +462,18 @@ __global__ void __launch_bounds__(kT8Threads, kTailBlocks) k_wf_tail8(SceneView 
           ray.flight = i < flying;
           if (ray.flight) {
             const uint32_t p = T.path[i];
-            const uint32_t bounce = meta_bounce(b.meta[p]);
-            const float4 o = b.o4[p], d = b.d4[p];
-            const uint2 k2 = b.key2[p];
-            ray.o = f3(o.x, o.y, o.z);
-            ray.d = f3(d.x, d.y, d.z);
-            ray.key = ((uint64_t)k2.y << 32) | k2.x;
-            ray.seed = bounce ? b.sg[p] : kNoGauss;
+            path_ray(b, p, ray.o, ray.d, ray.key);
+            ray.seed = meta_bounce(path_meta(b, p)) ? path_gauss(b, p) : kNoGauss;
           } else {
-            const uint32_t slot = T.query[i - flying];
-            const float4 o = b.so4[slot], d = b.sd4[slot];
-            ray.o = f3(o.x, o.y, o.z);
-            ray.d = f3(d.x, d.y, d.z);
-            ray.seed = __float_as_uint(d.w);
-            ray.seed_tau = o.w;
+            query_ray(b, T.query[i - flying], ray.o, ray.d, ray.seed, ray.seed_tau);
           }
           return true;
         },
         [&](uint32_t i, const Ray8&, const Hit8& h) {
           if (i < flying) {
-            const uint32_t p = T.path[i];
-            const float3 a = h.t < kInf ? S.albedo : f3(0.f, 0.f, 0.f);
-            b.alb4[p] = make_float4(a.x, a.y, a.z, h.t);
-            b.sg[p] = h.gauss;
+            set_scatter(b, T.path[i], h.t < kInf ? S.albedo : f3(0.f, 0.f, 0.f), h.t, h.gauss);
           } else {
-            const float tau = (float)h.w;
-            b.so4[T.query[i - flying]].w = tau >= kMaxOpticalDepth ? 0.0f : expf(-tau);
+            set_transmittance(b, T.query[i - flying], (float)h.w);
           }
         });
     __syncwarp();
@@ -601,16 +484,14 @@ __global__ void __launch_bounds__(kT8Threads, kTailBlocks) k_wf_tail8(SceneView 
           scene, S.depth8, smem, order, flying, &T.next, 1u, (int)min(32u, max(flying, 1u)), status,
           [&](uint32_t i, Ray8& ray) {
             const uint32_t p = T.path[i];
-            ray.t = b.alb4[p].w;
+            ray.t = path_scatter_t(b, p);
             if (!(ray.t < kInf)) return false;
-            const float4 o = b.o4[p], d = b.d4[p];
-            ray.o = f3(o.x, o.y, o.z);
-            ray.d = f3(d.x, d.y, d.z);
+            path_ray(b, p, ray.o, ray.d, ray.key);
             return true;
           },
           [&](uint32_t i, const Ray8& ray, const Hit8& h) {
             const float3 a = mean_albedo(h.w, h.r, h.g, h.b);
-            b.alb4[T.path[i]] = make_float4(a.x, a.y, a.z, ray.t);
+            b.st[4u * T.path[i] + 3u] = make_float4(a.x, a.y, a.z, ray.t);
           });
       __syncwarp();
     }
@@ -656,11 +537,11 @@ __device__ __forceinline__ uint32_t expand10(uint32_t v) {
   return v;
 }
 
-__global__ void k_wf_sort_keys(uint32_t n, const uint32_t* __restrict__ q, const float4* __restrict__ o4,
+__global__ void k_wf_sort_keys(uint32_t n, const uint32_t* __restrict__ q, const float4* __restrict__ ray,
                                float3 lo, float3 inv_ext, uint32_t* __restrict__ keys) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float4 o = o4[q[i]];
+  const float4 o = ray[2u * q[i]];
   auto quant = [](float x) { return (uint32_t)fminf(fmaxf(x, 0.0f), 1023.0f); };
   const uint32_t x = quant((o.x - lo.x) * inv_ext.x), y = quant((o.y - lo.y) * inv_ext.y),
                  z = quant((o.z - lo.z) * inv_ext.z);
@@ -684,7 +565,7 @@ vp_status ensure_workspace(vp_context* ctx, size_t paths) {
   WfWorkspace& w = ctx->wf;
   if (w.cap >= paths && w.base) return VP_OK;
   free_wavefront(ctx);
-  const size_t per_path = 4 * 16 + 16 + 8 + 4 + 16 + 4 + 3 * 48 + 16 + 4 * 3 + 3 * 4;
+  const size_t per_path = 2 * 16 + 4 * 16 + 3 * 48 + 16 + 4 * 3 + 3 * 4;
   const size_t bytes = paths * per_path + 64 * 256 + 4096;
   cudaError_t e = cudaMalloc(&w.base, bytes);
   if (e == cudaErrorMemoryAllocation) {  // give back what the context's pool keeps, and try again
@@ -704,18 +585,10 @@ vp_status ensure_workspace(vp_context* ctx, size_t paths) {
   }
   char* cur = static_cast<char*>(w.base);
   WfBuffers& b = w.b;
-  carve_buf(cur, b.o4, paths);
-  carve_buf(cur, b.d4, paths);
-  carve_buf(cur, b.thr4, paths);
-  carve_buf(cur, b.rad4, paths);
-  carve_buf(cur, b.rng4, paths);
-  carve_buf(cur, b.key2, paths);
-  carve_buf(cur, b.meta, paths);
-  carve_buf(cur, b.alb4, paths);
-  carve_buf(cur, b.sg, paths);
-  carve_buf(cur, b.so4, 3 * paths);
-  carve_buf(cur, b.sd4, 3 * paths);
-  carve_buf(cur, b.sw4, 3 * paths);
+  carve_buf(cur, b.ray, 2 * paths);
+  carve_buf(cur, b.st, 4 * paths);
+  carve_buf(cur, b.sq, 6 * paths);
+  carve_buf(cur, b.sw, 3 * paths);
   carve_buf(cur, b.L4, paths);
   carve_buf(cur, b.qa, paths);
   carve_buf(cur, b.qb, paths);
@@ -837,7 +710,7 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
     // path): the tail takes over.  The first bounce always runs as stages.
     if (it != 0u && (polled <= kTailMax || s->view.albedo_all_zero)) break;
     if (it != 0u && (it & 3u) == 0u && polled >= kSortMinPaths) {  // (camera rays share one origin)
-      k_wf_sort_keys<<<(polled + 255) / 256, 256, 0, st>>>(polled, qcur, b.o4, blo, binv, b.sk_a);
+      k_wf_sort_keys<<<(polled + 255) / 256, 256, 0, st>>>(polled, qcur, b.ray, blo, binv, b.sk_a);
       vp_status r = radix_sort_pairs(b.sk_a, qcur, polled, 30, ctx->wf.sort_tmp, ctx->wf.sort_tmp_bytes, st,
                                      &ctx->launches);
       if (r) return r;

@@ -1,8 +1,9 @@
 // Scene build on the device: per-Gaussian precompute, 3-sigma ellipsoid bounds, 63-bit Morton
 // codes, radix sort, then two binary trees over the sorted boxes -- a Karras radix tree with a
 // bottom-up refit (the thread-per-ray megakernel's tree) and a PLOC agglomerative clustering
-// (the warp engines' tree) -- and the collapse of the latter to a 32-wide BVH, whose depth-first
-// leaf order becomes the scene order of the Gaussians.
+// (the other engines' tree) -- and two collapses of the latter: a 32-wide BVH (the warp-per-ray queries'), whose
+// depth-first leaf order becomes the scene order of the Gaussians, and a compressed 8-wide one (the thread-per-ray
+// queries', vp_trace8.cuh).
 //
 // Replaces the reference's host Morton sort + OptiX unit-sphere GAS / instance IAS build
 // (src/thesis/host/app/renderer.cpp:85-173, include/thesis/host/utils/math.h:103-131,

@@ -17,10 +17,10 @@
 // with icf = M (2 pi)^(-3/2) / prod(s) * sqrt(pi/2) (the reference's inv_cdf_factor_).
 // Computing p_perp from o - c + t_c d in world space avoids the cancellation of the
 // reference's p + t w form (|p| ~ distance/scale), which bounds FP32 transmittance accuracy
-// well above 1e-5.  Everything here is FP32.  The ACCURATE variant carries the closest-approach
+// well above 1e-5.  Every chord is FP32; sums over chords are carried in FP64 and rounded once, so
+// that their order does not matter.  The ACCURATE variant carries the closest-approach
 // vector, p_perp and d2 as unevaluated float pairs (hi + lo, built from the error-free TwoSum and
-// FMA TwoProduct transforms), so 9 - d2 and the half-chord keep their bits on grazing chords,
-// and sums optical depth in float pairs too.
+// FMA TwoProduct transforms), so 9 - d2 and the half-chord keep their bits on grazing chords.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -657,27 +657,11 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
   return v;
 }
-// Sum of the lanes' float pairs, as a float.
-__device__ __forceinline__ float warp_sum_ff(FF v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    FF w;
-    w.hi = __shfl_xor_sync(0xFFFFFFFFu, v.hi, o);
-    w.lo = __shfl_xor_sync(0xFFFFFFFFu, v.lo, o);
-    v = ff_add(v, w);
-  }
-  return __fadd_rn(v.hi, v.lo);
-}
 // FP64 sum over the warp: sums carried in FP64 and rounded once give the same FP32 result whatever the
 // order of their terms.
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-  return v;
-}
-__device__ __forceinline__ float warp_min(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
   return v;
 }
 

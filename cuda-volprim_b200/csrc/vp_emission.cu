@@ -20,8 +20,9 @@
 //     dL/dS = C (T - a) / S - T env,  a = (1 - T) / S,      dL/dC = a
 //     g_tau_i = G . (dL/dS + a e_i),   dLoss/de_i = G a tau_i
 // and tau_i is differentiated in closed form through the whitening p = W (o - mu), w = W d,
-// W = diag(1/s) R(q)^T (see tau_grad below).  The backward kernel traverses each ray twice --
-// once for S and C, once to scatter per-Gaussian gradients -- instead of storing hit lists.
+// W = diag(1/s) R(q)^T (see tau_grad below).  The backward kernel meets each ray's Gaussians twice --
+// once for S and C, once to scatter per-Gaussian gradients -- and stores no per-ray hits: its first
+// traversal lists the Gaussians of a packet of rays (below), which the second pass goes through.
 // Per Gaussian it accumulates 16 floats (float4 atomics, internal order): dLoss/dW (9),
 // sum g_tau dtau/dp (3, for the mean), sum g_tau tau (1, for density and the scale
 // normaliser), dLoss/de (3); a finishing kernel maps them to mean / scale / quaternion /

@@ -123,7 +123,7 @@ _TAU_ORDERS = {"auto": _capi.VP_TAU_ORDER_AUTO, "lane": _capi.VP_TAU_ORDER_LANE,
 class Scene:
     """Gaussians + acceleration structure on the device (vp_scene_create_ex).
 
-    wide_builder / binary_builder pick the binary tree of the BVH32 (warp and wavefront engines)
+    wide_builder / binary_builder pick the binary tree of the BVH32 and the 8-wide BVH (warp and wavefront engines)
     and of the megakernel: "ploc" (clustering, the default) or "lbvh" (Karras radix tree);
     leaf_max is the largest BVH32 leaf (1..32); collapse cuts the BVH32 from its binary tree:
     "sah" (SAH-optimal slot assignment, the default) or "greedy" (largest area first);

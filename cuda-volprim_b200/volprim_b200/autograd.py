@@ -5,7 +5,7 @@
 
 returns (n_cameras, H, W, 3) absorption-plus-emission images (the model of
 include/volprim_b200.h) that are differentiable with respect to the five parameter tensors.  The
-forward pass builds the scene (LBVH + BVH32 from the current parameters) on the device and
+forward pass builds the scene (its trees from the current parameters) on the device and
 renders each camera; the backward pass traverses every ray again and adds the per-Gaussian
 gradients of all cameras.  PyTorch is only the plumbing here: both passes are the library's
 CUDA kernels.

@@ -62,25 +62,28 @@ typedef enum vp_engine {
   VP_ENGINE_WARP = 0,       /* persistent kernel, one path per warp, warp-cooperative BVH32 traversal */
   VP_ENGINE_MEGAKERNEL = 1, /* plain per-pixel megakernel, thread-per-ray binary-tree traversal */
   VP_ENGINE_WAVEFRONT = 2   /* wavefront of persistent stage kernels over compacted path queues,
-                               warp-cooperative BVH32 traversal; same results as VP_ENGINE_WARP */
+                               thread-per-ray traversal of a compressed 8-wide BVH (warp-cooperative
+                               BVH32 traversal while counting, and for trees too deep for it); same
+                               results as VP_ENGINE_WARP */
 } vp_engine;
 
 /* Precision of the per-(ray, Gaussian) chord set-up (whitening transform, closest approach,
- * 3-sigma chord) and of the optical-depth sums.  Both are FP32 arithmetic; no precision uses
- * FP64 (the only FP64 on the device is the environment table build).  Both meet the 1e-5
+ * 3-sigma chord).  Both evaluate chords in FP32; the sums over a ray's chords (optical depth,
+ * albedo weights) are carried in FP64 and rounded once, so a result does not depend on the order
+ * in which a traversal meets the Gaussians.  Both meet the 1e-5
  * relative per-pixel transmittance gate against the FP64 closed form on rays from outside the
  * Gaussians (FAST: 6e-6 worst on the 256-Gaussian absorption image, ACCURATE: 3e-6). */
 typedef enum vp_precision {
   VP_PRECISION_AUTO = 0,    /* ACCURATE for absorption-only scenes (albedo == 0), else FAST */
   VP_PRECISION_FAST = 1,    /* FP32, hardware exp/log approximations (the reference's fast math) */
   VP_PRECISION_ACCURATE = 2 /* FP32 with error-free transforms: o - c, the closest approach and d2
-                               as float pairs (TwoSum / FMA TwoProduct), correctly rounded exp,
-                               compensated optical-depth sums */
+                               as float pairs (TwoSum / FMA TwoProduct), correctly rounded exp */
 } vp_precision;
 
 /* Bits of vp_render_params.measure. */
 typedef enum vp_measure {
-  VP_MEASURE_COUNTERS = 1,  /* device counters (the reference's --measure-caps and more) */
+  VP_MEASURE_COUNTERS = 1,  /* device counters (the reference's --measure-caps and more), kept by the
+                               warp-per-ray traversal of the BVH32: same image, more device time */
   VP_MEASURE_STAGES = 2     /* per-stage CUDA-event timing of the wavefront launches */
 } vp_measure;
 
@@ -102,7 +105,9 @@ vp_status vp_version(int32_t* major, int32_t* minor);
 /* context                                                                                  */
 /* ---------------------------------------------------------------------------------------- */
 
-/* Binds a CUDA device and creates the context's stream.  Replaces cuda::Context + StreamDAG
+/* Binds a CUDA device and creates the context's stream and memory pool.  The pool serves the
+ * scenes', calls' and requests' device buffers in stream order, keeps at most 2 GiB of freed memory for
+ * the next of them, and is given back with the context.  Replaces cuda::Context + StreamDAG
  * construction in Renderer::Renderer (src/thesis/host/app/renderer.cpp:34-51). */
 vp_status vp_context_create(int32_t device, vp_context** out);
 vp_status vp_context_destroy(vp_context* ctx);
@@ -155,7 +160,7 @@ typedef struct vp_scene_info {
 /* Validates the primitives (positive finite scales, positive finite density, finite centres;
  * ply.cpp:146-172), precomputes the per-primitive whitening record (primitive.h:70-87), builds
  * the BVH over 3-sigma ellipsoid bounds on the device (Morton codes, radix sort, PLOC clustering
- * or Karras hierarchy + refit, collapse to a 32-wide BVH).  Replaces Renderer::initPrimsAndGAS
+ * or Karras hierarchy + refit, collapse to a 32-wide and a compressed 8-wide BVH).  Replaces Renderer::initPrimsAndGAS
  * (renderer.cpp:85-173: host Morton sort + OptiX GAS/IAS build).  No primitive-count cap below
  * 2^26 (the reference caps at 65,535, renderer.cpp:54-59).  count 0 makes an empty scene that
  * every ray misses (the reference's IAS over zero instances); the emission model rejects it. */
@@ -181,7 +186,8 @@ typedef enum vp_collapse {
 
 /* The order in which a transmittance query visits the hit children of a BVH32 node after the
  * nearest one.  The optical depth is the same sum either way; the order decides how soon a ray
- * reaches MAX_OPTICAL_DEPTH and stops. */
+ * reaches MAX_OPTICAL_DEPTH and stops.  (The thread-per-ray traversal of the 8-wide BVH always takes a
+ * node's children near to far by the ray's octant, at no cost.) */
 typedef enum vp_tau_order {
   VP_TAU_ORDER_AUTO = 0,    /* NEAREST when fewer than half of the Gaussians are opaque at their
                                core (central optical depth along their thinnest direction below
@@ -272,7 +278,7 @@ typedef struct vp_render_params {
   int32_t engine;          /* vp_engine */
   int32_t precision;       /* vp_precision */
   int32_t measure;         /* bit set: VP_MEASURE_COUNTERS counts crossings, bounces, shadow rays
-                              and maxima (costs atomics); VP_MEASURE_STAGES times the wavefront
+                              and maxima (warp-per-ray traversal, atomics); VP_MEASURE_STAGES times the wavefront
                               stages with CUDA events (no device-side cost) */
   /* Adaptive sampling (ADAPTIVE_THRESHOLD / ADAPTIVE_MIN_SAMPLES, device/core/constants.cuh:
    * 196-211; the test of device/entry/raygen.cuh:52-67).  Before each batch, a pixel that already
@@ -309,7 +315,8 @@ typedef struct vp_render_stats {
   uint64_t query_prim_tests[3];/* Gaussian boxes tested per query kind        (measure counters) */
   uint64_t query_geo_loads[3]; /* Gaussian records loaded per query kind       (measure counters) */
   double ms_stage[3];          /* device time of the wavefront's [0] extend (free-flight argmin),
-                                  [1] shadow (transmittance) and [2] all other launches; the
+                                  [1] shadow (transmittance) and [2] all other launches (the last
+                                  paths' launch, which does everything, among them); the
                                   warp and megakernel engines put their one kernel in [2]
                                                                              (measure stages) */
   uint32_t stage_launches[3];  /* launches in each ms_stage bucket            (measure stages) */
@@ -459,9 +466,9 @@ vp_status vp_render_emission_backward(vp_scene* scene, vp_env* env, const vp_cam
  * refills the slots freed by finished paths with new (pixel, sample) paths of the admitted
  * requests that still have unstarted paths (in the order the schedule gives), then extends,
  * shades, traces shadow rays and gathers every path in flight -- paths of different requests,
- * scenes, resolutions and sample counts share the same launches.  The iteration is captured once as a CUDA graph.  Requests wait in a FIFO until the
- * request table has a free entry and their image accumulator fits the memory budget.  A finished
- * path adds its sample to its request's per-pixel sum; a request completes when all its
+ * scenes, resolutions and sample counts share the same launches.  The
+ * iteration is captured once as a CUDA graph.  Requests wait in a FIFO until the request table has a
+ * free entry and their image accumulator fits the memory budget.  A finished path adds its sample to its request's per-pixel sum; a request completes when all its
  * width*height*spp paths have finished, and its mean image is written to its output buffer.
  * Each path's result is the one vp_render computes for the same scene, camera and params
  * (the same PCG32 stream per (pixel, sample)); only the order of the per-pixel FP32 sums differs. */

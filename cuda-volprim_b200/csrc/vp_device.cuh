@@ -290,6 +290,15 @@ struct PrimGeo {  // the record minus albedo
   float4 a, b, c;
   float icf;
 };
+// 32 bytes in one read-only load (p on a 32-byte boundary).  A gather costs the L1 a cycle per line and load
+// instruction, and the 8-wide BVH's transmittance kernel is closest to that limit (75 % of it, 57 % of the issue
+// slots), so its nodes and records are fetched by sectors: 2M-Gaussian stress image 62.9 -> 61.8 ms, showcase
+// 58.8 -> 58.6.  (The third pair of a record, read for its first half only, measured no better.)
+__device__ __forceinline__ void ldg256(const float4* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
 __device__ __forceinline__ PrimGeo load_geo(const float4* __restrict__ prims, uint32_t i) {
   PrimGeo g;
   g.a = __ldg(prims + 4u * i + 0u);

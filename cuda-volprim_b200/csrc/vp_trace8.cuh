@@ -266,8 +266,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
     Chord ch;
     if (hit) {
       PrimGeo g;
-      g.a = __ldg(sc.prims + 4u * gi);
-      g.b = __ldg(sc.prims + 4u * gi + 1u);
+      ldg256(sc.prims + 4u * gi, g.a, g.b);
       g.c = __ldg(sc.prims + 4u * gi + 2u);
       hit = chord_setup<kAcc>(g, o, d, ch);
       if constexpr (kKind == kScatter8) hit = hit && ch.t_in <= bound && bound <= ch.t_out;
@@ -412,9 +411,13 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
         }
       }
       const float4* p4 = reinterpret_cast<const float4*>(nodes + (size_t)cur * kNode8Words);
-      const float4 h = __ldg(p4);
-      const uint4 a = __ldg(reinterpret_cast<const uint4*>(p4) + 1), bq = __ldg(reinterpret_cast<const uint4*>(p4) + 2),
-                  c = __ldg(reinterpret_cast<const uint4*>(p4) + 3);
+      float4 h, wa, wb, wc;
+      ldg256(p4, h, wa);
+      ldg256(p4 + 2, wb, wc);
+      auto bits = [](float4 v) {
+        return make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+      };
+      const uint4 a = bits(wa), bq = bits(wb), c = bits(wc);
       const uint32_t ew = __float_as_uint(h.w);
       const float ax = __uint_as_float((ew & 0xFFu) << 23) * inv.x;
       const float ay = __uint_as_float((ew & 0xFF00u) << 15) * inv.y;

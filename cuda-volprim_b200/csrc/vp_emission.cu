@@ -43,8 +43,9 @@ namespace {
 // same Gaussians -- and walks the BVH32 once for all of them: at an inner node lane c tests child c's box
 // against the packet's frustum, at a leaf lane j tests the j-th Gaussian's, and each candidate is then met
 // by all 32 rays at once (its record one broadcast load, every lane setting up its own ray's chord).  One
-// ray a warp instead left about two lanes busy in the chord work, and the adjoint issued its 64 bytes of
-// atomics per (ray, Gaussian) where a packet reduces its rays' gradients first.
+// ray a warp instead leaves about two lanes busy in the chord work, and the adjoint issues its 64 bytes of
+// atomics per (ray, Gaussian) where a packet reduces its rays' gradients first; that form stays for images of
+// few rays (few_rays).
 //
 // Tile of the packet: k = min(spp, 32) samples of 2^floor(log2(32 / k)) pixels, near square.
 struct Tiling {
@@ -429,6 +430,125 @@ __global__ void __launch_bounds__(32 * kGroup, (kAcc ? 16 : kFwdWarps) / kGroup)
   if (P.measure) atomicAdd(&ctr->crossings, crossings);
 }
 
+// ---- a warp on each ray (images of few rays) ----
+// The Gaussians of one ray by the warp: f(index, record, chord) on the lane that set the chord up.
+template <bool kAcc, class F>
+__device__ void warp_visit(const SceneView& S, uint32_t* stack, float3 o, float3 d, uint32_t& status, F&& f) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  const RayBox rb = ray_box(o, d);
+  int sp = 0;
+  uint32_t ref = S.wide_root;
+  bool have = true;
+  while (true) {
+    if (!have) {
+      if (sp == 0) break;
+      ref = stack[--sp];
+      __syncwarp();
+    }
+    have = false;
+    if (ref_is_leaf(ref)) {
+      // leaves next on the stack join this step while their Gaussians fit in the 32 lanes
+      int total = (int)wide_leaf_count(ref);
+      uint32_t pi = wide_leaf_first(ref) + (uint32_t)lane;
+      while (sp > 0) {
+        const uint32_t r2 = stack[sp - 1];
+        if (!ref_is_leaf(r2)) break;
+        const int c2 = (int)wide_leaf_count(r2);
+        if (total + c2 > 32) break;
+        --sp;
+        if (lane >= total && lane < total + c2) pi = wide_leaf_first(r2) + (uint32_t)(lane - total);
+        total += c2;
+      }
+      __syncwarp();
+      if (lane < total) {
+        float tb;
+        if (slab(rb, __ldg(S.pbox + 2u * pi), __ldg(S.pbox + 2u * pi + 1u), 0.0f, kInf, tb)) {
+          const PrimGeo g = load_geo(S.prims, pi);
+          Chord ch;
+          if (chord_setup<kAcc>(g, o, d, ch) && ch.t_out > 0.0f) f(pi, g, ch);
+        }
+      }
+    } else {
+      const float4* node = S.wide + (size_t)ref * 64u;
+      const float4 lo = __ldg(node + lane);
+      const float4 hi = __ldg(node + 32 + lane);
+      const uint32_t cref = __float_as_uint(lo.w);
+      float tnear = 0.f;
+      const bool hit = (cref != kEmptyRef) && slab(rb, lo, hi, 0.0f, kInf, tnear);
+      const unsigned m = __ballot_sync(kFull, hit);
+      const int nh = __popc(m);
+      if (nh > 0) {
+        if ((uint32_t)(sp + nh) > S.stack_cap) {  // cannot happen for a BVH of the recorded depth
+          status |= kStatusStackOverflow;
+          break;
+        }
+        const int first = __ffs(m) - 1;
+        if (hit && lane != first) stack[sp + __popc(m & lt_mask) - 1] = cref;
+        sp += nh - 1;
+        ref = __shfl_sync(kFull, cref, first);
+        have = true;
+      }
+    }
+    __syncwarp();
+  }
+  __syncwarp();
+}
+
+template <bool kAcc>
+__device__ RaySums ray_sums(const SceneView& S, const float4* __restrict__ emis, uint32_t* stack, float3 o, float3 d,
+                            uint32_t& status, unsigned long long& crossings) {
+  double s = 0.0, r = 0.0, g = 0.0, b = 0.0;
+  warp_visit<kAcc>(S, stack, o, d, status, [&](uint32_t pi, const PrimGeo& geo, const Chord& ch) {
+    const float tau = chord_tau0<kAcc>(ch, geo.icf);
+    const float4 e = __ldg(emis + pi);
+    s += (double)tau;
+    r += (double)tau * (double)e.x;
+    g += (double)tau * (double)e.y;
+    b += (double)tau * (double)e.z;
+    ++crossings;
+  });
+  return RaySums{(float)warp_sum(s), (float)warp_sum(r), (float)warp_sum(g), (float)warp_sum(b)};
+}
+
+// A block of up to 8 warps takes a pixel, a warp each of its samples.
+template <bool kAcc>
+__global__ void __launch_bounds__(256, kAcc ? 2 : 4) k_emis_forward_ray(SceneView S, EnvView E, CameraView C, ParamsView P,
+                                                                       const float4* __restrict__ emis,
+                                                                       float4* __restrict__ out, unsigned int* work,
+                                                                       Counters* ctr) {
+  __shared__ float radiance[8][3];
+  __shared__ uint32_t taken;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  uint32_t* stack = reinterpret_cast<uint32_t*>(vp_dyn_smem) + warp * S.stack_cap;
+  uint32_t status = 0;
+  unsigned long long crossings = 0;
+  while (true) {
+    if (threadIdx.x == 0) taken = atomicAdd(work, 1u);
+    __syncthreads();
+    const uint32_t pix = taken;
+    if (pix >= P.width * P.height) break;
+    float3 sum = f3(0.f, 0.f, 0.f);
+    for (uint32_t s0 = 0; s0 < P.spp_total; s0 += warps) {
+      if (s0 + warp < P.spp_total) {
+        const PacketRay r = packet_ray(C, P, pix % P.width, pix / P.width, s0 + warp);
+        const RaySums rs = ray_sums<kAcc>(S, emis, stack, r.o, r.d, status, crossings);
+        const float3 L = ray_radiance(rs, env_lookup(E, r.d));
+        if (lane == 0) radiance[warp][0] = L.x, radiance[warp][1] = L.y, radiance[warp][2] = L.z;
+      }
+      __syncthreads();
+      for (uint32_t j = 0; j < min(warps, P.spp_total - s0); ++j)  // the pixel's samples in order
+        sum = add(sum, f3(radiance[j][0], radiance[j][1], radiance[j][2]));
+      __syncthreads();
+    }
+    const float inv = 1.0f / (float)P.spp_total;
+    if (threadIdx.x == 0) out[pix] = make_float4(sum.x * inv, sum.y * inv, sum.z * inv, 1.0f);
+    if (__syncthreads_or(status != 0u)) break;
+  }
+  if (status) atomicOr(&ctr->status, status);
+  if (P.measure) atomicAdd(&ctr->crossings, crossings);
+}
+
 // dtau/dp and dtau/dw of one chord, with tau itself, where p = W (x0 - mu), w = W d and x0 is a
 // point of the ray taken as fixed:
 //   tau = icf |w|^-1 exp(-d2/2) [erf(h/sqrt2) - erf(u/sqrt2)],  h = sqrt(9 - d2),
@@ -603,6 +723,58 @@ __global__ void __launch_bounds__(32 * kGroup, (kAcc ? 16 : kBwdWarps) / kGroup)
   if (P.measure) atomicAdd(&ctr->crossings, crossings);
 }
 
+// The adjoint with a warp on each ray: its second traversal adds every (ray, Gaussian) pair's terms by itself.
+template <bool kAcc>
+__global__ void __launch_bounds__(256, kAcc ? 2 : 4) k_emis_backward_ray(SceneView S, EnvView E, CameraView C, ParamsView P,
+                                                                        const float4* __restrict__ emis,
+                                                                        const float4* __restrict__ dl_dpix,
+                                                                        float4* __restrict__ acc, unsigned int* work,
+                                                                        Counters* ctr) {
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t* stack = reinterpret_cast<uint32_t*>(vp_dyn_smem) + warp * S.stack_cap;
+  const uint32_t n_rays = P.width * P.height * P.spp_total;
+  const float inv_spp = 1.0f / (float)P.spp_total;
+  uint32_t status = 0;
+  unsigned long long crossings = 0;
+  while (true) {
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(work, 1u);
+    item = __shfl_sync(kFull, item, 0);
+    if (item >= n_rays) break;
+    const uint32_t pix = item / P.spp_total;
+    const float4 gp = __ldg(dl_dpix + pix);
+    if (gp.x == 0.0f && gp.y == 0.0f && gp.z == 0.0f) continue;  // nothing flows back (e.g. a crop)
+    const float3 G = f3(gp.x * inv_spp, gp.y * inv_spp, gp.z * inv_spp);
+    const PacketRay ray = packet_ray(C, P, pix % P.width, pix / P.width, item % P.spp_total);
+    const float3 o = ray.o, d = ray.d;
+    const RaySums rs = ray_sums<kAcc>(S, emis, stack, o, d, status, crossings);
+    const float3 env = env_lookup(E, d);
+    float T, a, q;
+    opacity_terms(rs.S, T, a, q);
+    const float gS = G.x * fmaf(rs.r, q, -T * env.x) + G.y * fmaf(rs.g, q, -T * env.y) + G.z * fmaf(rs.b, q, -T * env.z);
+    const float3 gC = mul(G, a);
+    warp_visit<kAcc>(S, stack, o, d, status, [&](uint32_t pi, const PrimGeo& geo, const Chord& ch) {
+      float tau;
+      float3 v, dp, dw;
+      if (!tau_grad<kAcc>(geo, ch, o, d, tau, v, dp, dw)) return;
+      const float4 e = __ldg(emis + pi);
+      const float gt = gS + gC.x * e.x + gC.y * e.y + gC.z * e.z;
+      const float3 gp3 = mul(dp, gt), gw3 = mul(dw, gt);
+      // dLoss/dW_kl = gp_k v_l + gw_k d_l
+      float4* a4 = acc + 4u * pi;
+      atomicAdd(a4 + 0, make_float4(fmaf(gp3.x, v.x, gw3.x * d.x), fmaf(gp3.x, v.y, gw3.x * d.y),
+                                    fmaf(gp3.x, v.z, gw3.x * d.z), fmaf(gp3.y, v.x, gw3.y * d.x)));
+      atomicAdd(a4 + 1, make_float4(fmaf(gp3.y, v.y, gw3.y * d.y), fmaf(gp3.y, v.z, gw3.y * d.z),
+                                    fmaf(gp3.z, v.x, gw3.z * d.x), fmaf(gp3.z, v.y, gw3.z * d.y)));
+      atomicAdd(a4 + 2, make_float4(fmaf(gp3.z, v.z, gw3.z * d.z), gp3.x, gp3.y, gp3.z));
+      atomicAdd(a4 + 3, make_float4(gt * tau, gC.x * tau, gC.y * tau, gC.z * tau));
+    });
+    if (status) break;
+  }
+  if (status) atomicOr(&ctr->status, status);
+  if (P.measure) atomicAdd(&ctr->crossings, crossings);
+}
+
 // Per-Gaussian accumulators (internal order) -> gradients of the caller's parameters (caller
 // order), added to out[].  W_kl = R_lk / s_k with R = R(q / |q|) (the build's rotation matrix) and
 // icf proportional to density / (s_x s_y s_z):
@@ -699,6 +871,20 @@ vp_status with_group(uint32_t tiles, uint32_t stack_cap, F&& f) {
   if (tiles >= 10240u || packet_smem<4>(stack_cap, true) > kMost) return f(std::integral_constant<int, 2>{});
   if (tiles >= 1024u || packet_smem<8>(stack_cap, true) > kMost) return f(std::integral_constant<int, 4>{});
   return f(std::integral_constant<int, 8>{});
+}
+
+// Images of few rays take a warp on each ray: their packets are few, and wide at one or two samples a pixel, so
+// the chip waits for the densest.  Both sides at 12,800 / 40,000 / 65,536 / 180,000 rays, packets and then rays:
+// forward, 100k Gaussians 2.18 / 1.78 / 1.67 / 1.84 and 0.57 / 1.04 / 1.63 / 3.96 ms, 20k Gaussians 0.59 / 0.47 /
+// 0.45 / 0.49 and 0.17 / 0.30 / 0.44 / 1.06, 5k Gaussians 0.18 / 0.16 / 0.155 / 0.17 and 0.10 / 0.145 / 0.20 / 0.45;
+// ACCURATE crosses over at four fifths of that.  A gradient step at 38k / 154k rays (two views the latter; build
+// and forward in it): 100k Gaussians 9.4 / 15.0 and 5.7 / 20.5 ms, 5k 2.32 / 2.75 and 2.19 / 3.77: the adjoint's
+// packets, which it meets twice, pay later.
+bool few_rays(const ParamsView& P, uint32_t count, bool adjoint) {
+  uint64_t limit = count >= 16384u ? 65536u : 45056u;
+  if (P.accurate) limit = limit * 4u / 5u;
+  if (adjoint) limit = limit * 3u / 2u;
+  return (uint64_t)P.width * P.height * P.spp_total <= limit;
 }
 
 Tiling tiling(uint32_t width, uint32_t height, uint32_t spp) {
@@ -804,7 +990,16 @@ vp_status vp_render_emission(vp_scene* s, vp_env* e, const vp_camera* cam, const
   }
   if ((r = clear_counters(ctx))) return r;
   VP_CUDA(cudaEventRecord(ctx->ev0, st));
-  const vp_status lr = with_group(c.tiles.tiles, s->view.stack_cap, [&](auto group) -> vp_status {
+  auto per_ray = [&]() -> vp_status {
+    auto kern = c.P.accurate ? k_emis_forward_ray<true> : k_emis_forward_ray<false>;
+    const int warps = (int)std::min(std::max(c.P.spp_total, 1u), 8u);
+    const size_t smem = (size_t)warps * s->view.stack_cap * 4u;
+    if (smem > 47 * 1024) VP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int blocks = ctx->sm_count * blocks_per_sm(kern, 32 * warps, smem);
+    kern<<<blocks, 32 * warps, smem, st>>>(s->view, e->view, c.cv, c.P, s->emis, out, ctx->work_counter, ctx->counters);
+    return VP_OK;
+  };
+  auto packets = [&](auto group) -> vp_status {
     constexpr int G = decltype(group)::value;
     auto kern = c.P.accurate ? k_emis_forward<true, G> : k_emis_forward<false, G>;
     const size_t smem = packet_smem<G>(s->view.stack_cap, false);
@@ -813,8 +1008,12 @@ vp_status vp_render_emission(vp_scene* s, vp_env* e, const vp_camera* cam, const
     kern<<<blocks, 32 * G, smem, st>>>(s->view, e->view, c.cv, c.P, c.tiles, c.extent, s->emis, out, ctx->work_counter,
                                        ctx->counters);
     return VP_OK;
-  });
-  if (lr) return lr;
+  };
+  const vp_status lr = few_rays(c.P, s->info.count, false) ? per_ray() : with_group(c.tiles.tiles, s->view.stack_cap, packets);
+  if (lr) {
+    dev_free(tmp, st);
+    return lr;
+  }
   VP_CUDA(cudaGetLastError());
   r = finish_stats(ctx, p, 1, stats);
   if (tmp) {
@@ -874,7 +1073,15 @@ vp_status vp_render_emission_backward(vp_scene* s, vp_env* e, const vp_camera* c
   VP_CUDA(cudaMemsetAsync(acc, 0, 64ull * n, st));
   if ((r = clear_counters(ctx))) return cleanup(), r;
   VP_CUDA(cudaEventRecord(ctx->ev0, st));
-  const vp_status lr = with_group(c.tiles.tiles, s->view.stack_cap, [&](auto group) -> vp_status {
+  auto per_ray = [&]() -> vp_status {
+    auto kern = c.P.accurate ? k_emis_backward_ray<true> : k_emis_backward_ray<false>;
+    const size_t smem = 8u * (size_t)s->view.stack_cap * 4u;
+    if (smem > 48 * 1024) VP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int blocks = ctx->sm_count * blocks_per_sm(kern, 256, smem);
+    kern<<<blocks, 256, smem, st>>>(s->view, e->view, c.cv, c.P, s->emis, dsrc, acc, ctx->work_counter, ctx->counters);
+    return VP_OK;
+  };
+  auto packets = [&](auto group) -> vp_status {
     constexpr int G = decltype(group)::value;
     auto kern = c.P.accurate ? k_emis_backward<true, G> : k_emis_backward<false, G>;
     const size_t smem = packet_smem<G>(s->view.stack_cap, true);
@@ -883,7 +1090,8 @@ vp_status vp_render_emission_backward(vp_scene* s, vp_env* e, const vp_camera* c
     kern<<<blocks, 32 * G, smem, st>>>(s->view, e->view, c.cv, c.P, c.tiles, c.extent, s->emis, dsrc, acc, ctx->work_counter,
                                        ctx->counters);
     return VP_OK;
-  });
+  };
+  const vp_status lr = few_rays(c.P, s->info.count, true) ? per_ray() : with_group(c.tiles.tiles, s->view.stack_cap, packets);
   if (lr) return cleanup(), lr;
   VP_CUDA(cudaGetLastError());
   k_emis_finish<<<(n + 255) / 256, 256, 0, st>>>(n, s->perm, s->prims, s->raw, acc, s->scale_is_log, gm, gs, gq, gd, ge);

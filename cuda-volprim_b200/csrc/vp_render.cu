@@ -285,9 +285,10 @@ vp_status launch_transmittance(vp_scene* s, const float* o, const float* d, uint
   vp_context* ctx = s->ctx;
   cudaStream_t st = ctx->stream;
   if (n == 0) return VP_OK;
-  // Few rays through a small scene end sooner with a warp on each: 1,000 rays 59 / 71 us (1,000 Gaussians), 52 /
-  // 62 us (10k); at 65k rays it is 152 / 139 and 134 / 97 us, at 100k Gaussians 98 / 82 us for 1,000 rays.
-  const bool small = n <= 16384u && s->view.count < 32768u;
+  // Few rays through a small scene end sooner with a warp on each.  Warp / thread: 1,000 Gaussians, 1,000 rays 59 /
+  // 71 us, 18,000 83 / 96, 40,000 117 / 120, 80,000 175 / 148; 10,000 Gaussians, 1,000 rays 52 / 62, 65,000 134 /
+  // 97; from 16,384 Gaussians threads win at any count (30,000 in clusters, 16,000 rays 139 / 112).
+  const bool small = s->view.count < 2048u ? n <= 24576u : s->view.count < 16384u && n <= 16384u;
   if (engine == VP_ENGINE_WARP && s->view.depth8 != 0u && !small) {
     auto kern = accurate ? k_tau8<true> : k_tau8<false>;
     const size_t smem = trace8_smem_bytes(s->view.depth8, kT8Threads);

@@ -203,7 +203,7 @@ def run_reference(args):
     print(json.dumps(line), flush=True)
 
 
-# Algorithmic bytes of one traversal query's work: a Gaussian's 3-sigma box (2 float4) per box
+# Algorithmic bytes of one warp-per-ray or megakernel query's work: a Gaussian's 3-sigma box (2 float4) per box
 # test, its whitening record (4 float4) per box hit, a BVH32 inner node (32 child boxes, 64 float4)
 # per visit; binary LBVH nodes are 4 float4.
 BOX_BYTES, RECORD_BYTES, WIDE_NODE_BYTES, BINARY_NODE_BYTES = 32, 64, 1024, 64
@@ -252,11 +252,17 @@ def roofline(args, m, step_stats, sm_mhz=None):
     stage times of the timed steps (the steps are the same batch size over the same image) and the
     per-unit ncu figures of profiles/traffic.json (warp instructions and DRAM bytes per unit).
 
-    The traversal kernels are issue-bound (the scene is L2-resident, DRAM runs below 1% of peak),
-    so the binding roof is the SMs' issue rate: 148 SMs x 4 schedulers x one warp instruction per
-    cycle at the SM clock sampled during the timed region.  The bytes the traversal touches are
-    reported against a measured L2 copy rate (l2_demand) and the DRAM bytes against the measured
-    HBM copy rate (hbm)."""
+    The traversal kernels are bound inside the SM (the scene is L2-resident, DRAM runs at a few
+    percent of peak), so the roof reported is the SMs' issue rate: 148 SMs x 4 schedulers x one warp
+    instruction per cycle at the SM clock sampled during the timed region; lsu_frac_ncu is the
+    profiled share of the L1 / shared-memory data pipe, the other limit they come close to.  DRAM
+    bytes stand against the measured HBM copy rate (hbm).  For the warp and megakernel engines,
+    whose traversal the counters describe, the bytes it touches are reported against a measured L2
+    copy rate (l2_demand); the wavefront counts with the warp-per-ray form of its queries, so its
+    counters say how many queries a step has, not what the thread-per-ray kernels touch.
+
+    A batch's last paths run in one launch outside the stages: the per-unit figures are the stage
+    launches' totals over all of a profiled batch's units."""
     peak_hbm, peak_kind = measured_peaks()
 
     def query_bytes(k):
@@ -267,12 +273,13 @@ def roofline(args, m, step_stats, sm_mhz=None):
     if args.engine == "wavefront":
         ms = [sum(st["ms_stage"][k] for st in step_stats) / n for k in range(3)]
         nl = [sum(st["stage_launches"][k] for st in step_stats) / n for k in range(3)]
-        kern = [("k_wf_extend", query_bytes(0) + query_bytes(2) + m["bounces"] * EXTEND_STATE_BYTES,
-                 "free-flight argmin + scatter-point albedo", m["bounces"], "path bounces", EXTEND_STATE_BYTES),
-                ("k_wf_shadow", query_bytes(1) + m["shadow_rays"] * SHADOW_STATE_BYTES,
-                 "transmittance (NEE shadow rays)", m["shadow_rays"], "shadow rays", SHADOW_STATE_BYTES)]
+        kern = [("k_wf_extend8", "free-flight argmin + scatter-point albedo", m["bounces"], "path bounces",
+                 EXTEND_STATE_BYTES),
+                ("k_wf_shadow8", "transmittance (NEE shadow rays)", m["shadow_rays"], "shadow rays",
+                 SHADOW_STATE_BYTES)]
         k = 0 if ms[0] >= ms[1] else 1
-        name, alg, what, units, unit_name, state_bytes = kern[k]
+        name, what, units, unit_name, state_bytes = kern[k]
+        alg = None
         step_ms, launches = ms[k], nl[k]
         share = ms[k] / max(1e-9, sum(st["ms_kernels"] for st in step_stats) / n)
     else:
@@ -294,8 +301,6 @@ def roofline(args, m, step_stats, sm_mhz=None):
     issue_peak = 148 * 4 * clock * 1e6 / 1e9  # G warp-instructions / s
     inst = prof.get("warp_inst_per_unit")
     traffic = prof["dram_bytes_per_unit"] * units_per_launch if prof.get("dram_bytes_per_unit") else None
-    l2_peak = l2_copy_gbs()
-    l2_achieved = alg / launches / sec_per_launch / 1e9
     roof = {"kernel": name, "kernel_work": what, "kernel_share_of_step": share, "launches_per_step": launches,
             "kernel_ms_per_launch": step_ms / launches, "units_per_launch": units_per_launch, "units": unit_name}
     if inst:
@@ -312,13 +317,17 @@ def roofline(args, m, step_stats, sm_mhz=None):
     roof["traffic_source"] = prof.get("source")
     roof["traffic_per_unit"] = prof.get("dram_bytes_per_unit")
     roof["declared_state_bytes_per_unit"] = state_bytes
-    roof["l2_demand"] = {"achieved": l2_achieved, "peak": l2_peak, "unit": "GB/s", "frac": l2_achieved / l2_peak,
-                         "algorithmic_bytes_per_launch": alg / launches,
-                         "peak_source": "measured: L2-resident torch copy, 2 x 32 MiB, read + write bytes",
-                         "note": "3-sigma boxes tested x 32 B + Gaussian records loaded x 64 B + BVH32 inner nodes "
-                                 "x 1 KiB + per-item path state, per launch, over its CUDA-event time; the 70 MB "
-                                 "scene is L2-resident and L1 serves about half of the requests (ncu L1 hit rate "
-                                 "54-60%), so frac can exceed 1"}
+    if prof.get("lsu_pipe_frac") is not None:
+        roof["lsu_frac_ncu"] = prof["lsu_pipe_frac"]
+    if alg is not None:
+        l2_peak = l2_copy_gbs()
+        l2_achieved = alg / launches / sec_per_launch / 1e9
+        roof["l2_demand"] = {"achieved": l2_achieved, "peak": l2_peak, "unit": "GB/s",
+                             "frac": l2_achieved / l2_peak, "algorithmic_bytes_per_launch": alg / launches,
+                             "peak_source": "measured: L2-resident torch copy, 2 x 32 MiB, read + write bytes",
+                             "note": "3-sigma boxes tested x 32 B + Gaussian records loaded x 64 B + inner nodes "
+                                     "visited, over the launch's CUDA-event time; the scene is L2-resident and L1 "
+                                     "serves about half of the requests, so frac can exceed 1"}
     if traffic is not None:
         roof["hbm"] = {"achieved": traffic / sec_per_launch / 1e9, "peak": peak_hbm, "unit": "GB/s",
                        "frac": traffic / sec_per_launch / 1e9 / peak_hbm, "peak_source": peak_kind}
@@ -620,7 +629,7 @@ def other_configs(device):
         out["absorption_256" if prec == "auto" else "absorption_256_fast"] = {
             "mpaths_per_s": statistics.median(rates), "mpaths_per_s_spread": spread(rates), "ms": statistics.median(ms),
             "paths": st["paths"], "gaussians": sc.info()["count"],
-            "precision": "auto = ACCURATE: FP32 with float-pair set-up and sums" if prec == "auto" else
+            "precision": "auto = ACCURATE: FP32 chords with float-pair set-up, FP64 sums" if prec == "auto" else
                          "FAST: FP32, hardware exp/log approximations"}
     img.close()
     env.close()

@@ -104,8 +104,10 @@ def test_block_sizes(vp_ctx, w, h):
     check(vp_ctx, *scene_of(12, 2, 0.15), CAMERAS["outside"], w, h, spp)
 
 
-# More rays than the form with a warp on each takes (45,056 forward, 67,584 adjoint for a scene this small).
-@pytest.mark.parametrize("w, h, spp", [(263, 259, 1), (151, 150, 3), (93, 91, 8), (67, 60, 17), (47, 44, 33), (37, 29, 64)])
+# More rays than the form with a warp on each takes (45,056 forward, 67,584 adjoint for a scene this small); the last
+# has few enough tiles for blocks of 8 warps.
+@pytest.mark.parametrize("w, h, spp", [(263, 259, 1), (151, 150, 3), (93, 91, 8), (67, 60, 17), (47, 44, 33), (37, 29, 64),
+                                       (12, 9, 640)])
 @pytest.mark.parametrize("camera", list(CAMERAS))
 def test_packet_tiles(vp_ctx, w, h, spp, camera):
     check(vp_ctx, *scene_of(12, 2, 0.15), CAMERAS[camera], w, h, spp)

@@ -158,7 +158,7 @@ __global__ void k_srv_advance(SrvCtl* c, const SrvRequest* __restrict__ table, u
     const uint32_t off2 = block_exclusive_scan(r2, warp_tot, tot2);
     a = a1 + (off2 >= F2 ? 0u : min(r2, F2 - off2));
   } else {
-    // rank every entry by its key, then hand out the free slots in rank order
+    // rank the entries by their keys, then hand out the free slots in rank order
     const unsigned long long seq = mine ? table[e].seq : ~0ull;
     unsigned long long srpt_key = rem64;
     if (schedule == VP_SCHEDULE_SRPT && mine && srpt_aging > 0.0f) {
@@ -171,9 +171,16 @@ __global__ void k_srv_advance(SrvCtl* c, const SrvRequest* __restrict__ table, u
       const unsigned long long credit = (unsigned long long)((double)srpt_aging * (double)(now - base));
       srpt_key = rem64 > credit ? rem64 - credit : 0ull;
     }
-    const unsigned long long key = rem == 0 ? ~0ull : (schedule == VP_SCHEDULE_SRPT ? srpt_key : seq);
-    s_key[e] = key;
-    s_seq[e] = seq;
+    const unsigned long long key = schedule == VP_SCHEDULE_SRPT ? srpt_key : seq;
+    // only the entries that want slots are ranked, side by side in entry order: every thread going through the
+    // whole table took most of the launch's 26 us
+    uint32_t wanting = 0;
+    const uint32_t pos = block_exclusive_scan(rem ? 1u : 0u, warp_tot, wanting);
+    if (rem) {
+      s_key[pos] = key;
+      s_seq[pos] = seq;
+    }
+    s_by_rank[e] = 0u;
     // SRPT: a fraction of the free slots stays with the oldest request that has unstarted paths,
     // so a large request keeps progressing while smaller ones overtake it
     uint32_t reserve = 0, Fs = F;
@@ -194,19 +201,21 @@ __global__ void k_srv_advance(SrvCtl* c, const SrvRequest* __restrict__ table, u
     }
     __syncthreads();
     uint32_t rank = 0;
-    for (uint32_t j = 0; j < R; ++j) {
-      const unsigned long long kj = s_key[j], sj = s_seq[j];
-      rank += (kj < key || (kj == key && (sj < seq || (sj == seq && j < e)))) ? 1u : 0u;
+    if (rem) {
+      for (uint32_t j = 0; j < wanting; ++j) {
+        const unsigned long long kj = s_key[j], sj = s_seq[j];
+        rank += (kj < key || (kj == key && (sj < seq || (sj == seq && j < pos)))) ? 1u : 0u;
+      }
     }
     const uint32_t rest = rem - reserve;
-    s_by_rank[rank] = rest;
+    if (rem) s_by_rank[rank] = rest;
     __syncthreads();
     uint32_t tot = 0;
     const uint32_t before = block_exclusive_scan(s_by_rank[e], warp_tot, tot);  // thread e = rank e here
     __syncthreads();
     s_by_rank[e] = before;  // offset of rank e
     __syncthreads();
-    const uint32_t off = s_by_rank[rank];
+    const uint32_t off = s_by_rank[rank];  // (rank 0 and nothing to take where rem is 0)
     a = reserve + (off >= Fs ? 0u : min(rest, Fs - off));
   }
   uint32_t m = 0;

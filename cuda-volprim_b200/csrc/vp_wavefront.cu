@@ -92,15 +92,16 @@ __global__ void k_wf_generate(CameraView C, ParamsView P, uint32_t spp_offset, u
       live = !pixel_converged(P, count[pixel], mean[pixel], m2[pixel]);
       if (!live && p % batch == 0u) atomicAdd(&ctr->skipped, (unsigned long long)batch);
     }
-    slot = queue_reserve(b.ctr + 0, live ? 1u : 0u);  // all 32 lanes: blockDim is a multiple of 32
+    slot = queue_reserve(b.ctr + 0, live && P.max_bounces > 0 ? 1u : 0u);  // all 32 lanes: blockDim is a multiple of 32
     if (!live) return;
   }
+  b.L4[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (P.max_bounces == 0) return;  // no vertex: the sample is black
   const uint32_t pixel = p / batch, s = p % batch;
   PathState st = start_path(C, P, pixel % P.width, pixel / P.width, (uint64_t)spp_offset + s);
   const uint64_t key = draw_bounce_key(st.rng);
   store_path(b, p, st, key, kAliveBit, kNoGauss);
   b.qa[slot] = p;
-  b.L4[p] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // kMeasure = false compiles the statistics out (their registers would otherwise stay live

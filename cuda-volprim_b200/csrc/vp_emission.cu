@@ -77,8 +77,12 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 // extent: the largest |coordinate| of the scene's boxes.  The side planes go through the pixel coordinates
-// of the outermost samples, moved out by 0.02 pixels; their FP32 evaluation at a box corner is within
-// 1e-6 (|n|_1 extent + |w|), which the tolerance covers.
+// of the outermost samples, moved out by 0.02 pixels; w also holds what FP32 rounding may move a ray out of its plane.
+// With u = 2^-24 and D the distance to the scene's far side: the corner's and the rays' directions are off by 3 u
+// each and n by 3 u (divided by the sine of the angle between its factors), all of which tilt about the eye and so weigh
+// D, and n . x + w is off by 4 u (extent + |eye|) before it cancels; 2e-6 is 33 u.  From far away through a
+// narrow lens that is more than the 0.02 pixels: with a term in the extent alone, views from 1e5 times a Gaussian's
+// size lost some at the tiles' edges.
 __device__ __forceinline__ void packet_bounds(const CameraView& C, float extent, bool active, float x, float y, float3 o,
                                               float3 d, PacketBounds* B) {
   const int lane = threadIdx.x & 31;
@@ -95,12 +99,16 @@ __device__ __forceinline__ void packet_bounds(const CameraView& C, float extent,
     const float3 along = vertical ? C.dv : C.du;
     float3 inward = vertical ? C.du : C.dv;
     if (lane & 1) inward = mul(inward, -1.0f);
-    float3 n = cross3(C.ortho ? C.view_dir : corner, along);
-    n = mul(n, rsqrtf(fmaxf(dot3(n, n), 1e-37f)));
+    const float3 axis = C.ortho ? C.view_dir : corner;
+    float3 n = cross3(axis, along);
+    const float inv = rsqrtf(fmaxf(dot3(n, n), 1e-37f));
+    const float skew = sqrtf(dot3(axis, axis)) * sqrtf(dot3(along, along)) * inv;  // 1 / sin
+    n = mul(n, inv);
     if (dot3(n, inward) < 0.f) n = mul(n, -1.0f);
     const float3 at = C.ortho ? add(C.eye, corner) : C.eye;
     const float w = -dot3(n, at);
-    const float tol = 1e-6f * ((fabsf(n.x) + fabsf(n.y) + fabsf(n.z)) * extent + fabsf(w));
+    const float reach = sqrtf(dot3(at, at)) + 1.7321f * extent;
+    const float tol = 2e-6f * reach * fmaxf(skew, 1.0f);
     B->plane[lane] = make_float4(n.x, n.y, n.z, w + tol);
   }
   if (lane == 4) B->oc = make_float4(oc.x, oc.y, oc.z, r0 * 1.001f + 1e-6f * extent);

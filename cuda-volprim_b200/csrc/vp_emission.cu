@@ -321,7 +321,8 @@ __device__ __forceinline__ void expand_frontier(const SceneView& S, PacketShared
 }
 
 // Sums of this lane's ray over the packet's Gaussians, by the whole block: on every warp.  They run over up
-// to thousands of Gaussians one after the other, so they are carried in FP64 (eight terms at a time).
+// to thousands of Gaussians one after the other, so they are carried in FP64, eight FP32 terms at a time.  The eight
+// never span two subtrees: which warp takes which is a matter of timing, and an image is to be the same each time.
 template <bool kAcc, bool kList, int kGroup>
 __device__ __forceinline__ RaySums packet_sums(const SceneView& S, const float4* __restrict__ emis, uint32_t* stack,
                                                PacketShared<kGroup>& sh, float3 o, float3 d, bool active, uint32_t& status,
@@ -343,6 +344,8 @@ __device__ __forceinline__ RaySums packet_sums(const SceneView& S, const float4*
     if (lane == 0) i = atomicAdd(&sh.next, 1u);
     i = __shfl_sync(kFull, i, 0);
     if (i >= n_front) break;
+    flush();
+    met = 0u;
     if (lane == 0) {
       stack[0] = sh.front[i];
       if (kList) sh.owner[i] = (uint8_t)warp;

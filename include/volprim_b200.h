@@ -70,7 +70,8 @@ typedef enum vp_engine {
 /* Precision of the per-(ray, Gaussian) chord set-up (whitening transform, closest approach,
  * 3-sigma chord).  Both evaluate chords in FP32; the sums over a ray's chords (optical depth,
  * albedo weights) are carried in FP64 and rounded once, so a result does not depend on the order
- * in which a traversal meets the Gaussians.  Both meet the 1e-5
+ * in which a traversal meets the Gaussians (an emission image of many rays first adds up to eight
+ * neighbouring terms in FP32, always the same ones).  Both meet the 1e-5
  * relative per-pixel transmittance gate against the FP64 closed form on rays from outside the
  * Gaussians (FAST: 6e-6 worst on the 256-Gaussian absorption image, ACCURATE: 3e-6). */
 typedef enum vp_precision {

@@ -118,6 +118,12 @@ __device__ __forceinline__ const uint8_t* stage_order8() {
   return order.slot;
 }
 
+// A child is met where far x kFar8 >= near.  A plane's distance t is off by at most 4 u t, u = 2^-24, beyond what the
+// 1/64 quantum of its rounding outward covers: p - o, the reciprocal of the direction, their product and the final
+// FMA, u each.  So 8 u between a far and a near plane; 16 u is allowed.  Without it Gaussians of some ulps of their
+// distance were lost.  (An FMA in the place of the subtraction: no instruction more.)
+constexpr float kFar8 = 1.0f + 16.0f / 16777216.0f;
+
 // Two FMAs in one instruction (sm_100).
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   float2 d;
@@ -449,8 +455,8 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
           const float t1 = kKind == kScatter8 ? at_t : far_t;
           fz2 = make_float2(fminf(fz2.x, t1), fminf(fz2.y, t1));
         }  // a transmittance query has no far end
-        const float d1 = fmin3f(fx2.y, fy2.y, fz2.y) - fmax3f(nx2.y, ny2.y, fmaxf(nz2.y, t0));
-        const float d0 = fmin3f(fx2.x, fy2.x, fz2.x) - fmax3f(nx2.x, ny2.x, fmaxf(nz2.x, t0));
+        const float d1 = fmaf(fmin3f(fx2.y, fy2.y, fz2.y), kFar8, -fmax3f(nx2.y, ny2.y, fmaxf(nz2.y, t0)));
+        const float d0 = fmaf(fmin3f(fx2.x, fy2.x, fz2.x), kFar8, -fmax3f(nx2.x, ny2.x, fmaxf(nz2.x, t0)));
         miss = __funnelshift_l(__float_as_uint(d1), miss, 1);
         miss = __funnelshift_l(__float_as_uint(d0), miss, 1);
       }

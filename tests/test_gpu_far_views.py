@@ -58,3 +58,10 @@ def test_packets_lose_none(vp_ctx, view):
     env.close()
     lost = img - ref > 2e-6
     assert not lost.any(), (int(lost.sum()), float((img - ref).max()))
+
+
+def test_thread_per_ray_loses_none(view):
+    sc, _, _, o, d, prec, ref = view
+    got = sc.transmittance(o, d, precision=prec).astype(np.float64)
+    lost = got - ref > 2e-6
+    assert not lost.any(), (int(lost.sum()), float((got - ref).max()))

@@ -12,11 +12,10 @@ struct PathStats {
   unsigned int max_overlap = 0;
 };
 
-// Runs a path from its current vertex to its end; key: the free-flight key of this bounce, already drawn;
-// seed: the Gaussian that scattered the path to this vertex (kNoGauss at the camera).
+// Runs a path from its current vertex to its end; key: the free-flight key of this bounce, already drawn.
 template <class Q>
 __device__ __forceinline__ void run_path(const SceneView& S, const EnvView& E, const ParamsView& P, Q& q, PathState& s,
-                                         uint64_t key, uint32_t seed, PathStats& ps) {
+                                         uint64_t key, PathStats& ps) {
   while (true) {
     // Stages 1-3 of sample_scattering_event (sampling.cuh:474-540): ADT argmin over every
     // overlapped Gaussian, with the albedo of the rebuilt active set.  In a scene whose albedo
@@ -25,7 +24,7 @@ __device__ __forceinline__ void run_path(const SceneView& S, const EnvView& E, c
     float tstar = kInf;
     ScatterAlbedo sa;
     sa.valid = false;
-    if (!(s.bounce == 0 && S.albedo_all_zero)) tstar = q.argmin(s.o, s.d, key, &sa, seed);
+    if (!(s.bounce == 0 && S.albedo_all_zero)) tstar = q.argmin(s.o, s.d, key, &sa);
     const bool scattered = tstar < kInf;
     float3 albedo = f3(0.f, 0.f, 0.f);
     if (scattered) {
@@ -52,7 +51,6 @@ __device__ __forceinline__ void run_path(const SceneView& S, const EnvView& E, c
     }
     if (!alive) return;
     key = draw_bounce_key(s.rng);
-    seed = gauss;
   }
 }
 
@@ -63,7 +61,7 @@ __device__ float3 trace_path(const SceneView& S, const EnvView& E, const CameraV
   PathState s = start_path(C, P, px, py, sample_index);
   if (P.max_bounces > 0) {
     const uint64_t key = draw_bounce_key(s.rng);
-    run_path(S, E, P, q, s, key, kNoGauss, ps);
+    run_path(S, E, P, q, s, key, ps);
   }
   return finalize_sample(P, s.rad);
 }
@@ -75,8 +73,8 @@ struct WarpQueries {
   uint32_t& status;
   WarpStats& ws;
   bool measure;
-  __device__ float argmin(float3 o, float3 d, uint64_t key, ScatterAlbedo* sa, uint32_t seed) {
-    return warp_ray_query<kAcc, kArgmin>(S, W, o, d, key, status, ws, measure, sa, seed);
+  __device__ float argmin(float3 o, float3 d, uint64_t key, ScatterAlbedo* sa) {
+    return warp_ray_query<kAcc, kArgmin>(S, W, o, d, key, status, ws, measure, sa);
   }
   __device__ float transmittance(float3 o, float3 d, uint32_t seed = kNoGauss) {
     const float tau = warp_ray_query<kAcc, kTau>(S, W, o, d, 0ull, status, ws, measure, nullptr, seed);

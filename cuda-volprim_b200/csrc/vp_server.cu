@@ -287,8 +287,7 @@ __global__ void __launch_bounds__(256, 4) k_srv_extend(const SceneView* __restri
     ScatterAlbedo sa;
     sa.valid = false;
     if (!(bounce == 0 && S.albedo_all_zero))
-      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, key, status, ws, false, &sa,
-                                             bounce ? path_gauss(b, p) : kNoGauss);
+      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, key, status, ws, false, &sa);
     float3 albedo = f3(0.f, 0.f, 0.f);
     if (tstar < kInf) {
       uint32_t ov = sa.overlap;

@@ -137,8 +137,7 @@ __global__ void __launch_bounds__(256, VP_WF_MIN_BLOCKS) k_wf_extend(SceneView S
     ScatterAlbedo sa;
     sa.valid = false;
     if (!(bounce == 0 && S.albedo_all_zero))
-      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, key, status, ws, measure, &sa,
-                                             bounce ? path_gauss(b, p) : kNoGauss);
+      tstar = warp_ray_query<kAcc, kArgmin>(S, W, of, df, key, status, ws, measure, &sa);
     float3 albedo = f3(0.f, 0.f, 0.f);
     if (tstar < kInf) {
       uint32_t ov = sa.overlap;
@@ -394,7 +393,7 @@ __global__ void __launch_bounds__(256, kTailBlocks) k_wf_tail(SceneView S, EnvVi
     uint64_t key;
     uint32_t meta;
     PathState s = load_path(b, p, key, meta);
-    run_path(S, E, P, queries, s, key, s.bounce ? path_gauss(b, p) : kNoGauss, ps);
+    run_path(S, E, P, queries, s, key, ps);
     const float3 L = finalize_sample(P, s.rad);
     if (lane == 0) b.L4[p] = make_float4(L.x, L.y, L.z, 0.f);
     if (status) break;

@@ -399,8 +399,8 @@ __device__ float warp_ray_query(const SceneView& S, const WarpSmem& W, float3 o,
           const float v = hit ? chord_tau<kAcc>(ch.tc, ch.rw, ch.d2, ch.h, chord_u0(ch, 0.0f), fmaxf(ch.t_in, 0.0f),
                                                 ch.t_out, icf, ch.d2lo)
                               : 0.0f;
-          acc += warp_sum(v);
           lane_tau += (double)v;
+          acc = warp_sum((float)lane_tau);
           hits_seen += __popc(m);
           if (measure) ws.crossings += (unsigned)__popc(m);
           if (acc >= kMaxOpticalDepth) break;

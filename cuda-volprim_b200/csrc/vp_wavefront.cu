@@ -15,8 +15,9 @@
 //
 //   extend, shadow and tail run thread per ray over the compressed 8-wide BVH (vp_trace8.cuh); the scatter-point
 //   albedo is then the scene's, when all its Gaussians share one, or a second traversal.
-//   Their warp-per-ray forms over the BVH32 give the same results: they count (VP_MEASURE_COUNTERS) and
-//   serve scenes too deep for the 8-wide tree.
+//   Their warp-per-ray forms over the BVH32 give the same results: they count (VP_MEASURE_COUNTERS), serve scenes
+//   without an 8-wide tree (too deep) and take the last paths where
+//   Gaussians differ in albedo.
 //
 // Each kernel is a fraction of the fused path loop's code and registers, so more warps are
 // resident per SM to hide the latency of the dependent node loads.  The reference found a
@@ -64,6 +65,17 @@ constexpr uint32_t kSortMinPaths = VP_WF_SORT_MIN;
 // 1.9 / 1.8 (50k-Gaussian cloud), 5.3 / 2.5 / 2.4 / 2.4 (500k); 65k paths 5.6 / 3.5 / 3.0 / 3.2, 7.3 / 5.0 / 4.6 /
 // 4.4; a 12-bounce image of 361k paths 4.4 from 64k, 5.0 from 128k.
 constexpr uint32_t kTailMax = 65536;
+// With a warp on each path the tail takes as many as are resident at once, so that none waits for another; in an
+// image of more than kTailDeep bounces, whose paths mostly end on the way, twice as many.  12-bounce images of 4.2k / 10.8k
+// paths from one / two a resident warp on: 3,000 Gaussians of differing albedos 1.27 / 1.82 and 1.47 / 1.82 ms, 100k
+// ACCURATE 1.60 / 1.68 and 1.69 / 2.20; 64 bounces, 10k 1.51 / 2.16 and 1.41 / 1.87, 500k 2.79 / 5.83 and 2.61 / 5.07.
+constexpr uint32_t kTailDeep = 32;
+// Scenes whose Gaussians differ in albedo take their few paths with a warp on each, whose one traversal keeps
+// the chords at the scatter point: extend from this many paths on by threads (two traversals, at 2 blocks an SM),
+// shadow from this many.  12-bounce images of 11k / 30k / 60k paths, threads / warps / this: 3,000 Gaussians 1.15 / 1.62 /
+// 1.93, 0.66 / 1.02 / 1.33 and 0.65 / 1.03 / 1.29 ms; 10k in clusters 1.88 / 2.62 / 3.58, 1.22 / 1.74 / 2.52 and 1.22 /
+// 1.64 / 2.09.
+constexpr uint32_t kMixedExtendMin = 65536, kMixedShadowMin = 16384;
 // Resident blocks per SM of its register budget: 2 (128 registers) against 3: 4k paths 1.9 / 2.2 ms (50k), 2.4 /
 // 2.8 (500k).
 constexpr int kTailBlocks = 2;
@@ -363,7 +375,7 @@ __device__ __forceinline__ void welford_pixel(const ParamsView& P, const WfBuffe
 
 // The end of a batch, one cooperative launch: the paths still queued run to their ends, and once all have
 // finished the pixels' means take the batch's samples.  This form, a warp on each path over the BVH32 (the
-// warp engine's path loop), counts and serves scenes too deep for the 8-wide tree.
+// warp engine's path loop), counts and serves scenes without the 8-wide tree or of differing albedos.
 template <bool kAcc, bool kMeasure>
 __global__ void __launch_bounds__(256, kTailBlocks) k_wf_tail(SceneView S, EnvView E, ParamsView P, WfBuffers b, const uint32_t* q,
                                                  const uint32_t* count, unsigned int* work, Counters* ctr,
@@ -407,14 +419,14 @@ __global__ void __launch_bounds__(256, kTailBlocks) k_wf_tail(SceneView S, EnvVi
 // The same, thread per ray (vp_trace8.cuh): a warp keeps up to `share` of the queued paths and runs its own
 // little wavefront over them -- one traversal for the paths' next free flights and the transmittance
 // queries of their last vertices together, then a lane per path gathers and shades -- so no bounce waits for
-// another warp's.  kMixed: the scene's Gaussians differ in albedo.
+// another warp's.  For scenes of one albedo.
 constexpr uint32_t kTailShare = 16;
 struct TailWarp {  // in shared memory, after the traversal's
   uint32_t path[32];               // this round's paths: flying ones first, then those that only have queries left
   uint32_t query[3 * kTailShare];  // shadow-query slots to trace
   uint32_t next;
 };
-template <bool kAcc, bool kMixed>
+template <bool kAcc>
 __global__ void __launch_bounds__(kT8Threads, kTailBlocks) k_wf_tail8(SceneView S, EnvView E, ParamsView P, WfBuffers b,
                                                                      const uint32_t* q, const uint32_t* count,
                                                                      unsigned int* work, Counters* ctr, uint32_t batch,
@@ -477,24 +489,6 @@ __global__ void __launch_bounds__(kT8Threads, kTailBlocks) k_wf_tail8(SceneView 
           }
         });
     __syncwarp();
-    if constexpr (kMixed) {
-      if (lane == 0) T.next = 0u;
-      __syncwarp();
-      trace8<kAcc, kScatter8>(
-          scene, S.depth8, smem, order, flying, &T.next, 1u, (int)min(32u, max(flying, 1u)), status,
-          [&](uint32_t i, Ray8& ray) {
-            const uint32_t p = T.path[i];
-            ray.t = path_scatter_t(b, p);
-            if (!(ray.t < kInf)) return false;
-            path_ray(b, p, ray.o, ray.d, ray.key);
-            return true;
-          },
-          [&](uint32_t i, const Ray8& ray, const Hit8& h) {
-            const float3 a = mean_albedo(h.w, h.r, h.g, h.b);
-            b.st[4u * T.path[i] + 3u] = make_float4(a.x, a.y, a.z, ray.t);
-          });
-      __syncwarp();
-    }
     if (__any_sync(kFull, status != 0u)) break;
     // gather the last vertices' queries, shade the new ones
     const bool mine = (uint32_t)lane < flying + ending, fly = (uint32_t)lane < flying;
@@ -697,9 +691,13 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
   auto tail = P.accurate ? (P.measure ? k_wf_tail<true, true> : k_wf_tail<true, false>)
                          : (P.measure ? k_wf_tail<false, true> : k_wf_tail<false, false>);
   size_t smem_tail = smem;
-  if (use8) {
-    tail = P.accurate ? (mixed ? k_wf_tail8<true, true> : k_wf_tail8<true, false>)
-                      : (mixed ? k_wf_tail8<false, true> : k_wf_tail8<false, false>);
+  const bool tail8 = use8 && !mixed;
+  const bool deep = P.max_bounces > kTailDeep;
+  const uint32_t resident = (uint32_t)(ctx->sm_count * kTailBlocks * (threads / 32));
+  uint32_t tail_max = deep ? 2u * resident : resident;
+  if (tail8) {
+    tail_max = kTailMax;
+    tail = P.accurate ? k_wf_tail8<true> : k_wf_tail8<false>;
     smem_tail = smem8 + (kT8Threads / 32) * sizeof(TailWarp);
   }
   if (smem_tail > kSmem8Default)
@@ -708,7 +706,7 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
   for (uint32_t it = 0; it < P.max_bounces; ++it) {
     // Few paths left (the count last read), or none that can be (a scatter in an albedo-0 scene ends its
     // path): the tail takes over.  The first bounce always runs as stages.
-    if (it != 0u && (polled <= kTailMax || s->view.albedo_all_zero)) break;
+    if (it != 0u && (polled <= tail_max || s->view.albedo_all_zero)) break;
     if (it != 0u && (it & 3u) == 0u && polled >= kSortMinPaths) {  // (camera rays share one origin)
       k_wf_sort_keys<<<(polled + 255) / 256, 256, 0, st>>>(polled, qcur, b.ray, blo, binv, b.sk_a);
       vp_status r = radix_sort_pairs(b.sk_a, qcur, polled, 30, ctx->wf.sort_tmp, ctx->wf.sort_tmp_bytes, st,
@@ -717,7 +715,7 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
     }
     cudaEvent_t* e4 = ev + 4 * (it & 3u);
     if (timed) VP_CUDA(cudaEventRecord(e4[0], st));
-    if (use8) {
+    if (use8 && (!mixed || polled > kMixedExtendMin)) {
       ext8<<<ext8_blocks, kT8Threads, smem8, st>>>(s->view, b, qcur, b.ctr + 0, b.ctr + 3, ctx->counters);
     } else {
       ext<<<ext_blocks, threads, smem, st>>>(s->view, P, b, qcur, b.ctr + 0, b.ctr + 3, ctx->counters);
@@ -726,7 +724,7 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
     k_wf_shade<<<thr_blocks, threads, 0, st>>>(s->view, e->view, P, b, qcur, b.ctr + 0, qnext, b.ctr + 1,
                                                ctx->counters);
     if (timed) VP_CUDA(cudaEventRecord(e4[2], st));
-    if (use8)
+    if (use8 && (!mixed || polled > kMixedShadowMin))
       shd8<<<shd8_blocks, kT8Threads, smem8, st>>>(s->view, b, b.ctr + 2, b.ctr + 4, ctx->counters);
     else
       shd<<<shd_blocks, threads, smem_sh, st>>>(s->view, b, b.ctr + 2, b.ctr + 4, ctx->counters, P.measure);

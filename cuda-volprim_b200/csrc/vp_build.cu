@@ -29,6 +29,7 @@ struct ErrorWords {
   unsigned int opaque_cores;               // Gaussians opaque at their core (vp_tau_order AUTO)
   unsigned int mixed_albedo;               // 1 if some albedo differs from the first Gaussian's
   float albedo0[3];                        // the first Gaussian's
+  float overlap;                           // the share of the scene a Gaussian fills (k_overlap)
 };
 
 // A Gaussian is "opaque at its core" when the optical depth through its centre along its thinnest
@@ -622,6 +623,55 @@ __global__ void __launch_bounds__(kPlocTail) k_ploc_tail(uint32_t* __restrict__ 
     ctr[2] = passes;
     ctr[3] = m == 1u ? __float_as_uint(nlo[nodes - 1u].w) : 0u;
   }
+}
+
+// How much of the scene its Gaussians fill: with w the sides of a Gaussian's 3-sigma box and s those of the evenly
+// filled box that has the centres' spread, the mean over the Gaussians and the three faces of the product of
+// w / (w + s) along two axes -- about the share of them that a ray through the middle meets.  1: all in one place; 0.06:
+// scales of 0.1 in a box of side 2; 0.01 and 0.03 in the value-noise cloud and the dense clusters.  From at most
+// kOverlapSamples of them, evenly spaced in the caller's order, by one block.
+constexpr uint32_t kOverlapSamples = 4096;
+__global__ void __launch_bounds__(1024) k_overlap(uint32_t n, const float* __restrict__ mean, const float4* __restrict__ lo,
+                                                  const float4* __restrict__ hi, ErrorWords* __restrict__ err) {
+  __shared__ double part[32][6];
+  __shared__ double total[6];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  auto block_sums = [&](double (&v)[6]) {  // on every thread
+    for (int q = 0; q < 6; ++q) {
+      v[q] = warp_sum(v[q]);
+      if (lane == 0u) part[warp][q] = v[q];
+    }
+    __syncthreads();
+    if (warp == 0u)
+      for (int q = 0; q < 6; ++q) {
+        const double t = warp_sum(part[lane][q]);
+        if (lane == 0u) total[q] = t;
+      }
+    __syncthreads();
+    for (int q = 0; q < 6; ++q) v[q] = total[q];
+  };
+  const uint32_t m = min(n, kOverlapSamples);
+  auto sample = [&](uint32_t k) { return (uint32_t)((uint64_t)k * n / m); };
+  const float3 at = f3(mean[0], mean[1], mean[2]);  // (relative to the first centre: the spread of a far scene)
+  double c[6] = {};
+  for (uint32_t k = threadIdx.x; k < m; k += 1024u) {
+    const uint32_t i = sample(k);
+    const double x = mean[3 * i] - at.x, y = mean[3 * i + 1] - at.y, z = mean[3 * i + 2] - at.z;
+    c[0] += x, c[1] += y, c[2] += z, c[3] += x * x, c[4] += y * y, c[5] += z * z;
+  }
+  block_sums(c);
+  float s[3];
+  for (int a = 0; a < 3; ++a) s[a] = (float)sqrt(12.0 * fmax(c[3 + a] / m - (c[a] / m) * (c[a] / m), 0.0));
+  double f[6] = {};
+  for (uint32_t k = threadIdx.x; k < m; k += 1024u) {
+    const uint32_t i = sample(k);
+    const float4 l = lo[i], h = hi[i];
+    const float x = (h.x - l.x) / (h.x - l.x + s[0]), y = (h.y - l.y) / (h.y - l.y + s[1]),
+                z = (h.z - l.z) / (h.z - l.z + s[2]);
+    f[0] += x * y + y * z + z * x;
+  }
+  block_sums(f);
+  if (threadIdx.x == 0u) err->overlap = (float)(f[0] / (3.0 * m));
 }
 
 struct CollapseItem {
@@ -1255,6 +1305,14 @@ vp_status build_empty_scene(vp_context* ctx, const vp_gaussians* g, float sigma_
   return VP_OK;
 }
 
+// Above this overlap (k_overlap) a scene of more than one node's Gaussians goes without the 8-wide BVH: a ray meets so
+// many of them that there is nothing to cull, and a warp that takes 24 neighbouring records a step does better than
+// lanes that gather theirs.  Images of 11k / 60k / 217k paths, thread / warp per ray: 3,000 Gaussians in a
+// box of side 2, scales of 0.2 (overlap 0.16) 6.1 / 17.6 / 32.2 and 5.6 / 15.2 / 40.8 ms, of 0.3 (0.25) 17.7 / 52.7 /
+// 101.8 and 10.4 / 35.0 / 104.5 ms, of 0.8 (0.53) 48 / 177 / 392 and 23 / 112 / 380 ms; 300 in one place 2.2 / 5.4 / 7.9
+// and 1.1 / 2.3 / 5.4 ms.
+constexpr float kMaxOverlap8 = 0.2f;
+
 // The compressed 8-wide BVH of a scene (sc->nodes8, depth8 levels counting node 0), cut from the binary
 // tree the BVH32 comes from.  depth8 = 0: the tree is too deep or too large for it (kMaxDepth8,
 // kMaxNodes8) and the engines use the warp-cooperative queries.
@@ -1375,7 +1433,7 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
   if ((s = dev_alloc(&errw.p, 1, st))) return s;
   if ((s = dev_alloc(&bounds.p, 12, st))) return s;
   {
-    ErrorWords e0{0x7FFFFFFF, 0x7FFFFFFF, 0x7FFFFFFF, 0u, 0u, 0u, {0.f, 0.f, 0.f}};
+    ErrorWords e0{0x7FFFFFFF, 0x7FFFFFFF, 0x7FFFFFFF, 0u, 0u, 0u, {0.f, 0.f, 0.f}, 0.f};
     VP_CUDA(cudaMemcpyAsync(errw.p, &e0, sizeof(e0), cudaMemcpyHostToDevice, st));
     unsigned int b0[12];
     for (int k = 0; k < 3; ++k) {
@@ -1392,6 +1450,8 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
                                   rec0.p, lo0.p, hi0.p, errw.p);
   VP_CUDA(cudaGetLastError());
   k_bounds<<<std::min(nb, 1184u), TB, 0, st>>>(n, mean, lo0.p, hi0.p, bounds.p);
+  VP_CUDA(cudaGetLastError());
+  k_overlap<<<1, 1024, 0, st>>>(n, mean, lo0.p, hi0.p, errw.p);
   VP_CUDA(cudaGetLastError());
   ErrorWords eh{};
   unsigned int bh[12];
@@ -1642,7 +1702,9 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
     }
   }
   uint32_t depth8 = 0, nodes8 = 0;
-  if ((s = build_bvh8(ctx, n, wide_root, wl, wr, plo.p, phi.p, wlo, whi, par.p, par_leaf.p, pos.p, sc, depth8, nodes8)))
+  sc->overlap = eh.overlap;
+  if ((n <= 8u || eh.overlap <= kMaxOverlap8) &&
+      (s = build_bvh8(ctx, n, wide_root, wl, wr, plo.p, phi.p, wlo, whi, par.p, par_leaf.p, pos.p, sc, depth8, nodes8)))
     return s;
   // Scene order, then the records, boxes and adjoint inputs gathered into it.
   uint32_t* perm = nullptr;

@@ -111,6 +111,7 @@ struct vp_scene {
   float4* bin = nullptr;
   float4* pbox = nullptr;
   uint32_t* nodes8 = nullptr;
+  float overlap = 0.0f;  // the share of the scene that a Gaussian fills (vp_build.cu, k_overlap)
   // as given by the caller, in the scene's order: quaternion (w,x,y,z), then scale (log or
   // linear, as scale_is_log says) and density -- the chain-rule inputs of the adjoint
   float4* raw = nullptr;

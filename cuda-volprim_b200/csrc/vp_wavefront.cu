@@ -16,7 +16,7 @@
 //   extend, shadow and tail run thread per ray over the compressed 8-wide BVH (vp_trace8.cuh); the scatter-point
 //   albedo is then the scene's, when all its Gaussians share one, or a second traversal.
 //   Their warp-per-ray forms over the BVH32 give the same results: they count (VP_MEASURE_COUNTERS), serve scenes
-//   without an 8-wide tree (too deep) and take the last paths where
+//   without an 8-wide tree (too deep, or of Gaussians that fill most of it) and take the last paths where
 //   Gaussians differ in albedo.
 //
 // Each kernel is a fraction of the fused path loop's code and registers, so more warps are
@@ -70,6 +70,14 @@ constexpr uint32_t kTailMax = 65536;
 // paths from one / two a resident warp on: 3,000 Gaussians of differing albedos 1.27 / 1.82 and 1.47 / 1.82 ms, 100k
 // ACCURATE 1.60 / 1.68 and 1.69 / 2.20; 64 bounces, 10k 1.51 / 2.16 and 1.41 / 1.87, 500k 2.79 / 5.83 and 2.61 / 5.07.
 constexpr uint32_t kTailDeep = 32;
+// By threads it takes two a resident warp where Gaussians fill more of the scene than kTailOverlap (vp_build.cu,
+// k_overlap): its few paths a warp wait for one another's long rays.  20,000 Gaussians, scales of 0.15 in a
+// box of side 2 (0.11), 11k / 30k / 60k paths: 17.0 / 29.9 / 49.6 ms from 64k on, 15.6 / 27.4 / 42.1 from 4.7k; scales of
+// 0.1 (0.06) 5.2 / 9.8 / 16.2 and 5.4 / 9.6 / 15.6.  ACCURATE chords cost more, and the line lies lower: 10k Gaussians
+// in clusters (0.03), 12 bounces of 11k / 60k paths 1.58 / 3.03 ms from 64k on, 1.42 / 2.16 from 4.7k, 64 bounces of 8k / 60k
+// 2.10 / 4.00 from 64k, 1.97 / 3.48 from 16k.
+constexpr float kTailOverlap = 0.1f, kTailOverlapAccurate = 0.02f;
+constexpr uint32_t kTailMaxAccurate = 16384;
 // Scenes whose Gaussians differ in albedo take their few paths with a warp on each, whose one traversal keeps
 // the chords at the scatter point: extend from this many paths on by threads (two traversals, at 2 blocks an SM),
 // shadow from this many.  12-bounce images of 11k / 30k / 60k paths, threads / warps / this: 3,000 Gaussians 1.15 / 1.62 /
@@ -696,7 +704,9 @@ vp_status launch_wavefront(vp_scene* s, vp_env* e, const CameraView& cam, const 
   const uint32_t resident = (uint32_t)(ctx->sm_count * kTailBlocks * (threads / 32));
   uint32_t tail_max = deep ? 2u * resident : resident;
   if (tail8) {
-    tail_max = kTailMax;
+    tail_max = s->overlap > kTailOverlap ? 2u * resident
+               : !(P.accurate && s->overlap > kTailOverlapAccurate) ? kTailMax
+               : deep ? kTailMaxAccurate : 2u * resident;
     tail = P.accurate ? k_wf_tail8<true> : k_wf_tail8<false>;
     smem_tail = smem8 + (kT8Threads / 32) * sizeof(TailWarp);
   }

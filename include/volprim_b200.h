@@ -63,8 +63,9 @@ typedef enum vp_engine {
   VP_ENGINE_MEGAKERNEL = 1, /* plain per-pixel megakernel, thread-per-ray binary-tree traversal */
   VP_ENGINE_WAVEFRONT = 2   /* wavefront of persistent stage kernels over compacted path queues,
                                thread-per-ray traversal of a compressed 8-wide BVH (warp-cooperative
-                               BVH32 traversal while counting, and for trees too deep for it); same
-                               results as VP_ENGINE_WARP */
+                               BVH32 traversal while counting, for scenes without one -- too deep, or of
+                               Gaussians that fill most of the scene -- and for few paths of scenes whose
+                               Gaussians differ in albedo); same results as VP_ENGINE_WARP */
 } vp_engine;
 
 /* Precision of the per-(ray, Gaussian) chord set-up (whitening transform, closest approach,

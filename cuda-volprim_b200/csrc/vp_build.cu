@@ -1315,7 +1315,7 @@ constexpr float kMaxOverlap8 = 0.2f;
 
 // The compressed 8-wide BVH of a scene (sc->nodes8, depth8 levels counting node 0), cut from the binary
 // tree the BVH32 comes from.  depth8 = 0: the tree is too deep or too large for it (kMaxDepth8,
-// kMaxNodes8) and the engines use the warp-cooperative queries.
+// kMaxNodes8) and the engines use the warp-cooperative queries; the caller takes VP_ERROR_OUT_OF_MEMORY so, too.
 static vp_status build_bvh8(vp_context* ctx, uint32_t n, uint32_t root, const uint32_t* wl, const uint32_t* wr,
                             const float4* plo, const float4* phi, const float4* wlo, const float4* whi,
                             const uint32_t* par, const uint32_t* par_leaf, const uint32_t* pos, vp_scene* sc,
@@ -1701,11 +1701,6 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
       dp = false;
     }
   }
-  uint32_t depth8 = 0, nodes8 = 0;
-  sc->overlap = eh.overlap;
-  if ((n <= 8u || eh.overlap <= kMaxOverlap8) &&
-      (s = build_bvh8(ctx, n, wide_root, wl, wr, plo.p, phi.p, wlo, whi, par.p, par_leaf.p, pos.p, sc, depth8, nodes8)))
-    return s;
   // Scene order, then the records, boxes and adjoint inputs gathered into it.
   uint32_t* perm = nullptr;
   if ((s = dev_alloc(&perm, n, st))) return s;
@@ -1720,6 +1715,9 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
   sc->pbox = pbox;
   k_gather<<<nb, TB, 0, st>>>(n, perm, rec0.p, lo0.p, hi0.p, prims, pbox);
   VP_CUDA(cudaGetLastError());
+  dev_free(rec0.p, st);
+  dev_free(lo0.p, st);
+  dev_free(hi0.p, st);
   float4* raw = nullptr;
   if ((s = dev_alloc(&raw, 2ull * n, st))) return s;
   sc->raw = raw;
@@ -1749,6 +1747,18 @@ vp_status build_scene(vp_context* ctx, const vp_gaussians* g, float sigma_multip
     dev_free(wide, st);
     wide = tight;
     sc->wide = wide;
+  }
+  // Last, so that a device with room for the rest only goes without it.
+  uint32_t depth8 = 0, nodes8 = 0;
+  sc->overlap = eh.overlap;
+  if (n <= 8u || eh.overlap <= kMaxOverlap8) {
+    s = build_bvh8(ctx, n, wide_root, wl, wr, plo.p, phi.p, wlo, whi, par.p, par_leaf.p, pos.p, sc, depth8, nodes8);
+    if (s == VP_ERROR_OUT_OF_MEMORY) {
+      dev_free(sc->nodes8, st);
+      depth8 = nodes8 = 0u;
+    } else if (s) {
+      return s;
+    }
   }
   VP_CUDA(cudaEventRecord(ctx->ev1, st));
   VP_CUDA(cudaEventSynchronize(ctx->ev1));

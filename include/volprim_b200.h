@@ -109,7 +109,8 @@ vp_status vp_version(int32_t* major, int32_t* minor);
 
 /* Binds a CUDA device and creates the context's stream and memory pool.  The pool serves the
  * scenes', calls' and requests' device buffers in stream order, keeps at most 2 GiB of freed memory for
- * the next of them, and is given back with the context.  Replaces cuda::Context + StreamDAG
+ * the next of them (the driver takes it from the pool when another allocation of the process needs it),
+ * and is given back with the context.  Replaces cuda::Context + StreamDAG
  * construction in Renderer::Renderer (src/thesis/host/app/renderer.cpp:34-51). */
 vp_status vp_context_create(int32_t device, vp_context** out);
 vp_status vp_context_destroy(vp_context* ctx);

@@ -165,14 +165,6 @@ __device__ __forceinline__ void two_prod(float a, float b, float& p, float& e) {
 struct FF {
   float hi, lo;
 };
-// hi + lo of a + b, with a and b float pairs
-__device__ __forceinline__ FF ff_add(FF a, FF b) {
-  float s, e;
-  two_sum(a.hi, b.hi, s, e);
-  FF r;
-  fast_two_sum(s, __fadd_rn(e, __fadd_rn(a.lo, b.lo)), r.hi, r.lo);
-  return r;
-}
 // acc += v (float), compensated
 __device__ __forceinline__ void ff_accumulate(FF& acc, float v) {
   float s, e;

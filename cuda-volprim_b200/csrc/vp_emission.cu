@@ -885,12 +885,14 @@ vp_status with_group(uint32_t tiles, uint32_t stack_cap, F&& f) {
 }
 
 // Images of few rays take a warp on each ray: their packets are few, and wide at one or two samples a pixel, so
-// the chip waits for the densest.  Both sides at 12,800 / 40,000 / 65,536 / 180,000 rays, packets and then rays:
+// the chip waits for the densest.  Both sides at 12,800 / 40,000 / 65,536 / 180,000 rays (8, 1, 1 and 8 samples a pixel),
+// packets and then rays:
 // forward, 100k Gaussians 2.18 / 1.78 / 1.67 / 1.84 and 0.57 / 1.04 / 1.63 / 3.96 ms, 20k Gaussians 0.59 / 0.47 /
 // 0.45 / 0.49 and 0.17 / 0.30 / 0.44 / 1.06, 5k Gaussians 0.18 / 0.16 / 0.155 / 0.17 and 0.10 / 0.145 / 0.20 / 0.45;
 // ACCURATE crosses over at four fifths of that.  A gradient step at 38k / 154k rays (two views the latter; build
 // and forward in it): 100k Gaussians 9.4 / 15.0 and 5.7 / 20.5 ms, 5k 2.32 / 2.75 and 2.19 / 3.77: the adjoint's
-// packets, which it meets twice, pay later.
+// packets, which it meets twice, pay later.  Sample counts that fill a packet badly do not move the line: 70,000 rays through
+// 100k Gaussians take 1.68 ms in packets at 1 and at 17 samples a pixel, 2.37 at 33, which is a second pass for one ray.
 bool few_rays(const ParamsView& P, uint32_t count, bool adjoint) {
   uint64_t limit = count >= 16384u ? 65536u : 45056u;
   if (P.accurate) limit = limit * 4u / 5u;

@@ -205,7 +205,7 @@ __global__ void k_albedo_thread(SceneView S, const float* __restrict__ pts, uint
   if (status) atomicOr(&ctr->status, status);
 }
 
-// The same query, thread per ray (vp_trace8.cuh); k_tau_warp takes small calls and scenes too deep for the 8-wide BVH.
+// The same query, thread per ray (vp_trace8.cuh); k_tau_warp takes small calls and scenes without an 8-wide BVH.
 template <bool kAcc>
 __global__ void __launch_bounds__(kT8Threads, kT8Blocks) k_tau8(SceneView S, const float* __restrict__ org,
                                                                const float* __restrict__ dir, uint32_t n,
@@ -287,7 +287,9 @@ vp_status launch_transmittance(vp_scene* s, const float* o, const float* d, uint
   if (n == 0) return VP_OK;
   // Few rays through a small scene end sooner with a warp on each.  Warp / thread: 1,000 Gaussians, 1,000 rays 59 /
   // 71 us, 18,000 83 / 96, 40,000 117 / 120, 80,000 175 / 148; 10,000 Gaussians, 1,000 rays 52 / 62, 65,000 134 /
-  // 97; from 16,384 Gaussians threads win at any count (30,000 in clusters, 16,000 rays 139 / 112).
+  // 97.  How dense the scene is counts as well as its size, and the line at 16,384 Gaussians lies between: at 20,000,
+  // 1,000 / 4,000 / 16,000 rays through the value-noise cloud 61 / 62 / 86 and 63 / 73 / 85 us, through dense
+  // clusters 75 / 85 / 114 and 73 / 76 / 98; from 30,000 threads are level or win everywhere.
   const bool small = s->view.count < 2048u ? n <= 24576u : s->view.count < 16384u && n <= 16384u;
   if (engine == VP_ENGINE_WARP && s->view.depth8 != 0u && !small) {
     auto kern = accurate ? k_tau8<true> : k_tau8<false>;

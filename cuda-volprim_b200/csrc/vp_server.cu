@@ -8,7 +8,7 @@
 //   regen    (thread per path)   new paths: owning request from the share prefix sums, camera
 //                                ray, PCG32 stream, first free-flight key -- appended to the queue
 //   extend   (thread per path)   free-flight argmin + scatter albedo on the path's own scene (vp_trace8.cuh;
-//                                warp per path over the BVH32 when some scene is too deep for the 8-wide one)
+//                                warp per path over the BVH32 when some scene has no 8-wide one)
 //   shade    (thread per path)   phase / NEE / roulette with the request's own controls
 //   shadow   (thread per query)  transmittance on the query's scene, likewise
 //   gather   (thread per path)   radiance += weight x T; a finished path adds its sample to its

@@ -105,77 +105,73 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* __restrict__
 }
 
 // ---- exclusive scan of counts ---------------------------------------------------
-template <class T>
-__device__ __forceinline__ T block_scan_excl(T v, T* warp_tot, T& total) {
+__device__ __forceinline__ uint32_t block_scan_excl(uint32_t v, uint32_t* warp_tot, uint32_t& total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  T incl = v;
+  uint32_t incl = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const T t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
     if (lane >= o) incl += t;
   }
   if (lane == 31) warp_tot[w] = incl;
   __syncthreads();
   if (w == 0) {
-    T x = lane < nw ? warp_tot[lane] : T(0);
+    uint32_t x = lane < nw ? warp_tot[lane] : 0u;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const T t = __shfl_up_sync(0xFFFFFFFFu, x, o);
+      const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, x, o);
       if (lane >= o) x += t;
     }
     if (lane < nw) warp_tot[lane] = x;
   }
   __syncthreads();
   total = warp_tot[nw - 1];
-  const T r = (w ? warp_tot[w - 1] : T(0)) + incl - v;
+  const uint32_t r = (w ? warp_tot[w - 1] : 0u) + incl - v;
   __syncthreads();
   return r;
 }
 
-template <class T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const T* __restrict__ in, size_t n,
-                                                               T* __restrict__ partial) {
-  __shared__ T wt[32];
+__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* __restrict__ in, size_t n,
+                                                               uint32_t* __restrict__ partial) {
+  __shared__ uint32_t wt[32];
   const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
-  T s = 0;
+  uint32_t s = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k)
     if (base + k < n) s += in[base + k];
-  T total;
+  uint32_t total;
   (void)block_scan_excl(s, wt, total);
   if (threadIdx.x == 0) partial[blockIdx.x] = total;
 }
 
 // One block: exclusive scan of the m tile sums in place (each thread a contiguous chunk).
-template <class T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_partials(T* __restrict__ partial, uint32_t m) {
-  __shared__ T wt[32];
+__global__ void __launch_bounds__(kScanThreads) k_scan_partials(uint32_t* __restrict__ partial, uint32_t m) {
+  __shared__ uint32_t wt[32];
   const uint32_t per = (m + kScanThreads - 1) / kScanThreads;
   const uint32_t b = threadIdx.x * per, e = min(m, b + per);
-  T s = 0;
+  uint32_t s = 0;
   for (uint32_t i = b; i < e; ++i) s += partial[i];
-  T total;
-  T run = block_scan_excl(s, wt, total);
+  uint32_t total;
+  uint32_t run = block_scan_excl(s, wt, total);
   for (uint32_t i = b; i < e; ++i) {
-    const T v = partial[i];
+    const uint32_t v = partial[i];
     partial[i] = run;
     run += v;
   }
 }
 
-template <class T>
-__global__ void __launch_bounds__(kScanThreads) k_scan_down(const T* in, size_t n, const T* __restrict__ partial,
-                                                             T* out) {  // in may equal out
-  __shared__ T wt[32];
+__global__ void __launch_bounds__(kScanThreads) k_scan_down(const uint32_t* in, size_t n, const uint32_t* __restrict__ partial,
+                                                             uint32_t* out) {  // in may equal out
+  __shared__ uint32_t wt[32];
   const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
-  T v[kScanItems], s = 0;
+  uint32_t v[kScanItems], s = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    v[k] = base + k < n ? in[base + k] : T(0);
+    v[k] = base + k < n ? in[base + k] : 0u;
     s += v[k];
   }
-  T total;
-  T run = block_scan_excl(s, wt, total) + partial[blockIdx.x];
+  uint32_t total;
+  uint32_t run = block_scan_excl(s, wt, total) + partial[blockIdx.x];
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     if (base + k < n) out[base + k] = run;
@@ -183,11 +179,22 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const T* in, size_t 
   }
 }
 
-template <class T>
-vp_status exclusive_scan_t(const T* in, T* out, size_t n, void* tmp, size_t tmp_bytes, cudaStream_t st,
-                           uint32_t* launches);
+size_t scan_tmp_bytes(size_t n) { return ((n + kScanTile - 1) / kScanTile) * sizeof(uint32_t) + 256; }
 
-size_t scan_tmp_bytes(size_t n) { return ((n + kScanTile - 1) / kScanTile) * sizeof(unsigned long long) + 256; }
+vp_status exclusive_scan(const uint32_t* in, uint32_t* out, size_t n, void* tmp, size_t tmp_bytes, cudaStream_t st,
+                           uint32_t* launches) {
+  if (n == 0) return VP_OK;
+  const size_t tiles = (n + kScanTile - 1) / kScanTile;
+  if (tmp_bytes < scan_tmp_bytes(n)) return fail(VP_ERROR_INTERNAL, "scan scratch too small");
+  if (tiles > (size_t)0xFFFFFFFFu) return fail(VP_ERROR_LIMIT, "scan too large");
+  uint32_t* partial = static_cast<uint32_t*>(tmp);
+  k_scan_reduce<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, n, partial);
+  k_scan_partials<<<1, kScanThreads, 0, st>>>(partial, (uint32_t)tiles);
+  k_scan_down<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, n, partial, out);
+  VP_CUDA(cudaGetLastError());
+  if (launches) *launches += 3;
+  return VP_OK;
+}
 
 template <class K>
 size_t sort_tmp_bytes_t(size_t n) {
@@ -220,7 +227,7 @@ vp_status sort_pairs_t(K* keys, uint32_t* vals, uint32_t n, int end_bit, void* t
     const int shift = 8 * pass;
     k_rs_upsweep<K><<<tiles, kRsThreads, 0, st>>>(kin, n, shift, tiles, hist);
     VP_CUDA(cudaGetLastError());
-    vp_status r = exclusive_scan_t<uint32_t>(hist, hist, hist_n, scan_tmp, scan_tmp_bytes(hist_n), st, launches);
+    vp_status r = exclusive_scan(hist, hist, hist_n, scan_tmp, scan_tmp_bytes(hist_n), st, launches);
     if (r) return r;
     k_rs_scatter<K><<<tiles, kRsThreads, 0, st>>>(kin, vin, kout, vout, n, shift, tiles, hist);
     VP_CUDA(cudaGetLastError());
@@ -232,22 +239,6 @@ vp_status sort_pairs_t(K* keys, uint32_t* vals, uint32_t n, int end_bit, void* t
     VP_CUDA(cudaMemcpyAsync(keys, kin, (size_t)n * sizeof(K), cudaMemcpyDeviceToDevice, st));
     VP_CUDA(cudaMemcpyAsync(vals, vin, (size_t)n * 4, cudaMemcpyDeviceToDevice, st));
   }
-  return VP_OK;
-}
-
-template <class T>
-vp_status exclusive_scan_t(const T* in, T* out, size_t n, void* tmp, size_t tmp_bytes, cudaStream_t st,
-                           uint32_t* launches) {
-  if (n == 0) return VP_OK;
-  const size_t tiles = (n + kScanTile - 1) / kScanTile;
-  if (tmp_bytes < scan_tmp_bytes(n)) return fail(VP_ERROR_INTERNAL, "scan scratch too small");
-  if (tiles > (size_t)0xFFFFFFFFu) return fail(VP_ERROR_LIMIT, "scan too large");
-  T* partial = static_cast<T*>(tmp);
-  k_scan_reduce<T><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, n, partial);
-  k_scan_partials<T><<<1, kScanThreads, 0, st>>>(partial, (uint32_t)tiles);
-  k_scan_down<T><<<(unsigned)tiles, kScanThreads, 0, st>>>(in, n, partial, out);
-  VP_CUDA(cudaGetLastError());
-  if (launches) *launches += 3;
   return VP_OK;
 }
 

@@ -15,9 +15,11 @@
 // the 32 rays do.  A warp refills its finished lanes together, after draining both queues; once there is
 // nothing left to fetch, its idle lanes take over subtrees of the rays still walking.  Without that, a batch
 // ended with its longest rays, whose lanes walked alone, and below some 115k rays a whole warp on each ray
-// was sooner done; with it this form is the faster one at every size measured (transmittance of 1k / 65k /
-// 250k rays through a 100k-Gaussian cloud: 0.08 / 0.14 / 0.26 ms, 0.10 / 0.29 / 0.39 without, 0.10 / 0.24 /
-// 0.63 with a warp on each ray; the 2M-Gaussian stress image 64 / 77 / 180 ms).
+// was sooner done; with it this form is the faster one at every batch in scenes of many small Gaussians (transmittance
+// of 1k / 65k / 250k rays through a 100k-Gaussian cloud: 0.08 / 0.14 / 0.26 ms, 0.10 / 0.29 / 0.39 without, 0.10 /
+// 0.24 / 0.63 with a warp on each ray; the 2M-Gaussian stress image 64 / 77 / 180 ms).  A warp on each ray stays
+// better for short batches through small scenes (launch_transmittance, vp_render.cu), where the Gaussians are as large
+// as the scene (kMaxOverlap8, vp_build.cu) and for few paths through differing albedos (vp_wavefront.cu).
 //
 // Results do not depend on which rays share a warp or in which order chords are met: the argmin is a
 // minimum, and the sums (optical depth, albedo weights) are carried in FP64 and rounded once.
@@ -85,7 +87,6 @@ struct Hit8 {
   float t;          // kFlight8: free-flight minimum (kInf: escape)
   uint32_t gauss;   // kFlight8: its Gaussian
   double w, r, g, b;  // kTau8: w = optical depth; kScatter8: sums of weight, weight x albedo
-  uint32_t count;   // kScatter8: Gaussians containing the point
 };
 
 __device__ __forceinline__ float byte_plane(uint32_t word, uint32_t sel) {  // 1 + q / 32768
@@ -167,7 +168,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
   int sp = 0, sb = 0, owner = lane;  // its stack entries are [sb, sp)
   bool active = false, more = true;
   float t_hi = kInf;
-  uint32_t arg = kNoGauss, cnt = 0;
+  uint32_t arg = kNoGauss;
   double acc = 0.0, ar = 0.0, ag = 0.0, ab = 0.0;
   const unsigned used = rpw >= 32 ? kFull : ((1u << rpw) - 1u);
   const int refill = max(1, rpw / 4);
@@ -239,7 +240,6 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
           ar += (double)vj * (double)x;
           ag += (double)vj * (double)y;
           ab += (double)vj * (double)z;
-          ++cnt;
         }
       }
       m &= m - 1u;
@@ -310,7 +310,7 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
       if (q2n > 0) values(q2n);
       if (active && mask == 0u && sp == sb) {
         Hit8 h;
-        h.t = t_hi, h.gauss = arg, h.w = acc, h.r = ar, h.g = ag, h.b = ab, h.count = cnt;
+        h.t = t_hi, h.gauss = arg, h.w = acc, h.r = ar, h.g = ag, h.b = ab;
         sink(item, ray, h);
         active = false;
       }
@@ -335,7 +335,6 @@ __device__ __forceinline__ void trace8(const Scenes& scenes, uint32_t depth, uin
             sp = sb = 0;
             t_hi = kKind == kScatter8 ? ray.t : kInf;
             arg = kNoGauss;
-            cnt = 0u;
             acc = ar = ag = ab = 0.0;
             if constexpr (kTaus) {
               if (!ray.flight && ray.seed != kNoGauss) acc = (double)ray.seed_tau;

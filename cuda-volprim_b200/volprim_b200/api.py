@@ -127,8 +127,8 @@ class Scene:
     and of the megakernel: "ploc" (clustering, the default) or "lbvh" (Karras radix tree);
     leaf_max is the largest BVH32 leaf (1..32); collapse cuts the BVH32 from its binary tree:
     "sah" (SAH-optimal slot assignment, the default) or "greedy" (largest area first);
-    tau_order is the order transmittance queries visit a node's hit children after the nearest:
-    "lane", "nearest" or "auto" (nearest when fewer than half of the Gaussians are opaque at
+    tau_order is the order warp-per-ray transmittance queries visit a node's hit children after the
+    nearest (thread-per-ray ones always go near to far): "lane", "nearest" or "auto" (nearest when fewer than half of the Gaussians are opaque at
     their core and the BVH32 is at least 3 levels deep)."""
 
     def __init__(self, ctx: Context, g: Gaussians, sigma_multiplier: float = 1.0, wide_builder: str = "ploc",

@@ -157,7 +157,8 @@ typedef struct vp_scene_info {
   uint32_t binary_height;   /* height of the PLOC tree (0 when no PLOC tree was built) */
   uint32_t leaf_max;        /* largest BVH32 leaf the build allowed */
   int32_t wide_collapse;    /* vp_collapse the BVH32 was cut with */
-  int32_t tau_order;        /* vp_tau_order in use: VP_TAU_ORDER_LANE or VP_TAU_ORDER_NEAREST */
+  int32_t tau_order;        /* vp_tau_order of the warp-per-ray queries: VP_TAU_ORDER_LANE or
+                               VP_TAU_ORDER_NEAREST */
 } vp_scene_info;
 
 /* Validates the primitives (positive finite scales, positive finite density, finite centres;
@@ -212,7 +213,9 @@ typedef struct vp_scene_options {
   uint32_t leaf_max;      /* largest BVH32 leaf in Gaussians, 1..32 (default 24) */
   int32_t wide_collapse;  /* vp_collapse: how the binary tree becomes 32-wide nodes (default
                              VP_COLLAPSE_SAH) */
-  int32_t tau_order;      /* vp_tau_order of the scene's transmittance queries (default AUTO) */
+  int32_t tau_order;      /* vp_tau_order of the scene's warp-per-ray transmittance queries (default
+                             AUTO): vp_transmittance_static, the warp engine, counting renders, scenes
+                             without an 8-wide BVH, short vp_transmittance batches of small scenes */
 } vp_scene_options;
 
 vp_status vp_scene_options_default(vp_scene_options* out);
